@@ -158,7 +158,7 @@ int mcg_counters_read(mcg_context *ctx, mcg_counters *out);
 int mcg_last_kernel_ms(mcg_context *ctx, float *ms);
 
 /* Launch shape (0 = automatic): threads per block, resident blocks per SM,
- * steps between lane refills. */
+ * most steps a history takes before its warp looks at its other histories. */
 int mcg_set_launch(mcg_context *ctx, int32_t block, int32_t blocks_per_sm, int32_t refill_steps);
 
 /* Algorithm of the single-chain entry points: MCG_ALGO_HISTORY (default,
@@ -353,7 +353,7 @@ int mcg_fit_gradient(mcg_context *ctx, const double *h_weights, double *h_tally,
  * 8-byte aligned, updated in place), an optional device result array and the
  * device output d_tally_q[total cells], which is overwritten with the
  * fixed-point tally.  Everything else lives in one statically sized device
- * array inside the library (about 384 KiB, held by every GPU that loads the
+ * array inside the library (about 640 KiB, held by every GPU that loads the
  * library until the process exits), which holds chains of at most
  * MCG_NOALLOC_MAX_CELLS cells (larger chains are rejected with MCG_ERR_ARG
  * before any device work).  Every call looks up that array's device address

@@ -275,6 +275,45 @@ MCG_HD float mcg_exp_ff(float t, float *delta, const mcg_libm_tab *T)
  * of mcg_exp_ff_core(t) there. */
 #define MCG_EXP_SMALL_T 0.0054f
 
+/* 1 - expf(-u) for 0 <= u < 2^-8 (thin) and 0 <= u < 2^-4 (mid), without the
+ * float-float evaluator: below 1 the floats are the multiples of 2^-24, so
+ * 1 - expf(-u) is 1 - e^-u rounded to that grid.  z = u - u^2 (1/2 - u/6 + ...)
+ * in single precision is rounded to the grid by adding and subtracting 0.75
+ * (the floats of [3/4, 1) are that grid), and *r is the exact value minus
+ * the rounded one: u - om is exact (the two are within a factor of two, or
+ * om is 0), and the series is subtracted from that small difference, so r
+ * is known to about u^2 grid units (thin; truncation u^4/24) or
+ * 3e-4 of a unit (mid).  |r| below a half by more than that and by more than
+ * the table's largest exception distance (mcg_run_bounds) makes om the host
+ * library's 1 - expf(-u) bit for bit; the table generator checks it for
+ * every u of both ranges.  7 and 14 operations against 17 and 27 of the
+ * evaluator's small path with its midpoint test. */
+#define MCG_OM_THIN_MAX 0x1p-8f
+#define MCG_OM_MID_MAX 0x1p-4f
+MCG_HD float mcg_om_thin(float u, float uu, float *r)
+{
+  const float q = MCG_FMA(-u, 1.0f / 6.0f, 0.5f);
+  const float z = MCG_FMA(-uu, q, u);
+  const float om = MCG_SUB(MCG_ADD(z, 0.75f), 0.75f);
+  *r = MCG_FMA(-uu, q, MCG_SUB(u, om));
+  return om;
+}
+
+MCG_HD float mcg_om_mid(float u, float uu, float *r)
+{
+  float p = MCG_FMA(-u, 1.0f / 720.0f, 1.0f / 120.0f);
+  p = MCG_FMA(-u, p, 1.0f / 24.0f);
+  p = MCG_FMA(-u, p, 1.0f / 6.0f);
+  const float z = MCG_FMA(-uu, MCG_FMA(-u, p, 0.5f), u);
+  const float om = MCG_SUB(MCG_ADD(z, 0.75f), 0.75f);
+  /* u - om - u^2/2 with u^2 exact as uu + e, then + u^3 p */
+  const float e = MCG_FMA(u, u, -uu);
+  float d = MCG_FMA(-0.5f, uu, MCG_SUB(u, om));
+  d = MCG_FMA(-0.5f, e, d);
+  *r = MCG_FMA(MCG_MUL(uu, u), p, d);
+  return om;
+}
+
 /* Below this argument 1 - expf(t) rounds to exactly 1.0f whatever expf
  * returns (its result is below 2^-25); the table generator re-verifies this
  * against the host library for every float below the bound. */

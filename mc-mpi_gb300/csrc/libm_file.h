@@ -36,6 +36,56 @@ typedef struct mcg_libm_file {
   float tau_exp[MCG_TAU_BUCKETS];
 } mcg_libm_file;
 
+/* Acceptance bounds of mcg_om_thin and mcg_om_mid (exact_libm.h), from the
+ * exception table's per-bucket midpoint distances: |r| < b_mid, and
+ * |r| < b_thin - c_thin u^2, imply that u is no exception and that the
+ * form's error cannot have moved the result over a midpoint.  Near 0 the
+ * host library's distances shrink with u^2 (its polynomial's error does), so
+ * the thin bound follows them: c_thin is the largest tau / u^2 of the range's
+ * buckets plus 16 for the form's own error of about u^2 grid units. */
+typedef struct mcg_run_bounds_t {
+  float b_thin, c_thin, b_mid;
+} mcg_run_bounds_t;
+
+static inline mcg_run_bounds_t mcg_run_bounds(const float *tau_exp)
+{
+  const double grid = 1.0 / 16777216.0;
+  double c = 0.0, t = 0.0;
+  for (uint32_t b = MCG_TAU_BUCKETS / 2; b < MCG_TAU_BUCKETS; ++b) {
+    float lo; /* the bucket's smallest |argument| */
+    uint32_t u = (b << 19) & 0x7fffffffu;
+    memcpy(&lo, &u, 4);
+    if (tau_exp[b] < 0.0f || !(lo < MCG_OM_MID_MAX))
+      continue;
+    t = tau_exp[b] > t ? tau_exp[b] : t;
+    if (lo < MCG_OM_THIN_MAX) {
+      const double v = lo > 0.0f ? tau_exp[b] / ((double)lo * lo) : 1e30;
+      c = v > c ? v : c;
+    }
+  }
+  mcg_run_bounds_t r;
+  r.b_thin = (float)((0.5 - 1.0 / 262144.0) * grid);
+  r.c_thin = (float)((c + 16.0) * grid);
+  r.b_mid = (float)((0.5 - t - 1.0 / 2048.0) * grid);
+  return r;
+}
+
+/* Whether the forms accept u, and their value (the tracker's own tests). */
+static inline int mcg_om_thin_ok(float u, const mcg_run_bounds_t *B, float *om)
+{
+  float r;
+  const float uu = u * u;
+  *om = mcg_om_thin(u, uu, &r);
+  return u < MCG_OM_THIN_MAX && fabsf(r) < fmaf(uu, -B->c_thin, B->b_thin);
+}
+
+static inline int mcg_om_mid_ok(float u, const mcg_run_bounds_t *B, float *om)
+{
+  float r;
+  *om = mcg_om_mid(u, u * u, &r);
+  return u < MCG_OM_MID_MAX && fabsf(r) < B->b_mid;
+}
+
 static inline uint64_t mcg_fnv_word(uint64_t h, float v)
 {
   uint32_t u;

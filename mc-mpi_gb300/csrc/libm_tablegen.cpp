@@ -144,6 +144,35 @@ int main(int argc, char **argv)
     printf("%s: %zu exceptions, max midpoint distance %.4f ulp\n", fn == 0 ? "logf" : "expf",
            all.size(), (double)dmax);
   }
+  /* the tracker's short forms of 1 - expf(-u): wherever their acceptance
+   * test passes they must give the host library's value, for every u */
+  {
+    const mcg_run_bounds_t B = mcg_run_bounds(f.tau_exp);
+    long long bad = 0, rej_thin = 0, rej_mid = 0;
+    const uint32_t hi = asu(MCG_OM_MID_MAX), thin = asu(MCG_OM_THIN_MAX);
+#pragma omp parallel for reduction(+ : bad, rej_thin, rej_mid) schedule(dynamic, 1 << 16)
+    for (long long ui = 0; ui < (long long)hi; ++ui) {
+      const float u = asf((uint32_t)ui);
+      volatile float om = 1.0f - expf(-u);
+      float v;
+      if (!mcg_om_mid_ok(u, &B, &v))
+        ++rej_mid;
+      else if (asu(v) != asu(om))
+        ++bad;
+      if (ui < (long long)thin) {
+        if (!mcg_om_thin_ok(u, &B, &v))
+          ++rej_thin;
+        else if (asu(v) != asu(om))
+          ++bad;
+      }
+    }
+    if (bad) {
+      fprintf(stderr, "libm_tablegen: the short forms of 1 - expf(-u) accept %lld wrong values\n", bad);
+      return 1;
+    }
+    printf("short 1 - expf(-u): none wrong; left to the evaluator %lld thin, %lld mid arguments\n",
+           rej_thin, rej_mid);
+  }
   /* the host logf's largest relative error on (0, 1), against the double
    * log (itself within 1e-16): the strict tracker's certain-crossing test
    * assumes at most 2^-22 */

@@ -331,7 +331,7 @@ extern "C" int mcg_adjoint_run(mcg_context *ctx, const mcg_source *src, int64_t 
   P.counters = ctx->d_counters;
   P.libm = ctx->libm;
   P.libm_tab = ctx->libm_tab;
-  P.refill_steps = ctx->refill;
+  P.refill_steps = ctx->refill ? ctx->refill : 8;
   P.chunk = 64;
   P.with_grad = with_gradient ? 1 : 0;
   P.max_steps = ctx->max_steps;

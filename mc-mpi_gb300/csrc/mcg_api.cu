@@ -127,6 +127,10 @@ int mcg_load_libm(mcg_context *ctx)
   }
   ctx->libm.tau_log_max = tl;
   ctx->libm.tau_exp_max = te;
+  const mcg_run_bounds_t rb = mcg_run_bounds(hdr.tau_exp);
+  ctx->run_bounds[0] = rb.b_thin;
+  ctx->run_bounds[1] = rb.c_thin;
+  ctx->run_bounds[2] = rb.b_mid;
   cudaError_t e;
   float *dtl = nullptr, *dte = nullptr;
   uint2 *dhl = nullptr, *dhe = nullptr;
@@ -226,10 +230,11 @@ extern "C" int mcg_create(int device, int mode, mcg_context **out)
  * geometry: launches and tally reads then return MCG_ERR_STATE. */
 static void free_geometry(mcg_context *ctx)
 {
-  for (void *p : {(void *)ctx->d_cells_strict, (void *)ctx->d_cells_fast, (void *)ctx->d_tally})
+  for (void *p : {(void *)ctx->d_cells_strict, (void *)ctx->d_cells_fast, (void *)ctx->d_tab,
+                  (void *)ctx->d_tally})
     if (p)
       cudaFree(p);
-  ctx->d_cells_strict = ctx->d_cells_fast = nullptr;
+  ctx->d_cells_strict = ctx->d_cells_fast = ctx->d_tab = nullptr;
   ctx->d_tally = nullptr;
   ctx->n_layers = ctx->n_cells = ctx->cell_lo = 0;
   ctx->layer_start.clear();
@@ -239,7 +244,7 @@ static void free_geometry(mcg_context *ctx)
   ctx->rates.clear();
   ctx->cells_strict.clear();
   ctx->cells_fast.clear();
-  ctx->thin = false;
+  ctx->thin = ctx->thin_fast = false;
 }
 
 /* Allocations still to succeed before one is made to fail (-1: none). */
@@ -327,18 +332,56 @@ void mcg_cell_params(float sig, float rate, int gi, float dx, float4 &strict, fl
                      elo, ehi);
 }
 
-/* A chain is optically thin when every cell's absorption optical width
- * sig_a (edge_hi - edge_lo) is at most 5e-4: a crossing then has
- * |sig_a d_edge| >= MCG_EXP_SMALL_T (0.0054) only for |mu| < 0.093, which
- * takes under 1 % of the crossings (their share of directions is about
- * mu^2), so the strict tracker's certain-crossing path may evaluate the
- * small-argument exp form alone and send the others to the full step. */
+/* The tiles' parameters of n consecutive cells (mcg_tiles): {sig_a, sig_i, length
+ * of a flight that enters the cell by its left face, by its right face}, the
+ * float differences of the faces that mcg_step_cross forms (entered at a
+ * neighbour's face, which between layers of different spacing differs from
+ * the cell's own in the last bits).  Lengths outside the range in which the
+ * cached-reciprocal division is exact, and those of cells that would amplify
+ * the weight, are NaN: such steps take the full form.
+ * sig_i <= EPS is 0 in both arithmetics: the flight always crosses. */
+void mcg_tile_table(const float4 *c, int n, float4 *tab, float2 *right, float2 *left)
+{
+  for (int k = 0; k < n; ++k) {
+    auto length = [&](float a) { return a >= 0x1p-90f && a <= 0x1p90f && c[k].x >= 0.0f ? a : NAN; };
+    tab[k] = make_float4(c[k].x, c[k].y, length(c[k].w - (k ? c[k - 1].w : c[k].z)),
+                         length((k + 1 < n ? c[k + 1].z : c[k].w) - c[k].z));
+    if (right) {
+      right[k] = make_float2(tab[k].x, tab[k].z);
+      left[k] = make_float2(tab[k].x, tab[k].w);
+    }
+  }
+}
+
+/* thin: every cell's absorption optical width sig_a (edge_hi - edge_lo) is at
+ * most 2e-4, so that a crossing has u >= MCG_OM_THIN_MAX (2^-8) only for
+ * |mu| < 0.05, 0.3 % of the crossings (their share of directions is about
+ * mu^2), which go to the full step; thin_fast: both optical widths at most
+ * 4e-4 (the short series, below 2^-7, again for |mu| > 0.05). */
 static void update_thin(mcg_context *ctx)
 {
-  float widest = 0.0f;
-  for (const float4 &c : ctx->cells_strict)
-    widest = std::max(widest, std::fabs(c.x) * (c.w - c.z));
-  ctx->thin = !ctx->cells_strict.empty() && widest <= 5e-4f;
+  float wa = 0.0f, wi = 0.0f;
+  for (const float4 &c : ctx->cells_strict) {
+    wa = std::max(wa, std::fabs(c.x) * (c.w - c.z));
+    wi = std::max(wi, std::fabs(c.y) * (c.w - c.z));
+  }
+  /* 1 %: a cell entered at a neighbour's face may be a few ulps of x wider */
+  ctx->width_a = 1.01f * wa;
+  ctx->width_i = 1.01f * wi;
+  ctx->thin = !ctx->cells_strict.empty() && wa <= 2e-4f;
+  ctx->thin_fast = !ctx->cells_strict.empty() && std::max(wa, wi) <= 4e-4f;
+}
+
+static cudaError_t upload_tab(mcg_context *ctx)
+{
+  /* n + 2 PAD float4, then twice n + 2 PAD float2 */
+  const size_t n = ctx->cells_fast.size(), row = n + 2 * MCG_TAB_PAD;
+  std::vector<float4> tab(2 * row, make_float4(0, 0, 0, 0));
+  float2 *thin = reinterpret_cast<float2 *>(&tab[row]);
+  mcg_tile_table(ctx->cells_fast.data(), (int)n, &tab[MCG_TAB_PAD], thin + MCG_TAB_PAD,
+                 thin + row + MCG_TAB_PAD);
+  ctx->d_thin = reinterpret_cast<float2 *>(ctx->d_tab + row);
+  return cudaMemcpy(ctx->d_tab, tab.data(), tab.size() * sizeof(float4), cudaMemcpyHostToDevice);
 }
 
 extern "C" int mcg_set_layers(mcg_context *ctx, int n_layers, const int32_t *h_index_start,
@@ -378,6 +421,7 @@ extern "C" int mcg_set_layers(mcg_context *ctx, int n_layers, const int32_t *h_i
   cudaError_t e;
   if ((e = mcg_dev_malloc((void **)&ctx->d_cells_strict, total * sizeof(float4))) != cudaSuccess ||
       (e = mcg_dev_malloc((void **)&ctx->d_cells_fast, total * sizeof(float4))) != cudaSuccess ||
+      (e = mcg_dev_malloc((void **)&ctx->d_tab, 2 * (total + 2 * (size_t)MCG_TAB_PAD) * sizeof(float4))) != cudaSuccess ||
       (e = mcg_dev_malloc((void **)&ctx->d_tally, total * sizeof(unsigned long long))) != cudaSuccess) {
     free_geometry(ctx);
     return mcg_cuda_fail(e, "cudaMalloc(layers)");
@@ -396,6 +440,10 @@ extern "C" int mcg_set_layers(mcg_context *ctx, int n_layers, const int32_t *h_i
   ctx->cells_strict = cs;
   ctx->cells_fast = cf;
   update_thin(ctx);
+  if ((e = upload_tab(ctx)) != cudaSuccess) {
+    free_geometry(ctx);
+    return mcg_cuda_fail(e, "cudaMemcpy(layers)");
+  }
   ctx->n_cells = total;
   ctx->cell_lo = h_index_start[0];
   ctx->min_w = particle_min_weight;
@@ -442,7 +490,8 @@ extern "C" int mcg_set_layers_xs(mcg_context *ctx, int n_layers, const int32_t *
   if ((e = cudaMemcpy(ctx->d_cells_strict, ctx->cells_strict.data(), total * sizeof(float4),
                       cudaMemcpyHostToDevice)) != cudaSuccess ||
       (e = cudaMemcpy(ctx->d_cells_fast, ctx->cells_fast.data(), total * sizeof(float4),
-                      cudaMemcpyHostToDevice)) != cudaSuccess) {
+                      cudaMemcpyHostToDevice)) != cudaSuccess ||
+      (e = upload_tab(ctx)) != cudaSuccess) {
     free_geometry(ctx);
     return mcg_cuda_fail(e, "mcg_set_layers_xs: upload");
   }
@@ -563,7 +612,7 @@ extern "C" int mcg_set_launch(mcg_context *ctx, int32_t block, int32_t blocks_pe
     return mcg_fail(MCG_ERR_ARG, "mcg_set_launch: bad arguments");
   ctx->block = block; /* 0: chosen per launch from the chain length */
   ctx->blocks_per_sm = blocks_per_sm;
-  ctx->refill = refill_steps ? refill_steps : 8;
+  ctx->refill = refill_steps; /* 0: chosen per kernel */
   return MCG_OK;
 }
 
@@ -600,6 +649,7 @@ int mcg_track_launch(mcg_context *ctx, mcg_particle *d_particles, int64_t n, int
   mcg_track_params P;
   memset(&P, 0, sizeof(P));
   P.cells = strict ? ctx->d_cells_strict : ctx->d_cells_fast;
+  P.tab = {ctx->d_tab + MCG_TAB_PAD, ctx->d_thin + MCG_TAB_PAD, ctx->n_cells + 2 * MCG_TAB_PAD};
   P.n_cells = ctx->n_cells;
   P.cell_lo = ctx->cell_lo;
   P.min_w = ctx->min_w;
@@ -617,44 +667,52 @@ int mcg_track_launch(mcg_context *ctx, mcg_particle *d_particles, int64_t n, int
   P.counters = ctx->d_counters;
   P.libm = ctx->libm;
   P.libm_tab = ctx->libm_tab;
-  P.refill_steps = ctx->refill;
-  P.chunk = 64;
   P.max_steps = ctx->max_steps;
   if (ctx->algorithm == MCG_ALGO_EVENT) {
     ctx->launches++;
     return mcg_event_run(ctx, P);
   }
   /* default shape: short chains keep one tally copy per warp in 256-thread
-   * blocks; long chains share one copy per 1024-thread block */
-  int block = ctx->block;
-  if (block == 0)
-    block = ((size_t)ctx->n_cells * 8 * 8 <= 24 * 1024) ? 256 : 1024;
-  const int warps = block / 32;
-  const size_t base = sizeof(mcg_libm_tab) + 16 * sizeof(unsigned long long);
+   * blocks; long chains share one copy per block of 1024 threads (thin ones
+   * MCG_THIN_BLOCK), or of fewer where the copy and the warps' tiles would not
+   * fit; thin chains take the thin kernel with its tally unless the caller
+   * set another one or a larger block */
   int tmode = ctx->tally_mode;
-  /* one tally copy per warp while it stays small, else one per block */
-  int copies = ((size_t)ctx->n_cells * 8 * warps <= 24 * 1024) ? warps : 1;
-  if (tmode != MCG_TALLY_GLOBAL && base + (size_t)ctx->n_cells * 8 > (size_t)ctx->smem_optin)
+  bool thin = (strict ? ctx->thin : ctx->thin_fast) && tmode == MCG_TALLY_SMEM32 &&
+              ctx->block <= MCG_THIN_BLOCK;
+  auto copies_of = [&](int b) { /* one tally copy per warp while it stays small, else one per block */
+    return !thin && (size_t)ctx->n_cells * 8 * (b / 32) <= 24 * 1024 ? b / 32 : 1;
+  };
+  auto smem_of = [&](int b) {
+    return mcg_track_smem(tmode == MCG_TALLY_GLOBAL ? 0 : (size_t)ctx->n_cells * copies_of(b), b, thin);
+  };
+  int block = ctx->block;
+  if (block == 0) {
+    block = thin ? MCG_THIN_BLOCK : ((size_t)ctx->n_cells * 8 * 8 <= 24 * 1024) ? 256 : 1024;
+    while (tmode != MCG_TALLY_GLOBAL && block > 256 && smem_of(block) > (size_t)ctx->smem_optin)
+      block -= 128;
+  }
+  if (tmode != MCG_TALLY_GLOBAL && smem_of(block) > (size_t)ctx->smem_optin) {
     tmode = MCG_TALLY_GLOBAL; /* chain too long for a shared-memory copy */
-  size_t smem = base + (tmode == MCG_TALLY_GLOBAL ? 0 : (size_t)ctx->n_cells * 8 * copies);
-  P.tally_copies = copies;
+    thin = false;
+    block = ctx->block ? ctx->block : 1024;
+  }
+  const size_t smem = smem_of(block);
+  P.tally_copies = copies_of(block);
+  mcg_track_rounds(ctx, thin, P);
+  P.run = mcg_run_setup(ctx->log2_scale, ctx->min_w, thin, ctx->run_bounds, ctx->width_a,
+                        ctx->width_i);
   void (*kern)(mcg_track_params);
-  if (strict && mcg_strict_thin(ctx))
-    kern = tmode == MCG_TALLY_SMEM64 ? mcg_track_kernel<true, MCG_TALLY_SMEM64, true>
-         : tmode == MCG_TALLY_SMEM32 ? mcg_track_kernel<true, MCG_TALLY_SMEM32, true>
-                                     : mcg_track_kernel<true, MCG_TALLY_GLOBAL, true>;
-  else if (strict)
-    kern = tmode == MCG_TALLY_SMEM64 ? mcg_track_kernel<true, MCG_TALLY_SMEM64, false>
-         : tmode == MCG_TALLY_SMEM32 ? mcg_track_kernel<true, MCG_TALLY_SMEM32, false>
-                                     : mcg_track_kernel<true, MCG_TALLY_GLOBAL, false>;
-  else if (ctx->thin) /* the fast step ignores THIN but for the loop's unrolling */
-    kern = tmode == MCG_TALLY_SMEM64 ? mcg_track_kernel<false, MCG_TALLY_SMEM64, true>
-         : tmode == MCG_TALLY_SMEM32 ? mcg_track_kernel<false, MCG_TALLY_SMEM32, true>
-                                     : mcg_track_kernel<false, MCG_TALLY_GLOBAL, true>;
+  if (strict)
+    kern = thin ? mcg_track_kernel<true, MCG_TALLY_LO32, true>
+           : tmode == MCG_TALLY_SMEM64 ? mcg_track_kernel<true, MCG_TALLY_SMEM64, false>
+           : tmode == MCG_TALLY_SMEM32 ? mcg_track_kernel<true, MCG_TALLY_SMEM32, false>
+                                       : mcg_track_kernel<true, MCG_TALLY_GLOBAL, false>;
   else
-    kern = tmode == MCG_TALLY_SMEM64 ? mcg_track_kernel<false, MCG_TALLY_SMEM64, false>
-         : tmode == MCG_TALLY_SMEM32 ? mcg_track_kernel<false, MCG_TALLY_SMEM32, false>
-                                     : mcg_track_kernel<false, MCG_TALLY_GLOBAL, false>;
+    kern = thin ? mcg_track_kernel<false, MCG_TALLY_LO32, true>
+           : tmode == MCG_TALLY_SMEM64 ? mcg_track_kernel<false, MCG_TALLY_SMEM64, false>
+           : tmode == MCG_TALLY_SMEM32 ? mcg_track_kernel<false, MCG_TALLY_SMEM32, false>
+                                       : mcg_track_kernel<false, MCG_TALLY_GLOBAL, false>;
   /* the limit is raised to the device's opt-in maximum, the same value on
    * every call, so launches of the same kernel from other host threads (other
    * contexts, the no-allocation entry point) cannot lower it under this one */
@@ -669,8 +727,7 @@ int mcg_track_launch(mcg_context *ctx, mcg_particle *d_particles, int64_t n, int
       return mcg_cuda_fail(e, "occupancy");
     bps = std::max(bps, 1);
   }
-  long long want_blocks = (n + block - 1) / block;
-  int grid = (int)std::min<long long>((long long)ctx->sm_count * bps, std::max(want_blocks, 1LL));
+  const int grid = mcg_track_grid(ctx->sm_count * bps, block, n, P);
   if ((e = cudaMemsetAsync(ctx->d_next, 0, sizeof(unsigned long long), ctx->stream)) != cudaSuccess)
     return mcg_cuda_fail(e, "cudaMemsetAsync");
   cudaEventRecord(ctx->ev0, ctx->stream);

@@ -316,6 +316,7 @@ static mcg_batch_state *batch_of(mcg_context *ctx)
 static void batch_free(mcg_batch_state *B)
 {
   for (void *p : {B->d_slabs, B->d_items, (void *)B->d_cells_strict, (void *)B->d_cells_fast,
+                  (void *)B->d_tab,
                   (void *)B->d_tally, (void *)B->d_item_next, (void *)B->d_hist0})
     if (p)
       cudaFree(p);
@@ -360,11 +361,12 @@ extern "C" int mcg_batch_set(mcg_context *ctx, int32_t n_slabs, const mcg_slab *
   if (total > INT32_MAX || smem_need > (size_t)ctx->smem_optin)
     return mcg_fail(MCG_ERR_ARG, "mcg_batch_set: %lld cells / largest slab %d cells too large",
                     (long long)total, maxc);
-  std::vector<float4> cs, cf;
+  std::vector<float4> cs, cf, tab;
   std::vector<mcg_batch_slab_dev> sd;
   try {
     cs.resize(total);
     cf.resize(total);
+    tab.resize(total + 2 * MCG_TAB_PAD, make_float4(0, 0, 0, 0));
     sd.resize(n_slabs);
   } catch (const std::bad_alloc &) {
     return mcg_fail(MCG_ERR_ARG, "mcg_batch_set: no host memory for %lld cells", (long long)total);
@@ -394,6 +396,7 @@ extern "C" int mcg_batch_set(mcg_context *ctx, int32_t n_slabs, const mcg_slab *
     const float dx = (1.0f - 0.0f) / (float)sl.n_cells; /* Layer(0, 1, 0, m): src/layer.cpp:47 */
     for (int j = 0; j < sl.n_cells; ++j)
       mcg_cell_params(h_sigs[off + j], h_rates[off + j], j, dx, cs[off + j], cf[off + j]);
+    mcg_tile_table(&cf[off], sl.n_cells, &tab[MCG_TAB_PAD + off]);
     sd[s].cell_off = (int32_t)off;
     sd[s].m = sl.n_cells;
     sd[s].src.seed_mode = sl.seed_mode;
@@ -418,12 +421,14 @@ extern "C" int mcg_batch_set(mcg_context *ctx, int32_t n_slabs, const mcg_slab *
   cudaError_t e;
   if ((e = mcg_dev_malloc((void **)&B->d_cells_strict, total * sizeof(float4))) != cudaSuccess ||
       (e = mcg_dev_malloc((void **)&B->d_cells_fast, total * sizeof(float4))) != cudaSuccess ||
+      (e = mcg_dev_malloc((void **)&B->d_tab, (total + 2 * MCG_TAB_PAD) * sizeof(float4))) != cudaSuccess ||
       (e = mcg_dev_malloc((void **)&B->d_tally, total * sizeof(unsigned long long))) != cudaSuccess ||
       (e = mcg_dev_malloc(&B->d_slabs, n_slabs * sizeof(mcg_batch_slab_dev))) != cudaSuccess ||
       (e = mcg_dev_malloc((void **)&B->d_item_next, 64)) != cudaSuccess)
     return fail(e, "mcg_batch_set: cudaMalloc");
   if ((e = cudaMemcpy(B->d_cells_strict, cs.data(), total * sizeof(float4), cudaMemcpyHostToDevice)) != cudaSuccess ||
       (e = cudaMemcpy(B->d_cells_fast, cf.data(), total * sizeof(float4), cudaMemcpyHostToDevice)) != cudaSuccess ||
+      (e = cudaMemcpy(B->d_tab, tab.data(), tab.size() * sizeof(float4), cudaMemcpyHostToDevice)) != cudaSuccess ||
       (e = cudaMemcpy(B->d_slabs, sd.data(), n_slabs * sizeof(mcg_batch_slab_dev), cudaMemcpyHostToDevice)) != cudaSuccess ||
       (e = cudaMemset(B->d_tally, 0, total * sizeof(unsigned long long))) != cudaSuccess)
     return fail(e, "mcg_batch_set: upload");
@@ -500,7 +505,7 @@ static int batch_configure(mcg_context *ctx, mcg_batch_state *B, mcg_batch_launc
   P.libm_tab = ctx->libm_tab;
   P.min_w = B->min_w;
   P.q_log2 = ctx->log2_scale;
-  P.refill_steps = ctx->refill;
+  P.refill_steps = ctx->refill ? ctx->refill : 8;
   P.max_steps = ctx->max_steps;
   const int tm = B->tally_mode;
   L.smem = sizeof(mcg_libm_tab) + 16 * 8 + 4 * 8 +
@@ -663,6 +668,7 @@ extern "C" int mcg_batch_run_per_slab(mcg_context *ctx)
     mcg_track_params P;
     memset(&P, 0, sizeof(P));
     P.cells = (strict ? B->d_cells_strict : B->d_cells_fast) + B->cell_off[s];
+    P.tab = {B->d_tab + MCG_TAB_PAD + B->cell_off[s], nullptr, 0};
     P.n_cells = sl.n_cells;
     P.cell_lo = 0;
     P.min_w = B->min_w;
@@ -678,14 +684,14 @@ extern "C" int mcg_batch_run_per_slab(mcg_context *ctx)
     P.counters = ctx->d_counters;
     P.libm = ctx->libm;
     P.libm_tab = ctx->libm_tab;
-    P.refill_steps = ctx->refill;
-    P.chunk = 64;
+    mcg_track_rounds(ctx, false, P);
+    P.run = mcg_run_setup(ctx->log2_scale, B->min_w, false, ctx->run_bounds);
     P.max_steps = ctx->max_steps;
     const int block = ((size_t)sl.n_cells * 64 <= 24 * 1024) ? 256 : 1024;
     const int warps = block / 32;
     const int copies = ((size_t)sl.n_cells * 8 * warps <= 24 * 1024) ? warps : 1;
     P.tally_copies = copies;
-    const size_t smem = sizeof(mcg_libm_tab) + 16 * 8 + (size_t)sl.n_cells * 8 * copies;
+    const size_t smem = mcg_track_smem((size_t)sl.n_cells * copies, block, false);
     auto kern = strict ? mcg_track_kernel<true, MCG_TALLY_SMEM32, false>
                        : mcg_track_kernel<false, MCG_TALLY_SMEM32, false>;
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -693,8 +699,7 @@ extern "C" int mcg_batch_run_per_slab(mcg_context *ctx)
     int bps = 1;
     if (e == cudaSuccess)
       e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, kern, block, smem);
-    long long want = (sl.n_histories + block - 1) / block;
-    const int grid = (int)std::min<long long>((long long)ctx->sm_count * std::max(bps, 1), want);
+    const int grid = mcg_track_grid(ctx->sm_count * std::max(bps, 1), block, sl.n_histories, P);
     if (e == cudaSuccess)
       e = cudaMemsetAsync(ctx->d_next, 0, 8, ctx->stream);
     if (e == cudaSuccess) {

@@ -391,7 +391,7 @@ static int fit_launch_track(mcg_context *ctx, mcg_fit_state *F, int with_grad)
   P.step = F->step;
   P.min_w = F->min_w;
   P.q_log2 = ctx->log2_scale;
-  P.refill_steps = ctx->refill;
+  P.refill_steps = ctx->refill ? ctx->refill : 8;
   P.with_grad = with_grad;
   P.max_steps = ctx->max_steps;
   const size_t smem = 4 * 8 + (size_t)F->max_cells * 12;

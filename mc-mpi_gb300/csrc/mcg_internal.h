@@ -24,6 +24,7 @@ struct mcg_batch_state {
   void *d_items = nullptr;  /* mcg_batch_item[] */
   int n_items = 0, items_cap = 0;
   float4 *d_cells_strict = nullptr, *d_cells_fast = nullptr;
+  float4 *d_tab = nullptr; /* the tiles' per-cell parameters */
   unsigned long long *d_tally = nullptr;
   unsigned long long *d_item_next = nullptr;
   float min_w = 0.f;
@@ -107,8 +108,15 @@ struct mcg_context {
   std::vector<int32_t> layer_start, layer_m;
   std::vector<float> layer_dx, sigs, rates;
   std::vector<float4> cells_strict, cells_fast;
-  bool thin = false; /* every cell's sig_a width <= 5e-4 (mcg_step THIN) */
+  bool thin = false;      /* every cell's sig_a width <= 2e-4 (strict THIN) */
+  bool thin_fast = false; /* sig_a and sig_i widths <= 4e-4 (fast THIN) */
+  float width_a = 0.f, width_i = 0.f; /* those largest widths */
   float4 *d_cells_strict = nullptr, *d_cells_fast = nullptr;
+  /* the tiles' per-cell parameters (mcg_tile_table), MCG_TAB_PAD entries
+   * before and after; of the thin form one such array per direction, in the
+   * same allocation */
+  float4 *d_tab = nullptr;
+  float2 *d_thin = nullptr;
   unsigned long long *d_tally = nullptr;
   int log2_scale = 40;
   unsigned long long *d_counters = nullptr, *d_next = nullptr;
@@ -117,6 +125,7 @@ struct mcg_context {
   bool libm_loaded = false;
   mcg_libm_dev libm = {};
   mcg_libm_tab *libm_tab = nullptr;
+  float run_bounds[3] = {}; /* mcg_run_bounds of the table: b_thin, c_thin, b_mid */
   uint32_t libm_n_log = 0, libm_n_exp = 0;
 
   /* particle buffers of the host-pointer entry points */
@@ -126,7 +135,7 @@ struct mcg_context {
   size_t scratch_cap = 0;
 
   /* launch shape */
-  int block = 0, blocks_per_sm = 0, refill = 8;
+  int block = 0, blocks_per_sm = 0, refill = 0; /* refill 0: chosen per kernel */
   uint32_t max_steps = 1u << 28; /* per-history step limit (MCG_ERR_LIMIT) */
   int tally_mode = 1;            /* MCG_TALLY_SMEM32 */
 
@@ -147,6 +156,9 @@ int mcg_fail(int code, const char *fmt, ...);
  * it (mcg_testing_fail_allocation). */
 cudaError_t mcg_dev_malloc(void **p, size_t bytes);
 int mcg_cuda_fail(cudaError_t e, const char *what);
+#define MCG_TAB_PAD 32 /* a tile reads past its chain's ends (mcg_tiles) */
+void mcg_tile_table(const float4 *cells_fast, int n, float4 *tab, float2 *right = nullptr,
+                    float2 *left = nullptr);
 void mcg_cell_params(float sig, float rate, int gi, float dx, float4 &strict, float4 &fast);
 int mcg_track_launch(mcg_context *ctx, mcg_particle *d_particles, int64_t n, int32_t *d_results,
                      int64_t *d_steps, int64_t *d_scatters, const mcg_source *src, int64_t first);

@@ -28,10 +28,11 @@
 #include "mcg_internal.h"
 #include "mcg_track.cuh"
 
-/* Layout of the scratch array (bytes): step table, tally, counters, work
+/* Layout of the scratch array (bytes): step table, tile table, tally, counters, work
  * counter.  The tally region is sized as 8 bytes per cell. */
 #define MCG_NOALLOC_CELLS_OFF 0
-#define MCG_NOALLOC_TALLY_OFF (MCG_NOALLOC_CELLS_OFF + 16 * MCG_NOALLOC_MAX_CELLS)
+#define MCG_NOALLOC_TAB_OFF (MCG_NOALLOC_CELLS_OFF + 16 * MCG_NOALLOC_MAX_CELLS)
+#define MCG_NOALLOC_TALLY_OFF (MCG_NOALLOC_TAB_OFF + 16 * (MCG_NOALLOC_MAX_CELLS + 2 * MCG_TAB_PAD))
 #define MCG_NOALLOC_CNT_OFF (MCG_NOALLOC_TALLY_OFF + 8 * MCG_NOALLOC_MAX_CELLS)
 #define MCG_NOALLOC_NEXT_OFF (MCG_NOALLOC_CNT_OFF + 8 * 16)
 #define MCG_NOALLOC_BYTES (MCG_NOALLOC_NEXT_OFF + 256)
@@ -92,18 +93,21 @@ extern "C" int mcg_simulate_fast_noalloc(int n_layers, const int32_t *h_index_st
   if (rc != MCG_OK)
     return rc;
   float4 *cells = reinterpret_cast<float4 *>(base + MCG_NOALLOC_CELLS_OFF);
+  float4 *tab = reinterpret_cast<float4 *>(base + MCG_NOALLOC_TAB_OFF) + MCG_TAB_PAD;
   unsigned long long *tally = reinterpret_cast<unsigned long long *>(base + MCG_NOALLOC_TALLY_OFF);
   unsigned long long *cnt = reinterpret_cast<unsigned long long *>(base + MCG_NOALLOC_CNT_OFF);
   unsigned long long *next = reinterpret_cast<unsigned long long *>(base + MCG_NOALLOC_NEXT_OFF);
 
   /* step table on the host (as mcg_set_layers), then into the scratch */
-  std::vector<float4> cs(total), cf(total);
+  std::vector<float4> cs(total), cf(total), ct(total);
   int k = 0;
   for (int l = 0; l < n_layers; ++l)
     for (int j = 0; j < h_m[l]; ++j, ++k)
       mcg_cell_params(h_sigs[k], h_rates[k], h_index_start[l] + j, h_dx[l], cs[k], cf[k]);
+  mcg_tile_table(cf.data(), total, ct.data());
   cudaStream_t st = 0;
-  if ((e = cudaMemcpyAsync(cells, cf.data(), total * sizeof(float4), cudaMemcpyHostToDevice, st)) != cudaSuccess ||
+  if ((e = cudaMemcpyAsync(tab, ct.data(), total * sizeof(float4), cudaMemcpyHostToDevice, st)) != cudaSuccess ||
+      (e = cudaMemcpyAsync(cells, cf.data(), total * sizeof(float4), cudaMemcpyHostToDevice, st)) != cudaSuccess ||
       (e = cudaMemsetAsync(tally, 0, total * sizeof(unsigned long long), st)) != cudaSuccess ||
       (e = cudaMemsetAsync(cnt, 0, 16 * sizeof(unsigned long long), st)) != cudaSuccess ||
       (e = cudaMemsetAsync(next, 0, sizeof(unsigned long long), st)) != cudaSuccess)
@@ -113,6 +117,7 @@ extern "C" int mcg_simulate_fast_noalloc(int n_layers, const int32_t *h_index_st
     mcg_track_params P;
     memset(&P, 0, sizeof(P));
     P.cells = cells;
+    P.tab = {tab, nullptr, 0};
     P.n_cells = total;
     P.cell_lo = h_index_start[0];
     P.min_w = particle_min_weight;
@@ -123,22 +128,24 @@ extern "C" int mcg_simulate_fast_noalloc(int n_layers, const int32_t *h_index_st
     P.next = next;
     P.tally = tally;
     P.counters = cnt;
-    P.refill_steps = 8;
-    P.chunk = 64;
+    P.window = MCG_TW_MAX;
+    P.pool_lanes = 16;
+    P.refill_lanes = 8;
+    P.run = mcg_run_setup(log2_scale, particle_min_weight, false, nullptr);
     P.max_steps = 1u << 28;
-    const int block = ((size_t)total * 8 * 8 <= 24 * 1024) ? 256 : 1024;
-    const int warps = block / 32;
-    const int copies = ((size_t)total * 8 * warps <= 24 * 1024) ? warps : 1;
-    P.tally_copies = copies;
-    const size_t base_smem = sizeof(mcg_libm_tab) + 16 * sizeof(unsigned long long);
     int sms = 0, optin = 0, bps = 0;
     if ((e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess ||
         (e = cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev)) != cudaSuccess)
       return mcg_cuda_fail(e, "mcg_simulate_fast_noalloc: device attributes");
-    /* as the context path: a chain whose tally does not fit in the block's
-     * shared memory adds its deposits to the scratch tally directly */
-    const bool smem_tally = base_smem + (size_t)total * 8 * copies <= (size_t)optin;
-    const size_t smem = base_smem + (smem_tally ? (size_t)total * 8 * copies : 0);
+    /* as the context path: the block shrinks until the tally and the tiles
+     * fit in its shared memory (256 threads hold any chain of this entry) */
+    int block = ((size_t)total * 8 * 8 <= 24 * 1024) ? 256 : 1024;
+    auto copies_of = [&](int b) { return (size_t)total * 8 * (b / 32) <= 24 * 1024 ? b / 32 : 1; };
+    while (block > 256 && mcg_track_smem((size_t)total * copies_of(block), block, false) > (size_t)optin)
+      block /= 2;
+    P.tally_copies = copies_of(block);
+    const bool smem_tally = mcg_track_smem((size_t)total * P.tally_copies, block, false) <= (size_t)optin;
+    const size_t smem = mcg_track_smem(smem_tally ? (size_t)total * P.tally_copies : 0, block, false);
     auto kern = smem_tally ? mcg_track_kernel<false, MCG_TALLY_SMEM32, false>
                            : mcg_track_kernel<false, MCG_TALLY_GLOBAL, false>;
     /* the attribute is raised to the device's limit (the same value every
@@ -147,8 +154,7 @@ extern "C" int mcg_simulate_fast_noalloc(int n_layers, const int32_t *h_index_st
     if ((e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, optin)) != cudaSuccess ||
         (e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, kern, block, smem)) != cudaSuccess)
       return mcg_cuda_fail(e, "mcg_simulate_fast_noalloc: launch set-up");
-    long long want = (n + block - 1) / block;
-    int grid = (int)std::min<long long>((long long)sms * std::max(bps, 1), std::max(want, 1LL));
+    const int grid = mcg_track_grid(sms * std::max(bps, 1), block, n, P);
     kern<<<grid, block, smem, st>>>(P);
     if ((e = cudaGetLastError()) != cudaSuccess)
       return mcg_cuda_fail(e, "mcg_simulate_fast_noalloc: launch");

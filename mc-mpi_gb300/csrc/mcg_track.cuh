@@ -3,13 +3,14 @@
  *
  * One lane carries one particle history at a time through the whole chain of
  * layers (a sub-domain crossing is just the next cell's parameters, so the
- * hand-over between sub-domains costs nothing).  The grid is persistent:
- * every warp takes chunks of history indices from a global counter and
- * refills finished lanes from its chunk every `refill_steps` steps, so warps
- * stay full however uneven the history lengths are.  Deposits go to a
- * shared-memory 64-bit fixed-point histogram (one copy per block, or one per
- * warp when the chain is short) and are added to the global tally once per
- * block at the end; the sums are exact, hence order-independent.
+ * hand-over between sub-domains costs nothing), and the warp advances its 32
+ * histories together, a tile of certain crossings each (see "tiles" below).
+ * The grid is persistent: every warp takes chunks of history indices from a
+ * global counter and refills finished lanes from its chunk, so warps stay full
+ * however uneven the history lengths are.  Deposits go to a shared-memory
+ * fixed-point histogram (one copy per block, or one per warp when the chain is
+ * short) and are added to the global tally once per block at the end; the sums
+ * are exact, hence order-independent.
  *
  * The step follows Layer::particle_step (src/layer.cpp:123-190) and the loop
  * Layer::simulate_particle (src/layer.cpp:192-218).
@@ -17,8 +18,21 @@
 #ifndef MCG_TRACK_CUH
 #define MCG_TRACK_CUH
 
+#include <algorithm>
 #include "mcg_device.cuh"
 #include "mcgb300.h"
+#include "mcg_internal.h"
+
+/* Per-cell parameters of the tiles, readable MCG_TAB_PAD cells past both ends:
+ * cell: {sig_a, sig_i, length of a flight entering by the left face, by the
+ * right face}; thin (thin chains): {sig_a, that length} for flights to the
+ * right and, `left` entries on, for flights to the left: half the bytes of the
+ * other (the loads were a quarter of the L1's work on the 10,000-cell slab). */
+struct mcg_tab {
+  const float4 *cell;
+  const float2 *thin;
+  int32_t left;
+};
 
 /* Per-cell step parameters.  strict: {sig_a, sig_i, edge_lo, edge_hi}
  * fast: {sig_a, sig_i (0 when sig_i <= EPS), edge_lo, edge_hi}
@@ -26,6 +40,7 @@
  * GLOBAL cell index i and the cell's own layer spacing (src/layer.cpp:146,150). */
 struct mcg_track_params {
   const float4 *cells;
+  mcg_tab tab;
   int32_t n_cells, cell_lo;
   float min_w;
   int32_t q_log2;
@@ -39,16 +54,20 @@ struct mcg_track_params {
   unsigned long long *counters; /* mcg_counters fields */
   mcg_libm_dev libm;
   const mcg_libm_tab *libm_tab;
-  int32_t refill_steps;
+  int32_t window;       /* most steps of a tile (at most MCG_TW_MAX) */
+  int32_t pool_lanes;   /* lanes waiting for the full step that trigger it */
+  int32_t refill_lanes; /* lanes without a history that trigger a refill */
   int32_t tally_copies; /* 1 or warps per block */
-  int32_t chunk;        /* histories per warp grab (multiple of 32) */
+  int32_t chunk;        /* histories per warp grab (at most MCG_JUMPS) */
   uint32_t max_steps;
+  mcg_run_consts run;
 };
 
 /* Tally accumulation: shared-memory 64-bit atomics, shared-memory 32-bit
- * halves with an explicit carry, or 64-bit atomics straight to the global
- * tally (no shared memory, higher occupancy). */
-enum { MCG_TALLY_SMEM64 = 0, MCG_TALLY_SMEM32 = 1, MCG_TALLY_GLOBAL = 2 };
+ * halves with an explicit carry, 64-bit atomics straight to the global tally,
+ * or (thin chains) shared-memory low words with the carries going straight to
+ * the global tally. */
+enum { MCG_TALLY_SMEM64 = 0, MCG_TALLY_SMEM32 = 1, MCG_TALLY_GLOBAL = 2, MCG_TALLY_LO32 = 3 };
 
 template <int TALLY>
 __device__ __forceinline__ void mcg_tally_add(unsigned long long *t, long long q)
@@ -456,13 +475,10 @@ __device__ __forceinline__ void mcg_step_rest(uint64_t &seed, float &x, float &m
   const float edge = neg ? c.z : c.w;
   float om;
   if (STRICT) {
-    /* d_edge, and the crossing's absorption, do not depend on the flight
-     * sample: start them before the logarithm */
     const float a = __fsub_rn(edge, x), aa = fabsf(a);
     const float de = inv_mu == 0.0f ? MCG_MAXREAL
                      : (aa >= 0x1p-100f && aa <= 0x1p100f) ? mcg_div_by_rcp(a, mu, inv_mu)
                                                             : __fdiv_rn(a, mu);
-    const float om_cross = mcg_one_minus_expf_strict(__fmul_rn(-sig_a, de), T, LM);
     /* di = sig_i > EPS ? -log(h) / sig_i : MAXREAL; the exact value is
      * only needed when the flight may end inside the cell: the certified
      * test settles almost every crossing */
@@ -476,16 +492,16 @@ __device__ __forceinline__ void mcg_step_rest(uint64_t &seed, float &x, float &m
     } else {
       cross = !(di < de);
     }
+    /* one exponential, of the length that the step takes */
+    om = mcg_one_minus_expf_strict(__fmul_rn(-sig_a, cross ? de : di), T, LM);
     if (!cross) {
       inew = idx;
       x = __fadd_rn(x, __fmul_rn(di, mu));
       mu = __fsub_rn(__fmul_rn(2.0f, mcg_rnd_real(seed)), 1.0f);
       inv_mu = mcg_flight_rcp(mu);
-      om = mcg_one_minus_expf_strict(__fmul_rn(-sig_a, di), T, LM);
       ++nsc;
     } else {
       x = edge;
-      om = om_cross;
     }
     const float dw = __fmul_rn(om, wmc);
     wmc = __fsub_rn(wmc, dw);
@@ -526,18 +542,622 @@ __device__ __forceinline__ void mcg_step_rest(uint64_t &seed, float &x, float &m
   idx = inew;
 }
 
-/* THIN: the chain is optically thin (every |sig_a cell width| <= 5e-4):
- * the strict step's thin certain-crossing path, and, in both arithmetics,
- * four steps per pass of the step loop. */
+/* ---------------------------------------------------------------- tiles
+ * A tile is up to TW consecutive certain crossings of one flight.  Along a
+ * flight nothing but the weight is serial: the cells, the random numbers (the
+ * LCG jumps ahead), the face-to-face lengths and the absorbed fractions of the
+ * next TW cells are independent.  A warp holds 32 histories, one per lane,
+ * and advances each by one tile per round:
+ *   1. every lane with a history that can run puts its flight in shared memory;
+ *   2. a few flights at a time, G lanes each: lane j forms the absorbed
+ *      fractions of steps j and j + G, as pairs of the packed f32x2
+ *      operations, and whether each is certainly a crossing;
+ *   3. lane = history again: the weights in order, w <- w - RN(om w), up to the
+ *      first step that is not certain, which gives the deposits;
+ *   4. a few flights at a time, lane j adds the deposits of steps j and j + G
+ *      to the tally.
+ * Against one lane per history through the whole step this makes the cell
+ * loads and the tally atomics runs of consecutive cells (with scattered lanes
+ * the L1 was the bound: 18 of 19 cycles of a warp step on the 10,000-cell
+ * slab), keeps the lanes busy whatever the histories do, and a single history
+ * takes about 30 cycles per step instead of 300, which is what the end of a
+ * launch waits for.  Every step is exactly mcg_step_cross's. */
+/* Lanes per flight in phases 2 and 4 (G) and steps of a tile (2 G).  Thin chains
+ * take 16 and 32: fewer rounds and shared-memory rows per step; others 8 and
+ * 16: their flights are short, and what a tile has after its flight's end is
+ * lost. */
+template <bool THIN> struct mcg_tile_shape {
+  static constexpr int G = THIN ? 16 : 8, TW = 2 * G, F = 32 / G; /* F: flights at a time */
+  static constexpr int PLANE = G * 33;
+};
+#define MCG_TW_MAX 32
+#define MCG_THIN_BLOCK 768 /* most threads of a thin kernel: 85 registers */
+
+/* A warp's shared memory: the flights, and one fraction (then deposit) per
+ * step: step i of flight r at (i / G) PLANE + (r / F) 33 + (r % F) G + i % G,
+ * consecutive over the lanes of phases 2 and 4 and free of bank conflicts down
+ * the steps of 32 flights (phase 3). */
+template <bool THIN> struct mcg_tile_smem {
+  uint4 flight[32]; /* state << 1; THIN: the flight's bounds on g and |r| */
+  float4 slant[32]; /* |mu| twice, -|RN(1 / mu)| twice */
+  int4 place[32];   /* length to the first face (inf: the cell's), cell, direction, steps taken */
+  float step[2 * mcg_tile_shape<THIN>::PLANE];
+};
+
+/* Jumps of the sample stream in the shifted representation (state << 1, so the
+ * modulus is the word's): s -> A s + C after k steps. */
+struct mcg_real_jumps {
+  unsigned long long A[MCG_TW_MAX + 1], C[MCG_TW_MAX + 1];
+};
+
+__device__ __forceinline__ void mcg_fill_real_jumps(mcg_real_jumps *J)
+{
+  for (int k = threadIdx.x; k <= MCG_TW_MAX; k += blockDim.x) {
+    const uint64_t c = mcg_lcg_skip(0ull, (uint64_t)k, 0);
+    J->A[k] = (mcg_lcg_skip(1ull, (uint64_t)k, 0) - c) & MCG_MASK63;
+    J->C[k] = c << 1;
+  }
+}
+
+/* A warp's view: its shared memory, and its lanes' jumps of j + 1 and
+ * G + j + 1 steps. */
+template <bool THIN> struct mcg_tile_warp {
+  mcg_tile_smem<THIN> *S;
+  uint64_t A0, C0, A1, C1;
+
+  __device__ __forceinline__ mcg_tile_warp(mcg_tile_smem<THIN> *s, const mcg_real_jumps *J)
+  {
+    constexpr int G = mcg_tile_shape<THIN>::G;
+    const int lane = threadIdx.x & 31, j = lane & (G - 1);
+    S = s;
+    A0 = J->A[j + 1], C0 = J->C[j + 1], A1 = J->A[G + j + 1], C1 = J->C[G + j + 1];
+    S->place[lane] = make_int4(0, 0, 0, 0); /* a row not yet used reads cell 0 */
+  }
+};
+
+/* Pairs of floats in one 64-bit register: one instruction for two IEEE
+ * operations (round to nearest, subnormals kept). */
+typedef unsigned long long mcg_f2;
+__device__ __forceinline__ mcg_f2 f2_make(float a, float b)
+{
+  mcg_f2 r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+  return r;
+}
+__device__ __forceinline__ mcg_f2 f2_both(float a) { return f2_make(a, a); }
+__device__ __forceinline__ void f2_get(mcg_f2 v, float &a, float &b)
+{
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v));
+}
+__device__ __forceinline__ mcg_f2 f2_mul(mcg_f2 a, mcg_f2 b)
+{
+  mcg_f2 r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ mcg_f2 f2_add(mcg_f2 a, mcg_f2 b)
+{
+  mcg_f2 r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ mcg_f2 f2_fma(mcg_f2 a, mcg_f2 b, mcg_f2 c)
+{
+  mcg_f2 r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+
+/* Certain crossing by the linear bound: with g = 1 + floor(s / 2^40) 2^-23
+ * (the state's top 23 bits as the float of [1, 2) below 1 + h),
+ *     g < RN(K - sig_i de),  K = 2 - 2^-20,
+ * gives h <= g - 1 + 2^-23 <= 1 - T - 2^-20 + 2^-23 + 2^-24, T = sig_i de
+ * exactly (T <= 1, since g >= 1), hence -ln h >= 1 - h >= T + 2^-20.5 and
+ * -logf(h) >= (T + 2^-20.5)(1 - 2^-22) > T: the reference's flight passes the
+ * face (the reasoning of mcg_cross_threshold, with the tangent of e^-T
+ * instead of a MUFU operation).  FAST: 1 - h exceeds the computed collision
+ * probability, at most T (1 + 2^-20).  It fails on T + 1e-6 of the crossings
+ * where the exponential one fails on 1 - e^-T + 6e-5. */
+#define MCG_TILE_K (2.0f - 0x1p-20f)
+
+/* Two steps of a flight (packed): their absorbed fractions of the weight, NaN
+ * where a step is not certainly a crossing that this form reproduces bit for
+ * bit.  a: lengths to the faces along x; amu, ny: |mu| and -|RN(1 / mu)|, both
+ * twice.  With the reciprocal's sign turned every quantity that the series
+ * need negative comes out negative (roundings are symmetric): lengths and
+ * fractions are returned negated.
+ * THIN: the collision bound (thr) and the midpoint bound are the flight's,
+ * taken at the chain's widest cell, and its largest u is below the thin
+ * form's limit (mcg_thin_tests). */
+template <bool STRICT, bool THIN>
+__device__ __forceinline__ void mcg_tile_steps(mcg_f2 a, mcg_f2 amu, mcg_f2 ny, mcg_f2 sig_a,
+                                               mcg_f2 sig_i, uint32_t s_hi0, uint32_t s_hi1,
+                                               float thr, float bound, const mcg_run_consts &R,
+                                               float &nom0, float &nom1, mcg_f2 &nde)
+{
+  const float g0 = __uint_as_float(__funnelshift_r(s_hi0, 0x7fu, 9));
+  const float g1 = __uint_as_float(__funnelshift_r(s_hi1, 0x7fu, 9));
+  bool ok0, ok1;
+  mcg_f2 nom;
+  if (STRICT) {
+    /* mcg_div_by_rcp, mcg_om_thin / mcg_om_mid in pairs */
+    const mcg_f2 nq = f2_mul(a, ny);
+    nde = f2_fma(f2_fma(amu, nq, a), ny, nq);
+    const mcg_f2 nu = f2_mul(sig_a, nde), uu = f2_mul(nu, nu);
+    mcg_f2 r; /* of either sign */
+    if (THIN) {
+      const mcg_f2 w = f2_fma(nu, f2_both(1.0f / 6.0f), f2_both(0.5f));
+      nom = f2_add(f2_add(f2_fma(uu, w, nu), f2_both(-0.75f)), f2_both(0.75f));
+      r = f2_fma(uu, w, f2_fma(nom, f2_both(-1.0f), nu));
+    } else {
+      mcg_f2 p = f2_fma(nu, f2_both(1.0f / 720.0f), f2_both(1.0f / 120.0f));
+      p = f2_fma(nu, p, f2_both(1.0f / 24.0f));
+      p = f2_fma(nu, p, f2_both(1.0f / 6.0f));
+      nom = f2_fma(uu, f2_fma(nu, p, f2_both(0.5f)), nu);
+      nom = f2_add(f2_add(nom, f2_both(-0.75f)), f2_both(0.75f));
+      const mcg_f2 ne = f2_fma(f2_mul(nu, f2_both(-1.0f)), nu, uu); /* uu - u^2 */
+      mcg_f2 nd = f2_fma(f2_both(0.5f), uu, f2_fma(nom, f2_both(-1.0f), nu));
+      nd = f2_fma(f2_both(-0.5f), ne, nd);
+      r = f2_fma(f2_mul(uu, nu), p, nd);
+    }
+    float r0, r1;
+    f2_get(r, r0, r1);
+    if (THIN) {
+      ok0 = (fabsf(r0) < bound) & (g0 < thr);
+      ok1 = (fabsf(r1) < bound) & (g1 < thr);
+    } else {
+      float u0, u1, t0, t1;
+      f2_get(nu, u0, u1);
+      f2_get(f2_fma(sig_i, nde, f2_both(MCG_TILE_K)), t0, t1);
+      ok0 = (fabsf(r0) < R.b_mid) & (fabsf(u0) < MCG_OM_MID_MAX) & (g0 < t0);
+      ok1 = (fabsf(r1) < R.b_mid) & (fabsf(u1) < MCG_OM_MID_MAX) & (g1 < t1);
+    }
+  } else {
+    /* mcg_one_minus_exp_small and, not THIN, mcg_one_minus_exp_fast of -u */
+    nde = f2_mul(a, ny);
+    const mcg_f2 nu = f2_mul(sig_a, nde);
+    mcg_f2 p = f2_fma(nu, f2_both(1.0f / 6.0f), f2_both(0.5f));
+    p = f2_fma(nu, p, f2_both(1.0f));
+    nom = f2_mul(nu, p);
+    if (THIN) {
+      ok0 = g0 < thr;
+      ok1 = g1 < thr;
+    } else {
+      float u0, u1, t0, t1, s0, s1, l0, l1;
+      f2_get(nu, u0, u1);
+      f2_get(f2_mul(sig_i, nde), t0, t1);
+      p = f2_fma(nu, f2_both(1.0f / 5040.0f), f2_both(1.0f / 720.0f));
+      p = f2_fma(nu, p, f2_both(1.0f / 120.0f));
+      p = f2_fma(nu, p, f2_both(1.0f / 24.0f));
+      p = f2_fma(nu, p, f2_both(1.0f / 6.0f));
+      p = f2_fma(nu, p, f2_both(0.5f));
+      p = f2_fma(nu, p, f2_both(1.0f));
+      f2_get(f2_mul(nu, p), l0, l1);
+      f2_get(nom, s0, s1);
+      nom = f2_make(fminf(u0, t0) > -0x1p-7f ? s0 : l0, fminf(u1, t1) > -0x1p-7f ? s1 : l1);
+      ok0 = (u0 > -0.25f) & (g0 < __fadd_rn(MCG_TILE_K, t0));
+      ok1 = (u1 > -0.25f) & (g1 < __fadd_rn(MCG_TILE_K, t1));
+    }
+  }
+  f2_get(nom, nom0, nom1);
+  nom0 = ok0 ? nom0 : __int_as_float(0x7fc00000);
+  nom1 = ok1 ? nom1 : __int_as_float(0x7fc00000);
+}
+
+/* Two deposits (scaled values, exact conversions) of a lane, not THIN. */
+template <int TALLY>
+__device__ __forceinline__ void mcg_tile_deposit(bool in0, unsigned long long *t0, float v0,
+                                                 bool in1, unsigned long long *t1, float v1)
+{
+  if (in0) {
+    if (v0 < 0x1p31f)
+      mcg_deposit_u31<TALLY>(t0, v0);
+    else
+      mcg_tally_add<TALLY>(t0, __float2ll_rn(v0));
+  }
+  if (in1) {
+    if (v1 < 0x1p31f)
+      mcg_deposit_u31<TALLY>(t1, v1);
+    else
+      mcg_tally_add<TALLY>(t1, __float2ll_rn(v1));
+  }
+}
+
+/* The bounds of a flight on a thin chain from its widest cell (R.w_a, R.w_i:
+ * the chain's largest sig_a and sig_i widths): {thr, bound} of
+ * mcg_tile_steps, which no step passes when the flight is so slanted that its
+ * steps may leave the thin form's range or its first deposit 31 bits.  The
+ * factor covers the roundings of the lengths and products. */
+template <bool STRICT>
+__device__ __forceinline__ float2 mcg_thin_tests(float inv_mu, float wmc, const mcg_run_consts &R)
+{
+  const float y = fabsf(inv_mu) * (1.0f + 0x1p-20f);
+  const float u = __fmul_rn(R.w_a, y), ti = __fmul_rn(R.w_i, y);
+  const bool ok = (STRICT ? u < MCG_OM_THIN_MAX : fmaxf(u, ti) < 0x1p-7f) &
+                  (__fmul_rn(u, __fmul_rn(wmc, R.scale)) < 0x1p31f);
+  return make_float2(ok ? __fsub_rn(MCG_TILE_K, ti) : -1.0f,
+                     __fmaf_rn(__fmul_rn(u, u), -R.c_thin, R.b_thin));
+}
+
+/* Adds a deposit q to the 32-bit tally of a thin chain (MCG_TALLY_LO32): the
+ * low words are in shared memory, and what passes them goes to the global
+ * 64-bit tally at once.  A carry every 2^32 / q deposits (q about 2e6 at
+ * scale 2^35, 6e7 at 2^40) costs less than shared memory for 64 bits per cell,
+ * which takes it from the cell table's L1 and from more warps. */
+__device__ __forceinline__ void mcg_lo32_add(unsigned *lo, unsigned long long *global, long long q)
+{
+  const uint32_t v = (uint32_t)q, old = atomicAdd(lo, v);
+  const uint64_t hi = (uint64_t)(q >> 32) + ((uint32_t)(old + v) < old ? 1u : 0u);
+  if (hi)
+    atomicAdd(global, (unsigned long long)(hi << 32));
+}
+
+/* Shared-memory add under a predicate (no branch); the old value, or 0. */
+__device__ __forceinline__ uint32_t mcg_shared_add_if(bool p, uint32_t addr, uint32_t v)
+{
+  uint32_t old;
+  asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.s32 p, %3, 0;\n\tmov.u32 %0, 0;\n\t"
+               "@p atom.shared.add.u32 %0, [%1], %2;\n\t}"
+               : "=r"(old)
+               : "r"(addr), "r"(v), "r"((int)p)
+               : "memory");
+  return old;
+}
+
+/* Phase 2 for U passes of F flights from pass q0.  All loads come before the
+ * first store, which the compiler could not tell apart from the next pass's
+ * rows: 4 passes in flight instead of 1 took the 10,000-cell slab from 131 to
+ * 110 ms per 5e6 histories (the table's L1 misses).  Rows past the last flight
+ * are computed and never used. */
+template <bool STRICT, bool THIN, int U>
+__device__ __forceinline__ void mcg_tile_form(mcg_tile_smem<THIN> *S, int q0, const mcg_tab &tab,
+                                              const mcg_tile_warp<THIN> &B,
+                                              const mcg_run_consts &R)
+{
+  constexpr int G = mcg_tile_shape<THIN>::G, F = 32 / G, PLANE = mcg_tile_shape<THIN>::PLANE;
+  const int lane = threadIdx.x & 31, sub = lane / G, j = lane & (G - 1);
+  const int not_first = j ? 0x7f800000 : 0; /* makes the first length inf or NaN: not the least */
+  int4 pl[U];
+  uint4 fl[U];
+  ulonglong2 sl[U];
+  float a[U], b[U], sa0[U], sa1[U], si0[U], si1[U], om0[U], om1[U];
+#pragma unroll
+  for (int v = 0; v < U; ++v)
+    pl[v] = S->place[F * (q0 + v) + sub];
+#pragma unroll
+  for (int v = 0; v < U; ++v)
+    if (THIN) {
+      const float2 *p = tab.thin + (pl[v].y + j * pl[v].z);
+      const float2 c = __ldg(p), d = __ldg(p + G * pl[v].z);
+      sa0[v] = c.x, sa1[v] = d.x, a[v] = c.y, b[v] = d.y;
+      si0[v] = si1[v] = 0.0f;
+    } else {
+      const float4 *p = tab.cell + (pl[v].y + j * pl[v].z);
+      const float4 c = __ldg(p), d = __ldg(p + G * pl[v].z);
+      sa0[v] = c.x, sa1[v] = d.x, si0[v] = c.y, si1[v] = d.y;
+      a[v] = pl[v].z < 0 ? c.w : c.z, b[v] = pl[v].z < 0 ? d.w : d.z;
+    }
+#pragma unroll
+  for (int v = 0; v < U; ++v) {
+    fl[v] = S->flight[F * (q0 + v) + sub];
+    sl[v] = *reinterpret_cast<const ulonglong2 *>(&S->slant[F * (q0 + v) + sub]);
+  }
+#pragma unroll
+  for (int v = 0; v < U; ++v) {
+    const uint64_t s = (uint64_t)fl[v].y << 32 | fl[v].x;
+    const uint64_t n0 = B.A0 * s + B.C0, n1 = B.A1 * s + B.C1;
+    mcg_f2 nde;
+    mcg_tile_steps<STRICT, THIN>(
+        f2_make(fminf(a[v], __int_as_float(pl[v].x | not_first)), b[v]), sl[v].x, sl[v].y,
+        f2_make(sa0[v], sa1[v]), f2_make(si0[v], si1[v]), (uint32_t)(n0 >> 32),
+        (uint32_t)(n1 >> 32), __uint_as_float(fl[v].z), __uint_as_float(fl[v].w), R, om0[v], om1[v],
+        nde);
+  }
+#pragma unroll
+  for (int v = 0; v < U; ++v) {
+    S->step[33 * (q0 + v) + lane] = om0[v];
+    S->step[PLANE + 33 * (q0 + v) + lane] = om1[v];
+  }
+}
+
+/* Phase 4 for U passes from pass q0. */
+template <bool THIN, int TALLY, int U>
+__device__ __forceinline__ void mcg_tile_add(mcg_tile_smem<THIN> *S, int q0,
+                                             unsigned long long *tally, unsigned *lo32)
+{
+  constexpr int G = mcg_tile_shape<THIN>::G, F = 32 / G, PLANE = mcg_tile_shape<THIN>::PLANE;
+  const int lane = threadIdx.x & 31, sub = lane / G, j = lane & (G - 1);
+  int4 pl[U];
+  float v0[U], v1[U];
+#pragma unroll
+  for (int v = 0; v < U; ++v) {
+    pl[v] = S->place[F * (q0 + v) + sub];
+    v0[v] = S->step[33 * (q0 + v) + lane];
+    v1[v] = S->step[PLANE + 33 * (q0 + v) + lane];
+  }
+  if (THIN) {
+    uint32_t at[2 * U];
+    bool carry[2 * U], any = false;
+#pragma unroll
+    for (int v = 0; v < U; ++v) {
+      const uint32_t d0 = __float2uint_rn(v0[v]), d1 = __float2uint_rn(v1[v]);
+      at[2 * v] = (uint32_t)(pl[v].y + j * pl[v].z);
+      at[2 * v + 1] = at[2 * v] + G * pl[v].z;
+      const uint32_t o0 = mcg_shared_add_if(j < pl[v].w, at[2 * v], d0);
+      const uint32_t o1 = mcg_shared_add_if(j + G < pl[v].w, at[2 * v + 1], d1);
+      any |= carry[2 * v] = (uint32_t)(o0 + d0) < o0;
+      any |= carry[2 * v + 1] = (uint32_t)(o1 + d1) < o1;
+    }
+    if (__any_sync(0xffffffffu, any)) {
+      const uint32_t base = (uint32_t)__cvta_generic_to_shared(lo32);
+#pragma unroll
+      for (int v = 0; v < 2 * U; ++v)
+        if (carry[v])
+          atomicAdd(&tally[(at[v] - base) >> 2], 1ull << 32);
+    }
+  } else {
+#pragma unroll
+    for (int v = 0; v < U; ++v) {
+      unsigned long long *t = tally + (pl[v].y + j * pl[v].z);
+      mcg_tile_deposit<TALLY>(j < pl[v].w, t, v0[v], j + G < pl[v].w, t + G * pl[v].z, v1[v]);
+    }
+  }
+}
+
+/* One round over the warp (all lanes call): the lanes with `can` advance their
+ * flights by up to nmax (1 .. TW) certain crossings and return their
+ * number; a0: length to the first face when the flight starts inside the cell,
+ * else infinity; W is the weight times the tally scale, res (fast) its
+ * residue; test: mcg_thin_tests (THIN).  tab: the chain's tile table; lo32
+ * (THIN, with the global tally): see mcg_lo32_add. */
+template <bool STRICT, bool THIN, int TALLY>
+__device__ __forceinline__ int mcg_tiles(bool can, uint64_t s2, float amu, float ainv, float a0,
+                                         int dir, int idx, int nmax, float2 test, float &W,
+                                         float &res, const mcg_tab &tab,
+                                         unsigned long long *tally, unsigned *lo32,
+                                         const mcg_tile_warp<THIN> &B, const mcg_run_consts &R)
+{
+  constexpr int G = mcg_tile_shape<THIN>::G, TW = 2 * G, F = 32 / G;
+  constexpr int PLANE = mcg_tile_shape<THIN>::PLANE;
+  mcg_tile_smem<THIN> *S = B.S;
+  const int lane = threadIdx.x & 31;
+  const unsigned mask = __ballot_sync(0xffffffffu, can);
+  const int cnt = __popc(mask), rank = __popc(mask & lanemask_lt());
+  S->place[lane].w = 0; /* rows past the last flight: no deposits */
+  if (can) {
+    S->flight[rank] = make_uint4((uint32_t)s2, (uint32_t)(s2 >> 32), __float_as_uint(test.x),
+                                 __float_as_uint(test.y));
+    S->slant[rank] = make_float4(amu, amu, -ainv, -ainv);
+    S->place[rank] = make_int4(__float_as_int(a0), THIN && dir < 0 ? idx + tab.left : idx, dir, 0);
+  }
+  __syncwarp();
+  int q = 0;
+  if (THIN)
+    for (; F * (q + 2) < cnt; q += 4)
+      mcg_tile_form<STRICT, THIN, 4>(S, q, tab, B, R);
+  for (; F * q < cnt; q += 2)
+    mcg_tile_form<STRICT, THIN, 2>(S, q, tab, B, R);
+  __syncwarp();
+  int n = 0;
+  if (can) {
+    float *st = S->step + 33 * (rank / F) + G * (rank % F);
+    if (nmax < TW)
+      st[(nmax / G) * PLANE + nmax % G] = __int_as_float(0x7fc00000);
+    if (THIN) {
+      /* unconditionally, with the last valid weight kept every eight steps
+       * (from the first NaN on everything is NaN); the rest of an early end
+       * again from there */
+      float w = W, rs = res;
+#pragma unroll
+      for (int i = 0; i < TW; ++i) {
+        float *si = st + (i / G) * PLANE + i % G;
+        const float dv = __fmul_rn(-*si, w), w2 = __fsub_rn(w, dv);
+        if (!STRICT)
+          rs = __fadd_rn(rs, __fsub_rn(__fsub_rn(w, w2), dv));
+        w = w2;
+        *si = dv;
+        if (i % 8 == 7 && w == w) {
+          W = w;
+          res = rs;
+          n = i + 1;
+        }
+      }
+      for (; n < TW; ++n) {
+        const float dv = st[(n / G) * PLANE + n % G];
+        if (dv != dv)
+          break;
+        const float w2 = __fsub_rn(W, dv);
+        if (!STRICT)
+          res = __fadd_rn(res, __fsub_rn(__fsub_rn(W, w2), dv));
+        W = w2;
+      }
+      /* phase 4: the address of step j is y + j z */
+      S->place[rank] = make_int4(0, (int)__cvta_generic_to_shared(lo32) + 4 * idx, 4 * dir, n);
+    } else {
+      bool ok = true;
+#pragma unroll
+      for (int i = 0; i < TW; ++i) {
+        float *si = st + (i / G) * PLANE + i % G;
+        const float dv = __fmul_rn(-*si, W);
+        ok &= dv < 0x1p62f; /* false for NaN */
+        if (ok) {
+          const float w2 = __fsub_rn(W, dv);
+          if (!STRICT)
+            res = __fadd_rn(res, __fsub_rn(__fsub_rn(W, w2), dv));
+          W = w2;
+          *si = dv;
+          n = i + 1;
+        }
+      }
+      S->place[rank].w = n;
+    }
+  }
+  __syncwarp();
+  q = 0;
+  if (THIN)
+    for (; F * (q + 2) < cnt; q += 4)
+      mcg_tile_add<THIN, TALLY, 4>(S, q, tally, lo32);
+  for (; F * q < cnt; q += 2)
+    mcg_tile_add<THIN, TALLY, 2>(S, q, tally, lo32);
+  __syncwarp();
+  return n;
+}
+
+/* Length along x from x to the face ahead, for a flight that starts at x in a
+ * cell; NaN (no tile) outside the range in which the tiles' division is exact,
+ * without a direction, or beyond the cell's own length (x outside the cell, or
+ * a cell without one). */
+__device__ __forceinline__ float mcg_first_length(const float4 c, const float4 tab, float x,
+                                                  float mu, float inv_mu, float wmc)
+{
+  const float a = fabsf(mu < 0.0f ? __fsub_rn(x, c.z) : __fsub_rn(c.w, x));
+  const bool inside = mu < 0.0f ? x >= c.z : x <= c.w;
+  return inside & (inv_mu != 0.0f) & (wmc <= 0x1p60f) & ((a == 0.0f) | (a >= 0x1p-100f)) &
+                 (a <= (mu < 0.0f ? tab.w : tab.z))
+             ? a
+             : __int_as_float(0x7fc00000);
+}
+
+/* Most steps of a tile from cell idx of [lo, hi): to the end of the range, one
+ * while the weight is near the minimum (so no step passes it unseen), none
+ * (the full step) below the weights that scale exactly. */
+__device__ __forceinline__ int mcg_tile_limit(int width, int idx, int lo, int hi, float mu,
+                                              float wmc, uint32_t left, const mcg_run_consts &R)
+{
+  int n = min(width, mu < 0.0f ? idx - lo + 1 : hi - idx);
+  n = (int)min((uint32_t)n, left);
+  return wmc >= R.w_many ? n : wmc >= R.w_one ? min(n, 1) : 0;
+}
+
+/* The step that a tile left: the flight sample's state, then whatever the step
+ * is (mcg_step_rest). */
+template <bool STRICT, int TALLY>
+__device__ __forceinline__ void mcg_full(uint64_t &seed, float &x, float &mu, float &wmc,
+                                         float &inv_mu, int &idx, uint32_t &nsc, const float4 c,
+                                         unsigned long long *tally_cell, int qs,
+                                         const mcg_libm_tab *T, const mcg_libm_dev &LM,
+                                         float *l_out = nullptr, bool *coll_out = nullptr,
+                                         float *dep_out = nullptr, float *wres = nullptr)
+{
+  mcg_lcg_next(seed);
+  mcg_step_rest<STRICT, TALLY>(seed, x, mu, wmc, inv_mu, idx, nsc, c, tally_cell, qs, T, LM, l_out,
+                               coll_out, dep_out, wres);
+}
+
+/* A warp's share of a launch's histories: a chunk taken from a counter, handed
+ * to idle lanes in order.  The seed-chain state of a chunk's first history is
+ * found by one jump-ahead (`state_of`, run by all lanes together) and a
+ * lane's own by one multiply-add from jump[r], jump[MCG_JUMPS + r], the
+ * r-step jumps (instead of a jump-ahead of about 20 doublings per lane, run
+ * by the one or two lanes that refill). */
+#define MCG_JUMPS 32
+
+__device__ __forceinline__ void mcg_fill_jumps(unsigned long long *jump)
+{
+  for (int r = threadIdx.x; r < MCG_JUMPS; r += blockDim.x) {
+    const uint64_t c = mcg_lcg_skip(0ull, (uint64_t)r, 1);
+    jump[r] = (mcg_lcg_skip(1ull, (uint64_t)r, 1) - c) & MCG_MASK63;
+    jump[MCG_JUMPS + r] = c;
+  }
+}
+
+/* Shared memory of mcg_track_kernel: libm tables, counters, jumps, the tally's
+ * copies (an even number of words), the warps' tiles. */
+inline size_t mcg_track_smem(size_t tally_words, int block, bool thin)
+{
+  if (thin)
+    tally_words = (tally_words + 1) / 2; /* MCG_TALLY_LO32 */
+  return sizeof(mcg_libm_tab) + (16 + 2 * MCG_JUMPS + 2 * (MCG_TW_MAX + 1)) * 8 +
+         ((tally_words + 1) & ~(size_t)1) * 8 +
+         (size_t)(block / 32) * (thin ? sizeof(mcg_tile_smem<true>) : sizeof(mcg_tile_smem<false>));
+}
+
+struct mcg_pool {
+  long long next = 0, end = 0; /* what is left of the chunk */
+  long long base = 0;          /* the chunk's first history and its state */
+  uint64_t state = 0;
+  bool drained = false;
+
+  /* The history of this lane (in `need`), or -1, and its seed-chain state;
+   * chunks of at most MCG_JUMPS histories.  The whole warp calls. */
+  template <class F>
+  __device__ __forceinline__ long long take(unsigned need, unsigned long long *counter, long long n,
+                                            int chunk, const F &state_of,
+                                            const unsigned long long *jump, uint64_t &my_state)
+  {
+    const int cnt = __popc(need), rank = __popc(need & lanemask_lt());
+    const long long avail = end - next;
+    long long my = -1, my_base = base;
+    uint64_t st = state;
+    if (rank < avail)
+      my = next + rank;
+    if (cnt > avail && !drained) {
+      unsigned long long b = 0;
+      if ((threadIdx.x & 31) == 0)
+        b = atomicAdd(counter, (unsigned long long)chunk);
+      b = __shfl_sync(0xffffffffu, b, 0);
+      if ((long long)b >= n) {
+        drained = true;
+        next = end = 0;
+      } else {
+        end = min((long long)b + chunk, n);
+        base = (long long)b;
+        state = state_of(base);
+        const long long r2 = rank - avail;
+        if (rank >= avail && r2 < end - base) {
+          my = base + r2;
+          my_base = base;
+          st = state;
+        }
+        next = min(base + (cnt - avail), end);
+      }
+    } else {
+      next += min((long long)cnt, avail);
+    }
+    const int r = my >= 0 ? (int)(my - my_base) : 0;
+    my_state = (jump[r] * st + jump[MCG_JUMPS + r]) & MCG_MASK63;
+    return my;
+  }
+};
+
+/* Counters of a finished history: result r, final weight. */
+template <bool STRICT>
+__device__ __forceinline__ void mcg_count_end(unsigned long long *s_cnt, int r, float wmc,
+                                              float wres, int qs)
+{
+  atomicAdd(&s_cnt[MCG_CNT_HIST], 1ull);
+  long long wq = mcg_to_fixed(wmc, qs);
+  if (!STRICT)
+    wq += mcg_to_fixed(wres, qs); /* the weight's float-float remainder */
+  if (r == -1) {
+    atomicAdd(&s_cnt[MCG_CNT_LEFT], 1ull);
+    atomicAdd(&s_cnt[MCG_CNT_WLEFT], (unsigned long long)wq);
+  } else if (r == 1) {
+    atomicAdd(&s_cnt[MCG_CNT_RIGHT], 1ull);
+    atomicAdd(&s_cnt[MCG_CNT_WRIGHT], (unsigned long long)wq);
+  } else if (r == 0) {
+    atomicAdd(&s_cnt[MCG_CNT_KILL], 1ull);
+    atomicAdd(&s_cnt[MCG_CNT_WKILL], (unsigned long long)wq);
+  } else {
+    atomicOr(&s_cnt[MCG_CNT_ERR], 1ull);
+  }
+}
+
+/* THIN: the chain is optically thin (see update_thin in mcg_api.cu) and the
+ * tally is MCG_TALLY_LO32. */
 template <bool STRICT, int TALLY, bool THIN>
-__global__ void __launch_bounds__(1024) mcg_track_kernel(mcg_track_params P)
+__global__ void __launch_bounds__(THIN ? MCG_THIN_BLOCK : 1024) mcg_track_kernel(mcg_track_params P)
 {
   extern __shared__ __align__(16) unsigned char smem[];
   mcg_libm_tab *T = reinterpret_cast<mcg_libm_tab *>(smem);
   unsigned long long *s_cnt = reinterpret_cast<unsigned long long *>(smem + sizeof(mcg_libm_tab));
-  unsigned long long *s_tally = s_cnt + 16;
+  unsigned long long *s_jump = s_cnt + 16;
+  mcg_real_jumps *s_real = reinterpret_cast<mcg_real_jumps *>(s_jump + 2 * MCG_JUMPS);
+  unsigned long long *s_tally = s_jump + 2 * MCG_JUMPS + 2 * (MCG_TW_MAX + 1);
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int ncell = P.n_cells, lo = P.cell_lo;
+  mcg_fill_jumps(s_jump);
+  mcg_fill_real_jumps(s_real);
 
   if (STRICT) {
     const float *src = reinterpret_cast<const float *>(P.libm_tab);
@@ -547,88 +1167,41 @@ __global__ void __launch_bounds__(1024) mcg_track_kernel(mcg_track_params P)
   }
   if (tid < 16)
     s_cnt[tid] = 0ull;
-  if (TALLY != MCG_TALLY_GLOBAL)
-    for (int i = tid; i < ncell * P.tally_copies; i += blockDim.x)
-      s_tally[i] = 0ull;
+  /* the block's copy of the tally: 64-bit words, or low words (THIN) */
+  const int words = TALLY == MCG_TALLY_GLOBAL ? 0 : THIN ? (ncell + 1) / 2 : ncell * P.tally_copies;
+  for (int i = tid; i < words; i += blockDim.x)
+    s_tally[i] = 0ull;
+  mcg_tile_smem<THIN> *tile = reinterpret_cast<mcg_tile_smem<THIN> *>(
+      s_tally + ((words + 1) & ~1)) + warp;
   __syncthreads();
-  unsigned long long *my_tally = TALLY == MCG_TALLY_GLOBAL
+  unsigned *lo32 = THIN ? reinterpret_cast<unsigned *>(s_tally) : nullptr;
+  unsigned long long *my_tally = TALLY == MCG_TALLY_GLOBAL || THIN
                                      ? P.tally
                                      : s_tally + (size_t)(warp % P.tally_copies) * ncell;
 
-  uint64_t seed = 0;
+  uint64_t s2 = 0; /* the state, shifted left by one */
   float x = 0.f, mu = 0.f, wmc = 0.f, inv_mu = 0.f;
   float wres = 0.f; /* fast: the weight's rounding residue (mcg_fast_weight_update) */
+  float2 test = make_float2(0.f, 0.f); /* THIN: mcg_thin_tests */
+  float a0 = 0.f;   /* mcg_first_length; inf: x is the face the cell was entered by */
   int idx = 0;
   int64_t hid = -1;
   uint32_t nst = 0, nsc = 0;
-  bool active = false;
+  bool active = false, wait = false; /* wait: the lane's step needs the full form */
   unsigned long long tot_steps = 0, tot_scat = 0;
-  long long pool_next = 0, pool_end = 0;
-  bool drained = false;
+  mcg_pool pool;
   const float min_w = P.min_w;
   const int qs = P.q_log2;
+  const mcg_tile_warp<THIN> tiles(tile, s_real);
 
   for (;;) {
-    unsigned need = __ballot_sync(0xffffffffu, !active);
-    if (need) {
-      int cnt = __popc(need), rank = __popc(need & lanemask_lt());
-      long long avail = pool_end - pool_next, my = -1;
-      if (rank < avail)
-        my = pool_next + rank;
-      if (cnt > avail && !drained) {
-        unsigned long long base = 0;
-        if (lane == 0)
-          base = atomicAdd(P.next, (unsigned long long)P.chunk);
-        base = __shfl_sync(0xffffffffu, base, 0);
-        if ((long long)base >= P.n) {
-          drained = true;
-          pool_next = pool_end = 0;
-        } else {
-          long long end = min((long long)base + P.chunk, (long long)P.n);
-          long long r2 = rank - avail;
-          if (rank >= avail && r2 < end - (long long)base)
-            my = (long long)base + r2;
-          pool_next = min((long long)base + (cnt - avail), end);
-          pool_end = end;
-        }
-      } else {
-        pool_next += min((long long)cnt, avail);
-      }
-      if (!active && my >= 0) {
-        hid = my;
-        mcg_load_particle(P, hid, seed, x, mu, wmc, idx);
-        idx -= lo;
-        inv_mu = mcg_flight_rcp(mu);
-        wres = 0.f;
-        nst = nsc = 0;
-        active = true;
-      }
-    }
-    if (!__any_sync(0xffffffffu, active))
-      break;
-
-    if (active) {
-      /* up to refill_steps steps, never past the step limit; idx is the
-       * cell index local to the chain, so one unsigned compare is the
-       * range test of simulate_particle's loop */
-      const int kmax = (int)min((uint32_t)P.refill_steps, P.max_steps - nst);
-      int k = 0;
-      /* four steps per loop pass on thin chains: measured 3 % faster
-       * (strict) than one; on thicker chains, where crossings split between
-       * the exp evaluator's paths, one (four measured 36 % slower) */
-      constexpr int kUnroll = THIN ? 4 : 1;
-#pragma unroll kUnroll
-      for (; k < kmax;) {
-        if (!((wmc >= min_w) & ((unsigned)idx < (unsigned)ncell)))
-          break;
-        mcg_step<STRICT, TALLY, THIN>(seed, x, mu, wmc, inv_mu, idx, nsc, __ldg(P.cells + idx),
-                                      &my_tally[idx], qs, T, P.libm, nullptr, nullptr, nullptr,
-                                      STRICT ? nullptr : &wres);
-        ++k;
-      }
-      const bool going = (wmc >= min_w) & ((unsigned)idx < (unsigned)ncell);
-      nst += (uint32_t)k;
-      if (!going || nst >= P.max_steps) {
+    bool alive = active & (wmc >= min_w) & ((unsigned)idx < (unsigned)ncell) & (nst < P.max_steps);
+    const unsigned ab = __ballot_sync(0xffffffffu, alive);
+    /* ended histories leave and newborns come once refill_lanes lanes are
+     * without a living history, or no lane has one */
+    if (!ab || (__popc(~ab) >= P.refill_lanes &&
+                (!pool.drained || __any_sync(0xffffffffu, active & !alive)))) {
+      if (active & !alive) {
         /* history ends: classification of simulate_particle; a history
          * still alive in the chain here has reached the step limit */
         const bool in = (wmc >= min_w) && ((unsigned)idx < (unsigned)ncell);
@@ -643,9 +1216,11 @@ __global__ void __launch_bounds__(1024) mcg_track_kernel(mcg_track_params P)
           r = 0;
         else
           r = -1;
-        if (P.particles) {
+        if (P.particles && nst) {
+          if (a0 == INFINITY)
+            x = mu < 0.0f ? __ldg(&P.cells[idx + 1].z) : __ldg(&P.cells[idx - 1].w);
           unsigned long long *q = reinterpret_cast<unsigned long long *>(P.particles + hid);
-          q[0] = seed;
+          q[0] = s2 >> 1;
           q[1] = (unsigned long long)__float_as_uint(x) |
                  ((unsigned long long)__float_as_uint(mu) << 32);
           q[2] = (unsigned long long)__float_as_uint(wmc) |
@@ -657,25 +1232,90 @@ __global__ void __launch_bounds__(1024) mcg_track_kernel(mcg_track_params P)
           P.steps[hid] = nst;
         if (P.scatters)
           P.scatters[hid] = nsc;
-        atomicAdd(&s_cnt[MCG_CNT_HIST], 1ull);
-        long long wq = mcg_to_fixed(wmc, qs);
-        if (!STRICT)
-          wq += mcg_to_fixed(wres, qs); /* the weight's float-float remainder */
-        if (r == -1) {
-          atomicAdd(&s_cnt[MCG_CNT_LEFT], 1ull);
-          atomicAdd(&s_cnt[MCG_CNT_WLEFT], (unsigned long long)wq);
-        } else if (r == 1) {
-          atomicAdd(&s_cnt[MCG_CNT_RIGHT], 1ull);
-          atomicAdd(&s_cnt[MCG_CNT_WRIGHT], (unsigned long long)wq);
-        } else if (r == 0) {
-          atomicAdd(&s_cnt[MCG_CNT_KILL], 1ull);
-          atomicAdd(&s_cnt[MCG_CNT_WKILL], (unsigned long long)wq);
-        } else {
-          atomicOr(&s_cnt[MCG_CNT_ERR], 1ull);
-        }
+        mcg_count_end<STRICT>(s_cnt, r, wmc, wres, qs);
         tot_steps += nst;
         tot_scat += nsc;
         active = false;
+      }
+      const unsigned need = __ballot_sync(0xffffffffu, !active);
+      uint64_t my_seed = 0;
+      const long long my = pool.take(need, P.next, P.n, P.chunk, [&](long long base) {
+        return P.particles || P.src.seed_mode ? 0ull
+               : mcg_lcg_skip(P.src.base_seed, (uint64_t)(P.first + base) + 1, 1);
+      }, s_jump, my_seed);
+      if (!active && my >= 0) {
+        hid = my;
+        uint64_t seed;
+        if (!P.particles && P.src.seed_mode == 0)
+          mcg_source_particle_at(P.src, my_seed, seed, x, mu, wmc, idx);
+        else
+          mcg_load_particle(P, hid, seed, x, mu, wmc, idx);
+        s2 = seed << 1;
+        idx -= lo;
+        inv_mu = mcg_flight_rcp(mu);
+        wres = 0.f;
+        nst = nsc = 0;
+        active = true;
+        alive = (wmc >= min_w) & ((unsigned)idx < (unsigned)ncell) & (nst < P.max_steps);
+        if (THIN)
+          test = mcg_thin_tests<STRICT>(inv_mu, wmc, P.run);
+        if (alive)
+          a0 = mcg_first_length(__ldg(P.cells + idx), __ldg(P.tab.cell + idx), x, mu, inv_mu, wmc);
+      }
+      if (!__any_sync(0xffffffffu, active))
+        break;
+    }
+
+    /* one tile for every lane that can; the lanes whose step needs the full
+     * form wait until pool_lanes of them do (or no other lane can step) and
+     * take it together.  Each pass steps a lane, makes one wait, completes
+     * the waiting steps or ends a history, and no lane passes its step
+     * limit, so this ends. */
+    bool can = alive & !wait;
+    const int nmax = a0 == a0 ? mcg_tile_limit(min(P.window, mcg_tile_shape<THIN>::TW), idx, 0, ncell,
+                                               mu, wmc, P.max_steps - nst, P.run)
+                              : 0;
+    wait |= can & (nmax == 0);
+    can &= nmax != 0;
+    if (__any_sync(0xffffffffu, can)) {
+      const int dir = mu < 0.0f ? -1 : 1;
+      float W = __fmul_rn(wmc, P.run.scale), res = __fmul_rn(wres, P.run.scale);
+      const int n = mcg_tiles<STRICT, THIN, TALLY>(can, s2, fabsf(mu), fabsf(inv_mu), a0, dir, idx,
+                                                   nmax, test, W, res, P.tab, my_tally, lo32,
+                                                   tiles, P.run);
+      if (n > 0) {
+        s2 = s_real->A[n] * s2 + s_real->C[n];
+        wmc = __fmul_rn(W, P.run.inv_scale);
+        if (!STRICT)
+          wres = __fmul_rn(res, P.run.inv_scale);
+        idx += n * dir;
+        nst += (uint32_t)n;
+        a0 = INFINITY;
+      }
+      wait |= can & (n < nmax);
+    }
+    const unsigned wb = __ballot_sync(0xffffffffu, wait);
+    if (wb && (__popc(wb) >= P.pool_lanes || !__any_sync(0xffffffffu, alive & !wait))) {
+      if (wait) {
+        if (a0 == INFINITY)
+          x = mu < 0.0f ? __ldg(&P.cells[idx + 1].z) : __ldg(&P.cells[idx - 1].w);
+        uint64_t seed = s2 >> 1;
+        const int cell = idx;
+        float len, dep;
+        bool coll;
+        mcg_full<STRICT, TALLY>(seed, x, mu, wmc, inv_mu, idx, nsc, __ldg(P.cells + idx),
+                                THIN ? nullptr : &my_tally[idx], qs, T, P.libm, &len, &coll, &dep,
+                                STRICT ? nullptr : &wres);
+        if (THIN) {
+          mcg_lo32_add(lo32 + cell, my_tally + cell, mcg_to_fixed(dep, qs));
+          test = mcg_thin_tests<STRICT>(inv_mu, wmc, P.run);
+        }
+        s2 = seed << 1;
+        ++nst;
+        wait = false;
+        a0 = (unsigned)idx < (unsigned)ncell
+                 ? mcg_first_length(__ldg(P.cells + idx), __ldg(P.tab.cell + idx), x, mu, inv_mu, wmc)
+                 : 0.0f;
       }
     }
   }
@@ -690,7 +1330,11 @@ __global__ void __launch_bounds__(1024) mcg_track_kernel(mcg_track_params P)
     atomicAdd(&s_cnt[MCG_CNT_SCAT], tot_scat);
   }
   __syncthreads();
-  if (TALLY != MCG_TALLY_GLOBAL)
+  if (THIN) {
+    for (int i = tid; i < ncell; i += blockDim.x)
+      if (lo32[i])
+        atomicAdd(&P.tally[i], (unsigned long long)lo32[i]);
+  } else if (TALLY != MCG_TALLY_GLOBAL)
     for (int i = tid; i < ncell; i += blockDim.x) {
       unsigned long long s = 0;
       for (int c = 0; c < P.tally_copies; ++c)
@@ -706,6 +1350,24 @@ __global__ void __launch_bounds__(1024) mcg_track_kernel(mcg_track_params P)
       atomicAdd(&P.counters[tid], s_cnt[tid]);
     }
   }
+}
+
+/* Rounds of a launch (see the kernel's loop). */
+inline void mcg_track_rounds(const mcg_context *ctx, bool thin, mcg_track_params &P)
+{
+  P.window = ctx->refill ? ctx->refill : MCG_TW_MAX;
+  P.pool_lanes = 4;
+  P.refill_lanes = thin ? 1 : 2;
+}
+
+/* Grid of at most `resident` blocks, and the chunk of histories a warp takes:
+ * a warp advances its histories together, one tile of each per round, so few
+ * histories are spread over as many warps as there are. */
+inline int mcg_track_grid(int resident, int block, int64_t n, mcg_track_params &P)
+{
+  const int64_t warps = (int64_t)resident * (block / 32);
+  P.chunk = (int)std::min<int64_t>(MCG_JUMPS, (n + warps - 1) / warps);
+  return (int)std::min<int64_t>(resident, n);
 }
 
 #endif

@@ -358,7 +358,7 @@ extern "C" int mcg_worker_run(mcg_context *ctx, const mcg_source *src, int64_t n
   W.items = cnt + 4;
   W.cycles = cnt + 3;
   W.per_cycle = per_cycle;
-  W.refill_steps = ctx->refill;
+  W.refill_steps = ctx->refill ? ctx->refill : 8;
   W.min_w = ctx->min_w;
   W.q_log2 = ctx->log2_scale;
   W.tally = ctx->d_tally;
@@ -1006,7 +1006,7 @@ extern "C" int mcg_worker_run_async(mcg_context *ctx, const mcg_source *src, int
   A.src = *src;
   A.state = state;
   A.src_total = (unsigned long long)n;
-  A.refill_steps = ctx->refill;
+  A.refill_steps = ctx->refill ? ctx->refill : 8;
   A.min_w = ctx->min_w;
   A.q_log2 = ctx->log2_scale;
   A.tally = ctx->d_tally;

@@ -1,0 +1,71 @@
+"""The tiled tracker (a warp advances each of its histories by a tile of up to
+16 or 32 certain crossings) against the event-based tracker, whose single
+crossings and full steps are another path of the same arithmetic: per particle
+and per cell identical, over chain lengths around the tile sizes, thin and
+thick cells, one and several layers of different spacing, and particles inside
+and outside their cells, with directions, weights and seeds at the edges of
+what the tiles accept.  Results are exact, so nothing is tolerated."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+f32 = np.float32
+
+
+def _particles(mcg, rng, m, dx, n):
+    p = np.zeros(n, mcg.PARTICLE_DTYPE)
+    p["seed"] = rng.integers(0, 2 ** 63, n, dtype=np.uint64)
+    p["seed"][::17] |= np.uint64(1) << np.uint64(63)
+    p["index"] = rng.integers(0, m, n)
+    p["x"] = ((p["index"] + rng.random(n)) * dx).astype(f32)
+    p["x"][::5] = (p["index"][::5] * dx).astype(f32)            # on the left face
+    p["x"][1::11] = ((p["index"][1::11] + 1) * dx).astype(f32)  # on the right face
+    p["x"][2::13] = ((p["index"][2::13] - 0.5) * dx).astype(f32)  # outside the cell
+    p["mu"] = (2 * rng.random(n) - 1).astype(f32)
+    for k, v in enumerate((1.0, -1.0, 0.0, -0.0, 1e-4, -1e-4, 1.1e-4, 1e-3, -0.03, 0.06)):
+        p["mu"][k::29] = v
+    p["wmc"] = 1.0
+    for k, v in enumerate((1e-12, 2e-12, 0.9e-12, 1e-30, 0.3, 1e20, 0.0)):
+        p["wmc"][k::23] = v
+    p["index"][3::31] = -1
+    p["index"][4::37] = m
+    return p
+
+
+@pytest.mark.parametrize("mode", ["strict", "fast"])
+@pytest.mark.parametrize("thin", [False, True])
+@pytest.mark.parametrize("m,layers", [(1, 1), (2, 2), (15, 1), (16, 3), (17, 1), (31, 1), (32, 1),
+                                      (33, 7), (64, 1), (700, 9)])
+def test_tiles_match_event_mode(mcg, mode, thin, m, layers):
+    rng = np.random.default_rng(m * 100 + layers)
+    st, lm, dx, _, _ = mcg.layer_decomposition(0.0, 1.0, m, layers)
+    # optical widths: thin below 2e-4 in sigma_a and 4e-4 in sigma_s; thick from
+    # far below to far above the tiles' ranges, some cells empty or scattering only
+    if thin:
+        sa, ss = 1.9e-4 * m * rng.random(m), 2e-4 * m * rng.random(m)
+    else:
+        sa, ss = m * 10.0 ** rng.uniform(-5, 0.5, m), m * 10.0 ** rng.uniform(-5, 0, m)
+    sa[::7], ss[3::8] = 0.0, 5e-5
+    sigs = (sa + ss).astype(f32)
+    rates = np.where(sigs > 0, sa / np.where(sigs > 0, sigs, 1), 0).astype(f32)
+    with mcg.Context(mode=mode) as ctx:
+        for min_w, scale, n, launch in ((1e-12, 40, 2500, {}), (0.3, 35, 33, {}), (0.0, 20, 1, {}),
+                                        (-np.inf, 35, 400, dict(block=1024, refill_steps=3)),
+                                        (1e-12, 44, 999, dict(block=64, blocks_per_sm=1))):
+            ctx.set_layers(st, lm, dx, sigs, rates, min_w)
+            ctx.set_tally_scale(scale)
+            ctx.set_launch(**launch)
+            p = _particles(mcg, rng, m, 1.0 / m, n)
+            out = []
+            for algorithm in ("history", "event"):
+                ctx.set_algorithm(algorithm, 1)
+                ctx.tally_reset()
+                q = p.copy()
+                r = ctx.simulate(q)
+                out.append((q, r, ctx.tally_q(), ctx.counters()))
+            (pa, ra, qa, ca), (pb, rb, qb, cb) = out
+            assert pa.tobytes() == pb.tobytes()
+            for key in ("results", "steps", "scatters"):
+                assert np.array_equal(ra[key], rb[key]), key
+            assert np.array_equal(qa, qb)
+            assert ca == cb
