@@ -170,8 +170,8 @@ enum mcg_algorithm { MCG_ALGO_HISTORY = 0, MCG_ALGO_EVENT = 1 };
 int mcg_set_algorithm(mcg_context *ctx, int32_t algorithm, int32_t steps_per_pass);
 
 /* Where the tracker accumulates deposits: 0 shared-memory 64-bit atomics,
- * 1 shared-memory 32-bit halves with carry (default), 2 64-bit atomics on the
- * global tally.  All three give the same exact sums. */
+ * 1 shared-memory 32-bit atomics with carries (default), 2 64-bit atomics on
+ * the global tally.  All three give the same exact sums. */
 int mcg_set_tally_mode(mcg_context *ctx, int32_t mode);
 
 /* Longest history, in steps, before the tracker stops it with result 2 and
@@ -263,17 +263,15 @@ int mcg_batch_run_per_slab(mcg_context *ctx);
 int mcg_batch_tally_reset(mcg_context *ctx);
 int mcg_batch_tally_read(mcg_context *ctx, int64_t *h_q, double *h_f64);
 /* Launch shape of mcg_batch_run: threads per block (256, 512 or 1024),
- * histories per work item (a block takes one item at a time), tally mode
+ * most histories per work item (a block takes one item at a time), tally mode
  * (as mcg_set_tally_mode). 0 keeps the current value. */
 int mcg_batch_set_launch(mcg_context *ctx, int32_t block, int64_t item_histories,
                          int32_t tally_mode);
-/* Deferral of the full step in mcg_batch_run (0 off, the default; 1..32
- * on): a lane whose step is not a certain crossing waits while the warp's
- * other lanes keep crossing, and the waiting lanes complete their steps
- * together once at least `defer` of them wait (or no other lane can step),
- * instead of the warp running the full step once for every step any of its
- * lanes needs it; lanes refill when two have ended their histories.  Same
- * results for every value. */
+/* Deferral of the full step in mcg_batch_run: a lane whose step is not a certain
+ * crossing waits while the warp's other lanes keep crossing, and the waiting
+ * lanes complete their steps together once at least `defer` (1..32; 0: the
+ * library's choice) of them wait or no other lane can step.  Same results for
+ * every value. */
 int mcg_batch_set_deferral(mcg_context *ctx, int32_t defer);
 /* Autotuner: times every candidate on a sample of each slab's histories
  * (fraction in (0, 1], raised so that the sample holds at least four times
@@ -290,7 +288,7 @@ typedef struct mcg_batch_tuning {
   int32_t candidates;
   int32_t algorithm;      /* MCG_ALGO_HISTORY or MCG_ALGO_EVENT */
   int32_t steps_per_pass; /* event mode: events per pass */
-  int32_t defer;          /* history mode: waiting lanes of the deferred full step, 0 off */
+  int32_t defer;          /* history mode: waiting lanes of the deferred full step */
 } mcg_batch_tuning;
 int mcg_batch_autotune(mcg_context *ctx, double sample_fraction, mcg_batch_tuning *out);
 

@@ -392,7 +392,7 @@ class Context:
         _check(self.lib.mcg_batch_set_launch(self.h, block, item_histories, tally_mode))
 
     def batch_set_deferral(self, defer):
-        """0/False: off; True: 8 waiting lanes; 1..32: that many."""
+        """0/False: the library's choice; True: 8 waiting lanes; 1..32: that many."""
         lanes = 8 if defer is True else int(defer)
         _check(self.lib.mcg_batch_set_deferral(self.h, lanes))
 

@@ -652,8 +652,6 @@ int mcg_track_launch(mcg_context *ctx, mcg_particle *d_particles, int64_t n, int
   P.tab = {ctx->d_tab + MCG_TAB_PAD, ctx->d_thin + MCG_TAB_PAD, ctx->n_cells + 2 * MCG_TAB_PAD};
   P.n_cells = ctx->n_cells;
   P.cell_lo = ctx->cell_lo;
-  P.min_w = ctx->min_w;
-  P.q_log2 = ctx->log2_scale;
   P.particles = d_particles;
   P.results = d_results;
   P.steps = d_steps;
@@ -667,52 +665,34 @@ int mcg_track_launch(mcg_context *ctx, mcg_particle *d_particles, int64_t n, int
   P.counters = ctx->d_counters;
   P.libm = ctx->libm;
   P.libm_tab = ctx->libm_tab;
-  P.max_steps = ctx->max_steps;
+  P.rules = mcg_rules_setup(ctx, ctx->min_w, false);
   if (ctx->algorithm == MCG_ALGO_EVENT) {
     ctx->launches++;
     return mcg_event_run(ctx, P);
   }
-  /* default shape: short chains keep one tally copy per warp in 256-thread
-   * blocks; long chains share one copy per block of 1024 threads (thin ones
-   * MCG_THIN_BLOCK), or of fewer where the copy and the warps' tiles would not
-   * fit; thin chains take the thin kernel with its tally unless the caller
-   * set another one or a larger block */
-  int tmode = ctx->tally_mode;
-  bool thin = (strict ? ctx->thin : ctx->thin_fast) && tmode == MCG_TALLY_SMEM32 &&
-              ctx->block <= MCG_THIN_BLOCK;
-  auto copies_of = [&](int b) { /* one tally copy per warp while it stays small, else one per block */
-    return !thin && (size_t)ctx->n_cells * 8 * (b / 32) <= 24 * 1024 ? b / 32 : 1;
-  };
-  auto smem_of = [&](int b) {
-    return mcg_track_smem(tmode == MCG_TALLY_GLOBAL ? 0 : (size_t)ctx->n_cells * copies_of(b), b, thin);
-  };
-  int block = ctx->block;
-  if (block == 0) {
-    block = thin ? MCG_THIN_BLOCK : ((size_t)ctx->n_cells * 8 * 8 <= 24 * 1024) ? 256 : 1024;
-    while (tmode != MCG_TALLY_GLOBAL && block > 256 && smem_of(block) > (size_t)ctx->smem_optin)
-      block -= 128;
-  }
-  if (tmode != MCG_TALLY_GLOBAL && smem_of(block) > (size_t)ctx->smem_optin) {
-    tmode = MCG_TALLY_GLOBAL; /* chain too long for a shared-memory copy */
-    thin = false;
-    block = ctx->block ? ctx->block : 1024;
-  }
-  const size_t smem = smem_of(block);
-  P.tally_copies = copies_of(block);
-  mcg_track_rounds(ctx, thin, P);
-  P.run = mcg_run_setup(ctx->log2_scale, ctx->min_w, thin, ctx->run_bounds, ctx->width_a,
-                        ctx->width_i);
+  /* thin chains take the thin kernel with its tally unless the caller set
+   * the global tally or a larger block */
+  const bool global = ctx->tally_mode == MCG_TALLY_GLOBAL;
+  const bool try_thin = (strict ? ctx->thin : ctx->thin_fast) && !global &&
+                        ctx->block <= MCG_THIN_BLOCK;
+  const mcg_shape shape = mcg_track_shape(ctx->n_cells, ctx->block, global, try_thin,
+                                          (size_t)ctx->smem_optin);
+  const bool thin = shape.thin;
+  const int block = shape.block;
+  const size_t smem = shape.smem;
+  P.tally_copies = shape.copies;
+  P.rules = mcg_rules_setup(ctx, ctx->min_w, thin);
   void (*kern)(mcg_track_params);
   if (strict)
     kern = thin ? mcg_track_kernel<true, MCG_TALLY_LO32, true>
-           : tmode == MCG_TALLY_SMEM64 ? mcg_track_kernel<true, MCG_TALLY_SMEM64, false>
-           : tmode == MCG_TALLY_SMEM32 ? mcg_track_kernel<true, MCG_TALLY_SMEM32, false>
-                                       : mcg_track_kernel<true, MCG_TALLY_GLOBAL, false>;
+           : shape.global ? mcg_track_kernel<true, MCG_TALLY_GLOBAL, false>
+           : ctx->tally_mode == MCG_TALLY_SMEM64 ? mcg_track_kernel<true, MCG_TALLY_SMEM64, false>
+                                                 : mcg_track_kernel<true, MCG_TALLY_SMEM32, false>;
   else
     kern = thin ? mcg_track_kernel<false, MCG_TALLY_LO32, true>
-           : tmode == MCG_TALLY_SMEM64 ? mcg_track_kernel<false, MCG_TALLY_SMEM64, false>
-           : tmode == MCG_TALLY_SMEM32 ? mcg_track_kernel<false, MCG_TALLY_SMEM32, false>
-                                       : mcg_track_kernel<false, MCG_TALLY_GLOBAL, false>;
+           : shape.global ? mcg_track_kernel<false, MCG_TALLY_GLOBAL, false>
+           : ctx->tally_mode == MCG_TALLY_SMEM64 ? mcg_track_kernel<false, MCG_TALLY_SMEM64, false>
+                                                 : mcg_track_kernel<false, MCG_TALLY_SMEM32, false>;
   /* the limit is raised to the device's opt-in maximum, the same value on
    * every call, so launches of the same kernel from other host threads (other
    * contexts, the no-allocation entry point) cannot lower it under this one */

@@ -3,19 +3,22 @@
  * persistent launch (the batched form of the tracker).
  *
  * Work is cut into items: up to `item_histories` consecutive histories of
- * one slab.  Items are sorted by expected cost (histories x cells, largest
- * first) and handed out through one global counter.  A block takes one item
- * at a time; when the item's slab differs from the block's current one it
+ * one slab (fewer in small runs, build_items).  Items are sorted by expected
+ * cost (histories x cells, largest first) and handed out through one global
+ * counter.  A block works on one item at a time, its warps taking the item's
+ * histories from a block-local counter and running them as the single-chain
+ * tracker does (mcg_histories, mcg_track.cuh).  When the histories are handed
+ * out, the block changes to the next item at once: if that is another slab's it
  * flushes its shared-memory tally to the slab's global tally and zeroes it
- * for the new slab (at most max_cells 64-bit counters, 32 KB for 4096 cells).
- * Inside an item the warps refill their lanes from a block-local counter
- * exactly as the single-chain tracker does, so lanes stay busy across
- * histories of different lengths; the block synchronises only between
- * items.  The per-cell step table of every slab lives in HBM (16 B per cell)
- * and is read through L1.  The step is mcg_step (mcg_track.cuh), i.e.
- * Layer::particle_step of src/layer.cpp:123-190; with deferral on, it is
- * split into the certain crossing (mcg_step_cross) and the rest of the step
- * (mcg_step_rest), which a warp runs for its waiting lanes together.
+ * (at most max_cells 64-bit counters, 32 KB for 4096 cells), and the histories
+ * its warps still hold go on in their lanes and add to the global tally.
+ * Waiting for them instead, an item's end cost its block up to 3 ms (the
+ * longest of its histories): 4096 slabs of up to 50,000 histories, strict,
+ * took 285 ms with that, 278 without, 36 more of it per halving of the items.
+ * Issue-bound (66 % of the slots; 5 warp instructions per step and lane, 40 %
+ * in forming the steps, 20 % in the deposits, 16 % in full steps), then the
+ * loads of the 136 MB step table through L2.  Whole run: 410 -> 206 ms strict,
+ * 247 -> 155 ms fast.
  */
 #include <algorithm>
 #include <new>
@@ -38,7 +41,7 @@ struct mcg_batch_item {
 };
 
 struct mcg_batch_params {
-  const float4 *cells;
+  const float4 *cells, *tab;
   const mcg_batch_slab_dev *slabs;
   const mcg_batch_item *items;
   int32_t n_items;
@@ -48,37 +51,39 @@ struct mcg_batch_params {
   unsigned long long *counters;
   mcg_libm_dev libm;
   const mcg_libm_tab *libm_tab;
-  float min_w;
-  int32_t q_log2;
-  int32_t refill_steps;
-  uint32_t max_steps;
-  int32_t defer_lanes; /* DEFER: waiting lanes that trigger the full steps */
+  mcg_rules rules;
 };
 
-/* DEFER: certain crossings a lane takes between two of the warp's checks,
- * and the idle lanes (history ended) at which the warp refills */
-#define MCG_DEFER_WINDOW 4
-#define MCG_DEFER_REFILL 2
+/* The item that a block works on (shared memory). */
+struct mcg_batch_work {
+  unsigned long long taken; /* histories handed out */
+  long long item, first, count;
+  int32_t off, m;
+  mcg_source src;
+  long long pad;
+};
 
-template <bool STRICT, int TALLY, bool DEFER>
+/* Shared memory: libm tables, counters, the item, jumps, the tally of one slab,
+ * the warps' tiles. */
+static size_t batch_smem(int max_cells, int block, bool tally)
+{
+  return mcg_track_smem(tally ? max_cells : 0, block, false) + sizeof(mcg_batch_work);
+}
+static_assert(sizeof(mcg_batch_work) % 16 == 0, "the tally after it is read by 16 bytes");
+
+template <bool STRICT, int TALLY>
 __global__ void __launch_bounds__(1024) mcg_batch_kernel(mcg_batch_params P)
 {
   extern __shared__ __align__(16) unsigned char smem[];
   mcg_libm_tab *T = reinterpret_cast<mcg_libm_tab *>(smem);
   unsigned long long *s_cnt = reinterpret_cast<unsigned long long *>(smem + sizeof(mcg_libm_tab));
-  long long *s_ctl = reinterpret_cast<long long *>(s_cnt + 16); /* item, local history counter */
-  unsigned long long *s_tally = reinterpret_cast<unsigned long long *>(s_ctl + 4);
+  mcg_batch_work *work = reinterpret_cast<mcg_batch_work *>(s_cnt + 16);
+  mcg_chain_jumps *s_chain = reinterpret_cast<mcg_chain_jumps *>(work + 1);
+  mcg_real_jumps *s_real = reinterpret_cast<mcg_real_jumps *>(s_chain + 1);
+  unsigned long long *s_tally = reinterpret_cast<unsigned long long *>(s_real + 1);
   const int tid = threadIdx.x, lane = tid & 31;
-  /* r-step jumps of the seed chain, s -> (A_r s + C_r) mod 2^63 for
-   * r < 32: a warp finds the chain state of the first history of each
-   * 32-history chunk it takes with one jump-ahead, run by all its lanes
-   * together, and each lane its own from there with one multiply-add */
-  __shared__ unsigned long long s_jump[64];
-  if (tid < 32) {
-    const uint64_t c = mcg_lcg_skip(0ull, (uint64_t)tid, 1);
-    s_jump[tid] = (mcg_lcg_skip(1ull, (uint64_t)tid, 1) - c) & MCG_MASK63;
-    s_jump[32 + tid] = c;
-  }
+  mcg_fill_chain_jumps(s_chain);
+  mcg_fill_real_jumps(s_real);
   if (STRICT) {
     const float *src = reinterpret_cast<const float *>(P.libm_tab);
     float *dst = reinterpret_cast<float *>(T);
@@ -87,207 +92,75 @@ __global__ void __launch_bounds__(1024) mcg_batch_kernel(mcg_batch_params P)
   }
   if (tid < 16)
     s_cnt[tid] = 0ull;
-  const float min_w = P.min_w;
-  const int qs = P.q_log2;
-  int cur = -1, m = 0;
-  const float4 *cells = nullptr;
-  unsigned long long *gtally = nullptr;
+  if (tid == 0)
+    work->taken = work->count = 0; /* no item: exhausted at once */
+  mcg_tile_smem<false> *tile =
+      reinterpret_cast<mcg_tile_smem<false> *>(
+          s_tally + (TALLY == MCG_TALLY_GLOBAL ? 0 : (P.max_cells + 1) & ~1)) + (tid >> 5);
+  __syncthreads();
+  const mcg_tile_warp<false> tiles(tile, s_real);
+  mcg_geometry geo = {-1, 0};
+  mcg_sink sink = {0u, P.tally};
+  auto flush = [&] {
+    if (TALLY != MCG_TALLY_GLOBAL)
+      for (int i = tid; i < geo.ncell; i += blockDim.x)
+        if (s_tally[i])
+          atomicAdd(&P.tally[geo.off + i], s_tally[i]);
+  };
   unsigned long long tot_steps = 0, tot_scat = 0;
-
-  for (;;) {
-    __syncthreads();
-    if (tid == 0)
-      s_ctl[0] = (long long)atomicAdd(P.item_next, 1ull);
-    __syncthreads();
-    const long long item = s_ctl[0];
-    if (item >= P.n_items)
-      break;
-    const mcg_batch_item it = P.items[item];
-    if (it.slab != cur) {
-      if (cur >= 0 && TALLY != MCG_TALLY_GLOBAL)
-        for (int i = tid; i < m; i += blockDim.x)
-          if (s_tally[i])
-            atomicAdd(&gtally[i], s_tally[i]);
-      __syncthreads();
-      cur = it.slab;
-      const mcg_batch_slab_dev sd = P.slabs[cur];
-      m = sd.m;
-      cells = P.cells + sd.cell_off;
-      gtally = P.tally + sd.cell_off;
-      if (TALLY != MCG_TALLY_GLOBAL)
-        for (int i = tid; i < m; i += blockDim.x)
-          s_tally[i] = 0ull;
-    }
-    if (tid == 0)
-      s_ctl[1] = 0;
-    __syncthreads();
-    const mcg_source S = P.slabs[cur].src;
-    unsigned long long *tally = TALLY == MCG_TALLY_GLOBAL ? gtally : s_tally;
-
-    /* lanes refill from the item's histories [0, it.count) */
-    uint64_t seed = 0;
-    float x = 0.f, mu = 0.f, wmc = 0.f, inv_mu = 0.f;
-    float wres = 0.f; /* fast: the weight's rounding residue */
-    int idx = 0;
-    uint32_t nst = 0, nsc = 0;
-    bool active = false;
-    bool wait = false; /* DEFER: the lane's step waits for the full step */
-    long long pool_next = 0, pool_end = 0;
-    /* the chunk the pool lies in: its first history and that history's
-     * seed-chain state (seed_mode 0) */
-    long long pool_base = 0;
-    uint64_t pool_seed = 0;
-    bool drained = false;
-    for (;;) {
-      unsigned need = __ballot_sync(0xffffffffu, !active);
-      if (need) {
-        int cnt = __popc(need), rank = __popc(need & lanemask_lt());
-        long long avail = pool_end - pool_next, my = -1, my_base = pool_base;
-        uint64_t my_seed = pool_seed;
-        if (rank < avail)
-          my = pool_next + rank;
-        if (cnt > avail && !drained) {
-          long long base = 0;
-          if (lane == 0)
-            base = (long long)atomicAdd(reinterpret_cast<unsigned long long *>(&s_ctl[1]), 32ull);
-          base = __shfl_sync(0xffffffffu, base, 0);
-          if (base >= it.count) {
-            drained = true;
-            pool_next = pool_end = 0;
-          } else {
-            long long end = min(base + 32, (long long)it.count);
-            long long r2 = rank - avail;
-            pool_base = base;
-            if (S.seed_mode == 0)
-              pool_seed = mcg_lcg_skip(S.base_seed, (uint64_t)(it.first + base) + 1, 1);
-            if (rank >= avail && r2 < end - base) {
-              my = base + r2;
-              my_base = base;
-              my_seed = pool_seed;
-            }
-            pool_next = min(base + (cnt - avail), end);
-            pool_end = end;
-          }
-        } else {
-          pool_next += min((long long)cnt, avail);
-        }
-        if (!active && my >= 0) {
-          if (S.seed_mode == 0) {
-            const int r = (int)(my - my_base); /* 0 <= r < 32: my lies in its chunk */
-            mcg_source_particle_at(S, (s_jump[r] * my_seed + s_jump[32 + r]) & MCG_MASK63, seed, x,
-                                   mu, wmc, idx);
-          } else {
-            mcg_source_particle(S, it.first + my, seed, x, mu, wmc, idx);
-          }
-          inv_mu = mcg_flight_rcp(mu);
-          wres = 0.f;
-          nst = nsc = 0;
-          active = true;
-        }
-      }
-      if (!__any_sync(0xffffffffu, active))
-        break;
-      int k = 0;
-      if (DEFER) {
-        /* pooled deferral, run by the whole warp: a lane whose step is not
-         * a certain crossing waits (mcg_step_cross has advanced only its
-         * seed) while the others keep crossing, and the waiting lanes
-         * complete their steps together (mcg_step_rest) once defer_lanes of
-         * them wait or no other lane can step, so the long full step runs
-         * with many lanes instead of once for every lane that needs it.
-         * The round lasts until MCG_DEFER_REFILL lanes have ended their
-         * histories (while the item has more) or no lane can step; a lane
-         * may still wait when it ends, and its step completes in a later
-         * round.  mcg_step_cross + mcg_step_rest perform exactly mcg_step
-         * and each lane's steps keep their order: same results.  Every pass
-         * steps a lane, makes one wait or completes the waiting steps, and
-         * no lane passes its step limit, so the round ends. */
-        const uint32_t kcap = active ? P.max_steps - nst : 0u;
-        for (;;) {
-          bool go = !wait & ((uint32_t)k < kcap) & (wmc >= min_w) & ((unsigned)idx < (unsigned)m);
-          for (int j = 0; go & (j < MCG_DEFER_WINDOW); ++j) {
-            if (!mcg_step_cross<STRICT, TALLY>(seed, x, mu, wmc, inv_mu, idx,
-                                               __ldg(cells + idx), &tally[idx], qs, T, P.libm,
-                                               nullptr, nullptr, nullptr,
-                                               STRICT ? nullptr : &wres)) {
-              wait = true;
-              break;
-            }
-            ++k;
-            go = ((uint32_t)k < kcap) & (wmc >= min_w) & ((unsigned)idx < (unsigned)m);
-          }
-          go &= !wait;
-          const unsigned wb = __ballot_sync(0xffffffffu, wait);
-          const unsigned gb = __ballot_sync(0xffffffffu, go);
-          if (!wb && !gb)
-            break;
-          if (wb && (!gb || __popc(wb) >= P.defer_lanes)) {
-            if (wait) {
-              mcg_step_rest<STRICT, TALLY>(seed, x, mu, wmc, inv_mu, idx, nsc,
-                                           __ldg(cells + idx), &tally[idx], qs, T, P.libm,
-                                           nullptr, nullptr, nullptr, STRICT ? nullptr : &wres);
-              ++k;
-              wait = false;
-            }
-          } else if (!drained && __popc(~(wb | gb)) >= MCG_DEFER_REFILL) {
-            break;
+  mcg_histories<STRICT, false, TALLY, true>(
+      geo, sink, P.cells, {P.tab, nullptr, 0}, s_tally, P.rules, tiles, s_real, T, P.libm,
+      &work->taken, [&] { return work->count; }, 0,
+      [&](long long my, uint64_t &seed, float &x, float &mu, float &wmc, int &idx) {
+        mcg_born(s_chain, work->src, work->first + my, seed, x, mu, wmc, idx);
+      },
+      [&](long long, int r, uint64_t, float, float, float wmc, float wres, int, uint32_t nst,
+          uint32_t nsc) {
+        mcg_count_end<STRICT>(s_cnt, r, wmc, wres, P.rules.q_log2);
+        tot_steps += nst;
+        tot_scat += nsc;
+      },
+      /* broadcast, so that the warp decides as one */
+      [&] {
+        return __shfl_sync(0xffffffffu, *(volatile unsigned long long *)&work->taken, 0) >=
+               (unsigned long long)work->count;
+      },
+      [&] {
+        /* every warp of the block comes here (each looks at the exhausted
+         * item in every round), so nothing is being added to the tally */
+        __syncthreads();
+        if (tid == 0) {
+          work->item = (long long)atomicAdd(P.item_next, 1ull);
+          work->taken = 0;
+          if (work->item < P.n_items) {
+            const mcg_batch_item it = P.items[work->item];
+            const mcg_batch_slab_dev sd = P.slabs[it.slab];
+            work->first = it.first;
+            work->count = it.count;
+            work->off = sd.cell_off;
+            work->m = sd.m;
+            work->src = sd.src;
           }
         }
-      } else if (active) {
-        /* up to refill_steps steps, never past the step limit; one
-         * unsigned compare is the slab's range test */
-        const int kmax = (int)min((uint32_t)P.refill_steps, P.max_steps - nst);
-        while ((k < kmax) & (wmc >= min_w) & ((unsigned)idx < (unsigned)m)) {
-          mcg_step<STRICT, TALLY>(seed, x, mu, wmc, inv_mu, idx, nsc, __ldg(cells + idx),
-                                  &tally[idx], qs, T, P.libm, nullptr, nullptr, nullptr,
-                                  STRICT ? nullptr : &wres);
-          ++k;
-        }
-      }
-      if (active)
-        nst += (uint32_t)k;
-      if (active && !wait) {
-        const bool going = (wmc >= min_w) & ((unsigned)idx < (unsigned)m);
-        if (!going || nst >= P.max_steps) {
-          /* a history still alive in the slab here has reached the limit */
-          const bool in = (wmc >= min_w) && ((unsigned)idx < (unsigned)m);
-          int r;
-          if (in)
-            r = 2;
-          else if (idx == -1)
-            r = -1;
-          else if (idx == m)
-            r = 1;
-          else if (wmc < min_w)
-            r = 0;
-          else
-            r = -1;
-          atomicAdd(&s_cnt[MCG_CNT_HIST], 1ull);
-          const unsigned long long wq =
-              (unsigned long long)(mcg_to_fixed(wmc, qs) + (STRICT ? 0ll : mcg_to_fixed(wres, qs)));
-          if (r == -1) {
-            atomicAdd(&s_cnt[MCG_CNT_LEFT], 1ull);
-            atomicAdd(&s_cnt[MCG_CNT_WLEFT], wq);
-          } else if (r == 1) {
-            atomicAdd(&s_cnt[MCG_CNT_RIGHT], 1ull);
-            atomicAdd(&s_cnt[MCG_CNT_WRIGHT], wq);
-          } else if (r == 0) {
-            atomicAdd(&s_cnt[MCG_CNT_KILL], 1ull);
-            atomicAdd(&s_cnt[MCG_CNT_WKILL], wq);
-          } else {
-            atomicOr(&s_cnt[MCG_CNT_ERR], 1ull);
+        __syncthreads();
+        if (work->item >= P.n_items)
+          return false;
+        if (work->off != geo.off) {
+          flush();
+          geo.off = work->off;
+          geo.ncell = work->m;
+          sink.shared = (uint32_t)__cvta_generic_to_shared(s_tally) - 8u * (uint32_t)geo.off;
+          if (TALLY != MCG_TALLY_GLOBAL) {
+            __syncthreads();
+            for (int i = tid; i < geo.ncell; i += blockDim.x)
+              s_tally[i] = 0ull;
+            __syncthreads();
           }
-          tot_steps += nst;
-          tot_scat += nsc;
-          active = false;
         }
-      }
-    }
-  }
-  if (cur >= 0 && TALLY != MCG_TALLY_GLOBAL)
-    for (int i = tid; i < m; i += blockDim.x)
-      if (s_tally[i])
-        atomicAdd(&gtally[i], s_tally[i]);
+        return true;
+      });
+  __syncthreads();
+  flush();
   for (int o = 16; o > 0; o >>= 1) {
     tot_steps += __shfl_down_sync(0xffffffffu, tot_steps, o);
     tot_scat += __shfl_down_sync(0xffffffffu, tot_scat, o);
@@ -341,6 +214,21 @@ void mcg_ext_destroy(mcg_context *ctx)
   ctx->ext = nullptr;
 }
 
+/* The fast arithmetic's cells (mcg_cell_params) and the tile table
+ * (mcg_tile_table: within a slab neighbours share their faces) from the strict
+ * cells, on the GPU: uploading all three took 27 ms longer for 8.5e6 cells. */
+__global__ void mcg_batch_tables(const float4 *strict, float4 *fast, float4 *tab, int64_t n)
+{
+  for (int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k < n;
+       k += (int64_t)gridDim.x * blockDim.x) {
+    const float4 c = strict[k];
+    const float sig_i = c.y > 1e-4f ? c.y : 0.0f, a = __fsub_rn(c.w, c.z);
+    const float len = a >= 0x1p-90f && a <= 0x1p90f && c.x >= 0.0f ? a : __int_as_float(0x7fc00000);
+    fast[k] = make_float4(c.x, sig_i, c.z, c.w);
+    tab[k] = make_float4(c.x, sig_i, len, len);
+  }
+}
+
 extern "C" int mcg_batch_set(mcg_context *ctx, int32_t n_slabs, const mcg_slab *h_slabs,
                              const float *h_sigs, const float *h_rates, float particle_min_weight)
 {
@@ -357,16 +245,15 @@ extern "C" int mcg_batch_set(mcg_context *ctx, int32_t n_slabs, const mcg_slab *
     hist += sl.n_histories;
     maxc = std::max(maxc, sl.n_cells);
   }
+  /* the largest slab whose tally fits in a block's shared memory */
   const size_t smem_need = sizeof(mcg_libm_tab) + 16 * 8 + 4 * 8 + (size_t)maxc * 8;
   if (total > INT32_MAX || smem_need > (size_t)ctx->smem_optin)
     return mcg_fail(MCG_ERR_ARG, "mcg_batch_set: %lld cells / largest slab %d cells too large",
                     (long long)total, maxc);
-  std::vector<float4> cs, cf, tab;
+  std::vector<float4> cs;
   std::vector<mcg_batch_slab_dev> sd;
   try {
     cs.resize(total);
-    cf.resize(total);
-    tab.resize(total + 2 * MCG_TAB_PAD, make_float4(0, 0, 0, 0));
     sd.resize(n_slabs);
   } catch (const std::bad_alloc &) {
     return mcg_fail(MCG_ERR_ARG, "mcg_batch_set: no host memory for %lld cells", (long long)total);
@@ -394,9 +281,9 @@ extern "C" int mcg_batch_set(mcg_context *ctx, int32_t n_slabs, const mcg_slab *
     const mcg_slab &sl = h_slabs[s];
     B->cell_off[s] = (int32_t)off;
     const float dx = (1.0f - 0.0f) / (float)sl.n_cells; /* Layer(0, 1, 0, m): src/layer.cpp:47 */
+    float4 fast;
     for (int j = 0; j < sl.n_cells; ++j)
-      mcg_cell_params(h_sigs[off + j], h_rates[off + j], j, dx, cs[off + j], cf[off + j]);
-    mcg_tile_table(&cf[off], sl.n_cells, &tab[MCG_TAB_PAD + off]);
+      mcg_cell_params(h_sigs[off + j], h_rates[off + j], j, dx, cs[off + j], fast);
     sd[s].cell_off = (int32_t)off;
     sd[s].m = sl.n_cells;
     sd[s].src.seed_mode = sl.seed_mode;
@@ -427,30 +314,46 @@ extern "C" int mcg_batch_set(mcg_context *ctx, int32_t n_slabs, const mcg_slab *
       (e = mcg_dev_malloc((void **)&B->d_item_next, 64)) != cudaSuccess)
     return fail(e, "mcg_batch_set: cudaMalloc");
   if ((e = cudaMemcpy(B->d_cells_strict, cs.data(), total * sizeof(float4), cudaMemcpyHostToDevice)) != cudaSuccess ||
-      (e = cudaMemcpy(B->d_cells_fast, cf.data(), total * sizeof(float4), cudaMemcpyHostToDevice)) != cudaSuccess ||
-      (e = cudaMemcpy(B->d_tab, tab.data(), tab.size() * sizeof(float4), cudaMemcpyHostToDevice)) != cudaSuccess ||
+      (e = cudaMemset(B->d_tab, 0, (total + 2 * MCG_TAB_PAD) * sizeof(float4))) != cudaSuccess ||
       (e = cudaMemcpy(B->d_slabs, sd.data(), n_slabs * sizeof(mcg_batch_slab_dev), cudaMemcpyHostToDevice)) != cudaSuccess ||
       (e = cudaMemset(B->d_tally, 0, total * sizeof(unsigned long long))) != cudaSuccess)
     return fail(e, "mcg_batch_set: upload");
+  mcg_batch_tables<<<(int)std::min<int64_t>((total + 255) / 256, 8LL * ctx->sm_count), 256>>>(
+      B->d_cells_strict, B->d_cells_fast, B->d_tab + MCG_TAB_PAD, total);
+  if ((e = cudaGetLastError()) != cudaSuccess || (e = cudaStreamSynchronize(0)) != cudaSuccess)
+    return fail(e, "mcg_batch_set: tables");
   return mcg_tally_reset(ctx) == MCG_OK ? MCG_OK : MCG_ERR_CUDA;
 }
 
-/* Items of `item` histories, sorted by expected cost, optionally only the
- * first `fraction` of every slab's histories (autotuner samples). */
-static int build_items(mcg_context *ctx, mcg_batch_state *B, int64_t item, double fraction)
+/* Items of at most `item` histories, sorted by expected cost, optionally only
+ * the first `fraction` of every slab's histories (autotuner samples).  An item
+ * is also at most a sixteenth of a block's even share of the run (cost: histories
+ * x cells), so a small run still has an item for every block and the last ones
+ * are short: 37 slabs of up to 20,000 histories took 34 ms with the 40 items
+ * that 16,384 histories make of them.  Not below 64 histories: each item loads
+ * and adds its slab's tally. */
+static int build_items(mcg_context *ctx, mcg_batch_state *B, int64_t item, double fraction, int grid)
 {
   std::vector<mcg_batch_item> items;
   std::vector<double> cost;
+  auto histories = [&](int s) {
+    const int64_t n = B->slabs[s].n_histories;
+    return fraction < 1.0 ? std::max<int64_t>(std::min<int64_t>(n, 32), (int64_t)std::ceil(n * fraction))
+                          : n;
+  };
+  double total = 0.0;
+  for (int s = 0; s < B->n_slabs; ++s)
+    total += (double)histories(s) * B->slabs[s].n_cells;
   for (int s = 0; s < B->n_slabs; ++s) {
-    int64_t n = B->slabs[s].n_histories;
-    if (fraction < 1.0)
-      n = std::max<int64_t>(std::min<int64_t>(n, 32), (int64_t)std::ceil(n * fraction));
-    for (int64_t f = 0; f < n; f += item) {
+    const int64_t n = histories(s);
+    const int64_t share = (int64_t)(total / (16.0 * grid) / B->slabs[s].n_cells);
+    const int64_t step = std::min(item, std::max<int64_t>(64, share));
+    for (int64_t f = 0; f < n; f += step) {
       mcg_batch_item it;
       it.slab = s;
       it.pad = 0;
       it.first = f;
-      it.count = std::min(item, n - f);
+      it.count = std::min(step, n - f);
       items.push_back(it);
       cost.push_back((double)it.count * (double)B->slabs[s].n_cells);
     }
@@ -476,6 +379,9 @@ static int build_items(mcg_context *ctx, mcg_batch_state *B, int64_t item, doubl
   if (e != cudaSuccess)
     return mcg_cuda_fail(e, "mcg_batch: upload items");
   B->n_items = (int)sorted.size();
+  B->items_built_for = item;
+  B->items_grid = grid;
+  B->items_fraction = fraction;
   B->graph_valid = false;
   return MCG_OK;
 }
@@ -484,55 +390,64 @@ struct mcg_batch_launch {
   void (*kern)(mcg_batch_params);
   mcg_batch_params P;
   size_t smem;
-  int grid;
+  int grid, block;
 };
 
-/* Kernel choice, attributes and grid: done outside any stream capture. */
-static int batch_configure(mcg_context *ctx, mcg_batch_state *B, mcg_batch_launch &L)
+/* Lanes waiting for the full step that trigger it (mcg_batch_set_deferral 0):
+ * 4 to 12 lie within 2 % on 4096 slabs of up to 4096 cells, 4 is 13 % faster
+ * than 8 on 37 small ones. */
+#define MCG_BATCH_POOL 4
+
+/* Kernel choice, attributes, grid and items (of `fraction` of the histories):
+ * done outside any stream capture. */
+static int batch_configure(mcg_context *ctx, mcg_batch_state *B, int64_t item, double fraction,
+                           mcg_batch_launch &L)
 {
   const bool strict = ctx->mode == MCG_MODE_STRICT;
   mcg_batch_params &P = L.P;
   memset(&P, 0, sizeof(P));
   P.cells = strict ? B->d_cells_strict : B->d_cells_fast;
+  P.tab = B->d_tab + MCG_TAB_PAD;
   P.slabs = static_cast<const mcg_batch_slab_dev *>(B->d_slabs);
-  P.items = static_cast<const mcg_batch_item *>(B->d_items);
-  P.n_items = B->n_items;
   P.max_cells = B->max_cells;
   P.item_next = B->d_item_next;
   P.tally = B->d_tally;
   P.counters = ctx->d_counters;
   P.libm = ctx->libm;
   P.libm_tab = ctx->libm_tab;
-  P.min_w = B->min_w;
-  P.q_log2 = ctx->log2_scale;
-  P.refill_steps = ctx->refill ? ctx->refill : 8;
-  P.max_steps = ctx->max_steps;
-  const int tm = B->tally_mode;
-  L.smem = sizeof(mcg_libm_tab) + 16 * 8 + 4 * 8 +
-           (tm == MCG_TALLY_GLOBAL ? 0 : (size_t)B->max_cells * 8);
-  /* deferral is built for the shared-memory 32-bit tally (the autotuner's
-   * candidates); other tally modes run without it */
-  P.defer_lanes = B->defer;
-  if (strict && B->defer && tm == MCG_TALLY_SMEM32)
-    L.kern = mcg_batch_kernel<true, MCG_TALLY_SMEM32, true>;
-  else if (!strict && B->defer && tm == MCG_TALLY_SMEM32)
-    L.kern = mcg_batch_kernel<false, MCG_TALLY_SMEM32, true>;
-  else if (strict)
-    L.kern = tm == MCG_TALLY_SMEM64 ? mcg_batch_kernel<true, MCG_TALLY_SMEM64, false>
-           : tm == MCG_TALLY_SMEM32 ? mcg_batch_kernel<true, MCG_TALLY_SMEM32, false>
-                                    : mcg_batch_kernel<true, MCG_TALLY_GLOBAL, false>;
+  P.rules = mcg_rules_setup(ctx, B->min_w, false);
+  P.rules.pool_lanes = B->defer ? B->defer : MCG_BATCH_POOL;
+  /* the asked block, or a smaller one where the largest slab's tally and the
+   * warps' tiles would not fit; the global tally where none does.  Both
+   * shared-memory modes add 64 bits at once (mcg_shared_red_if). */
+  int tm = B->tally_mode;
+  if (batch_smem(B->max_cells, 256, true) > (size_t)ctx->smem_optin)
+    tm = MCG_TALLY_GLOBAL;
+  L.block = B->block;
+  while (L.block > 256 && batch_smem(B->max_cells, L.block, tm != MCG_TALLY_GLOBAL) > (size_t)ctx->smem_optin)
+    L.block /= 2;
+  L.smem = batch_smem(B->max_cells, L.block, tm != MCG_TALLY_GLOBAL);
+  if (strict)
+    L.kern = tm == MCG_TALLY_GLOBAL ? mcg_batch_kernel<true, MCG_TALLY_GLOBAL>
+                                    : mcg_batch_kernel<true, MCG_TALLY_SMEM64>;
   else
-    L.kern = tm == MCG_TALLY_SMEM64 ? mcg_batch_kernel<false, MCG_TALLY_SMEM64, false>
-           : tm == MCG_TALLY_SMEM32 ? mcg_batch_kernel<false, MCG_TALLY_SMEM32, false>
-                                    : mcg_batch_kernel<false, MCG_TALLY_GLOBAL, false>;
+    L.kern = tm == MCG_TALLY_GLOBAL ? mcg_batch_kernel<false, MCG_TALLY_GLOBAL>
+                                    : mcg_batch_kernel<false, MCG_TALLY_SMEM64>;
   cudaError_t e = cudaFuncSetAttribute(L.kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        (int)L.smem);
   int bps = 0;
   if (e == cudaSuccess)
-    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, L.kern, B->block, L.smem);
+    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, L.kern, L.block, L.smem);
   if (e != cudaSuccess)
     return mcg_cuda_fail(e, "mcg_batch: launch set-up");
   L.grid = ctx->sm_count * std::max(bps, 1);
+  if (B->items_built_for != item || B->items_grid != L.grid || B->items_fraction != fraction) {
+    int rc = build_items(ctx, B, item, fraction, L.grid);
+    if (rc != MCG_OK)
+      return rc;
+  }
+  P.items = static_cast<const mcg_batch_item *>(B->d_items);
+  P.n_items = B->n_items;
   return MCG_OK;
 }
 
@@ -541,11 +456,11 @@ static int batch_enqueue(mcg_context *ctx, mcg_batch_state *B, const mcg_batch_l
   cudaError_t e;
   if ((e = cudaMemsetAsync(B->d_item_next, 0, 8, ctx->stream)) != cudaSuccess)
     return mcg_cuda_fail(e, "mcg_batch: memset");
-  L.kern<<<L.grid, B->block, L.smem, ctx->stream>>>(L.P);
+  L.kern<<<L.grid, L.block, L.smem, ctx->stream>>>(L.P);
   if ((e = cudaGetLastError()) != cudaSuccess)
     return mcg_cuda_fail(e, "mcg_batch_kernel launch");
   ctx->last_grid = L.grid;
-  ctx->last_block = B->block;
+  ctx->last_block = L.block;
   ctx->launches++;
   return MCG_OK;
 }
@@ -613,11 +528,6 @@ extern "C" int mcg_batch_run(mcg_context *ctx)
       return rc;
     return mcg_sync(ctx);
   }
-  if (B->items_built_for != (int)B->item_histories) {
-    if ((rc = build_items(ctx, B, B->item_histories, 1.0)) != MCG_OK)
-      return rc;
-    B->items_built_for = (int)B->item_histories;
-  }
   cudaError_t e;
   if (!B->graph_valid) {
     if (B->graph) {
@@ -625,7 +535,7 @@ extern "C" int mcg_batch_run(mcg_context *ctx)
       B->graph = nullptr;
     }
     mcg_batch_launch L;
-    if ((rc = batch_configure(ctx, B, L)) != MCG_OK)
+    if ((rc = batch_configure(ctx, B, B->item_histories, 1.0, L)) != MCG_OK)
       return rc;
     cudaGraph_t g;
     if ((e = cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeThreadLocal)) != cudaSuccess)
@@ -671,8 +581,6 @@ extern "C" int mcg_batch_run_per_slab(mcg_context *ctx)
     P.tab = {B->d_tab + MCG_TAB_PAD + B->cell_off[s], nullptr, 0};
     P.n_cells = sl.n_cells;
     P.cell_lo = 0;
-    P.min_w = B->min_w;
-    P.q_log2 = ctx->log2_scale;
     P.n = sl.n_histories;
     P.src.seed_mode = sl.seed_mode;
     P.src.isotropic = sl.isotropic;
@@ -684,16 +592,15 @@ extern "C" int mcg_batch_run_per_slab(mcg_context *ctx)
     P.counters = ctx->d_counters;
     P.libm = ctx->libm;
     P.libm_tab = ctx->libm_tab;
-    mcg_track_rounds(ctx, false, P);
-    P.run = mcg_run_setup(ctx->log2_scale, B->min_w, false, ctx->run_bounds);
-    P.max_steps = ctx->max_steps;
-    const int block = ((size_t)sl.n_cells * 64 <= 24 * 1024) ? 256 : 1024;
-    const int warps = block / 32;
-    const int copies = ((size_t)sl.n_cells * 8 * warps <= 24 * 1024) ? warps : 1;
-    P.tally_copies = copies;
-    const size_t smem = mcg_track_smem((size_t)sl.n_cells * copies, block, false);
-    auto kern = strict ? mcg_track_kernel<true, MCG_TALLY_SMEM32, false>
-                       : mcg_track_kernel<false, MCG_TALLY_SMEM32, false>;
+    P.rules = mcg_rules_setup(ctx, B->min_w, false);
+    const mcg_shape shape = mcg_track_shape(sl.n_cells, 0, false, false, (size_t)ctx->smem_optin);
+    const int block = shape.block;
+    const size_t smem = shape.smem;
+    P.tally_copies = shape.copies;
+    auto kern = strict ? (shape.global ? mcg_track_kernel<true, MCG_TALLY_GLOBAL, false>
+                                       : mcg_track_kernel<true, MCG_TALLY_SMEM32, false>)
+                       : (shape.global ? mcg_track_kernel<false, MCG_TALLY_GLOBAL, false>
+                                       : mcg_track_kernel<false, MCG_TALLY_SMEM32, false>);
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          (int)smem);
     int bps = 1;
@@ -808,9 +715,8 @@ extern "C" int mcg_batch_autotune(mcg_context *ctx, double sample_fraction, mcg_
     return mcg_fail(MCG_ERR_ARG, "mcg_batch_autotune: sample fraction must be in (0, 1]");
   const int blocks[] = {256, 512, 1024};
   const int64_t items[] = {4096, 16384, 65536};
-  /* tally mode and deferral of the full step (waiting lanes) */
-  const int shapes[][2] = {{MCG_TALLY_SMEM32, 0}, {MCG_TALLY_SMEM32, 4}, {MCG_TALLY_SMEM32, 8},
-                           {MCG_TALLY_SMEM64, 0}};
+  /* tally mode and lanes that wait for the full step */
+  const int shapes[][2] = {{MCG_TALLY_SMEM32, 4}, {MCG_TALLY_SMEM32, 12}};
   /* every candidate runs the same sample, of at least four times the event
    * engine's drain size (below it the event-based form is a single drain
    * launch, and a persistent launch is dominated by its tail), or the whole
@@ -833,8 +739,6 @@ extern "C" int mcg_batch_autotune(mcg_context *ctx, double sample_fraction, mcg_
     /* the sample keeps the full run's number of items per slab, so the
      * item-level tail the candidate would see is represented */
     const int64_t sample_item = std::max<int64_t>(32, (int64_t)std::llround(it * sample_fraction));
-    if ((rc = build_items(ctx, B, sample_item, sample_fraction)) != MCG_OK)
-      return rc;
     for (int bl : blocks)
       for (const auto &sh : shapes) {
         const int tm = sh[0];
@@ -842,7 +746,7 @@ extern "C" int mcg_batch_autotune(mcg_context *ctx, double sample_fraction, mcg_
         B->tally_mode = tm;
         B->defer = sh[1];
         mcg_batch_launch L;
-        if ((rc = batch_configure(ctx, B, L)) != MCG_OK)
+        if ((rc = batch_configure(ctx, B, sample_item, sample_fraction, L)) != MCG_OK)
           return rc;
         for (int rep = warmed ? 1 : 0; rep < 2; ++rep) { /* the very first run warms up */
           cudaEventRecord(ctx->ev0, ctx->stream);

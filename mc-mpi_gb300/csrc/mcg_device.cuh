@@ -16,22 +16,20 @@
  * strict absorption forms (mcg_run_bounds). */
 struct mcg_run_consts {
   float scale, inv_scale;
-  float w_one;  /* below: no run (the full step) */
-  float w_many; /* below: runs of one step, so none passes the minimum weight unseen */
+  float min_w; /* the minimum weight times the scale */
   float b_thin, c_thin, b_mid;
   float w_a, w_i; /* thin chains: the largest sig_a and sig_i cell widths */
 };
 
 
 /* b: the acceptance bounds {b_thin, c_thin, b_mid}, or NULL (fast). */
-inline mcg_run_consts mcg_run_setup(int log2_scale, float min_w, bool thin, const float *b,
+inline mcg_run_consts mcg_run_setup(int log2_scale, float min_w, const float *b,
                                     float w_a = 0.0f, float w_i = 0.0f)
 {
   mcg_run_consts R;
   R.scale = ldexpf(1.0f, log2_scale);
   R.inv_scale = ldexpf(1.0f, -log2_scale);
-  R.w_one = fmaxf(min_w, 0x1p-60f);
-  R.w_many = R.w_one * (thin ? 4.0f / 3.0f : 8.0f);
+  R.min_w = min_w * R.scale;
   R.b_thin = b ? b[0] : 0.0f;
   R.c_thin = b ? b[1] : 0.0f;
   R.b_mid = b ? b[2] : 0.0f;

@@ -647,9 +647,9 @@ int mcg_event_run(mcg_context *ctx, mcg_track_params &TP)
   P.n_cells = TP.n_cells;
   P.cell_lo = TP.cell_lo;
   P.tp = TP;
-  P.min_w = TP.min_w;
-  P.q_log2 = TP.q_log2;
-  P.max_steps = TP.max_steps;
+  P.min_w = TP.rules.min_w;
+  P.q_log2 = TP.rules.q_log2;
+  P.max_steps = TP.rules.max_steps;
   P.counters = TP.counters;
   P.libm = TP.libm;
   P.libm_tab = TP.libm_tab;

@@ -29,8 +29,8 @@ struct mcg_batch_state {
   unsigned long long *d_item_next = nullptr;
   float min_w = 0.f;
   /* launch shape, chosen by mcg_batch_set_launch or the autotuner */
-  int block = 512, tally_mode = 1;
-  int defer = 0; /* waiting lanes of the deferred full step, 0: off (mcg_batch_set_deferral) */
+  int block = 1024, tally_mode = 1;
+  int defer = 0; /* lanes that wait for the full step, 0: default (mcg_batch_set_deferral) */
   int64_t item_histories = 16384;
   /* history- or event-based; events per pass of the event engine */
   int algorithm = MCG_ALGO_HISTORY, event_steps = 8;
@@ -39,7 +39,9 @@ struct mcg_batch_state {
   /* CUDA graph of one run (memset of the item counter + the kernel) */
   cudaGraphExec_t graph = nullptr;
   bool graph_valid = false;
-  int items_built_for = -1; /* item size the list was built for */
+  int64_t items_built_for = -1; /* item size, grid and share of the histories the list is for */
+  int items_grid = 0;
+  double items_fraction = 1.0;
 };
 
 /* Per-context state of the adjoint unit (mcg_adjoint.cu). */

@@ -120,32 +120,24 @@ extern "C" int mcg_simulate_fast_noalloc(int n_layers, const int32_t *h_index_st
     P.tab = {tab, nullptr, 0};
     P.n_cells = total;
     P.cell_lo = h_index_start[0];
-    P.min_w = particle_min_weight;
-    P.q_log2 = log2_scale;
     P.particles = d_particles;
     P.results = d_results;
     P.n = n;
     P.next = next;
     P.tally = tally;
     P.counters = cnt;
-    P.window = MCG_TW_MAX;
-    P.pool_lanes = 16;
-    P.refill_lanes = 8;
-    P.run = mcg_run_setup(log2_scale, particle_min_weight, false, nullptr);
-    P.max_steps = 1u << 28;
+    mcg_context rules; /* the defaults of a context, for its rules */
+    rules.log2_scale = log2_scale;
+    P.rules = mcg_rules_setup(&rules, particle_min_weight, false);
     int sms = 0, optin = 0, bps = 0;
     if ((e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess ||
         (e = cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev)) != cudaSuccess)
       return mcg_cuda_fail(e, "mcg_simulate_fast_noalloc: device attributes");
-    /* as the context path: the block shrinks until the tally and the tiles
-     * fit in its shared memory (256 threads hold any chain of this entry) */
-    int block = ((size_t)total * 8 * 8 <= 24 * 1024) ? 256 : 1024;
-    auto copies_of = [&](int b) { return (size_t)total * 8 * (b / 32) <= 24 * 1024 ? b / 32 : 1; };
-    while (block > 256 && mcg_track_smem((size_t)total * copies_of(block), block, false) > (size_t)optin)
-      block /= 2;
-    P.tally_copies = copies_of(block);
-    const bool smem_tally = mcg_track_smem((size_t)total * P.tally_copies, block, false) <= (size_t)optin;
-    const size_t smem = mcg_track_smem(smem_tally ? (size_t)total * P.tally_copies : 0, block, false);
+    const mcg_shape shape = mcg_track_shape(total, 0, false, false, (size_t)optin);
+    const bool smem_tally = !shape.global;
+    const int block = shape.block;
+    const size_t smem = shape.smem;
+    P.tally_copies = shape.copies;
     auto kern = smem_tally ? mcg_track_kernel<false, MCG_TALLY_SMEM32, false>
                            : mcg_track_kernel<false, MCG_TALLY_GLOBAL, false>;
     /* the attribute is raised to the device's limit (the same value every

@@ -34,6 +34,17 @@ struct mcg_tab {
   int32_t left;
 };
 
+/* How a warp runs its histories (mcg_histories). */
+struct mcg_rules {
+  float min_w;
+  int32_t q_log2;
+  uint32_t max_steps;
+  int32_t window;       /* most steps of a tile (at most MCG_TW_MAX) */
+  int32_t pool_lanes;   /* lanes waiting for the full step that trigger it */
+  int32_t refill_lanes; /* lanes without a history that trigger a refill */
+  mcg_run_consts run;
+};
+
 /* Per-cell step parameters.  strict: {sig_a, sig_i, edge_lo, edge_hi}
  * fast: {sig_a, sig_i (0 when sig_i <= EPS), edge_lo, edge_hi}
  * edge_lo = (float)i * dx_layer, edge_hi = (float)(i+1) * dx_layer with the
@@ -42,8 +53,6 @@ struct mcg_track_params {
   const float4 *cells;
   mcg_tab tab;
   int32_t n_cells, cell_lo;
-  float min_w;
-  int32_t q_log2;
   mcg_particle *particles; /* NULL: source mode */
   int32_t *results;
   int64_t *steps, *scatters;
@@ -54,13 +63,9 @@ struct mcg_track_params {
   unsigned long long *counters; /* mcg_counters fields */
   mcg_libm_dev libm;
   const mcg_libm_tab *libm_tab;
-  int32_t window;       /* most steps of a tile (at most MCG_TW_MAX) */
-  int32_t pool_lanes;   /* lanes waiting for the full step that trigger it */
-  int32_t refill_lanes; /* lanes without a history that trigger a refill */
   int32_t tally_copies; /* 1 or warps per block */
-  int32_t chunk;        /* histories per warp grab (at most MCG_JUMPS) */
-  uint32_t max_steps;
-  mcg_run_consts run;
+  int32_t chunk;        /* histories per warp grab */
+  mcg_rules rules;
 };
 
 /* Tally accumulation: shared-memory 64-bit atomics, shared-memory 32-bit
@@ -744,25 +749,6 @@ __device__ __forceinline__ void mcg_tile_steps(mcg_f2 a, mcg_f2 amu, mcg_f2 ny, 
   nom1 = ok1 ? nom1 : __int_as_float(0x7fc00000);
 }
 
-/* Two deposits (scaled values, exact conversions) of a lane, not THIN. */
-template <int TALLY>
-__device__ __forceinline__ void mcg_tile_deposit(bool in0, unsigned long long *t0, float v0,
-                                                 bool in1, unsigned long long *t1, float v1)
-{
-  if (in0) {
-    if (v0 < 0x1p31f)
-      mcg_deposit_u31<TALLY>(t0, v0);
-    else
-      mcg_tally_add<TALLY>(t0, __float2ll_rn(v0));
-  }
-  if (in1) {
-    if (v1 < 0x1p31f)
-      mcg_deposit_u31<TALLY>(t1, v1);
-    else
-      mcg_tally_add<TALLY>(t1, __float2ll_rn(v1));
-  }
-}
-
 /* The bounds of a flight on a thin chain from its widest cell (R.w_a, R.w_i:
  * the chain's largest sig_a and sig_i widths): {thr, bound} of
  * mcg_tile_steps, which no step passes when the flight is so slanted that its
@@ -860,46 +846,134 @@ __device__ __forceinline__ void mcg_tile_form(mcg_tile_smem<THIN> *S, int q0, co
   }
 }
 
+/* 64-bit shared-memory add under a predicate.  On batched slabs, whose
+ * deposits often pass 32 bits, it is the cheaper form (4096 slabs, 3.1e7
+ * histories, strict: 197 ms against 215 with 32-bit halves and a carry); on a
+ * chain where a point source makes many lanes add to the same cells it is the
+ * dearer one (1000 cells, 1e6 histories, fast: 2.34 ms against 2.02). */
+__device__ __forceinline__ void mcg_shared_red_if(bool p, uint32_t addr, uint64_t v)
+{
+  asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.s32 p, %2, 0;\n\t@p red.shared.add.u64 [%0], %1;\n\t}"
+               :
+               : "r"(addr), "l"(v), "r"((int)p)
+               : "memory");
+}
+
+/* A deposit of scaled value v, 0 <= v < 2^63, as the 64-bit integer
+ * llrint(v): from 2^31 on v is an integer, so it is its shifted significand
+ * (the 64-bit conversion issues on the FP64 pipe). */
+__device__ __forceinline__ uint64_t mcg_fixed_u63(float v)
+{
+  const uint32_t b = __float_as_uint(v);
+  return v < 0x1p31f ? (uint64_t)__float2uint_rn(v)
+                     : (uint64_t)((b & 0x007fffffu) | 0x00800000u) << (b >> 23) - 150u;
+}
+
+/* Where the deposits of a warp's tiles go: TALLY and its base, such that base
+ * + 8 cell is a cell's word in shared memory (MCG_TALLY_GLOBAL: unused), and
+ * the global tally for the rows marked so. */
+struct mcg_sink {
+  uint32_t shared;            /* shared-memory address of cell 0's word (THIN: of its low word) */
+  unsigned long long *global; /* cell 0's word of the global tally */
+};
+
 /* Phase 4 for U passes from pass q0. */
-template <bool THIN, int TALLY, int U>
-__device__ __forceinline__ void mcg_tile_add(mcg_tile_smem<THIN> *S, int q0,
-                                             unsigned long long *tally, unsigned *lo32)
+template <bool THIN, int TALLY, bool MULTI, int U>
+__device__ __forceinline__ void mcg_tile_add(mcg_tile_smem<THIN> *S, int q0, const mcg_sink &D)
 {
   constexpr int G = mcg_tile_shape<THIN>::G, F = 32 / G, PLANE = mcg_tile_shape<THIN>::PLANE;
   const int lane = threadIdx.x & 31, sub = lane / G, j = lane & (G - 1);
   int4 pl[U];
-  float v0[U], v1[U];
+  float v[2 * U];
+  int at[2 * U];
+  bool in[2 * U];
 #pragma unroll
-  for (int v = 0; v < U; ++v) {
-    pl[v] = S->place[F * (q0 + v) + sub];
-    v0[v] = S->step[33 * (q0 + v) + lane];
-    v1[v] = S->step[PLANE + 33 * (q0 + v) + lane];
+  for (int k = 0; k < U; ++k) {
+    pl[k] = S->place[F * (q0 + k) + sub];
+    v[2 * k] = S->step[33 * (q0 + k) + lane];
+    v[2 * k + 1] = S->step[PLANE + 33 * (q0 + k) + lane];
+    at[2 * k] = pl[k].y + j * pl[k].z;
+    at[2 * k + 1] = at[2 * k] + G * pl[k].z;
+    in[2 * k] = j < pl[k].w;
+    in[2 * k + 1] = j + G < pl[k].w;
   }
-  if (THIN) {
-    uint32_t at[2 * U];
+  if (TALLY == MCG_TALLY_LO32) {
     bool carry[2 * U], any = false;
 #pragma unroll
-    for (int v = 0; v < U; ++v) {
-      const uint32_t d0 = __float2uint_rn(v0[v]), d1 = __float2uint_rn(v1[v]);
-      at[2 * v] = (uint32_t)(pl[v].y + j * pl[v].z);
-      at[2 * v + 1] = at[2 * v] + G * pl[v].z;
-      const uint32_t o0 = mcg_shared_add_if(j < pl[v].w, at[2 * v], d0);
-      const uint32_t o1 = mcg_shared_add_if(j + G < pl[v].w, at[2 * v + 1], d1);
-      any |= carry[2 * v] = (uint32_t)(o0 + d0) < o0;
-      any |= carry[2 * v + 1] = (uint32_t)(o1 + d1) < o1;
+    for (int k = 0; k < 2 * U; ++k) {
+      const uint32_t d = __float2uint_rn(v[k]);
+      const uint32_t old = mcg_shared_add_if(in[k], D.shared + 4 * at[k], d);
+      any |= carry[k] = (uint32_t)(old + d) < old;
     }
     if (__any_sync(0xffffffffu, any)) {
-      const uint32_t base = (uint32_t)__cvta_generic_to_shared(lo32);
 #pragma unroll
-      for (int v = 0; v < 2 * U; ++v)
-        if (carry[v])
-          atomicAdd(&tally[(at[v] - base) >> 2], 1ull << 32);
+      for (int k = 0; k < 2 * U; ++k)
+        if (carry[k])
+          atomicAdd(D.global + at[k], 1ull << 32);
     }
   } else {
+    bool far[2 * U], any_far = false, wide = false;
+    uint64_t d[2 * U];
 #pragma unroll
-    for (int v = 0; v < U; ++v) {
-      unsigned long long *t = tally + (pl[v].y + j * pl[v].z);
-      mcg_tile_deposit<TALLY>(j < pl[v].w, t, v0[v], j + G < pl[v].w, t + G * pl[v].z, v1[v]);
+    for (int k = 0; k < 2 * U; ++k) {
+      far[k] = in[k] && (TALLY == MCG_TALLY_GLOBAL || (MULTI && pl[k / 2].x));
+      any_far |= far[k];
+      d[k] = __float2uint_rn(v[k]);
+      wide |= in[k] & !(v[k] < 0x1p31f);
+    }
+    if (__any_sync(0xffffffffu, wide)) {
+#pragma unroll
+      for (int k = 0; k < 2 * U; ++k)
+        d[k] = mcg_fixed_u63(v[k]);
+    }
+    if (TALLY == MCG_TALLY_SMEM64) {
+#pragma unroll
+      for (int k = 0; k < 2 * U; ++k)
+        mcg_shared_red_if(in[k] & !far[k], D.shared + 8 * at[k], d[k]);
+    }
+    if (TALLY == MCG_TALLY_SMEM32) {
+      uint32_t hi[2 * U], more = 0u;
+#pragma unroll
+      for (int k = 0; k < 2 * U; ++k) {
+        const bool here = in[k] & !far[k];
+        const uint32_t lo = (uint32_t)d[k];
+        const uint32_t old = mcg_shared_add_if(here, D.shared + 8 * at[k], lo);
+        hi[k] = (here ? (uint32_t)(d[k] >> 32) : 0u) + ((uint32_t)(old + lo) < old ? 1u : 0u);
+        more |= hi[k];
+      }
+      if (__any_sync(0xffffffffu, more != 0u)) {
+#pragma unroll
+        for (int k = 0; k < 2 * U; ++k)
+          if (hi[k])
+            mcg_shared_add_if(true, D.shared + 8 * at[k] + 4, hi[k]);
+      }
+    }
+    if (TALLY == MCG_TALLY_GLOBAL || (MULTI && __any_sync(0xffffffffu, any_far))) {
+#pragma unroll
+      for (int k = 0; k < 2 * U; ++k)
+        if (far[k])
+          atomicAdd(D.global + at[k], (unsigned long long)d[k]);
+    }
+  }
+}
+
+/* The tile ends at the step that takes the weight below the minimum (scaled):
+ * weights only fall, so the last one tells whether there is such a step. */
+template <bool STRICT, bool THIN>
+__device__ __forceinline__ void mcg_tile_cut(const float *st, int &n, float &W, float &res,
+                                             float W0, float res0, float min_w)
+{
+  constexpr int G = mcg_tile_shape<THIN>::G, PLANE = mcg_tile_shape<THIN>::PLANE;
+  if (W < min_w) {
+    W = W0;
+    res = res0;
+    for (int i = 0; i < n; ++i) {
+      const float dv = st[(i / G) * PLANE + i % G], w2 = __fsub_rn(W, dv);
+      if (!STRICT)
+        res = __fadd_rn(res, __fsub_rn(__fsub_rn(W, w2), dv));
+      W = w2;
+      if (W < min_w)
+        n = i + 1; /* ends the loop */
     }
   }
 }
@@ -908,14 +982,14 @@ __device__ __forceinline__ void mcg_tile_add(mcg_tile_smem<THIN> *S, int q0,
  * flights by up to nmax (1 .. TW) certain crossings and return their
  * number; a0: length to the first face when the flight starts inside the cell,
  * else infinity; W is the weight times the tally scale, res (fast) its
- * residue; test: mcg_thin_tests (THIN).  tab: the chain's tile table; lo32
- * (THIN, with the global tally): see mcg_lo32_add. */
-template <bool STRICT, bool THIN, int TALLY>
+ * residue; test: mcg_thin_tests (THIN); far (MULTI): this flight's deposits go
+ * to the global tally.  idx indexes tab, the tile table, and the tallies. */
+template <bool STRICT, bool THIN, int TALLY, bool MULTI>
 __device__ __forceinline__ int mcg_tiles(bool can, uint64_t s2, float amu, float ainv, float a0,
                                          int dir, int idx, int nmax, float2 test, float &W,
-                                         float &res, const mcg_tab &tab,
-                                         unsigned long long *tally, unsigned *lo32,
-                                         const mcg_tile_warp<THIN> &B, const mcg_run_consts &R)
+                                         float &res, bool far, const mcg_tab &tab,
+                                         const mcg_sink &D, const mcg_tile_warp<THIN> &B,
+                                         const mcg_run_consts &R)
 {
   constexpr int G = mcg_tile_shape<THIN>::G, TW = 2 * G, F = 32 / G;
   constexpr int PLANE = mcg_tile_shape<THIN>::PLANE;
@@ -940,6 +1014,7 @@ __device__ __forceinline__ int mcg_tiles(bool can, uint64_t s2, float amu, float
   __syncwarp();
   int n = 0;
   if (can) {
+    const float W0 = W, res0 = res;
     float *st = S->step + 33 * (rank / F) + G * (rank % F);
     if (nmax < TW)
       st[(nmax / G) * PLANE + nmax % G] = __int_as_float(0x7fc00000);
@@ -971,8 +1046,8 @@ __device__ __forceinline__ int mcg_tiles(bool can, uint64_t s2, float amu, float
           res = __fadd_rn(res, __fsub_rn(__fsub_rn(W, w2), dv));
         W = w2;
       }
-      /* phase 4: the address of step j is y + j z */
-      S->place[rank] = make_int4(0, (int)__cvta_generic_to_shared(lo32) + 4 * idx, 4 * dir, n);
+      mcg_tile_cut<STRICT, THIN>(st, n, W, res, W0, res0, R.min_w);
+      S->place[rank] = make_int4(0, idx, dir, n); /* phase 4: the cell, of either direction */
     } else {
       bool ok = true;
 #pragma unroll
@@ -989,16 +1064,17 @@ __device__ __forceinline__ int mcg_tiles(bool can, uint64_t s2, float amu, float
           n = i + 1;
         }
       }
-      S->place[rank].w = n;
+      mcg_tile_cut<STRICT, THIN>(st, n, W, res, W0, res0, R.min_w);
+      S->place[rank] = make_int4(MULTI && far, idx, dir, n);
     }
   }
   __syncwarp();
   q = 0;
   if (THIN)
     for (; F * (q + 2) < cnt; q += 4)
-      mcg_tile_add<THIN, TALLY, 4>(S, q, tally, lo32);
+      mcg_tile_add<THIN, TALLY, MULTI, 4>(S, q, D);
   for (; F * q < cnt; q += 2)
-    mcg_tile_add<THIN, TALLY, 2>(S, q, tally, lo32);
+    mcg_tile_add<THIN, TALLY, MULTI, 2>(S, q, D);
   __syncwarp();
   return n;
 }
@@ -1018,15 +1094,14 @@ __device__ __forceinline__ float mcg_first_length(const float4 c, const float4 t
              : __int_as_float(0x7fc00000);
 }
 
-/* Most steps of a tile from cell idx of [lo, hi): to the end of the range, one
- * while the weight is near the minimum (so no step passes it unseen), none
- * (the full step) below the weights that scale exactly. */
+/* Most steps of a tile from cell idx of [lo, hi): to the end of the range; none
+ * (the full step) below the weights that stay normal numbers, scaled or not,
+ * through a tile (each step keeps more than 3/4). */
 __device__ __forceinline__ int mcg_tile_limit(int width, int idx, int lo, int hi, float mu,
-                                              float wmc, uint32_t left, const mcg_run_consts &R)
+                                              float wmc, uint32_t left)
 {
-  int n = min(width, mu < 0.0f ? idx - lo + 1 : hi - idx);
-  n = (int)min((uint32_t)n, left);
-  return wmc >= R.w_many ? n : wmc >= R.w_one ? min(n, 1) : 0;
+  const int n = min(width, mu < 0.0f ? idx - lo + 1 : hi - idx);
+  return wmc >= 0x1p-60f ? (int)min((uint32_t)n, left) : 0;
 }
 
 /* The step that a tile left: the flight sample's state, then whatever the step
@@ -1044,81 +1119,128 @@ __device__ __forceinline__ void mcg_full(uint64_t &seed, float &x, float &mu, fl
                                coll_out, dep_out, wres);
 }
 
-/* A warp's share of a launch's histories: a chunk taken from a counter, handed
- * to idle lanes in order.  The seed-chain state of a chunk's first history is
- * found by one jump-ahead (`state_of`, run by all lanes together) and a
- * lane's own by one multiply-add from jump[r], jump[MCG_JUMPS + r], the
- * r-step jumps (instead of a jump-ahead of about 20 doublings per lane, run
- * by the one or two lanes that refill). */
-#define MCG_JUMPS 32
+/* Jumps of the seed chain by d 32^l steps, d < 32: A and C of s -> A s + C mod
+ * 2^63 at l 32 + d.  A newborn's state is one multiply-add per base-32 digit of
+ * its index (a jump-ahead by doubling takes about 500 instructions, run by the
+ * one or two lanes that refill). */
+#define MCG_JUMP_LEVELS 8
+struct mcg_chain_jumps {
+  unsigned long long A[32 * MCG_JUMP_LEVELS], C[32 * MCG_JUMP_LEVELS];
+};
 
-__device__ __forceinline__ void mcg_fill_jumps(unsigned long long *jump)
+__device__ __forceinline__ void mcg_fill_chain_jumps(mcg_chain_jumps *J)
 {
-  for (int r = threadIdx.x; r < MCG_JUMPS; r += blockDim.x) {
-    const uint64_t c = mcg_lcg_skip(0ull, (uint64_t)r, 1);
-    jump[r] = (mcg_lcg_skip(1ull, (uint64_t)r, 1) - c) & MCG_MASK63;
-    jump[MCG_JUMPS + r] = c;
+  for (int k = threadIdx.x; k < 32 * MCG_JUMP_LEVELS; k += blockDim.x) {
+    const uint64_t steps = (uint64_t)(k & 31) << (5 * (k >> 5)), c = mcg_lcg_skip(0ull, steps, 1);
+    J->A[k] = (mcg_lcg_skip(1ull, steps, 1) - c) & MCG_MASK63;
+    J->C[k] = c;
   }
 }
 
-/* Shared memory of mcg_track_kernel: libm tables, counters, jumps, the tally's
- * copies (an even number of words), the warps' tiles. */
-inline size_t mcg_track_smem(size_t tally_words, int block, bool thin)
+/* The seed chain's state n steps after s. */
+__device__ __forceinline__ uint64_t mcg_chain_jump(const mcg_chain_jumps *J, uint64_t s, uint64_t n)
 {
-  if (thin)
-    tally_words = (tally_words + 1) / 2; /* MCG_TALLY_LO32 */
-  return sizeof(mcg_libm_tab) + (16 + 2 * MCG_JUMPS + 2 * (MCG_TW_MAX + 1)) * 8 +
-         ((tally_words + 1) & ~(size_t)1) * 8 +
-         (size_t)(block / 32) * (thin ? sizeof(mcg_tile_smem<true>) : sizeof(mcg_tile_smem<false>));
+  for (int l = 0; l < MCG_JUMP_LEVELS && n; ++l, n >>= 5) {
+    const int k = 32 * l + (int)(n & 31);
+    s = J->A[k] * s + J->C[k];
+  }
+  if (n) /* indices from 2^40 on */
+    s = mcg_lcg_skip(s & MCG_MASK63, n << (5 * MCG_JUMP_LEVELS), 1);
+  return s & MCG_MASK63;
 }
 
+/* Particle k of a device-born source (see mcg_source). */
+__device__ __forceinline__ void mcg_born(const mcg_chain_jumps *J, const mcg_source &S, int64_t k,
+                                         uint64_t &seed, float &x, float &mu, float &wmc, int &idx)
+{
+  const uint64_t s = S.seed_mode == 0 ? mcg_chain_jump(J, S.base_seed, (uint64_t)k + 1)
+                                      : ((S.base_seed + (uint64_t)k) & MCG_MASK63);
+  mcg_source_particle_at(S, s, seed, x, mu, wmc, idx);
+}
+
+/* A warp's share of a launch's histories: a chunk taken from a counter, handed
+ * to idle lanes in order. */
 struct mcg_pool {
   long long next = 0, end = 0; /* what is left of the chunk */
-  long long base = 0;          /* the chunk's first history and its state */
-  uint64_t state = 0;
   bool drained = false;
 
-  /* The history of this lane (in `need`), or -1, and its seed-chain state;
-   * chunks of at most MCG_JUMPS histories.  The whole warp calls. */
-  template <class F>
+  /* The history of this lane (in `need`), or -1; chunk 0: no more than the
+   * lanes ask for.  The whole warp calls. */
   __device__ __forceinline__ long long take(unsigned need, unsigned long long *counter, long long n,
-                                            int chunk, const F &state_of,
-                                            const unsigned long long *jump, uint64_t &my_state)
+                                            int chunk)
   {
     const int cnt = __popc(need), rank = __popc(need & lanemask_lt());
     const long long avail = end - next;
-    long long my = -1, my_base = base;
-    uint64_t st = state;
+    long long my = -1;
     if (rank < avail)
       my = next + rank;
     if (cnt > avail && !drained) {
+      const int grab = chunk ? chunk : cnt;
       unsigned long long b = 0;
       if ((threadIdx.x & 31) == 0)
-        b = atomicAdd(counter, (unsigned long long)chunk);
+        b = atomicAdd(counter, (unsigned long long)grab);
       b = __shfl_sync(0xffffffffu, b, 0);
       if ((long long)b >= n) {
         drained = true;
         next = end = 0;
       } else {
-        end = min((long long)b + chunk, n);
-        base = (long long)b;
-        state = state_of(base);
+        end = min((long long)b + grab, n);
         const long long r2 = rank - avail;
-        if (rank >= avail && r2 < end - base) {
-          my = base + r2;
-          my_base = base;
-          st = state;
-        }
-        next = min(base + (cnt - avail), end);
+        if (rank >= avail && r2 < end - (long long)b)
+          my = (long long)b + r2;
+        next = min((long long)b + (cnt - avail), end);
+        drained = end == n; /* nothing more to ask for */
       }
     } else {
       next += min((long long)cnt, avail);
     }
-    const int r = my >= 0 ? (int)(my - my_base) : 0;
-    my_state = (jump[r] * st + jump[MCG_JUMPS + r]) & MCG_MASK63;
     return my;
   }
 };
+
+/* Shared memory of mcg_track_kernel: libm tables, counters, jumps, the tally's
+ * copies (an even number of words; thin: low words), the warps' tiles. */
+inline size_t mcg_track_smem(size_t tally_words, int block, bool thin)
+{
+  if (thin)
+    tally_words = (tally_words + 1) / 2; /* MCG_TALLY_LO32 */
+  return sizeof(mcg_libm_tab) + 16 * 8 + sizeof(mcg_chain_jumps) + sizeof(mcg_real_jumps) +
+         ((tally_words + 1) & ~(size_t)1) * 8 +
+         (size_t)(block / 32) * (thin ? sizeof(mcg_tile_smem<true>) : sizeof(mcg_tile_smem<false>));
+}
+
+/* Launch shape of a chain: short ones keep one tally copy per warp in
+ * 256-thread blocks; long ones share one copy per block of 1024 threads (thin
+ * ones MCG_THIN_BLOCK), or of fewer where the copy and the warps' tiles would
+ * not fit; a chain too long for any copy adds to the global tally.  block and
+ * global as asked (0: automatic). */
+struct mcg_shape {
+  int block, copies;
+  bool global, thin;
+  size_t smem;
+};
+
+inline mcg_shape mcg_track_shape(int n_cells, int block, bool global, bool thin, size_t optin)
+{
+  mcg_shape s = {block, 1, global, thin, 0};
+  auto fit = [&](int b) {
+    s.copies = !s.thin && (size_t)n_cells * 8 * (b / 32) <= 24 * 1024 ? b / 32 : 1;
+    s.smem = mcg_track_smem(s.global ? 0 : (size_t)n_cells * s.copies, b, s.thin);
+    return s.smem <= optin;
+  };
+  if (!block) {
+    s.block = thin ? MCG_THIN_BLOCK : ((size_t)n_cells * 8 * 8 <= 24 * 1024) ? 256 : 1024;
+    while (!s.global && s.block > 256 && !fit(s.block))
+      s.block -= 128;
+  }
+  if (!fit(s.block)) {
+    s.global = true;
+    s.thin = false;
+    s.block = block ? block : 1024;
+    fit(s.block);
+  }
+  return s;
+}
 
 /* Counters of a finished history: result r, final weight. */
 template <bool STRICT>
@@ -1143,6 +1265,170 @@ __device__ __forceinline__ void mcg_count_end(unsigned long long *s_cnt, int r, 
   }
 }
 
+/* The chain that a warp's newborns run in; with MULTI the slab, whose cells
+ * start at `off` of the concatenated ones. */
+struct mcg_geometry {
+  int32_t off, ncell;
+};
+
+/* A warp's histories, to the end of the source: n() histories handed out by
+ * *counter in chunks (mcg_pool::take).  birth(k, ...) makes history k's particle
+ * with its cell index local to the chain; end(k, result, ...) sees its final
+ * state.  cells and tab are the chain's, word its shared-memory tally (base
+ * of mcg_sink D) as a pointer.  The whole warp calls.
+ *
+ * MULTI: cells, tab and the global tally are those of all slabs; when a slab's
+ * histories are handed out (exhausted()), the block changes to the next work
+ * item together (more(), which returns false when there is none) while its
+ * warps keep the histories they have: such a history stays in its lane, with
+ * its own slab's cells, and its deposits go to the global tally.  So no warp
+ * waits for another's longest history. */
+template <bool STRICT, bool THIN, int TALLY, bool MULTI, class N, class BIRTH, class END, class GONE,
+          class MORE>
+__device__ __forceinline__ void mcg_histories(mcg_geometry &geo, mcg_sink &D, const float4 *cells,
+                                              const mcg_tab &tab, unsigned long long *word,
+                                              const mcg_rules &R, const mcg_tile_warp<THIN> &tiles,
+                                              const mcg_real_jumps *jumps, const mcg_libm_tab *T,
+                                              const mcg_libm_dev &libm, unsigned long long *counter,
+                                              const N &n, int chunk, const BIRTH &birth,
+                                              const END &end, const GONE &exhausted, const MORE &more)
+{
+  uint64_t s2 = 0; /* the state, shifted left by one */
+  float x = 0.f, mu = 0.f, wmc = 0.f, inv_mu = 0.f;
+  float wres = 0.f; /* fast: the weight's rounding residue (mcg_fast_weight_update) */
+  float2 test = make_float2(0.f, 0.f); /* THIN: mcg_thin_tests */
+  float a0 = 0.f;   /* mcg_first_length; inf: x is the face the cell was entered by */
+  int idx = 0;
+  int off = 0, ncell = geo.ncell; /* the history's chain: cells off .. off + ncell */
+  int64_t hid = -1;
+  uint32_t nst = 0, nsc = 0;
+  bool active = false, wait = false; /* wait: the lane's step needs the full form */
+  mcg_pool pool;
+  bool work = true; /* MULTI: more() has not yet returned false */
+  const float min_w = R.min_w;
+  auto living = [&] {
+    return active & (wmc >= min_w) & ((unsigned)(idx - off) < (unsigned)ncell) & (nst < R.max_steps);
+  };
+
+  for (;;) {
+    bool alive = living();
+    const unsigned ab = __ballot_sync(0xffffffffu, alive);
+    /* ended histories leave and newborns come once refill_lanes lanes are
+     * without a living history, or no lane has one */
+    const bool gone = MULTI && work && exhausted();
+    if (!ab || gone || (__popc(~ab) >= R.refill_lanes &&
+                        (!pool.drained || __any_sync(0xffffffffu, active & !alive)))) {
+      if (active & !alive) {
+        /* history ends: classification of simulate_particle; a history
+         * still alive in the chain here has reached the step limit */
+        const int c = idx - off;
+        const bool in = (wmc >= min_w) && ((unsigned)c < (unsigned)ncell);
+        int r;
+        if (in)
+          r = 2;
+        else if (c == -1)
+          r = -1;
+        else if (c == ncell)
+          r = 1;
+        else if (wmc < min_w)
+          r = 0;
+        else
+          r = -1;
+        if (a0 == INFINITY)
+          x = mu < 0.0f ? __ldg(&cells[idx + 1].z) : __ldg(&cells[idx - 1].w);
+        end(hid, r, s2 >> 1, x, mu, wmc, wres, c, nst, nsc);
+        active = false;
+      }
+      unsigned need = __ballot_sync(0xffffffffu, !active);
+      while (MULTI && work && exhausted()) {
+        work = more();
+        pool = mcg_pool();
+      }
+      if (MULTI && !work)
+        pool.drained = true;
+      const long long my = need ? pool.take(need, counter, n(), chunk) : -1;
+      if (!active && my >= 0) {
+        hid = my;
+        uint64_t seed;
+        birth(my, seed, x, mu, wmc, idx);
+        s2 = seed << 1;
+        off = MULTI ? geo.off : 0;
+        ncell = geo.ncell;
+        idx += off;
+        a0 = 0.0f;
+        inv_mu = mcg_flight_rcp(mu);
+        wres = 0.f;
+        nst = nsc = 0;
+        active = true;
+        alive = living();
+        if (THIN)
+          test = mcg_thin_tests<STRICT>(inv_mu, wmc, R.run);
+        if (alive)
+          a0 = mcg_first_length(__ldg(cells + idx), __ldg(tab.cell + idx), x, mu, inv_mu, wmc);
+      }
+      if (!__any_sync(0xffffffffu, active) && (!MULTI || !work))
+        break;
+    }
+
+    /* one tile for every lane that can; the lanes whose step needs the full
+     * form wait until pool_lanes of them do (or no other lane can step) and
+     * take it together.  Each pass steps a lane, makes one wait, completes
+     * the waiting steps, ends a history or hands out work, and no lane passes
+     * its step limit, so this ends. */
+    bool can = alive & !wait;
+    const bool far = MULTI && off != geo.off;
+    const int nmax = a0 == a0 ? mcg_tile_limit(min(R.window, mcg_tile_shape<THIN>::TW), idx, off,
+                                               off + ncell, mu, wmc, R.max_steps - nst)
+                              : 0;
+    wait |= can & (nmax == 0);
+    can &= nmax != 0;
+    if (__any_sync(0xffffffffu, can)) {
+      const int dir = mu < 0.0f ? -1 : 1;
+      float W = __fmul_rn(wmc, R.run.scale), res = __fmul_rn(wres, R.run.scale);
+      const int k = mcg_tiles<STRICT, THIN, TALLY, MULTI>(can, s2, fabsf(mu), fabsf(inv_mu), a0, dir,
+                                                          idx, nmax, test, W, res, far, tab, D,
+                                                          tiles, R.run);
+      if (k > 0) {
+        s2 = jumps->A[k] * s2 + jumps->C[k];
+        wmc = __fmul_rn(W, R.run.inv_scale);
+        if (!STRICT)
+          wres = __fmul_rn(res, R.run.inv_scale);
+        idx += k * dir;
+        nst += (uint32_t)k;
+        a0 = INFINITY;
+      }
+      wait |= can & (k < nmax) & (wmc >= min_w);
+    }
+    const unsigned wb = __ballot_sync(0xffffffffu, wait);
+    if (wb && (__popc(wb) >= R.pool_lanes || !__any_sync(0xffffffffu, alive & !wait))) {
+      if (wait) {
+        if (a0 == INFINITY)
+          x = mu < 0.0f ? __ldg(&cells[idx + 1].z) : __ldg(&cells[idx - 1].w);
+        uint64_t seed = s2 >> 1;
+        const int cell = idx;
+        float len, dep;
+        bool coll;
+        mcg_full<STRICT, TALLY>(seed, x, mu, wmc, inv_mu, idx, nsc, __ldg(cells + idx),
+                                THIN ? nullptr
+                                     : (TALLY == MCG_TALLY_GLOBAL || far ? D.global + idx
+                                                                         : word + (idx - geo.off)),
+                                R.q_log2, T, libm, &len, &coll, &dep, STRICT ? nullptr : &wres);
+        if (THIN) {
+          mcg_lo32_add(reinterpret_cast<unsigned *>(word) + cell, D.global + cell,
+                       mcg_to_fixed(dep, R.q_log2));
+          test = mcg_thin_tests<STRICT>(inv_mu, wmc, R.run);
+        }
+        s2 = seed << 1;
+        ++nst;
+        wait = false;
+        a0 = (unsigned)(idx - off) < (unsigned)ncell
+                 ? mcg_first_length(__ldg(cells + idx), __ldg(tab.cell + idx), x, mu, inv_mu, wmc)
+                 : 0.0f;
+      }
+    }
+  }
+}
+
 /* THIN: the chain is optically thin (see update_thin in mcg_api.cu) and the
  * tally is MCG_TALLY_LO32. */
 template <bool STRICT, int TALLY, bool THIN>
@@ -1151,12 +1437,12 @@ __global__ void __launch_bounds__(THIN ? MCG_THIN_BLOCK : 1024) mcg_track_kernel
   extern __shared__ __align__(16) unsigned char smem[];
   mcg_libm_tab *T = reinterpret_cast<mcg_libm_tab *>(smem);
   unsigned long long *s_cnt = reinterpret_cast<unsigned long long *>(smem + sizeof(mcg_libm_tab));
-  unsigned long long *s_jump = s_cnt + 16;
-  mcg_real_jumps *s_real = reinterpret_cast<mcg_real_jumps *>(s_jump + 2 * MCG_JUMPS);
-  unsigned long long *s_tally = s_jump + 2 * MCG_JUMPS + 2 * (MCG_TW_MAX + 1);
+  mcg_chain_jumps *s_chain = reinterpret_cast<mcg_chain_jumps *>(s_cnt + 16);
+  mcg_real_jumps *s_real = reinterpret_cast<mcg_real_jumps *>(s_chain + 1);
+  unsigned long long *s_tally = reinterpret_cast<unsigned long long *>(s_real + 1);
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int ncell = P.n_cells, lo = P.cell_lo;
-  mcg_fill_jumps(s_jump);
+  mcg_fill_chain_jumps(s_chain);
   mcg_fill_real_jumps(s_real);
 
   if (STRICT) {
@@ -1174,53 +1460,27 @@ __global__ void __launch_bounds__(THIN ? MCG_THIN_BLOCK : 1024) mcg_track_kernel
   mcg_tile_smem<THIN> *tile = reinterpret_cast<mcg_tile_smem<THIN> *>(
       s_tally + ((words + 1) & ~1)) + warp;
   __syncthreads();
-  unsigned *lo32 = THIN ? reinterpret_cast<unsigned *>(s_tally) : nullptr;
-  unsigned long long *my_tally = TALLY == MCG_TALLY_GLOBAL || THIN
-                                     ? P.tally
-                                     : s_tally + (size_t)(warp % P.tally_copies) * ncell;
+  unsigned long long *my_tally = s_tally + (THIN ? 0 : (size_t)(warp % P.tally_copies) * ncell);
 
-  uint64_t s2 = 0; /* the state, shifted left by one */
-  float x = 0.f, mu = 0.f, wmc = 0.f, inv_mu = 0.f;
-  float wres = 0.f; /* fast: the weight's rounding residue (mcg_fast_weight_update) */
-  float2 test = make_float2(0.f, 0.f); /* THIN: mcg_thin_tests */
-  float a0 = 0.f;   /* mcg_first_length; inf: x is the face the cell was entered by */
-  int idx = 0;
-  int64_t hid = -1;
-  uint32_t nst = 0, nsc = 0;
-  bool active = false, wait = false; /* wait: the lane's step needs the full form */
-  unsigned long long tot_steps = 0, tot_scat = 0;
-  mcg_pool pool;
-  const float min_w = P.min_w;
-  const int qs = P.q_log2;
   const mcg_tile_warp<THIN> tiles(tile, s_real);
-
-  for (;;) {
-    bool alive = active & (wmc >= min_w) & ((unsigned)idx < (unsigned)ncell) & (nst < P.max_steps);
-    const unsigned ab = __ballot_sync(0xffffffffu, alive);
-    /* ended histories leave and newborns come once refill_lanes lanes are
-     * without a living history, or no lane has one */
-    if (!ab || (__popc(~ab) >= P.refill_lanes &&
-                (!pool.drained || __any_sync(0xffffffffu, active & !alive)))) {
-      if (active & !alive) {
-        /* history ends: classification of simulate_particle; a history
-         * still alive in the chain here has reached the step limit */
-        const bool in = (wmc >= min_w) && ((unsigned)idx < (unsigned)ncell);
-        int r;
-        if (in)
-          r = 2;
-        else if (idx == -1)
-          r = -1;
-        else if (idx == ncell)
-          r = 1;
-        else if (wmc < min_w)
-          r = 0;
+  mcg_geometry geo = {0, ncell};
+  mcg_sink sink = {(uint32_t)__cvta_generic_to_shared(my_tally), P.tally};
+  unsigned long long tot_steps = 0, tot_scat = 0;
+  mcg_histories<STRICT, THIN, TALLY, false>(
+      geo, sink, P.cells, P.tab, my_tally, P.rules, tiles, s_real, T, P.libm, P.next,
+      [&] { return (long long)P.n; }, P.chunk,
+      [&](long long my, uint64_t &seed, float &x, float &mu, float &wmc, int &idx) {
+        if (P.particles)
+          mcg_load_particle(P, my, seed, x, mu, wmc, idx);
         else
-          r = -1;
-        if (P.particles && nst) {
-          if (a0 == INFINITY)
-            x = mu < 0.0f ? __ldg(&P.cells[idx + 1].z) : __ldg(&P.cells[idx - 1].w);
+          mcg_born(s_chain, P.src, P.first + my, seed, x, mu, wmc, idx);
+        idx -= lo;
+      },
+      [&](long long hid, int r, uint64_t seed, float x, float mu, float wmc, float wres, int idx,
+          uint32_t nst, uint32_t nsc) {
+        if (P.particles && nst) { /* without a step the particle stays as it is */
           unsigned long long *q = reinterpret_cast<unsigned long long *>(P.particles + hid);
-          q[0] = s2 >> 1;
+          q[0] = seed;
           q[1] = (unsigned long long)__float_as_uint(x) |
                  ((unsigned long long)__float_as_uint(mu) << 32);
           q[2] = (unsigned long long)__float_as_uint(wmc) |
@@ -1232,93 +1492,11 @@ __global__ void __launch_bounds__(THIN ? MCG_THIN_BLOCK : 1024) mcg_track_kernel
           P.steps[hid] = nst;
         if (P.scatters)
           P.scatters[hid] = nsc;
-        mcg_count_end<STRICT>(s_cnt, r, wmc, wres, qs);
+        mcg_count_end<STRICT>(s_cnt, r, wmc, wres, P.rules.q_log2);
         tot_steps += nst;
         tot_scat += nsc;
-        active = false;
-      }
-      const unsigned need = __ballot_sync(0xffffffffu, !active);
-      uint64_t my_seed = 0;
-      const long long my = pool.take(need, P.next, P.n, P.chunk, [&](long long base) {
-        return P.particles || P.src.seed_mode ? 0ull
-               : mcg_lcg_skip(P.src.base_seed, (uint64_t)(P.first + base) + 1, 1);
-      }, s_jump, my_seed);
-      if (!active && my >= 0) {
-        hid = my;
-        uint64_t seed;
-        if (!P.particles && P.src.seed_mode == 0)
-          mcg_source_particle_at(P.src, my_seed, seed, x, mu, wmc, idx);
-        else
-          mcg_load_particle(P, hid, seed, x, mu, wmc, idx);
-        s2 = seed << 1;
-        idx -= lo;
-        inv_mu = mcg_flight_rcp(mu);
-        wres = 0.f;
-        nst = nsc = 0;
-        active = true;
-        alive = (wmc >= min_w) & ((unsigned)idx < (unsigned)ncell) & (nst < P.max_steps);
-        if (THIN)
-          test = mcg_thin_tests<STRICT>(inv_mu, wmc, P.run);
-        if (alive)
-          a0 = mcg_first_length(__ldg(P.cells + idx), __ldg(P.tab.cell + idx), x, mu, inv_mu, wmc);
-      }
-      if (!__any_sync(0xffffffffu, active))
-        break;
-    }
-
-    /* one tile for every lane that can; the lanes whose step needs the full
-     * form wait until pool_lanes of them do (or no other lane can step) and
-     * take it together.  Each pass steps a lane, makes one wait, completes
-     * the waiting steps or ends a history, and no lane passes its step
-     * limit, so this ends. */
-    bool can = alive & !wait;
-    const int nmax = a0 == a0 ? mcg_tile_limit(min(P.window, mcg_tile_shape<THIN>::TW), idx, 0, ncell,
-                                               mu, wmc, P.max_steps - nst, P.run)
-                              : 0;
-    wait |= can & (nmax == 0);
-    can &= nmax != 0;
-    if (__any_sync(0xffffffffu, can)) {
-      const int dir = mu < 0.0f ? -1 : 1;
-      float W = __fmul_rn(wmc, P.run.scale), res = __fmul_rn(wres, P.run.scale);
-      const int n = mcg_tiles<STRICT, THIN, TALLY>(can, s2, fabsf(mu), fabsf(inv_mu), a0, dir, idx,
-                                                   nmax, test, W, res, P.tab, my_tally, lo32,
-                                                   tiles, P.run);
-      if (n > 0) {
-        s2 = s_real->A[n] * s2 + s_real->C[n];
-        wmc = __fmul_rn(W, P.run.inv_scale);
-        if (!STRICT)
-          wres = __fmul_rn(res, P.run.inv_scale);
-        idx += n * dir;
-        nst += (uint32_t)n;
-        a0 = INFINITY;
-      }
-      wait |= can & (n < nmax);
-    }
-    const unsigned wb = __ballot_sync(0xffffffffu, wait);
-    if (wb && (__popc(wb) >= P.pool_lanes || !__any_sync(0xffffffffu, alive & !wait))) {
-      if (wait) {
-        if (a0 == INFINITY)
-          x = mu < 0.0f ? __ldg(&P.cells[idx + 1].z) : __ldg(&P.cells[idx - 1].w);
-        uint64_t seed = s2 >> 1;
-        const int cell = idx;
-        float len, dep;
-        bool coll;
-        mcg_full<STRICT, TALLY>(seed, x, mu, wmc, inv_mu, idx, nsc, __ldg(P.cells + idx),
-                                THIN ? nullptr : &my_tally[idx], qs, T, P.libm, &len, &coll, &dep,
-                                STRICT ? nullptr : &wres);
-        if (THIN) {
-          mcg_lo32_add(lo32 + cell, my_tally + cell, mcg_to_fixed(dep, qs));
-          test = mcg_thin_tests<STRICT>(inv_mu, wmc, P.run);
-        }
-        s2 = seed << 1;
-        ++nst;
-        wait = false;
-        a0 = (unsigned)idx < (unsigned)ncell
-                 ? mcg_first_length(__ldg(P.cells + idx), __ldg(P.tab.cell + idx), x, mu, inv_mu, wmc)
-                 : 0.0f;
-      }
-    }
-  }
+      },
+      [] { return true; }, [] { return false; });
 
   /* per-thread counters -> block */
   for (int o = 16; o > 0; o >>= 1) {
@@ -1331,6 +1509,7 @@ __global__ void __launch_bounds__(THIN ? MCG_THIN_BLOCK : 1024) mcg_track_kernel
   }
   __syncthreads();
   if (THIN) {
+    const unsigned *lo32 = reinterpret_cast<const unsigned *>(s_tally);
     for (int i = tid; i < ncell; i += blockDim.x)
       if (lo32[i])
         atomicAdd(&P.tally[i], (unsigned long long)lo32[i]);
@@ -1352,12 +1531,21 @@ __global__ void __launch_bounds__(THIN ? MCG_THIN_BLOCK : 1024) mcg_track_kernel
   }
 }
 
-/* Rounds of a launch (see the kernel's loop). */
-inline void mcg_track_rounds(const mcg_context *ctx, bool thin, mcg_track_params &P)
+/* The rules of a launch.  Full steps are pooled for 4 lanes (thin chains need
+ * them on 1 % of the tiles, others on a third of them) and ended histories
+ * replaced for one or two; 2 to 16 and 1 to 8 were measured within 5 % of
+ * these on thin chains and within 10 % on a 1000-cell one. */
+inline mcg_rules mcg_rules_setup(const mcg_context *ctx, float min_w, bool thin)
 {
-  P.window = ctx->refill ? ctx->refill : MCG_TW_MAX;
-  P.pool_lanes = 4;
-  P.refill_lanes = thin ? 1 : 2;
+  mcg_rules R;
+  R.min_w = min_w;
+  R.q_log2 = ctx->log2_scale;
+  R.max_steps = ctx->max_steps;
+  R.window = ctx->refill ? ctx->refill : MCG_TW_MAX;
+  R.pool_lanes = 4;
+  R.refill_lanes = thin ? 1 : 2;
+  R.run = mcg_run_setup(ctx->log2_scale, min_w, ctx->run_bounds, ctx->width_a, ctx->width_i);
+  return R;
 }
 
 /* Grid of at most `resident` blocks, and the chunk of histories a warp takes:
@@ -1366,7 +1554,7 @@ inline void mcg_track_rounds(const mcg_context *ctx, bool thin, mcg_track_params
 inline int mcg_track_grid(int resident, int block, int64_t n, mcg_track_params &P)
 {
   const int64_t warps = (int64_t)resident * (block / 32);
-  P.chunk = (int)std::min<int64_t>(MCG_JUMPS, (n + warps - 1) / warps);
+  P.chunk = (int)std::min<int64_t>(32, (n + warps - 1) / warps);
   return (int)std::min<int64_t>(resident, n);
 }
 

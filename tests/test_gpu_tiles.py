@@ -69,3 +69,36 @@ def test_tiles_match_event_mode(mcg, mode, thin, m, layers):
                 assert np.array_equal(ra[key], rb[key]), key
             assert np.array_equal(qa, qb)
             assert ca == cb
+
+
+@pytest.mark.parametrize("mode", ["strict", "fast"])
+@pytest.mark.parametrize("sizes", [(1, 40), (15, 700), (20_000, 25_000)])
+def test_batch_items_match_event_mode(mcg, mode, sizes):
+    """Work items down to one history, so that blocks change slabs while their
+    warps keep histories of earlier ones (whose deposits then go to the global
+    tally), in every tally mode and block size: the event-based form's tallies
+    and counters.  The largest slabs are beyond the shared-memory tally."""
+    rng = np.random.default_rng(sizes[1])
+    n_slabs = 60 if sizes[1] < 1000 else 3
+    cells = rng.integers(sizes[0], sizes[1] + 1, n_slabs)
+    total = int(cells.sum())
+    sa = np.repeat(10.0 ** rng.uniform(-2, 1, n_slabs), cells) * rng.random(total)
+    ss = np.repeat(10.0 ** rng.uniform(-2, 1.3, n_slabs), cells) * rng.random(total)
+    sigs = (sa + ss).astype(f32)
+    rates = (sa / np.maximum(sa + ss, 1e-30)).astype(f32)
+    slabs = [dict(n_cells=int(cells[s]), n_histories=int(rng.integers(0, 300)), base_seed=17 + s,
+                  seed_mode=s % 2, isotropic=s % 3, mu0=1.0, w0=1.0) for s in range(n_slabs)]
+    with mcg.Context(mode=mode) as ctx:
+        ctx.batch_set(slabs, sigs, rates, 1e-12)
+        ctx.batch_set_algorithm("event", 2)
+        ctx.batch_run()
+        want, counters = ctx.batch_tally_q(), ctx.counters()
+        ctx.batch_set_algorithm("history")
+        for block, item, tally, defer in ((256, 1, 1, 0), (512, 7, 0, 1), (1024, 64, 2, 32),
+                                          (1024, 1 << 20, 1, 4)):
+            ctx.batch_set_launch(block, item, tally)
+            ctx.batch_set_deferral(defer)
+            ctx.batch_tally_reset()
+            ctx.batch_run()
+            assert np.array_equal(ctx.batch_tally_q(), want), (block, item, tally)
+            assert ctx.counters() == counters
