@@ -56,20 +56,25 @@ struct mcg_adj_params {
   double *grad_a, *grad_s;
   mcg_libm_dev libm;
   const mcg_libm_tab *libm_tab;
-  int32_t refill_steps, chunk, with_grad;
+  int32_t chunk, with_grad, jumps; /* jumps: the seed chain's table fits in shared memory */
+  float b_mid; /* mcg_run_consts */
   uint32_t max_steps;
 };
 
-/* float-float accumulation s += v (TwoSum) */
-__device__ __forceinline__ void ff_add(float &hi, float &lo, float v)
-{
-  const float s = __fadd_rn(hi, v);
-  const float bv = __fsub_rn(s, hi);
-  const float e = __fadd_rn(__fsub_rn(hi, __fsub_rn(s, bv)), __fsub_rn(v, bv));
-  hi = s;
-  lo = __fadd_rn(lo, e);
-}
-
+/*
+ * Bound: instruction issue (56 % of the slots) at 11 of 32 lanes, the histories
+ * of a warp being at different places; memory plays no part.  Almost every step
+ * is a crossing that the bounds of mcg_cross decide without the logarithm,
+ * the exponential's table or the new direction, so the few full steps are
+ * gathered (the rounds below) instead of stopping the whole warp for one lane.
+ * 1000 cells, 2e6 histories, forward and gradient, strict: 69.2 ms with the
+ * full step in every lane, 42 ms so; the start of a history by the seed chain's
+ * table instead of the doubling jump is 1 ms of that.  A history stays with
+ * a lane, and 512 lanes share one fp32 accumulator per cell: tiles of crossings
+ * per flight, as the tracker has, took 39.4 ms but add a cell's terms in
+ * another grouping, which moved the gradients by more than two runs of this
+ * kernel differ.
+ */
 template <bool STRICT>
 __global__ void __launch_bounds__(1024) mcg_adjoint_kernel(mcg_adj_params P)
 {
@@ -79,8 +84,17 @@ __global__ void __launch_bounds__(1024) mcg_adjoint_kernel(mcg_adj_params P)
   unsigned long long *s_tally = s_cnt + 16;
   float *s_ga = reinterpret_cast<float *>(s_tally + P.n_cells);
   float *s_gs = s_ga + P.n_cells;
+  mcg_chain_jumps *s_chain = reinterpret_cast<mcg_chain_jumps *>(s_gs + P.n_cells);
   const int tid = threadIdx.x, lane = tid & 31;
   const int ncell = P.n_cells, lo = P.cell_lo;
+  if (P.jumps)
+    mcg_fill_chain_jumps(s_chain);
+  auto born = [&](int64_t k, uint64_t &seed, float &x, float &mu, float &wmc, int &idx) {
+    if (P.jumps)
+      mcg_born(s_chain, P.src, k, seed, x, mu, wmc, idx);
+    else
+      mcg_source_particle(P.src, k, seed, x, mu, wmc, idx);
+  };
   if (STRICT) {
     const float *src = reinterpret_cast<const float *>(P.libm_tab);
     float *dst = reinterpret_cast<float *>(T);
@@ -100,8 +114,8 @@ __global__ void __launch_bounds__(1024) mcg_adjoint_kernel(mcg_adj_params P)
   int idx = 0, phase = 0;
   int64_t hid = -1;
   uint32_t nst = 0, nsc = 0;
-  float G_hi = 0.f, G_lo = 0.f, P_hi = 0.f, P_lo = 0.f;
-  bool active = false;
+  float G_hi = 0.f, G_lo = 0.f, P_hi = 0.f, P_lo = 0.f, v_before = 0.f;
+  bool active = false, wait = false; /* wait: the lane's step needs the full form */
   unsigned long long tot_steps = 0, tot_scat = 0;
   long long pool_next = 0, pool_end = 0;
   bool drained = false;
@@ -134,7 +148,7 @@ __global__ void __launch_bounds__(1024) mcg_adjoint_kernel(mcg_adj_params P)
       }
       if (!active && my >= 0) {
         hid = my;
-        mcg_source_particle(P.src, P.first + hid, seed, x, mu, wmc, idx);
+        born(P.first + hid, seed, x, mu, wmc, idx);
         idx -= lo;
         inv_mu = mcg_flight_rcp(mu);
         nst = nsc = 0;
@@ -146,60 +160,93 @@ __global__ void __launch_bounds__(1024) mcg_adjoint_kernel(mcg_adj_params P)
     if (!__any_sync(0xffffffffu, active))
       break;
 
-    if (active) {
-      /* up to refill_steps steps, never past the step limit; idx is local
-       * to the chain */
-      const int kmax = (int)min((uint32_t)P.refill_steps, P.max_steps - nst);
-      int k = 0;
-      bool going = true;
-      for (; k < kmax; ++k) {
-        if (!((wmc >= min_w) & ((unsigned)idx < (unsigned)ncell))) {
-          going = false;
-          break;
-        }
+    /* A round, run by the whole warp: a lane whose step is not a certain
+     * crossing waits while the others keep crossing, MCG_GRAD_WINDOW steps
+     * between two votes, and the waiting lanes take the full step together
+     * once MCG_GRAD_POOL of them wait or nothing else can step; the round
+     * lasts until MCG_GRAD_REFILL lanes have ended a pass or want a history.
+     * Every pass steps a lane, makes one wait or completes the waiting steps,
+     * and no lane passes its step limit, so it ends. */
+    auto account = [&](int c, float l, bool coll, float dep) {
+      const float2 ax = __ldg(P.aux + c);
+      /* the loss so far: G itself in the forward pass, P in the replay */
+      mcg_ff_add(P_hi, P_lo, __fmul_rn(ax.x, dep));
+      if (phase == 0) {
+        mcg_deposit<MCG_TALLY_SMEM32>(&s_tally[c], dep, qs);
+      } else {
+        /* suffix before this step, then after it */
+        const float v_after = __fadd_rn(__fsub_rn(G_hi, P_hi), __fsub_rn(G_lo, P_lo));
+        const float ga = l * (ax.x * wmc - v_after);
+        const float score = (coll ? ax.y : 0.0f) - l;
+        const float gsc = score * v_before;
+        atomicAdd(&s_ga[c], ga);
+        atomicAdd(&s_gs[c], gsc);
+        v_before = v_after;
+      }
+      ++nst;
+    };
+    auto living = [&] {
+      return active & (wmc >= min_w) & ((unsigned)idx < (unsigned)ncell) & (nst < P.max_steps);
+    };
+    for (;;) {
+      bool go = living() & !wait;
+      for (int j = 0; go & (j < MCG_GRAD_WINDOW); ++j) {
         const int c = idx;
-        const float2 ax = __ldg(P.aux + c);
         float l, dep;
-        bool coll;
-        mcg_step<STRICT, MCG_TALLY_SMEM32>(seed, x, mu, wmc, inv_mu, idx, nsc, __ldg(P.cells + c),
-                                           phase == 0 ? &s_tally[c] : nullptr, qs, T, P.libm, &l,
-                                           &coll, &dep);
-        const float g = __fmul_rn(ax.x, dep);
-        if (phase == 0) {
-          ff_add(G_hi, G_lo, g);
+        if (!mcg_cross<STRICT>(seed, x, mu, wmc, inv_mu, idx, __ldg(P.cells + c), P.b_mid, l, dep)) {
+          wait = true;
+          go = false;
         } else {
-          /* suffix before this step, then after it */
-          const float v_before = __fadd_rn(__fsub_rn(G_hi, P_hi), __fsub_rn(G_lo, P_lo));
-          ff_add(P_hi, P_lo, g);
-          const float v_after = __fadd_rn(__fsub_rn(G_hi, P_hi), __fsub_rn(G_lo, P_lo));
-          const float ga = l * (ax.x * wmc - v_after);
-          const float score = (coll ? ax.y : 0.0f) - l;
-          const float gsc = score * v_before;
-          atomicAdd(&s_ga[c], ga);
-          atomicAdd(&s_gs[c], gsc);
+          account(c, l, false, dep);
+          go = living();
         }
       }
-      nst += (uint32_t)k;
-      if (!going || nst >= P.max_steps) {
-        if ((wmc >= min_w) && ((unsigned)idx < (unsigned)ncell))
-          atomicOr(&s_cnt[MCG_CNT_ERR], 1ull); /* the step limit */
+      const unsigned wb = __ballot_sync(0xffffffffu, wait);
+      const unsigned gb = __ballot_sync(0xffffffffu, go);
+      if (wb && (!gb || __popc(wb) >= MCG_GRAD_POOL)) {
+        if (wait) {
+          const int c = idx;
+          float l, dep;
+          bool coll;
+          mcg_full<STRICT, MCG_TALLY_SMEM32>(seed, x, mu, wmc, inv_mu, idx, nsc, __ldg(P.cells + c),
+                                             nullptr, qs, T, P.libm, &l, &coll, &dep);
+          account(c, l, coll, dep);
+          wait = false;
+        }
+      } else {
+        /* ended passes, and idle lanes while the source has more */
+        const unsigned over = __ballot_sync(0xffffffffu, active ? !wait & !go : !drained);
+        if (!(wb | gb) || __popc(over) >= MCG_GRAD_REFILL)
+          break;
+      }
+    }
+    if (active & !wait & !living()) {
+      if ((wmc >= min_w) && ((unsigned)idx < (unsigned)ncell))
+        atomicOr(&s_cnt[MCG_CNT_ERR], 1ull); /* the step limit */
+      if (phase == 0) {
+        tot_steps += nst;
+        tot_scat += nsc;
+      }
+      if (phase == 0 && P.with_grad) {
+        /* replay the same history from its start */
+        born(P.first + hid, seed, x, mu, wmc, idx);
+        idx -= lo;
+        inv_mu = mcg_flight_rcp(mu);
+        nst = nsc = 0;
+        G_hi = P_hi;
+        G_lo = P_lo;
+        v_before = __fadd_rn(G_hi, G_lo);
+        P_hi = P_lo = 0.f;
+        phase = 1;
+      } else {
         if (phase == 0) {
-          tot_steps += nst;
-          tot_scat += nsc;
+          G_hi = P_hi;
+          G_lo = P_lo;
         }
-        if (phase == 0 && P.with_grad) {
-          /* replay the same history from its start */
-          mcg_source_particle(P.src, P.first + hid, seed, x, mu, wmc, idx);
-          idx -= lo;
-          inv_mu = mcg_flight_rcp(mu);
-          nst = nsc = 0;
-          phase = 1;
-        } else {
-          atomicAdd(&s_cnt[MCG_CNT_HIST], 1ull);
-          mcg_tally_add<MCG_TALLY_SMEM32>(&s_cnt[MCG_CNT_WLEFT],
-                                           mcg_to_fixed(G_hi, gs) + mcg_to_fixed(G_lo, gs));
-          active = false;
-        }
+        atomicAdd(&s_cnt[MCG_CNT_HIST], 1ull);
+        mcg_tally_add<MCG_TALLY_SMEM32>(&s_cnt[MCG_CNT_WLEFT],
+                                         mcg_to_fixed(G_hi, gs) + mcg_to_fixed(G_lo, gs));
+        active = false;
       }
     }
   }
@@ -331,20 +378,18 @@ extern "C" int mcg_adjoint_run(mcg_context *ctx, const mcg_source *src, int64_t 
   P.counters = ctx->d_counters;
   P.libm = ctx->libm;
   P.libm_tab = ctx->libm_tab;
-  P.refill_steps = ctx->refill ? ctx->refill : 8;
+  P.b_mid = ctx->run_bounds[2];
   P.chunk = 64;
   P.with_grad = with_gradient ? 1 : 0;
   P.max_steps = ctx->max_steps;
   const int block = ctx->block ? ctx->block : 512;
-  const size_t smem = sizeof(mcg_libm_tab) + 16 * 8 + 2 * (size_t)ctx->n_cells * 8;
+  size_t smem = sizeof(mcg_libm_tab) + 16 * 8 + 2 * (size_t)ctx->n_cells * 8;
   if (smem > (size_t)ctx->smem_optin)
     return mcg_fail(MCG_ERR_ARG, "mcg_adjoint_run: chain of %d cells too long (max %d)",
                     ctx->n_cells, (int)((ctx->smem_optin - 2048 - 128) / 16));
   auto kern = strict ? mcg_adjoint_kernel<true> : mcg_adjoint_kernel<false>;
-  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   int bps = 1;
-  if (e == cudaSuccess)
-    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, kern, block, smem);
+  cudaError_t e = mcg_grad_shape(kern, block, ctx->smem_optin, &smem, &P.jumps, &bps);
   if (e != cudaSuccess)
     return mcg_cuda_fail(e, "mcg_adjoint_run: launch set-up");
   long long want = (n + block - 1) / block;

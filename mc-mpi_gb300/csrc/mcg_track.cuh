@@ -665,6 +665,65 @@ __device__ __forceinline__ mcg_f2 f2_fma(mcg_f2 a, mcg_f2 b, mcg_f2 c)
  * where the exponential one fails on 1 - e^-T + 6e-5. */
 #define MCG_TILE_K (2.0f - 0x1p-20f)
 
+/* One certain crossing of a lane's particle (the gradient kernels): completes
+ * the step, with its length and deposit, when it is certainly a crossing that
+ * the tiles' forms reproduce bit for bit; otherwise changes nothing and returns
+ * false (the step is mcg_full's).  14 operations for the absorbed fraction
+ * instead of the evaluator's 17 to 40, and 3 for the collision bound. */
+template <bool STRICT>
+__device__ __forceinline__ bool mcg_cross(uint64_t &seed, float &x, float mu, float &wmc, float inv_mu,
+                                          int &idx, const float4 c, float b_mid, float &len, float &dep)
+{
+  const uint64_t s = MCG_RNG_G * seed + MCG_RNG_C;
+  const float g = __uint_as_float(0x3f800000u | ((uint32_t)(s >> 40) & 0x007fffffu));
+  const bool neg = mu < 0.0f;
+  const float edge = neg ? c.z : c.w;
+  const float a = __fsub_rn(edge, x), aa = fabsf(a);
+  bool easy = inv_mu != 0.0f;
+  float om;
+  if (STRICT) {
+    len = mcg_div_by_rcp(a, mu, inv_mu);
+    const float u = __fmul_rn(c.x, len);
+    float r;
+    om = mcg_om_mid(u, __fmul_rn(u, u), &r);
+    easy &= (aa >= 0x1p-100f) & (aa <= 0x1p100f) & (fabsf(r) < b_mid) &
+            (__float_as_uint(u) < __float_as_uint(MCG_OM_MID_MAX)) &
+            (g < __fmaf_rn(-c.y, len, MCG_TILE_K));
+  } else {
+    len = __fmul_rn(a, inv_mu);
+    const float u = __fmul_rn(c.x, len), ti = __fmul_rn(c.y, len);
+    om = fmaxf(u, ti) < 0x1p-7f ? mcg_one_minus_exp_small(-u) : mcg_one_minus_exp_fast(-u);
+    easy &= (__float_as_uint(u) < 0x3e800000u) & (g < __fsub_rn(MCG_TILE_K, ti));
+  }
+  if (!easy)
+    return false;
+  seed = s & MCG_MASK63;
+  x = edge;
+  dep = __fmul_rn(om, wmc);
+  wmc = __fsub_rn(wmc, dep);
+  idx = neg ? idx - 1 : idx + 1;
+  return true;
+}
+
+/* Rounds of the gradient kernels: certain crossings of a lane between two votes
+ * of the warp, lanes waiting for the full step that trigger it, lanes that have
+ * ended a pass or want a history that end the round.  Measured on 1000 cells and
+ * 2e6 histories (strict): windows of 2 to 16, pools of 3 to 12 and 1 to 4 lanes
+ * lie between 41.9 (these) and 48.6 ms. */
+#define MCG_GRAD_WINDOW 4
+#define MCG_GRAD_POOL 4
+#define MCG_GRAD_REFILL 1
+
+/* float-float accumulation s += v (TwoSum) */
+__device__ __forceinline__ void mcg_ff_add(float &hi, float &lo, float v)
+{
+  const float s = __fadd_rn(hi, v);
+  const float bv = __fsub_rn(s, hi);
+  const float e = __fadd_rn(__fsub_rn(hi, __fsub_rn(s, bv)), __fsub_rn(v, bv));
+  hi = s;
+  lo = __fadd_rn(lo, e);
+}
+
 /* Two steps of a flight (packed): their absorbed fractions of the weight, NaN
  * where a step is not certainly a crossing that this form reproduces bit for
  * bit.  a: lengths to the faces along x; amu, ny: |mu| and -|RN(1 / mu)|, both
@@ -1135,6 +1194,25 @@ __device__ __forceinline__ void mcg_fill_chain_jumps(mcg_chain_jumps *J)
     J->A[k] = (mcg_lcg_skip(1ull, steps, 1) - c) & MCG_MASK63;
     J->C[k] = c;
   }
+}
+
+/* Shared memory and resident blocks of a gradient kernel: the table of the seed
+ * chain (4 KB) goes after its arrays unless it does not fit or costs a block. */
+template <typename K>
+static cudaError_t mcg_grad_shape(K kern, int block, int limit, size_t *smem, int32_t *jumps, int *bps)
+{
+  const size_t more = (*smem + 7) / 8 * 8 + sizeof(mcg_chain_jumps);
+  const size_t top = more <= (size_t)limit ? more : *smem;
+  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)top);
+  if (e == cudaSuccess)
+    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(bps, kern, block, *smem);
+  int with = 0;
+  if (e == cudaSuccess && top == more)
+    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&with, kern, block, more);
+  *jumps = with > 0 && with == *bps;
+  if (*jumps)
+    *smem = more;
+  return e;
 }
 
 /* The seed chain's state n steps after s. */

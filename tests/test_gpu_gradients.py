@@ -1,0 +1,72 @@
+"""Gradient kernels: the lanes cross cells on their own and take the full steps
+together, so a history's terms are computed in rounds.  Checked at chain lengths
+and cross sections where the two kinds of step mix differently (thin cells:
+almost only crossings; thick ones: almost only full steps), at one history, a
+warp's worth and more than a block's share, with the step's weight cut-off, and
+for chains whose arrays leave no room for the seed chain's table.
+"""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+f32 = np.float32
+
+
+def _problem(m, low, high):
+    rng = np.random.default_rng(m)
+    sa, ss = (m * 10.0 ** rng.uniform(low, high, (2, m))).astype(f32)
+    return sa, ss, rng.standard_normal(m).astype(f32)
+
+
+def _ctx(mcg, mode, sa, ss, w, min_w=1e-12):
+    m = len(sa)
+    ctx = mcg.Context(mode=mode)
+    ctx.set_layers_xs([0], [m], [f32(1.0 / m)], sa, ss, min_w)
+    ctx.adjoint_set_weights(w)
+    return ctx
+
+
+@pytest.mark.parametrize("mode", ["strict", "fast"])
+@pytest.mark.parametrize("m,low,high", [(1, -2, 0), (2, -4, -2), (33, -3, 0.5), (40, -1, 0.5),
+                                        (1000, -3.5, -2), (6900, -4, -3.5)])
+@pytest.mark.parametrize("min_w", [1e-12, 0.5])
+def test_forward_pass_equals_event_mode(mcg, mode, m, low, high, min_w):
+    sa, ss, w = _problem(m, low, high)
+    with _ctx(mcg, mode, sa, ss, w, min_w) as ctx:
+        ctx.set_algorithm("event", 1)
+        for n in (1, 31, 3000):
+            ctx.tally_reset()
+            ctx.simulate_source(7, n)
+            ref, cnt = ctx.tally_q(), ctx.counters()
+            ctx.tally_reset()
+            ctx.adjoint_reset()
+            ctx.adjoint_run(7, n)
+            loss, _, _ = ctx.adjoint_read()
+            assert np.array_equal(ctx.tally_q(), ref)
+            assert [ctx.counters()[k] for k in ("steps", "scatters")] == [cnt[k] for k in ("steps", "scatters")]
+            # float-float sums of products rounded to 24 bits, over at most unit weight
+            assert abs(loss - (ctx.tally() * w).sum() / n) <= 2.0 ** -23 * np.abs(w).max()
+
+
+@pytest.mark.parametrize("mode", ["strict", "fast"])
+@pytest.mark.parametrize("m,low,high", [(1, -2, 0), (2, -4, -2), (33, -3, 0.5), (40, -1, 0.5)])
+def test_gradients_match_fp64_on_the_same_histories(mcg, oracle, mode, m, low, high):
+    """The 64-bit estimator follows the same random numbers, so all but a few
+    histories take the same path: a deposit's float32 rounding is at most about
+    1e-4 of it, and a step goes the other way in about 1e-6 of all cases, which
+    for 20000 histories of under 100 steps is two of them: sqrt(2 * 2 / 20000) =
+    1.4 % of a gradient that is all noise."""
+    n = 20000
+    sa, ss, w = _problem(m, low, high)
+    with _ctx(mcg, mode, sa, ss, w) as ctx:
+        ctx.adjoint_reset()
+        ctx.adjoint_run(0, n)
+        _, ga, gs = ctx.adjoint_read()
+    p = np.zeros(n, oracle.PARTICLE_DTYPE)
+    p["seed"] = oracle.rnd_seed_chain(5127801, n)
+    p["mu"], p["wmc"] = 1.0, 1.0
+    _, ra, rs = oracle.fp64_adjoint([oracle.layer_make(0.0, 1.0, 0, m)], sa.astype(float),
+                                    ss.astype(float), w, 1e-12, p)
+    for got, ref in ((ga, ra / n), (gs, rs / n)):
+        assert np.linalg.norm(got - ref) <= 0.05 * np.linalg.norm(ref)
