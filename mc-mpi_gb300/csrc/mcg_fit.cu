@@ -46,25 +46,24 @@ struct mcg_fit_params {
   double *grad;
   const long long *step;
   float min_w;
-  int32_t q_log2, refill_steps, with_grad;
+  int32_t q_log2, with_grad, jumps; /* jumps: the seed chain's table fits in shared memory */
   uint32_t max_steps;
 };
 
-__device__ __forceinline__ void fit_ff_add(float &hi, float &lo, float v)
-{
-  const float s = __fadd_rn(hi, v);
-  const float bv = __fsub_rn(s, hi);
-  const float e = __fadd_rn(__fsub_rn(hi, __fsub_rn(s, bv)), __fsub_rn(v, bv));
-  hi = s;
-  lo = __fadd_rn(lo, e);
-}
-
+/*
+ * Bound: instruction issue (76 % of the slots, 19 of 32 lanes), with the data
+ * pipe of the L1 at 64 % from the two atomics of a step.  Rounds, history starts
+ * and the reason for a lane per history are the adjoint kernel's.  64 slabs of up
+ * to 1024 cells, 1e5 histories each, five Adam steps: 337 ms with the full step
+ * in every lane, 272 ms so.
+ */
 __global__ void __launch_bounds__(512, 2) mcg_fit_kernel(mcg_fit_params P)
 {
   extern __shared__ __align__(16) unsigned char smem[];
   long long *s_ctl = reinterpret_cast<long long *>(smem);
   unsigned long long *s_tally = reinterpret_cast<unsigned long long *>(s_ctl + 4);
   float *s_g = reinterpret_cast<float *>(s_tally + P.max_cells);
+  mcg_chain_jumps *s_chain = reinterpret_cast<mcg_chain_jumps *>(s_g + ((P.max_cells + 1) & ~1));
   const int tid = threadIdx.x, lane = tid & 31;
   const long long step = *P.step;
   int cur = -1, m = 0;
@@ -72,7 +71,9 @@ __global__ void __launch_bounds__(512, 2) mcg_fit_kernel(mcg_fit_params P)
   const float2 *aux = nullptr;
   unsigned long long *gtally = nullptr;
   double *ggrad = nullptr;
-  mcg_libm_dev no_libm = {};
+  const mcg_libm_dev no_libm = {};
+  if (P.jumps)
+    mcg_fill_chain_jumps(s_chain);
   for (;;) {
     __syncthreads();
     if (tid == 0)
@@ -106,8 +107,14 @@ __global__ void __launch_bounds__(512, 2) mcg_fit_kernel(mcg_fit_params P)
     if (tid == 0)
       s_ctl[1] = 0;
     __syncthreads();
-    const mcg_fit_slab_dev sd = P.slabs[cur];
+    const mcg_fit_slab_dev &sd = P.slabs[cur];
     const int64_t src_base = step * sd.n_hist + it.first;
+    auto born = [&](long long h, uint64_t &seed, float &x, float &mu, float &wmc, int &idx) {
+      if (P.jumps)
+        mcg_born(s_chain, sd.src, src_base + h, seed, x, mu, wmc, idx);
+      else
+        mcg_source_particle(sd.src, src_base + h, seed, x, mu, wmc, idx);
+    };
 
     uint64_t seed = 0;
     float x = 0.f, mu = 0.f, wmc = 0.f, inv_mu = 0.f;
@@ -115,7 +122,7 @@ __global__ void __launch_bounds__(512, 2) mcg_fit_kernel(mcg_fit_params P)
     long long my_h = -1;
     uint32_t nst = 0, nsc = 0;
     float G_hi = 0.f, G_lo = 0.f, P_hi = 0.f, P_lo = 0.f;
-    bool active = false;
+    bool active = false, wait = false; /* wait: the lane's step needs the full form */
     long long pool_next = 0, pool_end = 0;
     bool drained = false;
     for (;;) {
@@ -146,7 +153,7 @@ __global__ void __launch_bounds__(512, 2) mcg_fit_kernel(mcg_fit_params P)
         }
         if (!active && my >= 0) {
           my_h = my;
-          mcg_source_particle(sd.src, src_base + my_h, seed, x, mu, wmc, idx);
+          born(my_h, seed, x, mu, wmc, idx);
           inv_mu = mcg_flight_rcp(mu);
           nst = nsc = 0;
           phase = 0;
@@ -156,36 +163,65 @@ __global__ void __launch_bounds__(512, 2) mcg_fit_kernel(mcg_fit_params P)
       }
       if (!__any_sync(0xffffffffu, active))
         break;
-      for (int k = 0; k < P.refill_steps; ++k) {
-        if (!active)
-          break;
-        if (!((wmc >= P.min_w) && (idx < m) && (idx >= 0)) || nst >= P.max_steps) {
-          if (phase == 0 && P.with_grad) {
-            mcg_source_particle(sd.src, src_base + my_h, seed, x, mu, wmc, idx);
-            inv_mu = mcg_flight_rcp(mu);
-            nst = nsc = 0;
-            phase = 1;
-            continue;
-          }
-          active = false;
-          break;
-        }
-        const int c = idx;
+      /* a round (the adjoint kernel's, mcg_adjoint.cu) */
+      auto account = [&](int c, float l, float dep) {
         const float wc = __ldg(&aux[c].x);
-        float l, dep;
-        bool coll;
-        mcg_step<false, MCG_TALLY_SMEM32>(seed, x, mu, wmc, inv_mu, idx, nsc, cells[c],
-                                          phase == 0 ? &s_tally[c] : nullptr, P.q_log2, nullptr,
-                                          no_libm, &l, &coll, &dep);
-        const float g = __fmul_rn(wc, dep);
+        mcg_ff_add(P_hi, P_lo, __fmul_rn(wc, dep));
         if (phase == 0) {
-          fit_ff_add(G_hi, G_lo, g);
+          mcg_deposit<MCG_TALLY_SMEM32>(&s_tally[c], dep, P.q_log2);
         } else {
-          fit_ff_add(P_hi, P_lo, g);
           const float v_after = __fadd_rn(__fsub_rn(G_hi, P_hi), __fsub_rn(G_lo, P_lo));
           atomicAdd(&s_g[c], l * (wc * wmc - v_after));
         }
         ++nst;
+      };
+      auto living = [&] {
+        return active & (wmc >= P.min_w) & ((unsigned)idx < (unsigned)m) & (nst < P.max_steps);
+      };
+      for (;;) {
+        bool go = living() & !wait;
+        for (int j = 0; go & (j < MCG_GRAD_WINDOW); ++j) {
+          const int c = idx;
+          float l, dep;
+          if (!mcg_cross<false>(seed, x, mu, wmc, inv_mu, idx, cells[c], 0.0f, l, dep)) {
+            wait = true;
+            go = false;
+          } else {
+            account(c, l, dep);
+            go = living();
+          }
+        }
+        const unsigned wb = __ballot_sync(0xffffffffu, wait);
+        const unsigned gb = __ballot_sync(0xffffffffu, go);
+        if (wb && (!gb || __popc(wb) >= MCG_GRAD_POOL)) {
+          if (wait) {
+            const int c = idx;
+            float l, dep;
+            bool coll;
+            mcg_full<false, MCG_TALLY_SMEM32>(seed, x, mu, wmc, inv_mu, idx, nsc, cells[c], nullptr,
+                                              P.q_log2, nullptr, no_libm, &l, &coll, &dep);
+            account(c, l, dep);
+            wait = false;
+          }
+        } else {
+          const unsigned over = __ballot_sync(0xffffffffu, active ? !wait & !go : !drained);
+          if (!(wb | gb) || __popc(over) >= MCG_GRAD_REFILL)
+            break;
+        }
+      }
+      if (active & !wait & !living()) {
+        if (phase == 0 && P.with_grad) {
+          /* replay the same history from its start */
+          born(my_h, seed, x, mu, wmc, idx);
+          inv_mu = mcg_flight_rcp(mu);
+          nst = nsc = 0;
+          G_hi = P_hi;
+          G_lo = P_lo;
+          P_hi = P_lo = 0.f;
+          phase = 1;
+        } else {
+          active = false;
+        }
       }
     }
   }
@@ -391,15 +427,11 @@ static int fit_launch_track(mcg_context *ctx, mcg_fit_state *F, int with_grad)
   P.step = F->step;
   P.min_w = F->min_w;
   P.q_log2 = ctx->log2_scale;
-  P.refill_steps = ctx->refill ? ctx->refill : 8;
   P.with_grad = with_grad;
   P.max_steps = ctx->max_steps;
-  const size_t smem = 4 * 8 + (size_t)F->max_cells * 12;
-  cudaError_t e = cudaFuncSetAttribute(mcg_fit_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       (int)smem);
+  size_t smem = 4 * 8 + (size_t)F->max_cells * 12;
   int bps = 1;
-  if (e == cudaSuccess)
-    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, mcg_fit_kernel, 512, smem);
+  cudaError_t e = mcg_grad_shape(mcg_fit_kernel, 512, ctx->smem_optin, &smem, &P.jumps, &bps);
   if (e != cudaSuccess)
     return mcg_cuda_fail(e, "mcg_fit: launch set-up");
   if ((e = cudaMemsetAsync(F->item_next, 0, 8, ctx->stream)) != cudaSuccess)

@@ -70,3 +70,36 @@ def test_gradients_match_fp64_on_the_same_histories(mcg, oracle, mode, m, low, h
                                     ss.astype(float), w, 1e-12, p)
     for got, ref in ((ga, ra / n), (gs, rs / n)):
         assert np.linalg.norm(got - ref) <= 0.05 * np.linalg.norm(ref)
+
+
+@pytest.mark.parametrize("cells,histories", [((1, 2, 33, 700), (1, 31, 9000, 20000)),
+                                             ((9000, 15000), (300, 300))])
+def test_fit_pass_equals_adjoint(mcg, cells, histories):
+    """Several slabs in one launch, one with two work items, two without room for
+    the seed chain's table: the tallies of the adjoint kernel and its gradients
+    but for the order of the float32 sums (a relative 1e-4 of the largest)."""
+    rng = np.random.default_rng(5)
+    slabs = [dict(n_cells=m, n_histories=n, base_seed=11 + m, seed_mode=0, isotropic=0, mu0=1.0,
+                  w0=1.0) for m, n in zip(cells, histories)]
+    total = sum(cells)
+    sa, ss = rng.uniform(0.2, 2, total).astype(f32), rng.uniform(0.5, 5, total).astype(f32)
+    w = rng.standard_normal(total).astype(f32)
+    with mcg.Context(mode="fast") as ctx:
+        ctx.fit_set(slabs, sa, ss, np.zeros(total), max_steps=1)
+        t, g = ctx.fit_gradient(w)
+    o = 0
+    for d in slabs:
+        m, n, k = d["n_cells"], d["n_histories"], slice(o, o + d["n_cells"])
+        o += m
+        if m > 14000:  # beyond the adjoint kernel's arrays: the tally alone
+            with mcg.Context(mode="fast") as ctx:
+                ctx.set_layers_xs([0], [m], [f32(1.0 / m)], sa[k], ss[k], 1e-12)
+                ctx.simulate_source(0, n, seed_mode=0, base_seed=d["base_seed"])
+                assert np.array_equal(t[k], ctx.tally() / n)
+            continue
+        with _ctx(mcg, "fast", sa[k], ss[k], w[k]) as ctx:
+            ctx.adjoint_reset()
+            ctx.adjoint_run(0, n, with_gradient=True, seed_mode=0, base_seed=d["base_seed"])
+            _, ref, _ = ctx.adjoint_read()
+            assert np.array_equal(t[k], ctx.tally() / n)
+        assert np.abs(g[k] - ref).max() <= 1e-4 * np.abs(ref).max()
