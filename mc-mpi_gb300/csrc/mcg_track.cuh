@@ -1349,6 +1349,108 @@ struct mcg_geometry {
   int32_t off, ncell;
 };
 
+/* A lane's history. */
+struct mcg_lane {
+  uint64_t s2 = 0; /* the state, shifted left by one */
+  float x = 0.f, mu = 0.f, wmc = 0.f, inv_mu = 0.f;
+  float wres = 0.f; /* fast: the weight's rounding residue (mcg_fast_weight_update) */
+  float2 test = {0.f, 0.f}; /* THIN: mcg_thin_tests */
+  float a0 = 0.f;   /* mcg_first_length; inf: x is the face the cell was entered by */
+  int idx = 0, off = 0, ncell = 0; /* its cell, of the range off .. off + ncell */
+  uint32_t nst = 0, nsc = 0;
+  bool wait = false; /* its step needs the full form */
+
+  __device__ __forceinline__ bool living(const mcg_rules &R) const
+  {
+    return (wmc >= R.min_w) & ((unsigned)(idx - off) < (unsigned)ncell) & (nst < R.max_steps);
+  }
+  /* x, when it is only known as a face */
+  __device__ __forceinline__ float place(const float4 *cells) const
+  {
+    return a0 != INFINITY ? x : mu < 0.0f ? __ldg(&cells[idx + 1].z) : __ldg(&cells[idx - 1].w);
+  }
+  /* A particle newly in the lane (state, x, mu, wmc, idx and range set). */
+  template <bool STRICT, bool THIN>
+  __device__ __forceinline__ void enter(const mcg_rules &R, const float4 *cells, const mcg_tab &tab)
+  {
+    a0 = 0.0f;
+    inv_mu = mcg_flight_rcp(mu);
+    wres = 0.f;
+    nst = nsc = 0;
+    if (THIN)
+      test = mcg_thin_tests<STRICT>(inv_mu, wmc, R.run);
+    if (living(R))
+      a0 = mcg_first_length(__ldg(cells + idx), __ldg(tab.cell + idx), x, mu, inv_mu, wmc);
+  }
+};
+
+/* One tile for every lane with `alive` that can; the lanes whose step needs the
+ * full form wait until pool_lanes of them do (or no other lane can step) and
+ * take it together.  Every call steps a lane, makes one wait or completes the
+ * waiting steps, if any lane is alive, and no lane passes its step limit.
+ * far (MULTI): the lane's deposits go to the global tally, the others' full
+ * steps to word[idx - word_off].  The whole warp calls. */
+template <bool STRICT, bool THIN, int TALLY, bool MULTI>
+__device__ __forceinline__ void mcg_advance(mcg_lane &p, bool alive, bool far, const float4 *cells,
+                                            const mcg_tab &tab, const mcg_sink &D,
+                                            unsigned long long *word, int word_off,
+                                            const mcg_rules &R, const mcg_tile_warp<THIN> &tiles,
+                                            const mcg_real_jumps *jumps, const mcg_libm_tab *T,
+                                            const mcg_libm_dev &libm)
+{
+  bool can = alive & !p.wait;
+  const int nmax = p.a0 == p.a0
+                       ? mcg_tile_limit(min(R.window, mcg_tile_shape<THIN>::TW), p.idx, p.off,
+                                        p.off + p.ncell, p.mu, p.wmc, R.max_steps - p.nst)
+                       : 0;
+  p.wait |= can & (nmax == 0);
+  can &= nmax != 0;
+  if (__any_sync(0xffffffffu, can)) {
+    const int dir = p.mu < 0.0f ? -1 : 1;
+    float W = __fmul_rn(p.wmc, R.run.scale), res = __fmul_rn(p.wres, R.run.scale);
+    const int k = mcg_tiles<STRICT, THIN, TALLY, MULTI>(can, p.s2, fabsf(p.mu), fabsf(p.inv_mu), p.a0,
+                                                        dir, p.idx, nmax, p.test, W, res, far, tab, D,
+                                                        tiles, R.run);
+    if (k > 0) {
+      p.s2 = jumps->A[k] * p.s2 + jumps->C[k];
+      p.wmc = __fmul_rn(W, R.run.inv_scale);
+      if (!STRICT)
+        p.wres = __fmul_rn(res, R.run.inv_scale);
+      p.idx += k * dir;
+      p.nst += (uint32_t)k;
+      p.a0 = INFINITY;
+    }
+    p.wait |= can & (k < nmax) & (p.wmc >= R.min_w);
+  }
+  const unsigned wb = __ballot_sync(0xffffffffu, p.wait);
+  if (wb && (__popc(wb) >= R.pool_lanes || !__any_sync(0xffffffffu, alive & !p.wait))) {
+    if (p.wait) {
+      p.x = p.place(cells);
+      uint64_t seed = p.s2 >> 1;
+      const int cell = p.idx;
+      float len, dep;
+      bool coll;
+      mcg_full<STRICT, TALLY>(seed, p.x, p.mu, p.wmc, p.inv_mu, p.idx, p.nsc, __ldg(cells + cell),
+                              THIN ? nullptr
+                                   : (TALLY == MCG_TALLY_GLOBAL || far ? D.global + cell
+                                                                       : word + (cell - word_off)),
+                              R.q_log2, T, libm, &len, &coll, &dep, STRICT ? nullptr : &p.wres);
+      if (THIN) {
+        mcg_lo32_add(reinterpret_cast<unsigned *>(word) + cell, D.global + cell,
+                     mcg_to_fixed(dep, R.q_log2));
+        p.test = mcg_thin_tests<STRICT>(p.inv_mu, p.wmc, R.run);
+      }
+      p.s2 = seed << 1;
+      ++p.nst;
+      p.wait = false;
+      p.a0 = (unsigned)(p.idx - p.off) < (unsigned)p.ncell
+                 ? mcg_first_length(__ldg(cells + p.idx), __ldg(tab.cell + p.idx), p.x, p.mu, p.inv_mu,
+                                    p.wmc)
+                 : 0.0f;
+    }
+  }
+}
+
 /* A warp's histories, to the end of the source: n() histories handed out by
  * *counter in chunks (mcg_pool::take).  birth(k, ...) makes history k's particle
  * with its cell index local to the chain; end(k, result, ...) sees its final
@@ -1371,25 +1473,14 @@ __device__ __forceinline__ void mcg_histories(mcg_geometry &geo, mcg_sink &D, co
                                               const N &n, int chunk, const BIRTH &birth,
                                               const END &end, const GONE &exhausted, const MORE &more)
 {
-  uint64_t s2 = 0; /* the state, shifted left by one */
-  float x = 0.f, mu = 0.f, wmc = 0.f, inv_mu = 0.f;
-  float wres = 0.f; /* fast: the weight's rounding residue (mcg_fast_weight_update) */
-  float2 test = make_float2(0.f, 0.f); /* THIN: mcg_thin_tests */
-  float a0 = 0.f;   /* mcg_first_length; inf: x is the face the cell was entered by */
-  int idx = 0;
-  int off = 0, ncell = geo.ncell; /* the history's chain: cells off .. off + ncell */
+  mcg_lane p;
   int64_t hid = -1;
-  uint32_t nst = 0, nsc = 0;
-  bool active = false, wait = false; /* wait: the lane's step needs the full form */
+  bool active = false;
   mcg_pool pool;
   bool work = true; /* MULTI: more() has not yet returned false */
-  const float min_w = R.min_w;
-  auto living = [&] {
-    return active & (wmc >= min_w) & ((unsigned)(idx - off) < (unsigned)ncell) & (nst < R.max_steps);
-  };
 
   for (;;) {
-    bool alive = living();
+    bool alive = active & p.living(R);
     const unsigned ab = __ballot_sync(0xffffffffu, alive);
     /* ended histories leave and newborns come once refill_lanes lanes are
      * without a living history, or no lane has one */
@@ -1399,22 +1490,21 @@ __device__ __forceinline__ void mcg_histories(mcg_geometry &geo, mcg_sink &D, co
       if (active & !alive) {
         /* history ends: classification of simulate_particle; a history
          * still alive in the chain here has reached the step limit */
-        const int c = idx - off;
-        const bool in = (wmc >= min_w) && ((unsigned)c < (unsigned)ncell);
+        const int c = p.idx - p.off;
+        const bool in = (p.wmc >= R.min_w) && ((unsigned)c < (unsigned)p.ncell);
         int r;
         if (in)
           r = 2;
         else if (c == -1)
           r = -1;
-        else if (c == ncell)
+        else if (c == p.ncell)
           r = 1;
-        else if (wmc < min_w)
+        else if (p.wmc < R.min_w)
           r = 0;
         else
           r = -1;
-        if (a0 == INFINITY)
-          x = mu < 0.0f ? __ldg(&cells[idx + 1].z) : __ldg(&cells[idx - 1].w);
-        end(hid, r, s2 >> 1, x, mu, wmc, wres, c, nst, nsc);
+        p.x = p.place(cells);
+        end(hid, r, p.s2 >> 1, p.x, p.mu, p.wmc, p.wres, c, p.nst, p.nsc);
         active = false;
       }
       unsigned need = __ballot_sync(0xffffffffu, !active);
@@ -1428,82 +1518,22 @@ __device__ __forceinline__ void mcg_histories(mcg_geometry &geo, mcg_sink &D, co
       if (!active && my >= 0) {
         hid = my;
         uint64_t seed;
-        birth(my, seed, x, mu, wmc, idx);
-        s2 = seed << 1;
-        off = MULTI ? geo.off : 0;
-        ncell = geo.ncell;
-        idx += off;
-        a0 = 0.0f;
-        inv_mu = mcg_flight_rcp(mu);
-        wres = 0.f;
-        nst = nsc = 0;
+        birth(my, seed, p.x, p.mu, p.wmc, p.idx);
+        p.s2 = seed << 1;
+        p.off = MULTI ? geo.off : 0;
+        p.ncell = geo.ncell;
+        p.idx += p.off;
+        p.enter<STRICT, THIN>(R, cells, tab);
         active = true;
-        alive = living();
-        if (THIN)
-          test = mcg_thin_tests<STRICT>(inv_mu, wmc, R.run);
-        if (alive)
-          a0 = mcg_first_length(__ldg(cells + idx), __ldg(tab.cell + idx), x, mu, inv_mu, wmc);
+        alive = p.living(R);
       }
       if (!__any_sync(0xffffffffu, active) && (!MULTI || !work))
         break;
     }
-
-    /* one tile for every lane that can; the lanes whose step needs the full
-     * form wait until pool_lanes of them do (or no other lane can step) and
-     * take it together.  Each pass steps a lane, makes one wait, completes
-     * the waiting steps, ends a history or hands out work, and no lane passes
-     * its step limit, so this ends. */
-    bool can = alive & !wait;
-    const bool far = MULTI && off != geo.off;
-    const int nmax = a0 == a0 ? mcg_tile_limit(min(R.window, mcg_tile_shape<THIN>::TW), idx, off,
-                                               off + ncell, mu, wmc, R.max_steps - nst)
-                              : 0;
-    wait |= can & (nmax == 0);
-    can &= nmax != 0;
-    if (__any_sync(0xffffffffu, can)) {
-      const int dir = mu < 0.0f ? -1 : 1;
-      float W = __fmul_rn(wmc, R.run.scale), res = __fmul_rn(wres, R.run.scale);
-      const int k = mcg_tiles<STRICT, THIN, TALLY, MULTI>(can, s2, fabsf(mu), fabsf(inv_mu), a0, dir,
-                                                          idx, nmax, test, W, res, far, tab, D,
-                                                          tiles, R.run);
-      if (k > 0) {
-        s2 = jumps->A[k] * s2 + jumps->C[k];
-        wmc = __fmul_rn(W, R.run.inv_scale);
-        if (!STRICT)
-          wres = __fmul_rn(res, R.run.inv_scale);
-        idx += k * dir;
-        nst += (uint32_t)k;
-        a0 = INFINITY;
-      }
-      wait |= can & (k < nmax) & (wmc >= min_w);
-    }
-    const unsigned wb = __ballot_sync(0xffffffffu, wait);
-    if (wb && (__popc(wb) >= R.pool_lanes || !__any_sync(0xffffffffu, alive & !wait))) {
-      if (wait) {
-        if (a0 == INFINITY)
-          x = mu < 0.0f ? __ldg(&cells[idx + 1].z) : __ldg(&cells[idx - 1].w);
-        uint64_t seed = s2 >> 1;
-        const int cell = idx;
-        float len, dep;
-        bool coll;
-        mcg_full<STRICT, TALLY>(seed, x, mu, wmc, inv_mu, idx, nsc, __ldg(cells + idx),
-                                THIN ? nullptr
-                                     : (TALLY == MCG_TALLY_GLOBAL || far ? D.global + idx
-                                                                         : word + (idx - geo.off)),
-                                R.q_log2, T, libm, &len, &coll, &dep, STRICT ? nullptr : &wres);
-        if (THIN) {
-          mcg_lo32_add(reinterpret_cast<unsigned *>(word) + cell, D.global + cell,
-                       mcg_to_fixed(dep, R.q_log2));
-          test = mcg_thin_tests<STRICT>(inv_mu, wmc, R.run);
-        }
-        s2 = seed << 1;
-        ++nst;
-        wait = false;
-        a0 = (unsigned)(idx - off) < (unsigned)ncell
-                 ? mcg_first_length(__ldg(cells + idx), __ldg(tab.cell + idx), x, mu, inv_mu, wmc)
-                 : 0.0f;
-      }
-    }
+    /* each pass advances a living lane, ends a history or hands out work, so
+     * this ends */
+    mcg_advance<STRICT, THIN, TALLY, MULTI>(p, alive, MULTI && p.off != geo.off, cells, tab, D, word,
+                                            geo.off, R, tiles, jumps, T, libm);
   }
 }
 

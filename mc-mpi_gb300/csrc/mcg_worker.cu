@@ -466,8 +466,7 @@ extern "C" int mcg_worker_run(mcg_context *ctx, const mcg_source *src, int64_t n
  * updated it) is all an idle warp polls, with an exponential back-off sleep
  * (up to 32 us); only when it is positive does the warp look at the rings,
  * each lane one or two rings at once, and try to claim from at most four.
- * The grid is no larger than the work needs (one 1024-thread block per 1024
- * histories).  Every loop of the kernel is bounded: a warp gives up with
+ * The grid is no larger than the work needs (a thread per history).  Every loop of the kernel is bounded: a warp gives up with
  * MCG_ERR_TIMEOUT after `idle_limit_ns` in which no history finished, and
  * every warp, busy or not, stops at the launch's deadline (`budget_ns` after
  * its start), recording how far the run got, so a run can fail but never
@@ -487,6 +486,7 @@ enum { MCG_AQ_SRC_NEXT = 0, MCG_AQ_DONE, MCG_AQ_HANDOFFS, MCG_AQ_PENDING, MCG_AQ
 
 struct mcg_async_params {
   const float4 *cells;
+  mcg_tab tab;
   int32_t n_layers, cell_lo, n_cells, src_layer;
   mcg_aq_ring *rings;
   mcg_particle *slots;          /* n_layers x cap */
@@ -495,13 +495,10 @@ struct mcg_async_params {
   mcg_source src;
   unsigned long long *state;    /* MCG_AQ_* counters */
   unsigned long long src_total;
-  int32_t refill_steps;
-  float min_w;
-  int32_t q_log2;
+  mcg_rules rules;
   unsigned long long *tally, *counters;
   mcg_libm_dev libm;
   const mcg_libm_tab *libm_tab;
-  uint32_t max_steps;
   unsigned long long idle_limit_ns, budget_ns;
   unsigned long long inflight; /* born and unfinished histories admitted */
 };
@@ -533,20 +530,37 @@ __device__ __forceinline__ unsigned long long mcg_globaltimer()
 }
 
 /* The block's own ring in shared memory: a leaver goes there while the
- * ring holds at most MCG_LQ - 1024 particles (then at most 1024 more can be
- * reserved by the block's lanes at once, so it never overfills), else to the
- * destination's global ring; idle lanes take from it first. */
-#define MCG_LQ 2048
+ * ring has room for one particle of every lane of the block besides those it
+ * holds (so it never overfills), else to the destination's global ring; idle
+ * lanes take from it first. */
+#define MCG_LQ 1024
 #define MCG_LQ_BYTES (16 + MCG_LQ * (4 + 4 + (int)sizeof(mcg_particle)))
 
-/* Rounds of the asynchronous workers: steps per lane between two warp
- * votes, lanes without a particle that end a round, longest round */
-#define MCG_AQ_WINDOW 16
-#define MCG_AQ_ROUND_IDLE 4
-#define MCG_AQ_ROUND_CAP 256
+/* Rounds of the asynchronous workers: lanes without a particle that end a
+ * round (8 to 20: within 1 % of each other; 4: 4 % slower), most tiles of a round;
+ * and most threads of a block: with 640 the shared memory of the 10,000-cell
+ * slab stays below 196 KB and leaves the tile table 60 KB of L1; 768 threads
+ * take 7 % longer, 512 9 %. */
+#define MCG_AQ_ROUND_IDLE 12
+#define MCG_AQ_ROUND_TILES 16
+#define MCG_AQ_BLOCK 640
 
-template <bool STRICT, bool SMEM, bool THIN>
-__global__ void __launch_bounds__(1024) mcg_worker_async(mcg_async_params P)
+/* Shared memory of the asynchronous workers: libm tables, the block's ring, the
+ * sub-domains' ranges, jumps, the tally (64-bit words, or low words), tiles. */
+static size_t async_smem(int layers, size_t cells, int block, bool global, bool thin)
+{
+  return mcg_track_smem(global ? 0 : cells, block, thin) + MCG_LQ_BYTES +
+         (size_t)((layers + 1) & ~1) * sizeof(int2);
+}
+
+/* TALLY and THIN as in mcg_track_kernel.  A warp advances its particles by the
+ * tracker's tiles (mcg_advance); it was one lane per particle through the whole
+ * step.  Bound: instruction issue, 80 warp instructions per step of 32 lanes (the
+ * tracker's 54, and the rows of tiles that a sub-domain's end cuts short), with
+ * the waits for the queues' global words.  10,000 cells in 64 sub-domains, 1e6
+ * histories, strict: 65.2 ms -> 34.2 ms for the call. */
+template <bool STRICT, int TALLY, bool THIN>
+__global__ void __launch_bounds__(MCG_AQ_BLOCK) mcg_worker_async(mcg_async_params P)
 {
   extern __shared__ __align__(16) unsigned char smem[];
   mcg_libm_tab *T = reinterpret_cast<mcg_libm_tab *>(smem);
@@ -557,37 +571,48 @@ __global__ void __launch_bounds__(1024) mcg_worker_async(mcg_async_params P)
   int *lq_L = reinterpret_cast<int *>(lq_seq + MCG_LQ);
   mcg_particle *lq_part = reinterpret_cast<mcg_particle *>(lq_L + MCG_LQ);
   int2 *s_rng = reinterpret_cast<int2 *>(smem + sizeof(mcg_libm_tab) + MCG_LQ_BYTES); /* [n_layers] lo, hi local */
-  unsigned long long *s_tally =
-      reinterpret_cast<unsigned long long *>(s_rng + ((P.n_layers + 1) & ~1));
+  mcg_chain_jumps *s_chain = reinterpret_cast<mcg_chain_jumps *>(s_rng + ((P.n_layers + 1) & ~1));
+  mcg_real_jumps *s_real = reinterpret_cast<mcg_real_jumps *>(s_chain + 1);
+  unsigned long long *s_tally = reinterpret_cast<unsigned long long *>(s_real + 1);
   const int tid = threadIdx.x, lane = tid & 31;
+  const int words = TALLY == MCG_TALLY_GLOBAL ? 0 : THIN ? (P.n_cells + 1) / 2 : P.n_cells;
+  mcg_tile_smem<THIN> *tile = reinterpret_cast<mcg_tile_smem<THIN> *>(
+      s_tally + ((words + 1) & ~1)) + (tid >> 5);
+  mcg_fill_chain_jumps(s_chain);
+  mcg_fill_real_jumps(s_real);
   const int gwarp = (int)((blockIdx.x * blockDim.x + tid) >> 5);
   if (STRICT)
     for (int i = tid; i < (int)(sizeof(mcg_libm_tab) / 4); i += blockDim.x)
       reinterpret_cast<float *>(T)[i] = reinterpret_cast<const float *>(P.libm_tab)[i];
   for (int l = tid; l < P.n_layers; l += blockDim.x)
     s_rng[l] = make_int2(P.rings[l].lo - P.cell_lo, P.rings[l].hi - P.cell_lo);
-  if (SMEM)
-    for (int i = tid; i < P.n_cells; i += blockDim.x)
-      s_tally[i] = 0ull;
+  for (int i = tid; i < words; i += blockDim.x)
+    s_tally[i] = 0ull;
   for (int i = tid; i < MCG_LQ; i += blockDim.x)
     lq_seq[i] = (unsigned)i; /* free for its first-lap ticket */
   if (tid < 4)
     lq_ctl[tid] = 0u;
   __syncthreads();
-  unsigned long long *tally = SMEM ? s_tally : P.tally;
-  const float min_w = P.min_w;
-  const int qs = P.q_log2;
+  const mcg_tile_warp<THIN> tiles(tile, s_real);
+  const mcg_sink sink = {(uint32_t)__cvta_generic_to_shared(s_tally), P.tally};
   const unsigned long long cap = P.cap;
   const int nl = P.n_layers;
   unsigned long long *const src_next = P.state + MCG_AQ_SRC_NEXT;
   unsigned long long *const done = P.state + MCG_AQ_DONE;
   long long *const pending = reinterpret_cast<long long *>(P.state + MCG_AQ_PENDING);
 
-  uint64_t seed = 0;
-  float x = 0.f, mu = 0.f, wmc = 0.f, inv_mu = 0.f;
-  int idx = 0, L = 0, llo = 0, lhi = 0;
-  uint32_t nst = 0, nsc = 0;
+  mcg_lane p;
+  int L = 0; /* its sub-domain: cells p.off .. p.off + p.ncell */
   bool active = false;
+  auto enter = [&](int sub, uint64_t seed) {
+    const int2 r = s_rng[sub];
+    L = sub;
+    p.s2 = seed << 1;
+    p.off = r.x;
+    p.ncell = r.y - r.x;
+    p.enter<STRICT, THIN>(P.rules, P.cells, P.tab);
+    active = true;
+  };
   unsigned long long n_hand = 0, steps = 0, scat = 0;
   unsigned long long seen_done = 0, seen_t = 0;
   /* every decision that steers the warp's control flow is taken on lane
@@ -635,13 +660,8 @@ __global__ void __launch_bounds__(1024) mcg_worker_async(mcg_async_params P)
                 const int ql = lq_L[sl];
                 __threadfence_block();
                 *(volatile unsigned *)&lq_seq[sl] = t + (unsigned)MCG_LQ; /* next lap */
-                seed = q.seed, x = q.x, mu = q.mu, wmc = q.wmc, idx = q.index - P.cell_lo;
-                L = ql;
-                llo = s_rng[ql].x;
-                lhi = s_rng[ql].y;
-                inv_mu = mcg_flight_rcp(mu);
-                nst = nsc = 0;
-                active = true;
+                p.x = q.x, p.mu = q.mu, p.wmc = q.wmc, p.idx = q.index - P.cell_lo;
+                enter(ql, q.seed);
               }
               need = __ballot_sync(0xffffffffu, !active);
             }
@@ -706,13 +726,8 @@ __global__ void __launch_bounds__(1024) mcg_worker_async(mcg_async_params P)
               atomicOr(&P.counters[MCG_CNT_ERR], 16ull);
             const mcg_particle q = P.slots[s];
             mcg_st_release(&P.seq[s], t + cap); /* free for the next lap */
-            seed = q.seed, x = q.x, mu = q.mu, wmc = q.wmc, idx = q.index - P.cell_lo;
-            L = l;
-            llo = s_rng[l].x;
-            lhi = s_rng[l].y;
-            inv_mu = mcg_flight_rcp(mu);
-            nst = nsc = 0;
-            active = true;
+            p.x = q.x, p.mu = q.mu, p.wmc = q.wmc, p.idx = q.index - P.cell_lo;
+            enter(l, q.seed);
           }
           need = __ballot_sync(0xffffffffu, !active);
         }
@@ -736,14 +751,10 @@ __global__ void __launch_bounds__(1024) mcg_worker_async(mcg_async_params P)
         base = __shfl_sync(0xffffffffu, base, 0);
         const int rank = __popc(need & lanemask_lt());
         if (((need >> lane) & 1u) && base + rank < P.src_total) {
-          mcg_source_particle(P.src, (int64_t)(base + rank), seed, x, mu, wmc, idx);
-          idx -= P.cell_lo;
-          L = P.src_layer;
-          llo = s_rng[L].x;
-          lhi = s_rng[L].y;
-          inv_mu = mcg_flight_rcp(mu);
-          nst = nsc = 0;
-          active = true;
+          uint64_t seed;
+          mcg_born(s_chain, P.src, (int64_t)(base + rank), seed, p.x, p.mu, p.wmc, p.idx);
+          p.idx -= P.cell_lo;
+          enter(P.src_layer, seed);
         }
       }
       scan = (scan + 1) % nl;
@@ -795,43 +806,31 @@ __global__ void __launch_bounds__(1024) mcg_worker_async(mcg_async_params P)
     sleep_ns = 128;
     int dir = 0;
     bool finished = false;
-    int k = 0;
-    {
-      /* the round: MCG_AQ_WINDOW steps per lane between two warp votes,
-       * until MCG_AQ_ROUND_IDLE lanes are without a particle to step, one of
-       * them newly (its particle left the sub-domain, ended, or reached the
-       * round's cap), or no lane can step: the queues are visited when
-       * there is something to hand over or to take, not every few steps */
-      const uint32_t kcap = active ? min((uint32_t)MCG_AQ_ROUND_CAP, P.max_steps - nst) : 0u;
-      for (;;) {
-        bool go = ((uint32_t)k < kcap) & (wmc >= min_w) &
-                  ((unsigned)(idx - llo) < (unsigned)(lhi - llo));
-        for (int j = 0; go & (j < MCG_AQ_WINDOW); ++j) {
-          mcg_step<STRICT, SMEM ? MCG_TALLY_SMEM32 : MCG_TALLY_GLOBAL, THIN>(
-              seed, x, mu, wmc, inv_mu, idx, nsc, __ldg(P.cells + idx), &tally[idx], qs, T,
-              P.libm);
-          ++k;
-          go = ((uint32_t)k < kcap) & (wmc >= min_w) &
-               ((unsigned)(idx - llo) < (unsigned)(lhi - llo));
-        }
-        const unsigned gb = __ballot_sync(0xffffffffu, go);
-        const unsigned fb = __ballot_sync(0xffffffffu, active & !go);
-        if (!gb || (fb && __popc(~gb) >= MCG_AQ_ROUND_IDLE))
-          break;
-      }
+    /* the round: tiles until MCG_AQ_ROUND_IDLE lanes are without a particle to
+     * step, one of them newly (its particle left the sub-domain or ended), or
+     * no lane can step: the queues are visited when there is something to
+     * hand over or to take, not every few steps */
+    bool alive = active & p.living(P.rules);
+    for (int r = 0; r < MCG_AQ_ROUND_TILES; ++r) {
+      mcg_advance<STRICT, THIN, TALLY, false>(p, alive, false, P.cells, P.tab, sink, s_tally, 0, P.rules,
+                                              tiles, s_real, T, P.libm);
+      alive = active & p.living(P.rules);
+      const unsigned gb = __ballot_sync(0xffffffffu, alive);
+      const unsigned fb = __ballot_sync(0xffffffffu, active & !alive);
+      if (!gb || (fb && __popc(~gb) >= MCG_AQ_ROUND_IDLE))
+        break;
     }
     if (active) {
-      nst += (uint32_t)k;
-      const bool going = (wmc >= min_w) & ((unsigned)(idx - llo) < (unsigned)(lhi - llo));
-      if (!going || nst >= P.max_steps) {
-        if (going)
+      if (!alive) {
+        const int c = p.idx - p.off;
+        if ((p.wmc >= P.rules.min_w) & ((unsigned)c < (unsigned)p.ncell))
           atomicOr(&P.counters[MCG_CNT_ERR], 1ull); /* the step limit */
-        else if (idx == llo - 1)
+        else if (c == -1)
           dir = L == 0 ? 0 : -1; /* the chain's ends leak (src/layer.cpp:47-48) */
-        else if (idx == lhi)
+        else if (c == p.ncell)
           dir = L == nl - 1 ? 0 : 1;
-        steps += nst;
-        scat += nsc;
+        steps += p.nst;
+        scat += p.nsc;
         finished = true;
         active = false;
       }
@@ -850,7 +849,7 @@ __global__ void __launch_bounds__(1024) mcg_worker_async(mcg_async_params P)
       }
       h = __shfl_sync(0xffffffffu, h, 0);
       e = __shfl_sync(0xffffffffu, e, 0);
-      local = e - h <= (unsigned)(MCG_LQ - 1024);
+      local = e - h <= MCG_LQ - blockDim.x;
     }
     if (local && finished && dir != 0) {
       const int leader = __ffs(movers) - 1;
@@ -867,7 +866,8 @@ __global__ void __launch_bounds__(1024) mcg_worker_async(mcg_async_params P)
         atomicOr(&P.counters[MCG_CNT_ERR], 16ull);
       } else {
         mcg_particle o;
-        o.seed = seed, o.x = x, o.mu = mu, o.wmc = wmc, o.index = idx + P.cell_lo;
+        o.seed = p.s2 >> 1, o.x = p.place(P.cells), o.mu = p.mu, o.wmc = p.wmc;
+        o.index = p.idx + P.cell_lo;
         lq_part[sl] = o;
         lq_L[sl] = L + dir;
         __threadfence_block();
@@ -889,7 +889,8 @@ __global__ void __launch_bounds__(1024) mcg_worker_async(mcg_async_params P)
         atomicOr(&P.counters[MCG_CNT_ERR], 2ull); /* the ring is full */
       } else {
         mcg_particle o;
-        o.seed = seed, o.x = x, o.mu = mu, o.wmc = wmc, o.index = idx + P.cell_lo;
+        o.seed = p.s2 >> 1, o.x = p.place(P.cells), o.mu = p.mu, o.wmc = p.wmc;
+        o.index = p.idx + P.cell_lo;
         P.slots[s] = o;
         mcg_st_release(&P.seq[s], t + 1); /* publish */
         published = true;
@@ -925,8 +926,13 @@ __global__ void __launch_bounds__(1024) mcg_worker_async(mcg_async_params P)
     atomicAdd(&P.counters[MCG_CNT_STEPS], steps);
     atomicAdd(&P.counters[MCG_CNT_SCAT], scat);
   }
-  if (SMEM) {
-    __syncthreads();
+  __syncthreads();
+  if (THIN) {
+    const unsigned *lo32 = reinterpret_cast<const unsigned *>(s_tally);
+    for (int i = tid; i < P.n_cells; i += blockDim.x)
+      if (lo32[i])
+        atomicAdd(&P.tally[i], (unsigned long long)lo32[i]);
+  } else if (TALLY != MCG_TALLY_GLOBAL) {
     for (int i = tid; i < P.n_cells; i += blockDim.x)
       if (s_tally[i])
         atomicAdd(&P.tally[i], s_tally[i]);
@@ -986,15 +992,27 @@ extern "C" int mcg_worker_run_async(mcg_context *ctx, const mcg_source *src, int
   mcg_aq_init<<<ctx->sm_count * 4, 256, 0, ctx->stream>>>(
       reinterpret_cast<unsigned long long *>(wb + o_seq), (unsigned long long)P_ * cap, cap);
 
-  const size_t smem_base =
-      sizeof(mcg_libm_tab) + MCG_LQ_BYTES + (size_t)((P_ + 1) & ~1) * sizeof(int2);
-  const bool use_smem = smem_base + (size_t)ctx->n_cells * 8 <= (size_t)ctx->smem_optin;
-  const size_t smem = smem_base + (use_smem ? (size_t)ctx->n_cells * 8 : 0);
+  /* the largest block whose tiles fit beside the tally; the global tally where
+   * not even 256 threads' do */
+  bool thin = strict ? ctx->thin : ctx->thin_fast, global = false;
+  int block = MCG_AQ_BLOCK;
+  auto smem_of = [&] { return async_smem(P_, (size_t)ctx->n_cells, block, global, thin); };
+  while (block > 256 && smem_of() > (size_t)ctx->smem_optin)
+    block -= 128;
+  if (smem_of() > (size_t)ctx->smem_optin) {
+    global = true;
+    thin = false;
+    block = MCG_AQ_BLOCK;
+    while (block > 128 && smem_of() > (size_t)ctx->smem_optin)
+      block -= 128;
+  }
+  const size_t smem = smem_of();
   if (smem > (size_t)ctx->smem_optin)
     return mcg_fail(MCG_ERR_ARG, "mcg_worker_run_async: %d sub-domains too many", P_);
   mcg_async_params A;
   memset(&A, 0, sizeof(A));
   A.cells = strict ? ctx->d_cells_strict : ctx->d_cells_fast;
+  A.tab = {ctx->d_tab + MCG_TAB_PAD, ctx->d_thin + MCG_TAB_PAD, ctx->n_cells + 2 * MCG_TAB_PAD};
   A.n_layers = P_;
   A.cell_lo = ctx->cell_lo;
   A.n_cells = ctx->n_cells;
@@ -1006,36 +1024,33 @@ extern "C" int mcg_worker_run_async(mcg_context *ctx, const mcg_source *src, int
   A.src = *src;
   A.state = state;
   A.src_total = (unsigned long long)n;
-  A.refill_steps = ctx->refill ? ctx->refill : 8;
-  A.min_w = ctx->min_w;
-  A.q_log2 = ctx->log2_scale;
+  A.rules = mcg_rules_setup(ctx, ctx->min_w, thin);
   A.tally = ctx->d_tally;
   A.counters = ctx->d_counters;
   A.libm = ctx->libm;
   A.libm_tab = ctx->libm_tab;
-  A.max_steps = ctx->max_steps;
   A.idle_limit_ns = 2000000000ull; /* 2 s without any history finishing */
   /* the launch's deadline: 30 s plus 2 us per history (the benchmark slab
    * runs a history in about 40 ns of GPU time) */
   A.budget_ns = 30000000000ull + 2000ull * (unsigned long long)n;
-  auto kern = strict ? (mcg_strict_thin(ctx) ? (use_smem ? mcg_worker_async<true, true, true>
-                                              : mcg_worker_async<true, false, true>)
-                                  : (use_smem ? mcg_worker_async<true, true, false>
-                                              : mcg_worker_async<true, false, false>))
-                     : (use_smem ? mcg_worker_async<false, true, false>
-                                 : mcg_worker_async<false, false, false>);
+  auto kern = strict ? (thin     ? mcg_worker_async<true, MCG_TALLY_LO32, true>
+                        : global ? mcg_worker_async<true, MCG_TALLY_GLOBAL, false>
+                                 : mcg_worker_async<true, MCG_TALLY_SMEM32, false>)
+                     : (thin     ? mcg_worker_async<false, MCG_TALLY_LO32, true>
+                        : global ? mcg_worker_async<false, MCG_TALLY_GLOBAL, false>
+                                 : mcg_worker_async<false, MCG_TALLY_SMEM32, false>);
   int bps = 1;
   if ((e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                 ctx->smem_optin)) != cudaSuccess ||
-      (e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, kern, 1024, smem)) != cudaSuccess)
+      (e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, kern, block, smem)) != cudaSuccess)
     return mcg_cuda_fail(e, "mcg_worker_run_async: launch set-up");
   /* no more blocks than the histories need (idle warps only poll) */
-  const long long want = std::max<long long>(1, (n + 1023) / 1024);
+  const long long want = std::max<long long>(1, (n + block - 1) / block);
   const int grid = (int)std::min<long long>((long long)ctx->sm_count * std::max(bps, 1), want);
   /* admission: a ring holds at most inflight + the grid's lanes particles,
    * so capacity - lanes histories in flight can never overflow a ring (a
    * smaller capacity still admits 32, and may overflow) */
-  const long long lanes = (long long)grid * 1024;
+  const long long lanes = (long long)grid * block;
   /* about one history per lane plus an eighth in transit: more would only
    * wait in the rings (and spill from the blocks' own rings to the global
    * ones) */
@@ -1045,7 +1060,7 @@ extern "C" int mcg_worker_run_async(mcg_context *ctx, const mcg_source *src, int
   if (!WS.monitor && (e = cudaStreamCreateWithFlags(&WS.monitor, cudaStreamNonBlocking)) != cudaSuccess)
     return mcg_cuda_fail(e, "mcg_worker_run_async: monitor stream");
   cudaEventRecord(ctx->ev0, ctx->stream);
-  kern<<<grid, 1024, smem, ctx->stream>>>(A);
+  kern<<<grid, block, smem, ctx->stream>>>(A);
   e = cudaGetLastError();
   cudaEventRecord(ctx->ev1, ctx->stream);
   if (e != cudaSuccess)

@@ -102,3 +102,27 @@ def test_batch_items_match_event_mode(mcg, mode, sizes):
             ctx.batch_run()
             assert np.array_equal(ctx.batch_tally_q(), want), (block, item, tally)
             assert ctx.counters() == counters
+
+
+@pytest.mark.parametrize("mode", ["strict", "fast"])
+@pytest.mark.parametrize("m,layers,width,n", [
+    (1, 1, 0.5, 5), (7, 7, 3.0, 2000), (20, 20, 1e-3, 120_000), (33, 2, 0.2, 700),
+    (700, 16, 1e-2, 5000), (3000, 5, 1.5e-4, 300), (16_000, 64, 1e-4, 300), (30_000, 3, 1e-4, 40)])
+def test_async_workers_match_event_mode(mcg, mode, m, layers, width, n):
+    """Sub-domains from one cell up, thin and thick chains (width: the largest
+    optical width of a cell), fewer histories than a warp has lanes and more than
+    the grid has, and chains beyond each form of the shared-memory tally."""
+    rng = np.random.default_rng(m)
+    st, lm, dx, _, _ = mcg.layer_decomposition(0.0, 1.0, m, layers)
+    sa, ss = rng.uniform(0.1, width * m / 2, (2, m)) if width * m > 0.4 else np.full((2, m), 0.1)
+    sigs = (sa + ss).astype(f32)
+    with mcg.Context(mode=mode) as ctx:
+        ctx.set_layers(st, lm, dx, sigs, (sa / sigs).astype(f32), 1e-12)
+        ctx.set_algorithm("event", 1)
+        ctx.simulate_source(0, n)
+        want, c = ctx.tally_q(), ctx.counters()
+        ctx.tally_reset()
+        ctx.worker_run_async(n)
+        assert np.array_equal(ctx.tally_q(), want)
+        got = ctx.counters()
+        assert all(got[k] == c[k] for k in ("histories", "steps", "scatters"))
