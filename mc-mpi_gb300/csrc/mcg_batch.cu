@@ -33,149 +33,12 @@
  * per-lane choice. */
 #define MCG_EXP_UNIFORM
 #include "mcg_internal.h"
-#include "mcg_track.cuh"
-
-struct mcg_batch_item {
-  int32_t slab, pad;
-  int64_t first, count;
-};
-
-struct mcg_batch_params {
-  const float4 *cells, *tab;
-  const mcg_batch_slab_dev *slabs;
-  const mcg_batch_item *items;
-  int32_t n_items;
-  int32_t max_cells;
-  unsigned long long *item_next;
-  unsigned long long *tally;
-  unsigned long long *counters;
-  mcg_libm_dev libm;
-  const mcg_libm_tab *libm_tab;
-  mcg_rules rules;
-};
-
-/* The item that a block works on (shared memory). */
-struct mcg_batch_work {
-  unsigned long long taken; /* histories handed out */
-  long long item, first, count;
-  int32_t off, m;
-  mcg_source src;
-  long long pad;
-};
-
-/* Shared memory: libm tables, counters, the item, jumps, the tally of one slab,
- * the warps' tiles. */
-static size_t batch_smem(int max_cells, int block, bool tally)
-{
-  return mcg_track_smem(tally ? max_cells : 0, block, false) + sizeof(mcg_batch_work);
-}
-static_assert(sizeof(mcg_batch_work) % 16 == 0, "the tally after it is read by 16 bytes");
+#include "mcg_batch.cuh"
 
 template <bool STRICT, int TALLY>
 __global__ void __launch_bounds__(1024) mcg_batch_kernel(mcg_batch_params P)
 {
-  extern __shared__ __align__(16) unsigned char smem[];
-  mcg_libm_tab *T = reinterpret_cast<mcg_libm_tab *>(smem);
-  unsigned long long *s_cnt = reinterpret_cast<unsigned long long *>(smem + sizeof(mcg_libm_tab));
-  mcg_batch_work *work = reinterpret_cast<mcg_batch_work *>(s_cnt + 16);
-  mcg_chain_jumps *s_chain = reinterpret_cast<mcg_chain_jumps *>(work + 1);
-  mcg_real_jumps *s_real = reinterpret_cast<mcg_real_jumps *>(s_chain + 1);
-  unsigned long long *s_tally = reinterpret_cast<unsigned long long *>(s_real + 1);
-  const int tid = threadIdx.x, lane = tid & 31;
-  mcg_fill_chain_jumps(s_chain);
-  mcg_fill_real_jumps(s_real);
-  if (STRICT) {
-    const float *src = reinterpret_cast<const float *>(P.libm_tab);
-    float *dst = reinterpret_cast<float *>(T);
-    for (int i = tid; i < (int)(sizeof(mcg_libm_tab) / 4); i += blockDim.x)
-      dst[i] = src[i];
-  }
-  if (tid < 16)
-    s_cnt[tid] = 0ull;
-  if (tid == 0)
-    work->taken = work->count = 0; /* no item: exhausted at once */
-  mcg_tile_smem<false> *tile =
-      reinterpret_cast<mcg_tile_smem<false> *>(
-          s_tally + (TALLY == MCG_TALLY_GLOBAL ? 0 : (P.max_cells + 1) & ~1)) + (tid >> 5);
-  __syncthreads();
-  const mcg_tile_warp<false> tiles(tile, s_real);
-  mcg_geometry geo = {-1, 0};
-  mcg_sink sink = {0u, P.tally};
-  auto flush = [&] {
-    if (TALLY != MCG_TALLY_GLOBAL)
-      for (int i = tid; i < geo.ncell; i += blockDim.x)
-        if (s_tally[i])
-          atomicAdd(&P.tally[geo.off + i], s_tally[i]);
-  };
-  unsigned long long tot_steps = 0, tot_scat = 0;
-  mcg_histories<STRICT, false, TALLY, true>(
-      geo, sink, P.cells, {P.tab, nullptr, 0}, s_tally, P.rules, tiles, s_real, T, P.libm,
-      &work->taken, [&] { return work->count; }, 0,
-      [&](long long my, uint64_t &seed, float &x, float &mu, float &wmc, int &idx) {
-        mcg_born(s_chain, work->src, work->first + my, seed, x, mu, wmc, idx);
-      },
-      [&](long long, int r, uint64_t, float, float, float wmc, float wres, int, uint32_t nst,
-          uint32_t nsc) {
-        mcg_count_end<STRICT>(s_cnt, r, wmc, wres, P.rules.q_log2);
-        tot_steps += nst;
-        tot_scat += nsc;
-      },
-      /* broadcast, so that the warp decides as one */
-      [&] {
-        return __shfl_sync(0xffffffffu, *(volatile unsigned long long *)&work->taken, 0) >=
-               (unsigned long long)work->count;
-      },
-      [&] {
-        /* every warp of the block comes here (each looks at the exhausted
-         * item in every round), so nothing is being added to the tally */
-        __syncthreads();
-        if (tid == 0) {
-          work->item = (long long)atomicAdd(P.item_next, 1ull);
-          work->taken = 0;
-          if (work->item < P.n_items) {
-            const mcg_batch_item it = P.items[work->item];
-            const mcg_batch_slab_dev sd = P.slabs[it.slab];
-            work->first = it.first;
-            work->count = it.count;
-            work->off = sd.cell_off;
-            work->m = sd.m;
-            work->src = sd.src;
-          }
-        }
-        __syncthreads();
-        if (work->item >= P.n_items)
-          return false;
-        if (work->off != geo.off) {
-          flush();
-          geo.off = work->off;
-          geo.ncell = work->m;
-          sink.shared = (uint32_t)__cvta_generic_to_shared(s_tally) - 8u * (uint32_t)geo.off;
-          if (TALLY != MCG_TALLY_GLOBAL) {
-            __syncthreads();
-            for (int i = tid; i < geo.ncell; i += blockDim.x)
-              s_tally[i] = 0ull;
-            __syncthreads();
-          }
-        }
-        return true;
-      });
-  __syncthreads();
-  flush();
-  for (int o = 16; o > 0; o >>= 1) {
-    tot_steps += __shfl_down_sync(0xffffffffu, tot_steps, o);
-    tot_scat += __shfl_down_sync(0xffffffffu, tot_scat, o);
-  }
-  if (lane == 0) {
-    atomicAdd(&s_cnt[MCG_CNT_STEPS], tot_steps);
-    atomicAdd(&s_cnt[MCG_CNT_SCAT], tot_scat);
-  }
-  __syncthreads();
-  if (tid < MCG_CNT_N && s_cnt[tid]) {
-    if (tid == MCG_CNT_ERR)
-      atomicOr(&P.counters[tid], s_cnt[tid]);
-    else
-      atomicAdd(&P.counters[tid], s_cnt[tid]);
-  }
+  mcg_batch_body<STRICT, TALLY, false>(P);
 }
 
 /* ------------------------------------------------------------ host side */
@@ -222,10 +85,8 @@ __global__ void mcg_batch_tables(const float4 *strict, float4 *fast, float4 *tab
   for (int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k < n;
        k += (int64_t)gridDim.x * blockDim.x) {
     const float4 c = strict[k];
-    const float sig_i = c.y > 1e-4f ? c.y : 0.0f, a = __fsub_rn(c.w, c.z);
-    const float len = a >= 0x1p-90f && a <= 0x1p90f && c.x >= 0.0f ? a : __int_as_float(0x7fc00000);
-    fast[k] = make_float4(c.x, sig_i, c.z, c.w);
-    tab[k] = make_float4(c.x, sig_i, len, len);
+    fast[k] = make_float4(c.x, c.y > 1e-4f ? c.y : 0.0f, c.z, c.w);
+    tab[k] = mcg_tile_cell(fast[k]);
   }
 }
 
@@ -286,6 +147,7 @@ extern "C" int mcg_batch_set(mcg_context *ctx, int32_t n_slabs, const mcg_slab *
       mcg_cell_params(h_sigs[off + j], h_rates[off + j], j, dx, cs[off + j], fast);
     sd[s].cell_off = (int32_t)off;
     sd[s].m = sl.n_cells;
+    sd[s].n_hist = sl.n_histories;
     sd[s].src.seed_mode = sl.seed_mode;
     sd[s].src.isotropic = sl.isotropic;
     sd[s].src.base_seed = sl.base_seed;
@@ -421,12 +283,12 @@ static int batch_configure(mcg_context *ctx, mcg_batch_state *B, int64_t item, d
    * warps' tiles would not fit; the global tally where none does.  Both
    * shared-memory modes add 64 bits at once (mcg_shared_red_if). */
   int tm = B->tally_mode;
-  if (batch_smem(B->max_cells, 256, true) > (size_t)ctx->smem_optin)
+  if (mcg_batch_smem(B->max_cells, 256, true, false) > (size_t)ctx->smem_optin)
     tm = MCG_TALLY_GLOBAL;
   L.block = B->block;
-  while (L.block > 256 && batch_smem(B->max_cells, L.block, tm != MCG_TALLY_GLOBAL) > (size_t)ctx->smem_optin)
+  while (L.block > 256 && mcg_batch_smem(B->max_cells, L.block, tm != MCG_TALLY_GLOBAL, false) > (size_t)ctx->smem_optin)
     L.block /= 2;
-  L.smem = batch_smem(B->max_cells, L.block, tm != MCG_TALLY_GLOBAL);
+  L.smem = mcg_batch_smem(B->max_cells, L.block, tm != MCG_TALLY_GLOBAL, false);
   if (strict)
     L.kern = tm == MCG_TALLY_GLOBAL ? mcg_batch_kernel<true, MCG_TALLY_GLOBAL>
                                     : mcg_batch_kernel<true, MCG_TALLY_SMEM64>;

@@ -48,8 +48,9 @@ struct mcg_batch_state {
 struct mcg_adj_state {
   float2 *d_aux = nullptr;               /* {w_c, 1/sig_s} per chain cell */
   unsigned long long *d_grad = nullptr;  /* grad_a[n], grad_s[n], loss */
+  float2 *d_sum = nullptr;               /* `sums` histories' losses (forward -> replay) */
   int n = 0;
-  int64_t histories = 0;
+  int64_t sums = 0, histories = 0;
   int g_log2 = 36;
 };
 
@@ -92,6 +93,7 @@ struct mcg_ev_ctl {
 /* One slab of the batched form (and of the event engine's slab mode). */
 struct mcg_batch_slab_dev {
   int32_t cell_off, m;
+  int64_t n_hist;
   mcg_source src;
 };
 

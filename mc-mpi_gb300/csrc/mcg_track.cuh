@@ -32,6 +32,7 @@ struct mcg_tab {
   const float4 *cell;
   const float2 *thin;
   int32_t left;
+  const float2 *aux; /* LOSS: {w_c, .}, readable as far */
 };
 
 /* How a warp runs its histories (mcg_histories). */
@@ -589,6 +590,11 @@ template <bool THIN> struct mcg_tile_smem {
   float step[2 * mcg_tile_shape<THIN>::PLANE];
 };
 
+/* LOSS (not THIN): and the loss weight of each step's cell. */
+struct mcg_loss_smem : mcg_tile_smem<false> {
+  float weight[2 * mcg_tile_shape<false>::PLANE];
+};
+
 /* Jumps of the sample stream in the shifted representation (state << 1, so the
  * modulus is the word's): s -> A s + C after k steps. */
 struct mcg_real_jumps {
@@ -707,10 +713,11 @@ __device__ __forceinline__ bool mcg_cross(uint64_t &seed, float &x, float mu, fl
 
 /* Rounds of the gradient kernels: certain crossings of a lane between two votes
  * of the warp, lanes waiting for the full step that trigger it, lanes that have
- * ended a pass or want a history that end the round.  Measured on 1000 cells and
- * 2e6 histories (strict): windows of 2 to 16, pools of 3 to 12 and 1 to 4 lanes
- * lie between 41.9 (these) and 48.6 ms. */
-#define MCG_GRAD_WINDOW 4
+ * ended a pass or want a history that end the round.  1000 cells, 2e6 histories:
+ * windows of 1 to 8 and pools of 2 to 8 lie within 4 % of these, pools of 1 or 12
+ * are 6 to 13 % slower.  Long windows with small pools let colliding histories fall
+ * behind, and the gradients' float sums notice (mcg_adjoint_fused). */
+#define MCG_GRAD_WINDOW 2
 #define MCG_GRAD_POOL 4
 #define MCG_GRAD_REFILL 1
 
@@ -854,7 +861,7 @@ __device__ __forceinline__ uint32_t mcg_shared_add_if(bool p, uint32_t addr, uin
  * rows: 4 passes in flight instead of 1 took the 10,000-cell slab from 131 to
  * 110 ms per 5e6 histories (the table's L1 misses).  Rows past the last flight
  * are computed and never used. */
-template <bool STRICT, bool THIN, int U>
+template <bool STRICT, bool THIN, int U, bool LOSS>
 __device__ __forceinline__ void mcg_tile_form(mcg_tile_smem<THIN> *S, int q0, const mcg_tab &tab,
                                               const mcg_tile_warp<THIN> &B,
                                               const mcg_run_consts &R)
@@ -865,7 +872,7 @@ __device__ __forceinline__ void mcg_tile_form(mcg_tile_smem<THIN> *S, int q0, co
   int4 pl[U];
   uint4 fl[U];
   ulonglong2 sl[U];
-  float a[U], b[U], sa0[U], sa1[U], si0[U], si1[U], om0[U], om1[U];
+  float a[U], b[U], sa0[U], sa1[U], si0[U], si1[U], om0[U], om1[U], w0[U], w1[U];
 #pragma unroll
   for (int v = 0; v < U; ++v)
     pl[v] = S->place[F * (q0 + v) + sub];
@@ -881,6 +888,10 @@ __device__ __forceinline__ void mcg_tile_form(mcg_tile_smem<THIN> *S, int q0, co
       const float4 c = __ldg(p), d = __ldg(p + G * pl[v].z);
       sa0[v] = c.x, sa1[v] = d.x, si0[v] = c.y, si1[v] = d.y;
       a[v] = pl[v].z < 0 ? c.w : c.z, b[v] = pl[v].z < 0 ? d.w : d.z;
+      if (LOSS) {
+        const float2 *w = tab.aux + (pl[v].y + j * pl[v].z);
+        w0[v] = __ldg(&w->x), w1[v] = __ldg(&(w + G * pl[v].z)->x);
+      }
     }
 #pragma unroll
   for (int v = 0; v < U; ++v) {
@@ -902,6 +913,11 @@ __device__ __forceinline__ void mcg_tile_form(mcg_tile_smem<THIN> *S, int q0, co
   for (int v = 0; v < U; ++v) {
     S->step[33 * (q0 + v) + lane] = om0[v];
     S->step[PLANE + 33 * (q0 + v) + lane] = om1[v];
+    if (LOSS) {
+      float *w = static_cast<mcg_loss_smem *>((mcg_tile_smem<false> *)S)->weight;
+      w[33 * (q0 + v) + lane] = w0[v];
+      w[PLANE + 33 * (q0 + v) + lane] = w1[v];
+    }
   }
 }
 
@@ -1042,12 +1058,14 @@ __device__ __forceinline__ void mcg_tile_cut(const float *st, int &n, float &W, 
  * number; a0: length to the first face when the flight starts inside the cell,
  * else infinity; W is the weight times the tally scale, res (fast) its
  * residue; test: mcg_thin_tests (THIN); far (MULTI): this flight's deposits go
- * to the global tally.  idx indexes tab, the tile table, and the tallies. */
-template <bool STRICT, bool THIN, int TALLY, bool MULTI>
+ * to the global tally.  idx indexes tab, the tile table, and the tallies.  LOSS:
+ * adds w_c dep of every step to the float-float sum (G_hi, G_lo), in order; res
+ * is left alone. */
+template <bool STRICT, bool THIN, int TALLY, bool MULTI, bool LOSS>
 __device__ __forceinline__ int mcg_tiles(bool can, uint64_t s2, float amu, float ainv, float a0,
                                          int dir, int idx, int nmax, float2 test, float &W,
-                                         float &res, bool far, const mcg_tab &tab,
-                                         const mcg_sink &D, const mcg_tile_warp<THIN> &B,
+                                         float &res, float &G_hi, float &G_lo, bool far,
+                                         const mcg_tab &tab, const mcg_sink &D, const mcg_tile_warp<THIN> &B,
                                          const mcg_run_consts &R)
 {
   constexpr int G = mcg_tile_shape<THIN>::G, TW = 2 * G, F = 32 / G;
@@ -1067,9 +1085,9 @@ __device__ __forceinline__ int mcg_tiles(bool can, uint64_t s2, float amu, float
   int q = 0;
   if (THIN)
     for (; F * (q + 2) < cnt; q += 4)
-      mcg_tile_form<STRICT, THIN, 4>(S, q, tab, B, R);
+      mcg_tile_form<STRICT, THIN, 4, LOSS>(S, q, tab, B, R);
   for (; F * q < cnt; q += 2)
-    mcg_tile_form<STRICT, THIN, 2>(S, q, tab, B, R);
+    mcg_tile_form<STRICT, THIN, 2, LOSS>(S, q, tab, B, R);
   __syncwarp();
   int n = 0;
   if (can) {
@@ -1109,6 +1127,10 @@ __device__ __forceinline__ int mcg_tiles(bool can, uint64_t s2, float amu, float
       S->place[rank] = make_int4(0, idx, dir, n); /* phase 4: the cell, of either direction */
     } else {
       bool ok = true;
+      const float *wt = nullptr;
+      const float G0_hi = G_hi, G0_lo = G_lo;
+      if (LOSS)
+        wt = static_cast<mcg_loss_smem *>((mcg_tile_smem<false> *)S)->weight + (st - S->step);
 #pragma unroll
       for (int i = 0; i < TW; ++i) {
         float *si = st + (i / G) * PLANE + i % G;
@@ -1116,14 +1138,26 @@ __device__ __forceinline__ int mcg_tiles(bool can, uint64_t s2, float amu, float
         ok &= dv < 0x1p62f; /* false for NaN */
         if (ok) {
           const float w2 = __fsub_rn(W, dv);
-          if (!STRICT)
+          if (!STRICT && !LOSS)
             res = __fadd_rn(res, __fsub_rn(__fsub_rn(W, w2), dv));
           W = w2;
           *si = dv;
           n = i + 1;
+          if (LOSS)
+            mcg_ff_add(G_hi, G_lo,
+                       __fmul_rn(wt[(i / G) * PLANE + i % G], __fmul_rn(dv, R.inv_scale)));
         }
       }
+      const bool cut = W < R.min_w;
       mcg_tile_cut<STRICT, THIN>(st, n, W, res, W0, res0, R.min_w);
+      if (LOSS && cut) {
+        G_hi = G0_hi;
+        G_lo = G0_lo;
+        for (int i = 0; i < n; ++i) {
+          const int at = (i / G) * PLANE + i % G;
+          mcg_ff_add(G_hi, G_lo, __fmul_rn(wt[at], __fmul_rn(st[at], R.inv_scale)));
+        }
+      }
       S->place[rank] = make_int4(MULTI && far, idx, dir, n);
     }
   }
@@ -1358,6 +1392,7 @@ struct mcg_lane {
   float a0 = 0.f;   /* mcg_first_length; inf: x is the face the cell was entered by */
   int idx = 0, off = 0, ncell = 0; /* its cell, of the range off .. off + ncell */
   uint32_t nst = 0, nsc = 0;
+  float G_hi = 0.f, G_lo = 0.f; /* LOSS: sum of w_c dep */
   bool wait = false; /* its step needs the full form */
 
   __device__ __forceinline__ bool living(const mcg_rules &R) const
@@ -1377,6 +1412,7 @@ struct mcg_lane {
     inv_mu = mcg_flight_rcp(mu);
     wres = 0.f;
     nst = nsc = 0;
+    G_hi = G_lo = 0.f;
     if (THIN)
       test = mcg_thin_tests<STRICT>(inv_mu, wmc, R.run);
     if (living(R))
@@ -1390,7 +1426,7 @@ struct mcg_lane {
  * waiting steps, if any lane is alive, and no lane passes its step limit.
  * far (MULTI): the lane's deposits go to the global tally, the others' full
  * steps to word[idx - word_off].  The whole warp calls. */
-template <bool STRICT, bool THIN, int TALLY, bool MULTI>
+template <bool STRICT, bool THIN, int TALLY, bool MULTI, bool LOSS = false>
 __device__ __forceinline__ void mcg_advance(mcg_lane &p, bool alive, bool far, const float4 *cells,
                                             const mcg_tab &tab, const mcg_sink &D,
                                             unsigned long long *word, int word_off,
@@ -1408,9 +1444,9 @@ __device__ __forceinline__ void mcg_advance(mcg_lane &p, bool alive, bool far, c
   if (__any_sync(0xffffffffu, can)) {
     const int dir = p.mu < 0.0f ? -1 : 1;
     float W = __fmul_rn(p.wmc, R.run.scale), res = __fmul_rn(p.wres, R.run.scale);
-    const int k = mcg_tiles<STRICT, THIN, TALLY, MULTI>(can, p.s2, fabsf(p.mu), fabsf(p.inv_mu), p.a0,
-                                                        dir, p.idx, nmax, p.test, W, res, far, tab, D,
-                                                        tiles, R.run);
+    const int k = mcg_tiles<STRICT, THIN, TALLY, MULTI, LOSS>(
+        can, p.s2, fabsf(p.mu), fabsf(p.inv_mu), p.a0, dir, p.idx, nmax, p.test, W, res, p.G_hi, p.G_lo,
+        far, tab, D, tiles, R.run);
     if (k > 0) {
       p.s2 = jumps->A[k] * p.s2 + jumps->C[k];
       p.wmc = __fmul_rn(W, R.run.inv_scale);
@@ -1434,7 +1470,10 @@ __device__ __forceinline__ void mcg_advance(mcg_lane &p, bool alive, bool far, c
                               THIN ? nullptr
                                    : (TALLY == MCG_TALLY_GLOBAL || far ? D.global + cell
                                                                        : word + (cell - word_off)),
-                              R.q_log2, T, libm, &len, &coll, &dep, STRICT ? nullptr : &p.wres);
+                              R.q_log2, T, libm, &len, &coll, &dep,
+                              STRICT || LOSS ? nullptr : &p.wres);
+      if (LOSS)
+        mcg_ff_add(p.G_hi, p.G_lo, __fmul_rn(__ldg(&tab.aux[cell].x), dep));
       if (THIN) {
         mcg_lo32_add(reinterpret_cast<unsigned *>(word) + cell, D.global + cell,
                      mcg_to_fixed(dep, R.q_log2));
@@ -1453,8 +1492,8 @@ __device__ __forceinline__ void mcg_advance(mcg_lane &p, bool alive, bool far, c
 
 /* A warp's histories, to the end of the source: n() histories handed out by
  * *counter in chunks (mcg_pool::take).  birth(k, ...) makes history k's particle
- * with its cell index local to the chain; end(k, result, ...) sees its final
- * state.  cells and tab are the chain's, word its shared-memory tally (base
+ * with its cell index local to the chain and returns its number; end(number,
+ * result, p, cell) sees its final state.  cells and tab are the chain's, word its shared-memory tally (base
  * of mcg_sink D) as a pointer.  The whole warp calls.
  *
  * MULTI: cells, tab and the global tally are those of all slabs; when a slab's
@@ -1463,8 +1502,8 @@ __device__ __forceinline__ void mcg_advance(mcg_lane &p, bool alive, bool far, c
  * warps keep the histories they have: such a history stays in its lane, with
  * its own slab's cells, and its deposits go to the global tally.  So no warp
  * waits for another's longest history. */
-template <bool STRICT, bool THIN, int TALLY, bool MULTI, class N, class BIRTH, class END, class GONE,
-          class MORE>
+template <bool STRICT, bool THIN, int TALLY, bool MULTI, bool LOSS, class N, class BIRTH, class END,
+          class GONE, class MORE>
 __device__ __forceinline__ void mcg_histories(mcg_geometry &geo, mcg_sink &D, const float4 *cells,
                                               const mcg_tab &tab, unsigned long long *word,
                                               const mcg_rules &R, const mcg_tile_warp<THIN> &tiles,
@@ -1504,7 +1543,7 @@ __device__ __forceinline__ void mcg_histories(mcg_geometry &geo, mcg_sink &D, co
         else
           r = -1;
         p.x = p.place(cells);
-        end(hid, r, p.s2 >> 1, p.x, p.mu, p.wmc, p.wres, c, p.nst, p.nsc);
+        end(hid, r, p, c);
         active = false;
       }
       unsigned need = __ballot_sync(0xffffffffu, !active);
@@ -1516,9 +1555,8 @@ __device__ __forceinline__ void mcg_histories(mcg_geometry &geo, mcg_sink &D, co
         pool.drained = true;
       const long long my = need ? pool.take(need, counter, n(), chunk) : -1;
       if (!active && my >= 0) {
-        hid = my;
         uint64_t seed;
-        birth(my, seed, p.x, p.mu, p.wmc, p.idx);
+        hid = birth(my, seed, p.x, p.mu, p.wmc, p.idx);
         p.s2 = seed << 1;
         p.off = MULTI ? geo.off : 0;
         p.ncell = geo.ncell;
@@ -1532,7 +1570,7 @@ __device__ __forceinline__ void mcg_histories(mcg_geometry &geo, mcg_sink &D, co
     }
     /* each pass advances a living lane, ends a history or hands out work, so
      * this ends */
-    mcg_advance<STRICT, THIN, TALLY, MULTI>(p, alive, MULTI && p.off != geo.off, cells, tab, D, word,
+    mcg_advance<STRICT, THIN, TALLY, MULTI, LOSS>(p, alive, MULTI && p.off != geo.off, cells, tab, D, word,
                                             geo.off, R, tiles, jumps, T, libm);
   }
 }
@@ -1574,7 +1612,7 @@ __global__ void __launch_bounds__(THIN ? MCG_THIN_BLOCK : 1024) mcg_track_kernel
   mcg_geometry geo = {0, ncell};
   mcg_sink sink = {(uint32_t)__cvta_generic_to_shared(my_tally), P.tally};
   unsigned long long tot_steps = 0, tot_scat = 0;
-  mcg_histories<STRICT, THIN, TALLY, false>(
+  mcg_histories<STRICT, THIN, TALLY, false, false>(
       geo, sink, P.cells, P.tab, my_tally, P.rules, tiles, s_real, T, P.libm, P.next,
       [&] { return (long long)P.n; }, P.chunk,
       [&](long long my, uint64_t &seed, float &x, float &mu, float &wmc, int &idx) {
@@ -1583,26 +1621,26 @@ __global__ void __launch_bounds__(THIN ? MCG_THIN_BLOCK : 1024) mcg_track_kernel
         else
           mcg_born(s_chain, P.src, P.first + my, seed, x, mu, wmc, idx);
         idx -= lo;
+        return my;
       },
-      [&](long long hid, int r, uint64_t seed, float x, float mu, float wmc, float wres, int idx,
-          uint32_t nst, uint32_t nsc) {
-        if (P.particles && nst) { /* without a step the particle stays as it is */
+      [&](long long hid, int r, const mcg_lane &p, int idx) {
+        if (P.particles && p.nst) { /* without a step the particle stays as it is */
           unsigned long long *q = reinterpret_cast<unsigned long long *>(P.particles + hid);
-          q[0] = seed;
-          q[1] = (unsigned long long)__float_as_uint(x) |
-                 ((unsigned long long)__float_as_uint(mu) << 32);
-          q[2] = (unsigned long long)__float_as_uint(wmc) |
+          q[0] = p.s2 >> 1;
+          q[1] = (unsigned long long)__float_as_uint(p.x) |
+                 ((unsigned long long)__float_as_uint(p.mu) << 32);
+          q[2] = (unsigned long long)__float_as_uint(p.wmc) |
                  ((unsigned long long)(uint32_t)(idx + lo) << 32);
         }
         if (P.results)
           P.results[hid] = r;
         if (P.steps)
-          P.steps[hid] = nst;
+          P.steps[hid] = p.nst;
         if (P.scatters)
-          P.scatters[hid] = nsc;
-        mcg_count_end<STRICT>(s_cnt, r, wmc, wres, P.rules.q_log2);
-        tot_steps += nst;
-        tot_scat += nsc;
+          P.scatters[hid] = p.nsc;
+        mcg_count_end<STRICT>(s_cnt, r, p.wmc, p.wres, P.rules.q_log2);
+        tot_steps += p.nst;
+        tot_scat += p.nsc;
       },
       [] { return true; }, [] { return false; });
 

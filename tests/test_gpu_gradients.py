@@ -50,13 +50,14 @@ def test_forward_pass_equals_event_mode(mcg, mode, m, low, high, min_w):
 
 
 @pytest.mark.parametrize("mode", ["strict", "fast"])
-@pytest.mark.parametrize("m,low,high", [(1, -2, 0), (2, -4, -2), (33, -3, 0.5), (40, -1, 0.5)])
+@pytest.mark.parametrize("m,low,high", [(1, -2, 0), (2, -4, -2), (33, -3, 0.5), (40, -1, 0.5),
+                                        (256, -3, -1.5), (257, -3, -1.5), (400, -2, 0.5)])
 def test_gradients_match_fp64_on_the_same_histories(mcg, oracle, mode, m, low, high):
     """The 64-bit estimator follows the same random numbers, so all but a few
     histories take the same path: a deposit's float32 rounding is at most about
     1e-4 of it, and a step goes the other way in about 1e-6 of all cases, which
-    for 20000 histories of under 100 steps is two of them: sqrt(2 * 2 / 20000) =
-    1.4 % of a gradient that is all noise."""
+    for 20000 histories of under 500 steps is ten of them: sqrt(2 * 10 / 20000) =
+    3.2 % of a gradient that is all noise."""
     n = 20000
     sa, ss, w = _problem(m, low, high)
     with _ctx(mcg, mode, sa, ss, w) as ctx:
@@ -70,6 +71,28 @@ def test_gradients_match_fp64_on_the_same_histories(mcg, oracle, mode, m, low, h
                                     ss.astype(float), w, 1e-12, p)
     for got, ref in ((ga, ra / n), (gs, rs / n)):
         assert np.linalg.norm(got - ref) <= 0.05 * np.linalg.norm(ref)
+
+
+def test_more_histories_than_one_part(mcg):
+    """Above 2^24 histories the forward pass and the replay take turns: the sums
+    over two shorter runs, and the tracker's tally."""
+    m, n = 257, (1 << 24) + 777
+    sa, ss, w = _problem(m, -2, -1)
+    with _ctx(mcg, "fast", sa, ss, w) as ctx:
+        ctx.simulate_source(0, n)
+        ref = ctx.tally_q()
+        out = []
+        for cuts in ((0, n), (0, 9_000_000, n)):
+            ctx.tally_reset()
+            ctx.adjoint_reset()
+            for a, b in zip(cuts, cuts[1:]):
+                ctx.adjoint_run(a, b - a)
+            out.append(ctx.adjoint_read())
+            assert np.array_equal(ctx.tally_q(), ref)
+    (la, a0, s0), (lb, a1, s1) = out
+    assert la == lb
+    for x, y in ((a0, a1), (s0, s1)):
+        assert np.abs(x - y).max() <= 1e-3 * np.abs(y).max()
 
 
 @pytest.mark.parametrize("cells,histories", [((1, 2, 33, 700), (1, 31, 9000, 20000)),
