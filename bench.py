@@ -548,10 +548,14 @@ def bench_fit(mcg, device, scale=1.0, n_steps=200):
         ms = ctx.last_kernel_ms()
         sig, loss = ctx.fit_read()
     hist = n_steps * sum(d["n_histories"] for d in slabs)
+    # a step: forward pass and replay (in turns of 2048 items of 8192
+    # histories), the weights and the Adam update
+    items = sum(-(-d["n_histories"] // 8192) for d in slabs)
+    per_step = 2 * -(-items // 2048) + 2
     err0 = float(np.linalg.norm(1.0 - hidden) / np.linalg.norm(hidden))
     err = float(np.linalg.norm(sig - hidden) / np.linalg.norm(hidden))
     return {"value": hist / (ms / 1e3), "unit": "histories/s", "adam_steps": n_steps,
-            "histories": hist, "ms_per_adam_step": ms / n_steps, "gpu_launches": 3 * n_steps,
+            "histories": hist, "ms_per_adam_step": ms / n_steps, "gpu_launches": per_step * n_steps,
             "rel_l2_error": err, "rel_l2_error_start": err0, "loss_first": float(loss[0]),
             "loss_last": float(loss[-1]), "mode": "fast",
             "workload": f"configuration 4: 64 slabs, cells U{{64..1024}}, hidden "

@@ -5,15 +5,14 @@
  * cross sections and measured absorption tallies t_c (weight absorbed per
  * history); the fit minimises L = sum over all cells of (a_c - t_c)^2, a_c the
  * simulated tally, over every cell's sig_a by Adam.  One Adam step is:
- *   1. one launch of the batched forward + adjoint kernel: each lane runs a
- *      history of its work item's slab forward (tally + G = sum w_c dep)
- *      and replays it from its seed accumulating dG/dsig_a (the pathwise
- *      derivative of mcg_adjoint.cu); the loss weights are
+ *   1. the batched forward pass (tally + G = sum w_c dep of every history) and
+ *      the replay of every history from its seed accumulating dG/dsig_a (the
+ *      pathwise derivative of mcg_adjoint.cu); the loss weights are
  *      w_c = 2 (a_c - t_c) from the previous step's tally (lagged by one
- *      step, so a single pass per step suffices);
+ *      step, so one set of histories per step suffices);
  *   2. a kernel forming the new weights and the loss from this step's tally;
  *   3. the Adam update of every sig_a, written straight into the step table.
- * The three kernels are captured once in a CUDA graph and replayed for every
+ * The kernels are captured once in a CUDA graph and replayed for every
  * step; each step simulates fresh histories (source indices step * n + i).
  */
 #include <algorithm>
@@ -22,168 +21,130 @@
 #include <vector>
 
 #include "mcg_internal.h"
-#include "mcg_track.cuh"
-
-struct mcg_fit_slab_dev {
-  int32_t cell_off, m;
-  int64_t n_hist;
-  mcg_source src;
-};
-
-struct mcg_fit_item {
-  int32_t slab, pad;
-  int64_t first, count;
-};
+#include "mcg_batch.cuh"
 
 struct mcg_fit_params {
-  float4 *cells;  /* fast step table; .x = sig_a, updated by the Adam kernel */
-  float2 *aux;    /* {w_c, unused} */
-  const mcg_fit_slab_dev *slabs;
-  const mcg_fit_item *items;
+  const float4 *cells;  /* fast step table; .x = sig_a, updated by the Adam kernel */
+  const float2 *aux;    /* {w_c, unused} */
+  const mcg_batch_slab_dev *slabs;
+  const mcg_batch_item *items;
   int32_t n_items, max_cells;
   unsigned long long *item_next;
-  unsigned long long *tally;
+  const float2 *sum; /* the forward pass's losses (mcg_batch_params::loss) */
   double *grad;
   const long long *step;
   float min_w;
-  int32_t q_log2, with_grad, jumps; /* jumps: the seed chain's table fits in shared memory */
+  int32_t q_log2, jumps; /* jumps: the seed chain's table fits in shared memory */
   uint32_t max_steps;
 };
 
+/* Forward pass: the batched tracker with the losses.  64 slabs of up to 1024
+ * cells, 1e5 histories each: 17.5 ms; 24 ms with a lane per history. */
+__global__ void __launch_bounds__(1024) mcg_fit_forward(mcg_batch_params P)
+{
+  mcg_batch_body<false, MCG_TALLY_SMEM64, true>(P);
+}
+
 /*
- * Bound: instruction issue (76 % of the slots, 19 of 32 lanes), with the data
- * pipe of the L1 at 64 % from the two atomics of a step.  Rounds, history starts
- * and the reason for a lane per history are the adjoint kernel's.  64 slabs of up
- * to 1024 cells, 1e5 histories each, five Adam steps: 337 ms with the full step
- * in every lane, 272 ms so.
+ * Replay of every history for dG/dsig_a: rounds, history starts and the reason
+ * for a lane per history are those of the adjoint's replay.  Bound: instruction
+ * issue, with the float atomics' compare-and-swap loops.  64 slabs of up to 1024
+ * cells, 1e5 histories each: 26 ms.  Five Adam steps, with the forward pass that
+ * starts them: 337 ms with forward pass and replay in one kernel of full steps,
+ * 235 ms so.
  */
-__global__ void __launch_bounds__(512, 2) mcg_fit_kernel(mcg_fit_params P)
+__global__ void __launch_bounds__(512, 2) mcg_fit_replay(mcg_fit_params P)
 {
   extern __shared__ __align__(16) unsigned char smem[];
   long long *s_ctl = reinterpret_cast<long long *>(smem);
-  unsigned long long *s_tally = reinterpret_cast<unsigned long long *>(s_ctl + 4);
-  float *s_g = reinterpret_cast<float *>(s_tally + P.max_cells);
+  float *s_g = reinterpret_cast<float *>(s_ctl + 4);
   mcg_chain_jumps *s_chain = reinterpret_cast<mcg_chain_jumps *>(s_g + ((P.max_cells + 1) & ~1));
-  const int tid = threadIdx.x, lane = tid & 31;
+  const int tid = threadIdx.x;
   const long long step = *P.step;
   int cur = -1, m = 0;
   const float4 *cells = nullptr;
   const float2 *aux = nullptr;
-  unsigned long long *gtally = nullptr;
   double *ggrad = nullptr;
   const mcg_libm_dev no_libm = {};
   if (P.jumps)
     mcg_fill_chain_jumps(s_chain);
+  auto flush = [&] {
+    if (cur >= 0)
+      for (int i = tid; i < m; i += blockDim.x)
+        if (s_g[i] != 0.0f)
+          atomicAdd(&ggrad[i], (double)s_g[i]);
+  };
   for (;;) {
     __syncthreads();
-    if (tid == 0)
+    if (tid == 0) {
       s_ctl[0] = (long long)atomicAdd(P.item_next, 1ull);
+      s_ctl[1] = 0;
+    }
     __syncthreads();
     const long long item = s_ctl[0];
     if (item >= P.n_items)
       break;
-    const mcg_fit_item it = P.items[item];
+    const mcg_batch_item it = P.items[item];
+    const mcg_batch_slab_dev &sd = P.slabs[it.slab];
     if (it.slab != cur) {
-      if (cur >= 0)
-        for (int i = tid; i < m; i += blockDim.x) {
-          if (s_tally[i])
-            atomicAdd(&gtally[i], s_tally[i]);
-          if (s_g[i] != 0.0f)
-            atomicAdd(&ggrad[i], (double)s_g[i]);
-        }
+      flush();
       __syncthreads();
       cur = it.slab;
-      const mcg_fit_slab_dev sd = P.slabs[cur];
       m = sd.m;
       cells = P.cells + sd.cell_off;
       aux = P.aux + sd.cell_off;
-      gtally = P.tally + sd.cell_off;
       ggrad = P.grad + sd.cell_off;
-      for (int i = tid; i < m; i += blockDim.x) {
-        s_tally[i] = 0ull;
+      for (int i = tid; i < m; i += blockDim.x)
         s_g[i] = 0.0f;
-      }
+      __syncthreads();
     }
-    if (tid == 0)
-      s_ctl[1] = 0;
-    __syncthreads();
-    const mcg_fit_slab_dev &sd = P.slabs[cur];
     const int64_t src_base = step * sd.n_hist + it.first;
-    auto born = [&](long long h, uint64_t &seed, float &x, float &mu, float &wmc, int &idx) {
-      if (P.jumps)
-        mcg_born(s_chain, sd.src, src_base + h, seed, x, mu, wmc, idx);
-      else
-        mcg_source_particle(sd.src, src_base + h, seed, x, mu, wmc, idx);
-    };
+    const float2 *sum = P.sum + item * MCG_ITEM_MOST;
 
     uint64_t seed = 0;
     float x = 0.f, mu = 0.f, wmc = 0.f, inv_mu = 0.f;
-    int idx = 0, phase = 0;
-    long long my_h = -1;
+    int idx = 0;
     uint32_t nst = 0, nsc = 0;
     float G_hi = 0.f, G_lo = 0.f, P_hi = 0.f, P_lo = 0.f;
     bool active = false, wait = false; /* wait: the lane's step needs the full form */
-    long long pool_next = 0, pool_end = 0;
-    bool drained = false;
+    mcg_pool pool;
     for (;;) {
-      unsigned need = __ballot_sync(0xffffffffu, !active);
+      const unsigned need = __ballot_sync(0xffffffffu, !active);
       if (need) {
-        int cnt = __popc(need), rank = __popc(need & lanemask_lt());
-        long long avail = pool_end - pool_next, my = -1;
-        if (rank < avail)
-          my = pool_next + rank;
-        if (cnt > avail && !drained) {
-          long long base = 0;
-          if (lane == 0)
-            base = (long long)atomicAdd(reinterpret_cast<unsigned long long *>(&s_ctl[1]), 32ull);
-          base = __shfl_sync(0xffffffffu, base, 0);
-          if (base >= it.count) {
-            drained = true;
-            pool_next = pool_end = 0;
-          } else {
-            long long end = min(base + 32, (long long)it.count);
-            long long r2 = rank - avail;
-            if (rank >= avail && r2 < end - base)
-              my = base + r2;
-            pool_next = min(base + (cnt - avail), end);
-            pool_end = end;
-          }
-        } else {
-          pool_next += min((long long)cnt, avail);
-        }
+        const long long my = pool.take(need, reinterpret_cast<unsigned long long *>(&s_ctl[1]), it.count, 32);
         if (!active && my >= 0) {
-          my_h = my;
-          born(my_h, seed, x, mu, wmc, idx);
+          if (P.jumps)
+            mcg_born(s_chain, sd.src, src_base + my, seed, x, mu, wmc, idx);
+          else
+            mcg_source_particle(sd.src, src_base + my, seed, x, mu, wmc, idx);
           inv_mu = mcg_flight_rcp(mu);
-          nst = nsc = 0;
-          phase = 0;
-          G_hi = G_lo = P_hi = P_lo = 0.f;
+          nst = 0;
+          const float2 g = sum[my];
+          G_hi = g.x;
+          G_lo = g.y;
+          P_hi = P_lo = 0.f;
           active = true;
         }
       }
       if (!__any_sync(0xffffffffu, active))
         break;
-      /* a round (the adjoint kernel's, mcg_adjoint.cu) */
+      /* a round (the adjoint's replay, mcg_adjoint.cu) */
       auto account = [&](int c, float l, float dep) {
         const float wc = __ldg(&aux[c].x);
         mcg_ff_add(P_hi, P_lo, __fmul_rn(wc, dep));
-        if (phase == 0) {
-          mcg_deposit<MCG_TALLY_SMEM32>(&s_tally[c], dep, P.q_log2);
-        } else {
-          const float v_after = __fadd_rn(__fsub_rn(G_hi, P_hi), __fsub_rn(G_lo, P_lo));
-          atomicAdd(&s_g[c], l * (wc * wmc - v_after));
-        }
+        const float v_after = __fadd_rn(__fsub_rn(G_hi, P_hi), __fsub_rn(G_lo, P_lo));
+        atomicAdd(&s_g[c], l * (wc * wmc - v_after));
         ++nst;
       };
       auto living = [&] {
         return active & (wmc >= P.min_w) & ((unsigned)idx < (unsigned)m) & (nst < P.max_steps);
       };
-      for (;;) {
+      auto cross = [&](int most) {
         bool go = living() & !wait;
-        for (int j = 0; go & (j < MCG_GRAD_WINDOW); ++j) {
+        for (int j = 0; go & (j < most); ++j) {
           const int c = idx;
           float l, dep;
-          if (!mcg_cross<false>(seed, x, mu, wmc, inv_mu, idx, cells[c], 0.0f, l, dep)) {
+          if (!mcg_cross<false>(seed, x, mu, wmc, inv_mu, idx, __ldg(cells + c), 0.0f, l, dep)) {
             wait = true;
             go = false;
           } else {
@@ -191,53 +152,41 @@ __global__ void __launch_bounds__(512, 2) mcg_fit_kernel(mcg_fit_params P)
             go = living();
           }
         }
+        return go;
+      };
+      auto full = [&] {
+        if (wait) {
+          const int c = idx;
+          float l, dep;
+          bool coll;
+          mcg_full<false, MCG_TALLY_SMEM32>(seed, x, mu, wmc, inv_mu, idx, nsc, __ldg(cells + c), nullptr,
+                                            P.q_log2, nullptr, no_libm, &l, &coll, &dep);
+          account(c, l, dep);
+          wait = false;
+        }
+      };
+      for (;;) {
+        const bool go = cross(MCG_GRAD_WINDOW);
         const unsigned wb = __ballot_sync(0xffffffffu, wait);
         const unsigned gb = __ballot_sync(0xffffffffu, go);
         if (wb && (!gb || __popc(wb) >= MCG_GRAD_POOL)) {
-          if (wait) {
-            const int c = idx;
-            float l, dep;
-            bool coll;
-            mcg_full<false, MCG_TALLY_SMEM32>(seed, x, mu, wmc, inv_mu, idx, nsc, cells[c], nullptr,
-                                              P.q_log2, nullptr, no_libm, &l, &coll, &dep);
-            account(c, l, dep);
-            wait = false;
-          }
+          full();
         } else {
-          const unsigned over = __ballot_sync(0xffffffffu, active ? !wait & !go : !drained);
+          const unsigned over = __ballot_sync(0xffffffffu, active ? !wait & !go : !pool.drained);
           if (!(wb | gb) || __popc(over) >= MCG_GRAD_REFILL)
             break;
         }
       }
-      if (active & !wait & !living()) {
-        if (phase == 0 && P.with_grad) {
-          /* replay the same history from its start */
-          born(my_h, seed, x, mu, wmc, idx);
-          inv_mu = mcg_flight_rcp(mu);
-          nst = nsc = 0;
-          G_hi = P_hi;
-          G_lo = P_lo;
-          P_hi = P_lo = 0.f;
-          phase = 1;
-        } else {
-          active = false;
-        }
-      }
+      active &= wait | living();
     }
   }
-  if (cur >= 0)
-    for (int i = tid; i < m; i += blockDim.x) {
-      if (s_tally[i])
-        atomicAdd(&gtally[i], s_tally[i]);
-      if (s_g[i] != 0.0f)
-        atomicAdd(&ggrad[i], (double)s_g[i]);
-    }
+  flush();
 }
 
 /* w_c = 2 (a_c - t_c) from this step's tally, the step's loss, and the
  * accumulators cleared for the next step. */
 __global__ void mcg_fit_weights_kernel(int n_cells, const int32_t *cell_slab,
-                                       const mcg_fit_slab_dev *slabs, const double *target,
+                                       const mcg_batch_slab_dev *slabs, const double *target,
                                        unsigned long long *tally, float2 *aux, double *loss_hist,
                                        const long long *step, int q_log2, int max_steps)
 {
@@ -259,8 +208,8 @@ __global__ void mcg_fit_weights_kernel(int n_cells, const int32_t *cell_slab,
 
 /* Adam on every sig_a; the new value goes straight into the step table. */
 __global__ void mcg_fit_adam_kernel(int n_cells, const int32_t *cell_slab,
-                                    const mcg_fit_slab_dev *slabs, double *grad, float *sig_a,
-                                    float4 *cells, float *m1, float *m2, long long *step, float lr,
+                                    const mcg_batch_slab_dev *slabs, double *grad, float *sig_a,
+                                    float4 *cells, float4 *tab, float *m1, float *m2, long long *step, float lr,
                                     float b1, float b2, float eps, float sig_min)
 {
   const long long t = *step + 1;
@@ -275,6 +224,7 @@ __global__ void mcg_fit_adam_kernel(int n_cells, const int32_t *cell_slab,
     const float s = fmaxf(sig_a[c] - lr * (a / c1) / (sqrtf(v / c2) + eps), sig_min);
     sig_a[c] = s;
     cells[c].x = s;
+    tab[c] = mcg_tile_cell(cells[c]);
   }
   __syncthreads();
   if (blockIdx.x == 0 && threadIdx.x == 0)
@@ -282,14 +232,18 @@ __global__ void mcg_fit_adam_kernel(int n_cells, const int32_t *cell_slab,
 }
 
 /* ------------------------------------------------------------ host side */
+#define MCG_FIT_PART 2048 /* most items between a forward pass and its replay: 128 MB of losses */
+
 struct mcg_fit_state {
   int n_slabs = 0, n_cells = 0, max_cells = 0, n_items = 0, max_steps = 0;
   std::vector<int32_t> cell_off;
   void *dev = nullptr; /* one allocation for everything below */
-  float4 *cells = nullptr;
+  void *dev_sum = nullptr; /* losses of `part` items, forward pass -> replay */
+  int part = 0;
+  float4 *cells = nullptr, *tab = nullptr; /* tab: mcg_tile_cell of cells */
   float2 *aux = nullptr;
-  mcg_fit_slab_dev *slabs = nullptr;
-  mcg_fit_item *items = nullptr;
+  mcg_batch_slab_dev *slabs = nullptr;
+  mcg_batch_item *items = nullptr;
   int32_t *cell_slab = nullptr;
   double *target = nullptr, *grad = nullptr, *loss_hist = nullptr;
   float *sig_a = nullptr, *m1 = nullptr, *m2 = nullptr;
@@ -316,6 +270,8 @@ extern "C" int mcg_fit_release(mcg_context *ctx)
     return MCG_OK;
   if (ctx->ext->fit->dev)
     cudaFree(ctx->ext->fit->dev);
+  if (ctx->ext->fit->dev_sum)
+    cudaFree(ctx->ext->fit->dev_sum);
   delete ctx->ext->fit;
   ctx->ext->fit = nullptr;
   return MCG_OK;
@@ -339,31 +295,42 @@ extern "C" int mcg_fit_set(mcg_context *ctx, int32_t n_slabs, const mcg_slab *h_
   }
   if (16 * 4 + (size_t)maxc * 12 > (size_t)ctx->smem_optin)
     return mcg_fail(MCG_ERR_ARG, "mcg_fit_set: slab of %d cells too large", maxc);
-  /* items of up to 8192 histories, largest first */
-  std::vector<mcg_fit_item> items;
+  /* items of up to MCG_ITEM_MOST histories, largest first */
+  std::vector<mcg_batch_item> items;
   for (int s = 0; s < n_slabs; ++s)
-    for (int64_t f = 0; f < h_slabs[s].n_histories; f += 8192)
-      items.push_back({s, 0, f, std::min<int64_t>(8192, h_slabs[s].n_histories - f)});
-  std::stable_sort(items.begin(), items.end(), [&](const mcg_fit_item &a, const mcg_fit_item &b) {
+    for (int64_t f = 0; f < h_slabs[s].n_histories; f += MCG_ITEM_MOST)
+      items.push_back({s, 0, f, std::min<int64_t>(MCG_ITEM_MOST, h_slabs[s].n_histories - f)});
+  std::stable_sort(items.begin(), items.end(), [&](const mcg_batch_item &a, const mcg_batch_item &b) {
     return a.count * h_slabs[a.slab].n_cells > b.count * h_slabs[b.slab].n_cells;
   });
   /* carve one allocation */
   size_t off = 0;
   auto take = [&](size_t bytes) { size_t o = off; off += (bytes + 255) & ~(size_t)255; return o; };
-  const size_t o_cells = take(total * sizeof(float4)), o_aux = take(total * sizeof(float2));
-  const size_t o_slabs = take(n_slabs * sizeof(mcg_fit_slab_dev));
-  const size_t o_items = take(items.size() * sizeof(mcg_fit_item));
+  const size_t padded = total + 2 * (size_t)MCG_TAB_PAD; /* the tiles read past the ends */
+  const size_t o_cells = take(total * sizeof(float4)), o_aux = take(padded * sizeof(float2));
+  const size_t o_tab = take(padded * sizeof(float4));
+  const size_t o_slabs = take(n_slabs * sizeof(mcg_batch_slab_dev));
+  const size_t o_items = take(items.size() * sizeof(mcg_batch_item));
   const size_t o_cs = take(total * 4), o_t = take(total * 8), o_g = take(total * 8);
   const size_t o_lh = take(max_steps * 8), o_sa = take(total * 4), o_m1 = take(total * 4);
-  const size_t o_m2 = take(total * 4), o_ta = take(total * 8), o_in = take(8), o_st = take(8);
+  const size_t o_m2 = take(total * 4), o_ta = take(total * 8), o_in = take(16), o_st = take(8);
   cudaError_t e = cudaMalloc(&F->dev, off);
   if (e != cudaSuccess)
     return mcg_cuda_fail(e, "mcg_fit_set: cudaMalloc");
+  for (F->part = (int)std::min<size_t>(items.size(), MCG_FIT_PART);; F->part /= 2) {
+    if ((e = cudaMalloc(&F->dev_sum, (size_t)F->part * MCG_ITEM_MOST * sizeof(float2))) == cudaSuccess)
+      break;
+    cudaGetLastError();
+    F->dev_sum = nullptr;
+    if (F->part <= 1)
+      return mcg_cuda_fail(e, "mcg_fit_set: cudaMalloc");
+  }
   char *b = static_cast<char *>(F->dev);
   F->cells = reinterpret_cast<float4 *>(b + o_cells);
-  F->aux = reinterpret_cast<float2 *>(b + o_aux);
-  F->slabs = reinterpret_cast<mcg_fit_slab_dev *>(b + o_slabs);
-  F->items = reinterpret_cast<mcg_fit_item *>(b + o_items);
+  F->aux = reinterpret_cast<float2 *>(b + o_aux) + MCG_TAB_PAD;
+  F->tab = reinterpret_cast<float4 *>(b + o_tab) + MCG_TAB_PAD;
+  F->slabs = reinterpret_cast<mcg_batch_slab_dev *>(b + o_slabs);
+  F->items = reinterpret_cast<mcg_batch_item *>(b + o_items);
   F->cell_slab = reinterpret_cast<int32_t *>(b + o_cs);
   F->target = reinterpret_cast<double *>(b + o_t);
   F->grad = reinterpret_cast<double *>(b + o_g);
@@ -375,9 +342,8 @@ extern "C" int mcg_fit_set(mcg_context *ctx, int32_t n_slabs, const mcg_slab *h_
   F->item_next = reinterpret_cast<unsigned long long *>(b + o_in);
   F->step = reinterpret_cast<long long *>(b + o_st);
   cudaMemset(F->dev, 0, off);
-  std::vector<float4> cf(total);
-  std::vector<float2> ax(total, make_float2(0.f, 0.f));
-  std::vector<mcg_fit_slab_dev> sd(n_slabs);
+  std::vector<float4> cf(total), ct(total);
+  std::vector<mcg_batch_slab_dev> sd(n_slabs);
   std::vector<int32_t> cs(total);
   int k = 0;
   for (int s = 0; s < n_slabs; ++s) {
@@ -391,13 +357,14 @@ extern "C" int mcg_fit_set(mcg_context *ctx, int32_t n_slabs, const mcg_slab *h_
       const float sig_s = h_sig_s[k];
       cf[k] = make_float4(h_sig_a0[k], sig_s > 1e-4f ? sig_s : 0.0f,
                           (float)j * dx, (float)(j + 1) * dx);
+      ct[k] = mcg_tile_cell(cf[k]);
       cs[k] = s;
     }
   }
   if ((e = cudaMemcpy(F->cells, cf.data(), total * sizeof(float4), cudaMemcpyHostToDevice)) != cudaSuccess ||
-      (e = cudaMemcpy(F->aux, ax.data(), total * sizeof(float2), cudaMemcpyHostToDevice)) != cudaSuccess ||
-      (e = cudaMemcpy(F->slabs, sd.data(), n_slabs * sizeof(mcg_fit_slab_dev), cudaMemcpyHostToDevice)) != cudaSuccess ||
-      (e = cudaMemcpy(F->items, items.data(), items.size() * sizeof(mcg_fit_item), cudaMemcpyHostToDevice)) != cudaSuccess ||
+      (e = cudaMemcpy(F->tab, ct.data(), total * sizeof(float4), cudaMemcpyHostToDevice)) != cudaSuccess ||
+      (e = cudaMemcpy(F->slabs, sd.data(), n_slabs * sizeof(mcg_batch_slab_dev), cudaMemcpyHostToDevice)) != cudaSuccess ||
+      (e = cudaMemcpy(F->items, items.data(), items.size() * sizeof(mcg_batch_item), cudaMemcpyHostToDevice)) != cudaSuccess ||
       (e = cudaMemcpy(F->cell_slab, cs.data(), total * 4, cudaMemcpyHostToDevice)) != cudaSuccess ||
       (e = cudaMemcpy(F->target, h_target, total * 8, cudaMemcpyHostToDevice)) != cudaSuccess ||
       (e = cudaMemcpy(F->sig_a, h_sig_a0, total * 4, cudaMemcpyHostToDevice)) != cudaSuccess)
@@ -411,35 +378,64 @@ extern "C" int mcg_fit_set(mcg_context *ctx, int32_t n_slabs, const mcg_slab *h_
   return MCG_OK;
 }
 
+/* The forward pass and (with_grad) the replay, in turns of F->part items. */
 static int fit_launch_track(mcg_context *ctx, mcg_fit_state *F, int with_grad)
 {
+  mcg_batch_params B;
+  memset(&B, 0, sizeof(B));
+  B.cells = F->cells;
+  B.tab = F->tab;
+  B.aux = F->aux;
+  B.loss = with_grad ? static_cast<float2 *>(F->dev_sum) : nullptr;
+  B.step = F->step;
+  B.slabs = F->slabs;
+  B.max_cells = F->max_cells;
+  B.item_next = F->item_next;
+  B.tally = F->tally;
+  B.rules = mcg_rules_setup(ctx, F->min_w, false);
   mcg_fit_params P;
   memset(&P, 0, sizeof(P));
   P.cells = F->cells;
   P.aux = F->aux;
   P.slabs = F->slabs;
-  P.items = F->items;
-  P.n_items = F->n_items;
   P.max_cells = F->max_cells;
-  P.item_next = F->item_next;
-  P.tally = F->tally;
+  P.item_next = F->item_next + 1;
+  P.sum = static_cast<const float2 *>(F->dev_sum);
   P.grad = F->grad;
   P.step = F->step;
   P.min_w = F->min_w;
   P.q_log2 = ctx->log2_scale;
-  P.with_grad = with_grad;
   P.max_steps = ctx->max_steps;
-  size_t smem = 4 * 8 + (size_t)F->max_cells * 12;
-  int bps = 1;
-  cudaError_t e = mcg_grad_shape(mcg_fit_kernel, 512, ctx->smem_optin, &smem, &P.jumps, &bps);
+  int block = 1024, f_bps = 1, bps = 1;
+  while (block > 128 && mcg_batch_smem(F->max_cells, block, true, true) > (size_t)ctx->smem_optin)
+    block -= 128;
+  const size_t f_smem = mcg_batch_smem(F->max_cells, block, true, true);
+  size_t smem = 4 * 8 + (((size_t)F->max_cells + 1) & ~(size_t)1) * 4;
+  cudaError_t e = cudaFuncSetAttribute(mcg_fit_forward, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                       ctx->smem_optin);
+  if (e == cudaSuccess)
+    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&f_bps, mcg_fit_forward, block, f_smem);
+  if (e == cudaSuccess)
+    e = mcg_grad_shape(mcg_fit_replay, 512, ctx->smem_optin, &smem, &P.jumps, &bps);
   if (e != cudaSuccess)
     return mcg_cuda_fail(e, "mcg_fit: launch set-up");
-  if ((e = cudaMemsetAsync(F->item_next, 0, 8, ctx->stream)) != cudaSuccess)
-    return mcg_cuda_fail(e, "mcg_fit: memset");
-  mcg_fit_kernel<<<ctx->sm_count * std::max(bps, 1), 512, smem, ctx->stream>>>(P);
-  if ((e = cudaGetLastError()) != cudaSuccess)
-    return mcg_cuda_fail(e, "mcg_fit_kernel launch");
-  ctx->launches++;
+  /* two blocks: their accumulators take what they took before the forward
+   * pass had its own kernel */
+  bps = std::min(std::max(bps, 1), 2);
+  for (int i = 0; i < F->n_items; i += F->part) {
+    B.items = P.items = F->items + i;
+    B.n_items = P.n_items = std::min(F->part, F->n_items - i);
+    if ((e = cudaMemsetAsync(F->item_next, 0, 16, ctx->stream)) != cudaSuccess)
+      return mcg_cuda_fail(e, "mcg_fit: memset");
+    mcg_fit_forward<<<ctx->sm_count * std::max(f_bps, 1), block, f_smem, ctx->stream>>>(B);
+    ctx->launches++;
+    if (with_grad) {
+      mcg_fit_replay<<<ctx->sm_count * bps, 512, smem, ctx->stream>>>(P);
+      ctx->launches++;
+    }
+    if ((e = cudaGetLastError()) != cudaSuccess)
+      return mcg_cuda_fail(e, "mcg_fit: launch");
+  }
   return MCG_OK;
 }
 
@@ -477,7 +473,7 @@ extern "C" int mcg_fit_run(mcg_context *ctx, int32_t n_steps, float lr, float be
                                                       F->tally, F->aux, F->loss_hist, F->step,
                                                       ctx->log2_scale, F->max_steps);
   mcg_fit_adam_kernel<<<1, 1024, 0, ctx->stream>>>(F->n_cells, F->cell_slab, F->slabs, F->grad,
-                                                   F->sig_a, F->cells, F->m1, F->m2, F->step, lr,
+                                                   F->sig_a, F->cells, F->tab, F->m1, F->m2, F->step, lr,
                                                    beta1, beta2, eps, sig_min);
   e = cudaStreamEndCapture(ctx->stream, &g);
   if (rc != MCG_OK)
@@ -497,7 +493,7 @@ extern "C" int mcg_fit_run(mcg_context *ctx, int32_t n_steps, float lr, float be
   if (e != cudaSuccess || e2 != cudaSuccess)
     return mcg_cuda_fail(e != cudaSuccess ? e : e2, "mcg_fit_run");
   cudaEventElapsedTime(&ctx->last_ms, ctx->ev0, ctx->ev1);
-  ctx->launches += 3LL * n_steps;
+  ctx->launches += (2LL * ((F->n_items + F->part - 1) / F->part) + 2) * n_steps;
   return MCG_OK;
 }
 
@@ -542,7 +538,7 @@ extern "C" int mcg_fit_gradient(mcg_context *ctx, const double *h_weights, doubl
   std::vector<float2> saved(n), ax(n);
   std::vector<double> keep_grad(n);
   std::vector<unsigned long long> keep_tally(n), q(n);
-  std::vector<mcg_fit_slab_dev> sd(F->n_slabs);
+  std::vector<mcg_batch_slab_dev> sd(F->n_slabs);
   std::vector<int32_t> cs(n);
   for (int c = 0; c < n; ++c)
     ax[c] = make_float2((float)h_weights[c], 0.0f);
@@ -550,7 +546,7 @@ extern "C" int mcg_fit_gradient(mcg_context *ctx, const double *h_weights, doubl
   if ((e = cudaMemcpy(saved.data(), F->aux, n * sizeof(float2), cudaMemcpyDeviceToHost)) != cudaSuccess ||
       (e = cudaMemcpy(keep_grad.data(), F->grad, n * 8, cudaMemcpyDeviceToHost)) != cudaSuccess ||
       (e = cudaMemcpy(keep_tally.data(), F->tally, n * 8, cudaMemcpyDeviceToHost)) != cudaSuccess ||
-      (e = cudaMemcpy(sd.data(), F->slabs, F->n_slabs * sizeof(mcg_fit_slab_dev), cudaMemcpyDeviceToHost)) != cudaSuccess ||
+      (e = cudaMemcpy(sd.data(), F->slabs, F->n_slabs * sizeof(mcg_batch_slab_dev), cudaMemcpyDeviceToHost)) != cudaSuccess ||
       (e = cudaMemcpy(cs.data(), F->cell_slab, n * 4, cudaMemcpyDeviceToHost)) != cudaSuccess ||
       (e = cudaMemcpy(F->aux, ax.data(), n * sizeof(float2), cudaMemcpyHostToDevice)) != cudaSuccess ||
       (e = cudaMemset(F->grad, 0, n * 8)) != cudaSuccess ||
