@@ -513,21 +513,8 @@ extern "C" int mcg_batch_tally_read(mcg_context *ctx, int64_t *h_q, double *h_f6
   int rc = batch_prepare(ctx, &B);
   if (rc != MCG_OK)
     return rc;
-  std::vector<int64_t> q(B->total_cells);
-  cudaError_t e = cudaMemcpyAsync(q.data(), B->d_tally, q.size() * sizeof(int64_t),
-                                  cudaMemcpyDeviceToHost, ctx->stream);
-  if (e == cudaSuccess)
-    e = cudaStreamSynchronize(ctx->stream);
-  if (e != cudaSuccess)
-    return mcg_cuda_fail(e, "mcg_batch_tally_read");
-  const double inv = std::ldexp(1.0, -ctx->log2_scale);
-  for (size_t i = 0; i < q.size(); ++i) {
-    if (h_q)
-      h_q[i] = q[i];
-    if (h_f64)
-      h_f64[i] = (double)q[i] * inv;
-  }
-  return MCG_OK;
+  cudaError_t e = mcg_read_tally(ctx, B->d_tally, (size_t)B->total_cells, h_q, h_f64);
+  return e == cudaSuccess ? MCG_OK : mcg_cuda_fail(e, "mcg_batch_tally_read");
 }
 
 extern "C" int mcg_batch_set_launch(mcg_context *ctx, int32_t block, int64_t item_histories,

@@ -124,6 +124,7 @@ struct mcg_context {
   unsigned long long *d_tally = nullptr;
   int log2_scale = 40;
   unsigned long long *d_counters = nullptr, *d_next = nullptr;
+  unsigned long long *h_err = nullptr; /* page-locked: the error flags after a run (mcg_sync) */
 
   /* strict libm */
   bool libm_loaded = false;
@@ -161,6 +162,8 @@ int mcg_fail(int code, const char *fmt, ...);
 cudaError_t mcg_dev_malloc(void **p, size_t bytes);
 int mcg_cuda_fail(cudaError_t e, const char *what);
 #define MCG_TAB_PAD 32 /* a tile reads past its chain's ends (mcg_tiles) */
+cudaError_t mcg_read_tally(mcg_context *ctx, const unsigned long long *d, size_t n, int64_t *h_q,
+                           double *h_f64);
 void mcg_tile_table(const float4 *cells_fast, int n, float4 *tab, float2 *right = nullptr,
                     float2 *left = nullptr);
 void mcg_cell_params(float sig, float rate, int gi, float dx, float4 &strict, float4 &fast);

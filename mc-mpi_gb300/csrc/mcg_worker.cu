@@ -1081,8 +1081,11 @@ extern "C" int mcg_worker_run_async(mcg_context *ctx, const mcg_source *src, int
       e = cudaStreamQuery(ctx->stream);
       if (e != cudaErrorNotReady)
         break;
-      std::this_thread::sleep_for(std::chrono::milliseconds(2));
+      /* asleep for a 64th of the time so far, so that a short launch is not
+       * waited for longer than it runs (it was 2 ms at a time) */
       const double el = std::chrono::duration<double>(std::chrono::steady_clock::now() - t0).count();
+      std::this_thread::sleep_for(std::chrono::microseconds(
+          std::min<long long>(2000, std::max<long long>(10, (long long)(el * 1e6 / 64)))));
       if (trace && el >= next_trace) {
         next_trace += 1.0;
         if (cudaMemcpyAsync(host, state, sizeof(host), cudaMemcpyDeviceToHost, WS.monitor) == cudaSuccess &&
