@@ -263,15 +263,17 @@ __global__ void __launch_bounds__(1024) mcg_adjoint_replay(mcg_adj_params P)
       }
     };
     /* a lane that waits does so while the others cross, MCG_GRAD_WINDOW steps
-     * between two votes, until MCG_GRAD_POOL of them wait or nothing else can
-     * step; the round lasts until MCG_GRAD_REFILL lanes have ended a history
-     * or want one.  Every pass steps a lane, makes one wait or completes the
-     * waiting steps, and no lane passes its step limit, so it ends. */
+     * between two votes, until MCG_GRAD_POOL of 32 with a history wait, and as
+     * many fewer as there are (a fixed number: 34.1 ms for 32.9, the last
+     * histories waiting for one another); the round lasts until
+     * MCG_GRAD_REFILL lanes have ended a history or want one.  Every pass
+     * steps a lane, makes one wait or completes the waiting steps, and no lane
+     * passes its step limit, so it ends. */
     for (;;) {
       const bool go = cross(MCG_GRAD_WINDOW);
       const unsigned wb = __ballot_sync(0xffffffffu, wait);
       const unsigned gb = __ballot_sync(0xffffffffu, go);
-      if (wb && (!gb || __popc(wb) >= MCG_GRAD_POOL)) {
+      if (wb && 32 * __popc(wb) >= MCG_GRAD_POOL * __popc(wb | gb)) {
         full();
       } else {
         const unsigned over = __ballot_sync(0xffffffffu, active ? !wait & !go : !pool.drained);

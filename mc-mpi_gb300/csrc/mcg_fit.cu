@@ -169,7 +169,7 @@ __global__ void __launch_bounds__(512, 2) mcg_fit_replay(mcg_fit_params P)
         const bool go = cross(MCG_GRAD_WINDOW);
         const unsigned wb = __ballot_sync(0xffffffffu, wait);
         const unsigned gb = __ballot_sync(0xffffffffu, go);
-        if (wb && (!gb || __popc(wb) >= MCG_GRAD_POOL)) {
+        if (wb && 32 * __popc(wb) >= MCG_GRAD_POOL * __popc(wb | gb)) {
           full();
         } else {
           const unsigned over = __ballot_sync(0xffffffffu, active ? !wait & !go : !pool.drained);

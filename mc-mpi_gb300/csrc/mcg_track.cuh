@@ -712,8 +712,8 @@ __device__ __forceinline__ bool mcg_cross(uint64_t &seed, float &x, float mu, fl
 }
 
 /* Rounds of the gradient kernels: certain crossings of a lane between two votes
- * of the warp, lanes waiting for the full step that trigger it, lanes that have
- * ended a pass or want a history that end the round.  1000 cells, 2e6 histories:
+ * of the warp, lanes (of 32 with a history) waiting for the full step that
+ * trigger it, lanes that have ended a pass or want a history that end the round.  1000 cells, 2e6 histories:
  * windows of 1 to 8 and pools of 2 to 8 lie within 4 % of these, pools of 1 or 12
  * are 6 to 13 % slower.  Long windows with small pools let colliding histories fall
  * behind, and the gradients' float sums notice (mcg_adjoint_fused). */
@@ -1430,8 +1430,11 @@ struct mcg_lane {
 };
 
 /* One tile for every lane with `alive` that can; the lanes whose step needs the
- * full form wait until pool_lanes of them do (or no other lane can step) and
- * take it together.  Every call steps a lane, makes one wait or completes the
+ * full form wait until pool_lanes of 32 alive ones do, and as many fewer as are
+ * alive, and take it together: a fixed number made the last histories of a warp
+ * wait for one another (10,000 cells, 1e5 histories, strict: 7.05 ms -> 5.85 ms).
+ * MULTI, whose warps stay full, keeps the number until nothing else can step
+ * (4096 slabs: 201 ms against 204).  Every call steps a lane, makes one wait or completes the
  * waiting steps, if any lane is alive, and no lane passes its step limit.
  * far (MULTI): the lane's deposits go to the global tally, the others' full
  * steps to word[idx - word_off].  The whole warp calls. */
@@ -1468,7 +1471,8 @@ __device__ __forceinline__ void mcg_advance(mcg_lane &p, bool alive, bool far, c
     p.wait |= can & (k < nmax) & (p.wmc >= R.min_w);
   }
   const unsigned wb = __ballot_sync(0xffffffffu, p.wait);
-  if (wb && (__popc(wb) >= R.pool_lanes || !__any_sync(0xffffffffu, alive & !p.wait))) {
+  if (wb && (MULTI ? __popc(wb) >= R.pool_lanes || wb == __ballot_sync(0xffffffffu, alive)
+                   : 32 * __popc(wb) >= R.pool_lanes * __popc(__ballot_sync(0xffffffffu, alive)))) {
     if (p.wait) {
       p.x = p.place(cells);
       uint64_t seed = p.s2 >> 1;
@@ -1686,10 +1690,10 @@ __global__ void __launch_bounds__(THIN ? MCG_THIN_BLOCK : 1024) mcg_track_kernel
   }
 }
 
-/* The rules of a launch.  Full steps are pooled for 4 lanes (thin chains need
- * them on 1 % of the tiles, others on a third of them) and ended histories
- * replaced for one or two; 2 to 16 and 1 to 8 were measured within 5 % of
- * these on thin chains and within 10 % on a 1000-cell one. */
+/* The rules of a launch.  Full steps are pooled for 4 lanes of 32 (thin chains
+ * need them on 1 % of the tiles, others on a third of them) and ended histories
+ * replaced for two; 2 to 16 and 1 to 8 were measured within 5 % of these on thin
+ * chains and within 10 % on a 1000-cell one. */
 inline mcg_rules mcg_rules_setup(const mcg_context *ctx, float min_w, bool thin)
 {
   mcg_rules R;
@@ -1698,7 +1702,7 @@ inline mcg_rules mcg_rules_setup(const mcg_context *ctx, float min_w, bool thin)
   R.max_steps = ctx->max_steps;
   R.window = ctx->refill ? ctx->refill : MCG_TW_MAX;
   R.pool_lanes = 4;
-  R.refill_lanes = thin ? 1 : 2;
+  R.refill_lanes = 2;
   R.run = mcg_run_setup(ctx->log2_scale, min_w, ctx->run_bounds, ctx->width_a, ctx->width_i);
   return R;
 }
