@@ -553,7 +553,7 @@ extern "C" int mcg_adjoint_run(mcg_context *ctx, const mcg_source *src, int64_t 
   P.n_cells = ctx->n_cells;
   P.cell_lo = ctx->cell_lo;
   P.g_log2 = A->g_log2;
-  P.rules = mcg_rules_setup(ctx, ctx->min_w, false);
+  P.rules = mcg_rules_setup(ctx, ctx->min_w);
   P.src = *src;
   P.next = ctx->d_next;
   P.tally = ctx->d_tally;

@@ -692,7 +692,7 @@ int mcg_track_launch(mcg_context *ctx, mcg_particle *d_particles, int64_t n, int
   P.counters = ctx->d_counters;
   P.libm = ctx->libm;
   P.libm_tab = ctx->libm_tab;
-  P.rules = mcg_rules_setup(ctx, ctx->min_w, false);
+  P.rules = mcg_rules_setup(ctx, ctx->min_w);
   if (ctx->algorithm == MCG_ALGO_EVENT) {
     ctx->launches++;
     return mcg_event_run(ctx, P);
@@ -708,7 +708,6 @@ int mcg_track_launch(mcg_context *ctx, mcg_particle *d_particles, int64_t n, int
   const int block = shape.block;
   const size_t smem = shape.smem;
   P.tally_copies = shape.copies;
-  P.rules = mcg_rules_setup(ctx, ctx->min_w, thin);
   void (*kern)(mcg_track_params);
   if (strict)
     kern = thin ? mcg_track_kernel<true, MCG_TALLY_LO32, true>

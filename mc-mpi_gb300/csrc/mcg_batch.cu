@@ -277,7 +277,7 @@ static int batch_configure(mcg_context *ctx, mcg_batch_state *B, int64_t item, d
   P.counters = ctx->d_counters;
   P.libm = ctx->libm;
   P.libm_tab = ctx->libm_tab;
-  P.rules = mcg_rules_setup(ctx, B->min_w, false);
+  P.rules = mcg_rules_setup(ctx, B->min_w);
   P.rules.pool_lanes = B->defer ? B->defer : MCG_BATCH_POOL;
   /* the asked block, or a smaller one where the largest slab's tally and the
    * warps' tiles would not fit; the global tally where none does.  Both
@@ -454,7 +454,7 @@ extern "C" int mcg_batch_run_per_slab(mcg_context *ctx)
     P.counters = ctx->d_counters;
     P.libm = ctx->libm;
     P.libm_tab = ctx->libm_tab;
-    P.rules = mcg_rules_setup(ctx, B->min_w, false);
+    P.rules = mcg_rules_setup(ctx, B->min_w);
     const mcg_shape shape = mcg_track_shape(sl.n_cells, 0, false, false, (size_t)ctx->smem_optin);
     const int block = shape.block;
     const size_t smem = shape.smem;

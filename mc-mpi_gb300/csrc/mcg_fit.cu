@@ -392,7 +392,7 @@ static int fit_launch_track(mcg_context *ctx, mcg_fit_state *F, int with_grad)
   B.max_cells = F->max_cells;
   B.item_next = F->item_next;
   B.tally = F->tally;
-  B.rules = mcg_rules_setup(ctx, F->min_w, false);
+  B.rules = mcg_rules_setup(ctx, F->min_w);
   mcg_fit_params P;
   memset(&P, 0, sizeof(P));
   P.cells = F->cells;

@@ -128,7 +128,7 @@ extern "C" int mcg_simulate_fast_noalloc(int n_layers, const int32_t *h_index_st
     P.counters = cnt;
     mcg_context rules; /* the defaults of a context, for its rules */
     rules.log2_scale = log2_scale;
-    P.rules = mcg_rules_setup(&rules, particle_min_weight, false);
+    P.rules = mcg_rules_setup(&rules, particle_min_weight);
     int sms = 0, optin = 0, bps = 0;
     if ((e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess ||
         (e = cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev)) != cudaSuccess)

@@ -1694,7 +1694,7 @@ __global__ void __launch_bounds__(THIN ? MCG_THIN_BLOCK : 1024) mcg_track_kernel
  * need them on 1 % of the tiles, others on a third of them) and ended histories
  * replaced for two; 2 to 16 and 1 to 8 were measured within 5 % of these on thin
  * chains and within 10 % on a 1000-cell one. */
-inline mcg_rules mcg_rules_setup(const mcg_context *ctx, float min_w, bool thin)
+inline mcg_rules mcg_rules_setup(const mcg_context *ctx, float min_w)
 {
   mcg_rules R;
   R.min_w = min_w;

@@ -1024,7 +1024,7 @@ extern "C" int mcg_worker_run_async(mcg_context *ctx, const mcg_source *src, int
   A.src = *src;
   A.state = state;
   A.src_total = (unsigned long long)n;
-  A.rules = mcg_rules_setup(ctx, ctx->min_w, thin);
+  A.rules = mcg_rules_setup(ctx, ctx->min_w);
   A.tally = ctx->d_tally;
   A.counters = ctx->d_counters;
   A.libm = ctx->libm;
