@@ -213,9 +213,6 @@ extern "C" int mcg_create(int device, int mode, mcg_context **out)
       rc = mcg_cuda_fail(e, "cudaMalloc(counters)");
     else
       cudaMemset(ctx->d_counters, 0, 16 * sizeof(unsigned long long));
-    if (rc == MCG_OK &&
-        (e = cudaHostAlloc(&ctx->h_err, sizeof(*ctx->h_err), cudaHostAllocDefault)) != cudaSuccess)
-      rc = mcg_cuda_fail(e, "cudaHostAlloc(error word)");
   }
   if (rc == MCG_OK && mode == MCG_MODE_STRICT)
     rc = mcg_load_libm(ctx);
@@ -306,8 +303,6 @@ extern "C" int mcg_destroy(mcg_context *ctx)
     cudaEventDestroy(ctx->ev1);
   if (ctx->stream)
     cudaStreamDestroy(ctx->stream);
-  if (ctx->h_err)
-    cudaFreeHost(ctx->h_err);
   delete ctx;
   return MCG_OK;
 }
@@ -751,7 +746,8 @@ int mcg_track_launch(mcg_context *ctx, mcg_particle *d_particles, int64_t n, int
 int mcg_sync(mcg_context *ctx)
 {
   /* the error flags come with the same synchronisation */
-  cudaError_t e = cudaMemcpyAsync(ctx->h_err, ctx->d_counters + MCG_CNT_ERR, sizeof(*ctx->h_err),
+  unsigned long long err = 0;
+  cudaError_t e = cudaMemcpyAsync(&err, ctx->d_counters + MCG_CNT_ERR, sizeof(err),
                                   cudaMemcpyDeviceToHost, ctx->stream);
   const cudaError_t e2 = cudaStreamSynchronize(ctx->stream);
   if (e2 != cudaSuccess)
@@ -759,7 +755,6 @@ int mcg_sync(mcg_context *ctx)
   if (e != cudaSuccess)
     return mcg_cuda_fail(e, "read error flags");
   cudaEventElapsedTime(&ctx->last_ms, ctx->ev0, ctx->ev1);
-  const unsigned long long err = *ctx->h_err;
   if (err)
     return mcg_fail(MCG_ERR_LIMIT, "a history exceeded the step limit (error flags %llx)", err);
   return MCG_OK;

@@ -124,7 +124,6 @@ struct mcg_context {
   unsigned long long *d_tally = nullptr;
   int log2_scale = 40;
   unsigned long long *d_counters = nullptr, *d_next = nullptr;
-  unsigned long long *h_err = nullptr; /* page-locked: the error flags after a run (mcg_sync) */
 
   /* strict libm */
   bool libm_loaded = false;
