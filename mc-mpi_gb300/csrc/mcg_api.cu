@@ -370,6 +370,23 @@ static void update_thin(mcg_context *ctx)
   ctx->width_i = 1.01f * wi;
   ctx->thin = !ctx->cells_strict.empty() && wa <= 2e-4f;
   ctx->thin_fast = !ctx->cells_strict.empty() && std::max(wa, wi) <= 4e-4f;
+  ctx->thick = mcg_thick(ctx->cells_strict.data(), (int)ctx->cells_strict.size(), true);
+  ctx->thick_fast = mcg_thick(ctx->cells_strict.data(), (int)ctx->cells_strict.size(), false);
+}
+
+/* Chains on which a lane per history is faster than tiles: by the cells' mean
+ * optical widths, in absorption (strict, whose tiles need u < 2^-4) or both
+ * together.  Kernel times of 2e6 histories, lanes / tiles, at mean widths
+ * sig_a (+ sig_i): strict .069 753 / 1454 us, .031 1053 / 1308, .028 1351 / 1709,
+ * .021 1338 / 1247, .014 tiles; fast .131 424 / 610, .156 555 / 792,
+ * .088 569 / 611, .104 797 / 775, .053 tiles. */
+bool mcg_thick(const float4 *cells, int n, bool strict)
+{
+  double sum = 0.0;
+  for (int c = 0; c < n; ++c)
+    sum += (std::fabs((double)cells[c].x) + (strict ? 0.0 : std::fabs((double)cells[c].y))) *
+           ((double)cells[c].w - cells[c].z);
+  return n > 0 && sum > (strict ? 0.02 : 0.08) * n;
 }
 
 /* The cells and their tile table to the device; `tab` holds the latter until
@@ -703,8 +720,17 @@ int mcg_track_launch(mcg_context *ctx, mcg_particle *d_particles, int64_t n, int
   const int block = shape.block;
   const size_t smem = shape.smem;
   P.tally_copies = shape.copies;
+  const bool lanes = strict ? ctx->thick : ctx->thick_fast;
   void (*kern)(mcg_track_params);
-  if (strict)
+  if (lanes && strict)
+    kern = shape.global ? mcg_track_kernel<true, MCG_TALLY_GLOBAL, false, true>
+           : ctx->tally_mode == MCG_TALLY_SMEM64 ? mcg_track_kernel<true, MCG_TALLY_SMEM64, false, true>
+                                                 : mcg_track_kernel<true, MCG_TALLY_SMEM32, false, true>;
+  else if (lanes)
+    kern = shape.global ? mcg_track_kernel<false, MCG_TALLY_GLOBAL, false, true>
+           : ctx->tally_mode == MCG_TALLY_SMEM64 ? mcg_track_kernel<false, MCG_TALLY_SMEM64, false, true>
+                                                 : mcg_track_kernel<false, MCG_TALLY_SMEM32, false, true>;
+  else if (strict)
     kern = thin ? mcg_track_kernel<true, MCG_TALLY_LO32, true>
            : shape.global ? mcg_track_kernel<true, MCG_TALLY_GLOBAL, false>
            : ctx->tally_mode == MCG_TALLY_SMEM64 ? mcg_track_kernel<true, MCG_TALLY_SMEM64, false>
@@ -728,7 +754,7 @@ int mcg_track_launch(mcg_context *ctx, mcg_particle *d_particles, int64_t n, int
       return mcg_cuda_fail(e, "occupancy");
     bps = std::max(bps, 1);
   }
-  const int grid = mcg_track_grid(ctx->sm_count * bps, block, n, P);
+  const int grid = mcg_track_grid(ctx->sm_count * bps, block, n, lanes, P);
   if ((e = cudaMemsetAsync(ctx->d_next, 0, sizeof(unsigned long long), ctx->stream)) != cudaSuccess)
     return mcg_cuda_fail(e, "cudaMemsetAsync");
   cudaEventRecord(ctx->ev0, ctx->stream);

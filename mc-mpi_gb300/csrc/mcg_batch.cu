@@ -468,7 +468,7 @@ extern "C" int mcg_batch_run_per_slab(mcg_context *ctx)
     int bps = 1;
     if (e == cudaSuccess)
       e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, kern, block, smem);
-    const int grid = mcg_track_grid(ctx->sm_count * std::max(bps, 1), block, sl.n_histories, P);
+    const int grid = mcg_track_grid(ctx->sm_count * std::max(bps, 1), block, sl.n_histories, false, P);
     if (e == cudaSuccess)
       e = cudaMemsetAsync(ctx->d_next, 0, 8, ctx->stream);
     if (e == cudaSuccess) {

@@ -114,6 +114,7 @@ struct mcg_context {
   std::vector<float4> cells_strict, cells_fast;
   bool thin = false;      /* every cell's sig_a width <= 2e-4 (strict THIN) */
   bool thin_fast = false; /* sig_a and sig_i widths <= 4e-4 (fast THIN) */
+  bool thick = false, thick_fast = false; /* mcg_thick, strict and fast */
   float width_a = 0.f, width_i = 0.f; /* those largest widths */
   float4 *d_cells_strict = nullptr, *d_cells_fast = nullptr;
   /* the tiles' per-cell parameters (mcg_tile_table), MCG_TAB_PAD entries
@@ -161,6 +162,7 @@ int mcg_fail(int code, const char *fmt, ...);
 cudaError_t mcg_dev_malloc(void **p, size_t bytes);
 int mcg_cuda_fail(cudaError_t e, const char *what);
 #define MCG_TAB_PAD 32 /* a tile reads past its chain's ends (mcg_tiles) */
+bool mcg_thick(const float4 *cells, int n, bool strict);
 cudaError_t mcg_read_tally(mcg_context *ctx, const unsigned long long *d, size_t n, int64_t *h_q,
                            double *h_f64);
 void mcg_tile_table(const float4 *cells_fast, int n, float4 *tab, float2 *right = nullptr,

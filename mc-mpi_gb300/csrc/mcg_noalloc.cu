@@ -138,15 +138,18 @@ extern "C" int mcg_simulate_fast_noalloc(int n_layers, const int32_t *h_index_st
     const int block = shape.block;
     const size_t smem = shape.smem;
     P.tally_copies = shape.copies;
-    auto kern = smem_tally ? mcg_track_kernel<false, MCG_TALLY_SMEM32, false>
-                           : mcg_track_kernel<false, MCG_TALLY_GLOBAL, false>;
+    const bool lanes = mcg_thick(cf.data(), total, false);
+    auto kern = lanes ? (smem_tally ? mcg_track_kernel<false, MCG_TALLY_SMEM32, false, true>
+                                    : mcg_track_kernel<false, MCG_TALLY_GLOBAL, false, true>)
+                      : (smem_tally ? mcg_track_kernel<false, MCG_TALLY_SMEM32, false>
+                                    : mcg_track_kernel<false, MCG_TALLY_GLOBAL, false>);
     /* the attribute is raised to the device's limit (the same value every
      * caller of this library sets), so a concurrent launch of the same kernel
      * from another host thread can never lower it below this launch's need */
     if ((e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, optin)) != cudaSuccess ||
         (e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, kern, block, smem)) != cudaSuccess)
       return mcg_cuda_fail(e, "mcg_simulate_fast_noalloc: launch set-up");
-    const int grid = mcg_track_grid(sms * std::max(bps, 1), block, n, P);
+    const int grid = mcg_track_grid(sms * std::max(bps, 1), block, n, lanes, P);
     kern<<<grid, block, smem, st>>>(P);
     if ((e = cudaGetLastError()) != cudaSuccess)
       return mcg_cuda_fail(e, "mcg_simulate_fast_noalloc: launch");

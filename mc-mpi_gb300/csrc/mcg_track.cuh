@@ -1408,6 +1408,15 @@ struct mcg_lane {
   {
     return (wmc >= R.min_w) & ((unsigned)(idx - off) < (unsigned)ncell) & (nst < R.max_steps);
   }
+  /* Classification of simulate_particle for an ended history; one still alive
+   * in the chain has reached the step limit (2). */
+  __device__ __forceinline__ int outcome(const mcg_rules &R) const
+  {
+    const int c = idx - off;
+    if ((wmc >= R.min_w) && ((unsigned)c < (unsigned)ncell))
+      return 2;
+    return c == -1 ? -1 : c == ncell ? 1 : wmc < R.min_w ? 0 : -1;
+  }
   /* x, when it is only known as a face */
   __device__ __forceinline__ float place(const float4 *cells) const
   {
@@ -1540,23 +1549,8 @@ __device__ __forceinline__ void mcg_histories(mcg_geometry &geo, mcg_sink &D, co
     if (!ab || gone || (__popc(~ab) >= R.refill_lanes &&
                         (!pool.drained || __any_sync(0xffffffffu, active & !alive)))) {
       if (active & !alive) {
-        /* history ends: classification of simulate_particle; a history
-         * still alive in the chain here has reached the step limit */
-        const int c = p.idx - p.off;
-        const bool in = (p.wmc >= R.min_w) && ((unsigned)c < (unsigned)p.ncell);
-        int r;
-        if (in)
-          r = 2;
-        else if (c == -1)
-          r = -1;
-        else if (c == p.ncell)
-          r = 1;
-        else if (p.wmc < R.min_w)
-          r = 0;
-        else
-          r = -1;
         p.x = p.place(cells);
-        end(hid, r, p, c);
+        end(hid, p.outcome(R), p, p.idx - p.off);
         active = false;
       }
       unsigned need = __ballot_sync(0xffffffffu, !active);
@@ -1588,9 +1582,58 @@ __device__ __forceinline__ void mcg_histories(mcg_geometry &geo, mcg_sink &D, co
   }
 }
 
+/* Histories of a chain of thick cells (update_thin in mcg_api.cu): one lane
+ * each through every step, MCG_LANES_STEPS of them between two looks for new
+ * ones.  Collisions and steep absorptions leave the tiles a step or two each. */
+#define MCG_LANES_STEPS 8
+template <bool STRICT, int TALLY, class BIRTH, class END>
+__device__ __forceinline__ void mcg_lane_histories(int ncell, const float4 *cells,
+                                                   unsigned long long *tally, const mcg_rules &R,
+                                                   const mcg_libm_tab *T, const mcg_libm_dev &libm,
+                                                   unsigned long long *counter, long long n, int chunk,
+                                                   const BIRTH &birth, const END &end)
+{
+  mcg_lane p;
+  uint64_t seed = 0;
+  int64_t hid = -1;
+  bool active = false;
+  mcg_pool pool;
+  p.ncell = ncell;
+  for (;;) {
+    const unsigned need = __ballot_sync(0xffffffffu, !active);
+    if (need) {
+      const long long my = pool.take(need, counter, n, chunk);
+      if (!active && my >= 0) {
+        hid = birth(my, seed, p.x, p.mu, p.wmc, p.idx);
+        p.inv_mu = mcg_flight_rcp(p.mu);
+        p.wres = 0.f;
+        p.nst = p.nsc = 0;
+        active = true;
+      }
+    }
+    if (!__any_sync(0xffffffffu, active))
+      break;
+    if (active) {
+      const int kmax = (int)min((uint32_t)MCG_LANES_STEPS, R.max_steps - p.nst);
+      int k = 0;
+#pragma unroll 1
+      for (; k < kmax && (p.wmc >= R.min_w) & ((unsigned)p.idx < (unsigned)ncell); ++k)
+        mcg_step<STRICT, TALLY, false>(seed, p.x, p.mu, p.wmc, p.inv_mu, p.idx, p.nsc,
+                                       __ldg(cells + p.idx), tally + p.idx, R.q_log2, T, libm, nullptr,
+                                       nullptr, nullptr, STRICT ? nullptr : &p.wres);
+      p.nst += (uint32_t)k;
+      if (!p.living(R)) {
+        p.s2 = seed << 1;
+        end(hid, p.outcome(R), p, p.idx);
+        active = false;
+      }
+    }
+  }
+}
+
 /* THIN: the chain is optically thin (see update_thin in mcg_api.cu) and the
- * tally is MCG_TALLY_LO32. */
-template <bool STRICT, int TALLY, bool THIN>
+ * tally is MCG_TALLY_LO32.  LANES: mcg_lane_histories instead of tiles. */
+template <bool STRICT, int TALLY, bool THIN, bool LANES = false>
 __global__ void __launch_bounds__(THIN ? MCG_THIN_BLOCK : 1024) mcg_track_kernel(mcg_track_params P)
 {
   extern __shared__ __align__(16) unsigned char smem[];
@@ -1625,37 +1668,40 @@ __global__ void __launch_bounds__(THIN ? MCG_THIN_BLOCK : 1024) mcg_track_kernel
   mcg_geometry geo = {0, ncell};
   mcg_sink sink = {(uint32_t)__cvta_generic_to_shared(my_tally), P.tally};
   unsigned long long tot_steps = 0, tot_scat = 0;
-  mcg_histories<STRICT, THIN, TALLY, false, false>(
-      geo, sink, P.cells, P.tab, my_tally, P.rules, tiles, s_real, T, P.libm, P.next,
-      [&] { return (long long)P.n; }, P.chunk,
-      [&](long long my, uint64_t &seed, float &x, float &mu, float &wmc, int &idx) {
-        if (P.particles)
-          mcg_load_particle(P, my, seed, x, mu, wmc, idx);
-        else
-          mcg_born(s_chain, P.src, P.first + my, seed, x, mu, wmc, idx);
-        idx -= lo;
-        return my;
-      },
-      [&](long long hid, int r, const mcg_lane &p, int idx) {
-        if (P.particles && p.nst) { /* without a step the particle stays as it is */
-          unsigned long long *q = reinterpret_cast<unsigned long long *>(P.particles + hid);
-          q[0] = p.s2 >> 1;
-          q[1] = (unsigned long long)__float_as_uint(p.x) |
-                 ((unsigned long long)__float_as_uint(p.mu) << 32);
-          q[2] = (unsigned long long)__float_as_uint(p.wmc) |
-                 ((unsigned long long)(uint32_t)(idx + lo) << 32);
-        }
-        if (P.results)
-          P.results[hid] = r;
-        if (P.steps)
-          P.steps[hid] = p.nst;
-        if (P.scatters)
-          P.scatters[hid] = p.nsc;
-        mcg_count_end<STRICT>(s_cnt, r, p.wmc, p.wres, P.rules.q_log2);
-        tot_steps += p.nst;
-        tot_scat += p.nsc;
-      },
-      [] { return true; }, [] { return false; });
+  auto birth = [&](long long my, uint64_t &seed, float &x, float &mu, float &wmc, int &idx) {
+    if (P.particles)
+      mcg_load_particle(P, my, seed, x, mu, wmc, idx);
+    else
+      mcg_born(s_chain, P.src, P.first + my, seed, x, mu, wmc, idx);
+    idx -= lo;
+    return my;
+  };
+  auto end = [&](long long hid, int r, const mcg_lane &p, int idx) {
+    if (P.particles && p.nst) { /* without a step the particle stays as it is */
+      unsigned long long *q = reinterpret_cast<unsigned long long *>(P.particles + hid);
+      q[0] = p.s2 >> 1;
+      q[1] = (unsigned long long)__float_as_uint(p.x) |
+             ((unsigned long long)__float_as_uint(p.mu) << 32);
+      q[2] = (unsigned long long)__float_as_uint(p.wmc) |
+             ((unsigned long long)(uint32_t)(idx + lo) << 32);
+    }
+    if (P.results)
+      P.results[hid] = r;
+    if (P.steps)
+      P.steps[hid] = p.nst;
+    if (P.scatters)
+      P.scatters[hid] = p.nsc;
+    mcg_count_end<STRICT>(s_cnt, r, p.wmc, p.wres, P.rules.q_log2);
+    tot_steps += p.nst;
+    tot_scat += p.nsc;
+  };
+  if constexpr (LANES)
+    mcg_lane_histories<STRICT, TALLY>(ncell, P.cells, TALLY == MCG_TALLY_GLOBAL ? P.tally : my_tally,
+                                      P.rules, T, P.libm, P.next, P.n, P.chunk, birth, end);
+  else
+    mcg_histories<STRICT, THIN, TALLY, false, false>(
+        geo, sink, P.cells, P.tab, my_tally, P.rules, tiles, s_real, T, P.libm, P.next,
+        [&] { return (long long)P.n; }, P.chunk, birth, end, [] { return true; }, [] { return false; });
 
   /* per-thread counters -> block */
   for (int o = 16; o > 0; o >>= 1) {
@@ -1710,8 +1756,12 @@ inline mcg_rules mcg_rules_setup(const mcg_context *ctx, float min_w)
 /* Grid of at most `resident` blocks, and the chunk of histories a warp takes:
  * a warp advances its histories together, one tile of each per round, so few
  * histories are spread over as many warps as there are. */
-inline int mcg_track_grid(int resident, int block, int64_t n, mcg_track_params &P)
+inline int mcg_track_grid(int resident, int block, int64_t n, bool lanes, mcg_track_params &P)
 {
+  if (lanes) { /* a lane per history */
+    P.chunk = 64;
+    return (int)std::min<int64_t>(resident, (n + block - 1) / block);
+  }
   const int64_t warps = (int64_t)resident * (block / 32);
   P.chunk = (int)std::min<int64_t>(32, (n + warps - 1) / warps);
   return (int)std::min<int64_t>(resident, n);

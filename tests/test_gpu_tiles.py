@@ -126,3 +126,37 @@ def test_async_workers_match_event_mode(mcg, mode, m, layers, width, n):
         assert np.array_equal(ctx.tally_q(), want)
         got = ctx.counters()
         assert all(got[k] == c[k] for k in ("histories", "steps", "scatters"))
+
+
+@pytest.mark.parametrize("mode", ["strict", "fast"])
+@pytest.mark.parametrize("m,layers,width", [(1, 1, 2.0), (16, 1, 0.3), (40, 3, 0.021), (40, 3, 0.019),
+                                            (300, 2, 0.1), (5000, 1, 1.0), (27_000, 1, 0.5)])
+def test_thick_chains_match_event_mode(mcg, mode, m, layers, width):
+    """Chains of thick cells run a lane per history (width: every cell's optical
+    width, on both sides of the rule's line and beyond the shared tally): host
+    particles and born ones, the weight cut-off and the tally modes."""
+    rng = np.random.default_rng(m)
+    st, lm, dx, _, _ = mcg.layer_decomposition(0.0, 1.0, m, layers)
+    sigs = np.full(m, 2 * width * m, f32)
+    rates = np.full(m, 0.5, f32)
+    with mcg.Context(mode=mode) as ctx:
+        for min_w, tally, launch in ((1e-12, 0, {}), (0.2, 1, dict(block=128)),
+                                     (1e-12, 2, dict(block=1024, blocks_per_sm=1))):
+            ctx.set_layers(st, lm, dx, sigs, rates, min_w)
+            ctx.set_tally_mode(tally)
+            ctx.set_launch(**launch)
+            p = _particles(mcg, rng, m, 1.0 / m, 700)
+            out = []
+            for algorithm in ("history", "event"):
+                ctx.set_algorithm(algorithm, 1)
+                ctx.tally_reset()
+                q = p.copy()
+                r = ctx.simulate(q)
+                ctx.simulate_source(3, 1500)
+                out.append((q, r, ctx.tally_q(), ctx.counters()))
+            (pa, ra, qa, ca), (pb, rb, qb, cb) = out
+            assert pa.tobytes() == pb.tobytes()
+            for key in ("results", "steps", "scatters"):
+                assert np.array_equal(ra[key], rb[key]), key
+            assert np.array_equal(qa, qb)
+            assert ca == cb
