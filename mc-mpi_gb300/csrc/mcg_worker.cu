@@ -27,6 +27,7 @@
 #include <cstdio>
 #include <cstdlib>
 #include <thread>
+#include <type_traits>
 #include <cstring>
 #include <vector>
 
@@ -533,8 +534,11 @@ __device__ __forceinline__ unsigned long long mcg_globaltimer()
  * ring has room for one particle of every lane of the block besides those it
  * holds (so it never overfills), else to the destination's global ring; idle
  * lanes take from it first. */
-#define MCG_LQ 1024
-#define MCG_LQ_BYTES (16 + MCG_LQ * (4 + 4 + (int)sizeof(mcg_particle)))
+static __host__ __device__ constexpr unsigned mcg_lq(bool tiles) { return tiles ? 1024u : 2048u; } /* its slots */
+static constexpr size_t mcg_lq_bytes(bool tiles)
+{
+  return 16 + mcg_lq(tiles) * (4 + 4 + sizeof(mcg_particle));
+}
 
 /* Rounds of the asynchronous workers: lanes without a particle that end a
  * round (8 to 20: within 1 % of each other; 4: 4 % slower), most tiles of a round;
@@ -543,41 +547,63 @@ __device__ __forceinline__ unsigned long long mcg_globaltimer()
  * take 7 % longer, 512 9 %. */
 #define MCG_AQ_ROUND_IDLE 12
 #define MCG_AQ_ROUND_TILES 16
+/* ... and of short sub-domains (fewer than MCG_AQ_SHORT cells each on average),
+ * where a tile is a few steps and a hand-over follows: a lane per particle through
+ * every step, MCG_AQ_WINDOW of them between two votes, at most
+ * MCG_AQ_ROUND_STEPS, and MCG_AQ_LANES_IDLE lanes that end the round, in blocks
+ * of 1024 threads.  2e6 histories, lanes / tiles: 8 cells each 2.0 / 3.5 ms
+ * (strict) and 2.2 / 3.9 (fast), 13 cells 2.2 / 2.9, 40 cells 4.2 / 2.7. */
+#define MCG_AQ_SHORT 24
+#define MCG_AQ_WINDOW 16
+#define MCG_AQ_ROUND_STEPS 256
+#define MCG_AQ_LANES_IDLE 4
 #define MCG_AQ_BLOCK 640
 
 /* Shared memory of the asynchronous workers: libm tables, the block's ring, the
  * sub-domains' ranges, jumps, the tally (64-bit words, or low words), tiles. */
-static size_t async_smem(int layers, size_t cells, int block, bool global, bool thin)
+static size_t async_smem(int layers, size_t cells, int block, bool global, bool thin, bool tiles)
 {
-  return mcg_track_smem(global ? 0 : cells, block, thin) + MCG_LQ_BYTES +
+  return mcg_track_smem(global ? 0 : cells, tiles ? block : 0, thin) + mcg_lq_bytes(tiles) +
          (size_t)((layers + 1) & ~1) * sizeof(int2);
 }
 
-/* TALLY and THIN as in mcg_track_kernel.  A warp advances its particles by the
+/* A warp's tiles, or nothing. */
+template <bool THIN, bool TILES> struct mcg_async_tiles : mcg_tile_warp<THIN> {
+  __device__ __forceinline__ mcg_async_tiles(mcg_tile_smem<THIN> *s, const mcg_real_jumps *J)
+      : mcg_tile_warp<THIN>(s, J)
+  {
+  }
+};
+template <bool THIN> struct mcg_async_tiles<THIN, false> {
+  __device__ __forceinline__ mcg_async_tiles(mcg_tile_smem<THIN> *, const mcg_real_jumps *) {}
+};
+
+/* TALLY and THIN as in mcg_track_kernel; TILES: see MCG_AQ_SHORT.  A warp advances its particles by the
  * tracker's tiles (mcg_advance); it was one lane per particle through the whole
  * step.  Bound: instruction issue, 80 warp instructions per step of 32 lanes (the
  * tracker's 54, and the rows of tiles that a sub-domain's end cuts short), with
  * the waits for the queues' global words.  10,000 cells in 64 sub-domains, 1e6
  * histories, strict: 65.2 ms -> 34.2 ms for the call. */
-template <bool STRICT, int TALLY, bool THIN>
-__global__ void __launch_bounds__(MCG_AQ_BLOCK) mcg_worker_async(mcg_async_params P)
+template <bool STRICT, int TALLY, bool THIN, bool TILES>
+__global__ void __launch_bounds__(TILES ? MCG_AQ_BLOCK : 1024) mcg_worker_async(mcg_async_params P)
 {
+  constexpr unsigned LQ = mcg_lq(TILES);
   extern __shared__ __align__(16) unsigned char smem[];
   mcg_libm_tab *T = reinterpret_cast<mcg_libm_tab *>(smem);
   /* local ring: head and tail tickets, publication words, sub-domain and
    * particle of every slot */
   unsigned *lq_ctl = reinterpret_cast<unsigned *>(smem + sizeof(mcg_libm_tab));
   unsigned *lq_seq = lq_ctl + 4;
-  int *lq_L = reinterpret_cast<int *>(lq_seq + MCG_LQ);
-  mcg_particle *lq_part = reinterpret_cast<mcg_particle *>(lq_L + MCG_LQ);
-  int2 *s_rng = reinterpret_cast<int2 *>(smem + sizeof(mcg_libm_tab) + MCG_LQ_BYTES); /* [n_layers] lo, hi local */
+  int *lq_L = reinterpret_cast<int *>(lq_seq + LQ);
+  mcg_particle *lq_part = reinterpret_cast<mcg_particle *>(lq_L + LQ);
+  int2 *s_rng = reinterpret_cast<int2 *>(lq_part + LQ); /* [n_layers] lo, hi local */
   mcg_chain_jumps *s_chain = reinterpret_cast<mcg_chain_jumps *>(s_rng + ((P.n_layers + 1) & ~1));
   mcg_real_jumps *s_real = reinterpret_cast<mcg_real_jumps *>(s_chain + 1);
   unsigned long long *s_tally = reinterpret_cast<unsigned long long *>(s_real + 1);
   const int tid = threadIdx.x, lane = tid & 31;
   const int words = TALLY == MCG_TALLY_GLOBAL ? 0 : THIN ? (P.n_cells + 1) / 2 : P.n_cells;
   mcg_tile_smem<THIN> *tile = reinterpret_cast<mcg_tile_smem<THIN> *>(
-      s_tally + ((words + 1) & ~1)) + (tid >> 5);
+      s_tally + ((words + 1) & ~1)) + (TILES ? tid >> 5 : 0);
   mcg_fill_chain_jumps(s_chain);
   mcg_fill_real_jumps(s_real);
   const int gwarp = (int)((blockIdx.x * blockDim.x + tid) >> 5);
@@ -588,13 +614,13 @@ __global__ void __launch_bounds__(MCG_AQ_BLOCK) mcg_worker_async(mcg_async_param
     s_rng[l] = make_int2(P.rings[l].lo - P.cell_lo, P.rings[l].hi - P.cell_lo);
   for (int i = tid; i < words; i += blockDim.x)
     s_tally[i] = 0ull;
-  for (int i = tid; i < MCG_LQ; i += blockDim.x)
-    lq_seq[i] = (unsigned)i; /* free for its first-lap ticket */
+  for (unsigned i = tid; i < LQ; i += blockDim.x)
+    lq_seq[i] = i; /* free for its first-lap ticket */
   if (tid < 4)
     lq_ctl[tid] = 0u;
   __syncthreads();
-  const mcg_tile_warp<THIN> tiles(tile, s_real);
   const mcg_sink sink = {(uint32_t)__cvta_generic_to_shared(s_tally), P.tally};
+  mcg_async_tiles<THIN, TILES> tiles(tile, s_real);
   const unsigned long long cap = P.cap;
   const int nl = P.n_layers;
   unsigned long long *const src_next = P.state + MCG_AQ_SRC_NEXT;
@@ -638,7 +664,7 @@ __global__ void __launch_bounds__(MCG_AQ_BLOCK) mcg_worker_async(mcg_async_param
         if ((int)(e - h) > 0) {
           const unsigned want = min((unsigned)__popc(need), e - h);
           const bool pub = (unsigned)lane < want &&
-                           *(volatile unsigned *)&lq_seq[(h + lane) % MCG_LQ] == h + lane + 1u;
+                           *(volatile unsigned *)&lq_seq[(h + lane) % LQ] == h + lane + 1u;
           const unsigned pm = __ballot_sync(0xffffffffu, pub);
           const int m = pm == 0xffffffffu ? 32 : __ffs(~pm) - 1;
           if (m > 0) {
@@ -649,7 +675,7 @@ __global__ void __launch_bounds__(MCG_AQ_BLOCK) mcg_worker_async(mcg_async_param
             if (got == h) {
               const int rank = __popc(need & lanemask_lt());
               if (((need >> lane) & 1u) && rank < m) {
-                const unsigned t = h + (unsigned)rank, sl = t % MCG_LQ;
+                const unsigned t = h + (unsigned)rank, sl = t % LQ;
                 int polls = 0;
                 while (*(volatile unsigned *)&lq_seq[sl] != t + 1u && ++polls < (1 << 16))
                   ;
@@ -659,7 +685,7 @@ __global__ void __launch_bounds__(MCG_AQ_BLOCK) mcg_worker_async(mcg_async_param
                 const mcg_particle q = lq_part[sl];
                 const int ql = lq_L[sl];
                 __threadfence_block();
-                *(volatile unsigned *)&lq_seq[sl] = t + (unsigned)MCG_LQ; /* next lap */
+                *(volatile unsigned *)&lq_seq[sl] = t + LQ; /* next lap */
                 p.x = q.x, p.mu = q.mu, p.wmc = q.wmc, p.idx = q.index - P.cell_lo;
                 enter(ql, q.seed);
               }
@@ -811,14 +837,37 @@ __global__ void __launch_bounds__(MCG_AQ_BLOCK) mcg_worker_async(mcg_async_param
      * no lane can step: the queues are visited when there is something to
      * hand over or to take, not every few steps */
     bool alive = active & p.living(P.rules);
-    for (int r = 0; r < MCG_AQ_ROUND_TILES; ++r) {
-      mcg_advance<STRICT, THIN, TALLY, false>(p, alive, false, P.cells, P.tab, sink, s_tally, 0, P.rules,
-                                              tiles, s_real, T, P.libm);
-      alive = active & p.living(P.rules);
-      const unsigned gb = __ballot_sync(0xffffffffu, alive);
-      const unsigned fb = __ballot_sync(0xffffffffu, active & !alive);
-      if (!gb || (fb && __popc(~gb) >= MCG_AQ_ROUND_IDLE))
-        break;
+    if constexpr (TILES) {
+      for (int r = 0; r < MCG_AQ_ROUND_TILES; ++r) {
+        mcg_advance<STRICT, THIN, TALLY, false>(p, alive, false, P.cells, P.tab, sink, s_tally, 0,
+                                                P.rules, tiles, s_real, T, P.libm);
+        alive = active & p.living(P.rules);
+        const unsigned gb = __ballot_sync(0xffffffffu, alive);
+        const unsigned fb = __ballot_sync(0xffffffffu, active & !alive);
+        if (!gb || (fb && __popc(~gb) >= MCG_AQ_ROUND_IDLE))
+          break;
+      }
+    } else {
+      unsigned long long *const tally = TALLY == MCG_TALLY_GLOBAL ? P.tally : s_tally;
+      const uint32_t stop_at = p.nst + min(P.rules.max_steps - p.nst, (uint32_t)MCG_AQ_ROUND_STEPS);
+      uint64_t seed = p.s2 >> 1;
+      p.a0 = 0.0f; /* x is always known */
+      for (;;) {
+        bool go = alive & (p.nst < stop_at);
+        for (int j = 0; go & (j < MCG_AQ_WINDOW); ++j) {
+          mcg_step<STRICT, TALLY, false>(seed, p.x, p.mu, p.wmc, p.inv_mu, p.idx, p.nsc,
+                                         __ldg(P.cells + p.idx), &tally[p.idx], P.rules.q_log2, T,
+                                         P.libm);
+          ++p.nst;
+          alive = p.living(P.rules);
+          go = alive & (p.nst < stop_at);
+        }
+        const unsigned gb = __ballot_sync(0xffffffffu, go);
+        const unsigned fb = __ballot_sync(0xffffffffu, active & !go);
+        if (!gb || (fb && __popc(~gb) >= MCG_AQ_LANES_IDLE))
+          break;
+      }
+      p.s2 = seed << 1;
     }
     if (active) {
       if (!alive) {
@@ -849,7 +898,7 @@ __global__ void __launch_bounds__(MCG_AQ_BLOCK) mcg_worker_async(mcg_async_param
       }
       h = __shfl_sync(0xffffffffu, h, 0);
       e = __shfl_sync(0xffffffffu, e, 0);
-      local = e - h <= MCG_LQ - blockDim.x;
+      local = e - h <= LQ - blockDim.x;
     }
     if (local && finished && dir != 0) {
       const int leader = __ffs(movers) - 1;
@@ -857,7 +906,7 @@ __global__ void __launch_bounds__(MCG_AQ_BLOCK) mcg_worker_async(mcg_async_param
       if (lane == leader)
         base = atomicAdd(&lq_ctl[1], (unsigned)__popc(movers));
       base = __shfl_sync(movers, base, leader);
-      const unsigned t = base + __popc(movers & lanemask_lt()), sl = t % MCG_LQ;
+      const unsigned t = base + __popc(movers & lanemask_lt()), sl = t % LQ;
       /* the slot's previous occupant is claimed; its reader frees it at once */
       int polls = 0;
       while (*(volatile unsigned *)&lq_seq[sl] != t && ++polls < (1 << 16))
@@ -995,18 +1044,25 @@ extern "C" int mcg_worker_run_async(mcg_context *ctx, const mcg_source *src, int
   /* the largest block whose tiles fit beside the tally; the global tally where
    * not even 256 threads' do */
   bool thin = strict ? ctx->thin : ctx->thin_fast, global = false;
-  int block = MCG_AQ_BLOCK;
-  auto smem_of = [&] { return async_smem(P_, (size_t)ctx->n_cells, block, global, thin); };
-  while (block > 256 && smem_of() > (size_t)ctx->smem_optin)
-    block -= 128;
-  if (smem_of() > (size_t)ctx->smem_optin) {
+  int block = 1024;
+  auto smem_of = [&](bool t) { return async_smem(P_, (size_t)ctx->n_cells, block, global, thin, t); };
+  const bool tiled = (int64_t)ctx->n_cells >= (int64_t)MCG_AQ_SHORT * P_ ||
+                     async_smem(P_, 0, 1024, true, false, false) > (size_t)ctx->smem_optin;
+  if (tiled) {
+    block = MCG_AQ_BLOCK;
+    while (block > 256 && smem_of(true) > (size_t)ctx->smem_optin)
+      block -= 128;
+  } else {
+    thin = false;
+  }
+  if (smem_of(tiled) > (size_t)ctx->smem_optin) {
     global = true;
     thin = false;
-    block = MCG_AQ_BLOCK;
-    while (block > 128 && smem_of() > (size_t)ctx->smem_optin)
+    block = tiled ? MCG_AQ_BLOCK : 1024;
+    while (tiled && block > 128 && smem_of(true) > (size_t)ctx->smem_optin)
       block -= 128;
   }
-  const size_t smem = smem_of();
+  const size_t smem = smem_of(tiled);
   if (smem > (size_t)ctx->smem_optin)
     return mcg_fail(MCG_ERR_ARG, "mcg_worker_run_async: %d sub-domains too many", P_);
   mcg_async_params A;
@@ -1033,12 +1089,15 @@ extern "C" int mcg_worker_run_async(mcg_context *ctx, const mcg_source *src, int
   /* the launch's deadline: 30 s plus 2 us per history (the benchmark slab
    * runs a history in about 40 ns of GPU time) */
   A.budget_ns = 30000000000ull + 2000ull * (unsigned long long)n;
-  auto kern = strict ? (thin     ? mcg_worker_async<true, MCG_TALLY_LO32, true>
-                        : global ? mcg_worker_async<true, MCG_TALLY_GLOBAL, false>
-                                 : mcg_worker_async<true, MCG_TALLY_SMEM32, false>)
-                     : (thin     ? mcg_worker_async<false, MCG_TALLY_LO32, true>
-                        : global ? mcg_worker_async<false, MCG_TALLY_GLOBAL, false>
-                                 : mcg_worker_async<false, MCG_TALLY_SMEM32, false>);
+  auto pick = [&](auto S) {
+    constexpr bool X = decltype(S)::value;
+    return thin     ? mcg_worker_async<X, MCG_TALLY_LO32, true, true>
+           : tiled  ? (global ? mcg_worker_async<X, MCG_TALLY_GLOBAL, false, true>
+                              : mcg_worker_async<X, MCG_TALLY_SMEM32, false, true>)
+           : global ? mcg_worker_async<X, MCG_TALLY_GLOBAL, false, false>
+                    : mcg_worker_async<X, MCG_TALLY_SMEM32, false, false>;
+  };
+  auto kern = strict ? pick(std::true_type()) : pick(std::false_type());
   int bps = 1;
   if ((e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                 ctx->smem_optin)) != cudaSuccess ||
