@@ -157,7 +157,7 @@ __global__ void __launch_bounds__(1024) mcg_adjoint_forward(mcg_adj_params P)
  * mcg_cross decide without the logarithm, the exponential's table or the new
  * direction, so the few full steps are gathered (the rounds below) instead of
  * stopping the whole warp for one lane.  1000 cells, 2e6 histories, strict:
- * 20 ms; with the full step in every lane, forward pass and replay took 69.2 ms.
+ * 19 ms; with the full step in every lane, forward pass and replay took 69.2 ms.
  * A history stays with a lane, and 512 lanes share one fp32 accumulator per
  * cell: tiles, as the forward pass has, add a cell's terms in another grouping,
  * which moved the gradients by more than two runs of this kernel differ (and

@@ -49,9 +49,9 @@ __global__ void __launch_bounds__(1024) mcg_fit_forward(mcg_batch_params P)
  * Replay of every history for dG/dsig_a: rounds, history starts and the reason
  * for a lane per history are those of the adjoint's replay.  Bound: instruction
  * issue, with the float atomics' compare-and-swap loops.  64 slabs of up to 1024
- * cells, 1e5 histories each: 26 ms.  Five Adam steps, with the forward pass that
+ * cells, 1e5 histories each: 25 ms.  Five Adam steps, with the forward pass that
  * starts them: 337 ms with forward pass and replay in one kernel of full steps,
- * 235 ms so.
+ * 230 ms so.
  */
 __global__ void __launch_bounds__(512, 2) mcg_fit_replay(mcg_fit_params P)
 {
