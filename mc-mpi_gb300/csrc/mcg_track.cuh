@@ -856,11 +856,21 @@ __device__ __forceinline__ uint32_t mcg_shared_add_if(bool p, uint32_t addr, uin
   return old;
 }
 
+/* The lesser of two floats, NaN if either is. */
+__device__ __forceinline__ float mcg_min_nan(float a, float b)
+{
+  float r;
+  asm("min.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
+  return r;
+}
+
 /* Phase 2 for U passes of F flights from pass q0.  All loads come before the
  * first store, which the compiler could not tell apart from the next pass's
  * rows: 4 passes in flight instead of 1 took the 10,000-cell slab from 131 to
  * 110 ms per 5e6 histories (the table's L1 misses).  Rows past the last flight
- * are computed and never used. */
+ * are computed and never used.  The minimum keeps a cell's NaN length (a step for
+ * the full form): on flights under way fminf made it inf, which the fast thin
+ * form, testing the collision bound alone, accepted. */
 template <bool STRICT, bool THIN, int U, bool LOSS>
 __device__ __forceinline__ void mcg_tile_form(mcg_tile_smem<THIN> *S, int q0, const mcg_tab &tab,
                                               const mcg_tile_warp<THIN> &B,
@@ -868,7 +878,6 @@ __device__ __forceinline__ void mcg_tile_form(mcg_tile_smem<THIN> *S, int q0, co
 {
   constexpr int G = mcg_tile_shape<THIN>::G, F = 32 / G, PLANE = mcg_tile_shape<THIN>::PLANE;
   const int lane = threadIdx.x & 31, sub = lane / G, j = lane & (G - 1);
-  const int not_first = j ? 0x7f800000 : 0; /* makes the first length inf or NaN: not the least */
   int4 pl[U];
   uint4 fl[U];
   ulonglong2 sl[U];
@@ -904,7 +913,7 @@ __device__ __forceinline__ void mcg_tile_form(mcg_tile_smem<THIN> *S, int q0, co
     const uint64_t n0 = B.A0 * s + B.C0, n1 = B.A1 * s + B.C1;
     mcg_f2 nde;
     mcg_tile_steps<STRICT, THIN>(
-        f2_make(fminf(a[v], __int_as_float(pl[v].x | not_first)), b[v]), sl[v].x, sl[v].y,
+        f2_make(mcg_min_nan(a[v], __int_as_float(j ? 0x7f800000 : pl[v].x)), b[v]), sl[v].x, sl[v].y,
         f2_make(sa0[v], sa1[v]), f2_make(si0[v], si1[v]), (uint32_t)(n0 >> 32),
         (uint32_t)(n1 >> 32), __uint_as_float(fl[v].z), __uint_as_float(fl[v].w), R, om0[v], om1[v],
         nde);
