@@ -340,12 +340,17 @@ void mcg_cell_params(float sig, float rate, int gi, float dx, float4 &strict, fl
  * cached-reciprocal division is exact, and those of cells that would amplify
  * the weight, are NaN: such steps take the full form.
  * sig_i <= EPS is 0 in both arithmetics: the flight always crosses. */
+static inline float4 tile_entry(const float4 *c, int n, int k)
+{
+  auto length = [&](float a) { return a >= 0x1p-90f && a <= 0x1p90f && c[k].x >= 0.0f ? a : NAN; };
+  return make_float4(c[k].x, c[k].y, length(c[k].w - (k ? c[k - 1].w : c[k].z)),
+                     length((k + 1 < n ? c[k + 1].z : c[k].w) - c[k].z));
+}
+
 void mcg_tile_table(const float4 *c, int n, float4 *tab, float2 *right, float2 *left)
 {
   for (int k = 0; k < n; ++k) {
-    auto length = [&](float a) { return a >= 0x1p-90f && a <= 0x1p90f && c[k].x >= 0.0f ? a : NAN; };
-    tab[k] = make_float4(c[k].x, c[k].y, length(c[k].w - (k ? c[k - 1].w : c[k].z)),
-                         length((k + 1 < n ? c[k + 1].z : c[k].w) - c[k].z));
+    tab[k] = tile_entry(c, n, k);
     if (right) {
       right[k] = make_float2(tab[k].x, tab[k].z);
       left[k] = make_float2(tab[k].x, tab[k].w);
@@ -353,8 +358,8 @@ void mcg_tile_table(const float4 *c, int n, float4 *tab, float2 *right, float2 *
   }
 }
 
-/* thin: every cell's absorption optical width sig_a (edge_hi - edge_lo) is at
- * most 2e-4, so that a crossing has u >= MCG_OM_THIN_MAX (2^-8) only for
+/* thin: every cell's absorption optical width, sig_a times the longer of its
+ * tile lengths, is at most 2e-4, so that a crossing has u >= MCG_OM_THIN_MAX (2^-8) only for
  * |mu| < 0.05, 0.3 % of the crossings (their share of directions is about
  * mu^2), which go to the full step; thin_fast: both optical widths at most
  * 4e-4 (the short series, below 2^-7, again for |mu| > 0.05).  A transparent
@@ -368,12 +373,21 @@ static void update_thin(mcg_context *ctx)
   double depth = 0.0; /* of the chain, both cross sections */
   for (const float4 &c : ctx->cells_strict) {
     depth += ((double)std::fabs(c.x) + std::fabs(c.y)) * ((double)c.w - c.z);
-    wa = std::max(wa, std::fabs(c.x) * (c.w - c.z));
-    wi = std::max(wi, std::fabs(c.y) * (c.w - c.z));
   }
-  /* 1 %: a cell entered at a neighbour's face may be a few ulps of x wider */
-  ctx->width_a = 1.01f * wa;
-  ctx->width_i = 1.01f * wi;
+  /* the widths that bound a whole flight (mcg_thin_tests): of the lengths that
+   * the tiles use, since a cell entered from another layer's face may be wider
+   * than its own faces are apart (3.7 % at some sub-domains' ends of 10,000
+   * cells in 64, without limit between layers of different spacing).  A NaN
+   * length has no step in the tiles. */
+  const int n = (int)ctx->cells_strict.size();
+  for (int k = 0; k < n; ++k) {
+    const float4 t = tile_entry(ctx->cells_strict.data(), n, k);
+    const float len = std::fmax(std::fmax(t.z, t.w), 0.0f);
+    wa = std::max(wa, std::fabs(t.x) * len);
+    wi = std::max(wi, std::fabs(t.y) * len);
+  }
+  ctx->width_a = wa;
+  ctx->width_i = wi;
   ctx->thin = !ctx->cells_strict.empty() && wa <= (depth < 1.2 ? 7e-5f : 2e-4f);
   ctx->thin_fast = !ctx->cells_strict.empty() && std::max(wa, wi) <= 4e-4f;
   ctx->thick = mcg_thick(ctx->cells_strict.data(), (int)ctx->cells_strict.size(), true);

@@ -816,7 +816,7 @@ __device__ __forceinline__ void mcg_tile_steps(mcg_f2 a, mcg_f2 amu, mcg_f2 ny, 
 }
 
 /* The bounds of a flight on a thin chain from its widest cell (R.w_a, R.w_i:
- * the chain's largest sig_a and sig_i widths): {thr, bound} of
+ * the chain's largest sig_a and sig_i widths, over the lengths of the table): {thr, bound} of
  * mcg_tile_steps, which no step passes when the flight is so slanted that its
  * steps may leave the thin form's range or its first deposit 31 bits.  The
  * factor covers the roundings of the lengths and products. */

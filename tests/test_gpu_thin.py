@@ -64,3 +64,51 @@ def test_cells_without_a_tile_length(mcg, mode, m, sign):
         assert c["histories"] == 3000
         if sign < 0:
             assert (q < 0).sum() == (sa < 0).sum()
+
+
+@pytest.mark.parametrize("mode", ["strict", "fast"])
+def test_fine_decomposition(mcg, mode):
+    """1000 sub-domains of 20 cells, as the library decomposes the slab: the
+    layers' float32 faces do not meet, and some cells have no length."""
+    m, layers = 20_000, 1000
+    st, lm, dx, _, _ = mcg.layer_decomposition(0.0, 1.0, m, layers)
+    left, right = _entry_widths(st, lm, dx)
+    assert min(left.min(), right.min()) <= 0
+    rng = np.random.default_rng(3)
+    sa, ss = rng.uniform(0.2, 1.0, (2, m)) * 1e-4 * m
+    with mcg.Context(mode=mode) as ctx:
+        ctx.set_layers_xs(st, lm, dx, sa, ss, 1e-12)
+        _same_as_event_mode(ctx, 2000)
+
+
+@pytest.mark.parametrize("mode", ["strict", "fast"])
+@pytest.mark.parametrize("gap", [0.5, 3.0])
+def test_cells_wider_from_the_next_layer(mcg, mode, gap):
+    """50 layers, each a little coarser than the one before, so that a layer
+    starts `gap` cells after the previous one ends: those cells are entered from
+    farther away than they are wide, in both directions."""
+    m, k = 1000, 20
+    st = np.arange(0, m, k)
+    dx = (1.0 / m) * np.cumprod(np.concatenate([[1.0], 1 + gap / st[1:]]))
+    left, right = _entry_widths(st, np.full(m // k, k), dx)
+    assert min((w > 1 + 0.9 * gap).sum() for w in (left, right)) >= m // k - 3
+    wide = dx.repeat(k)
+    # strict thin chains may scatter strongly, fast ones are thin in both
+    wa, ws = (1e-4, 2e-2) if mode == "strict" else (3e-4, 3e-4)
+    with mcg.Context(mode=mode) as ctx:
+        ctx.set_layers_xs(st, np.full(m // k, k), dx, wa / wide, ws / wide, 1e-12)
+        _same_as_event_mode(ctx, 2000 if mode == "strict" else 400_000)
+
+
+@pytest.mark.parametrize("mode", ["strict", "fast"])
+def test_uniform_decomposed_slab(mcg, mode):
+    """12,000 equal cells in 64 sub-domains: a few per cent wider at some of the
+    sub-domains' ends."""
+    m = 12_000
+    st, lm, dx, _, _ = mcg.layer_decomposition(0.0, 1.0, m, 64)
+    left, right = _entry_widths(st, lm, dx)
+    assert max(left.max(), right.max()) > 1.02
+    wa, ws = (5e-5, 2e-3) if mode == "strict" else (5e-5, 3.9e-4)
+    with mcg.Context(mode=mode) as ctx:
+        ctx.set_layers_xs(st, lm, dx, np.full(m, wa * m), np.full(m, ws * m), 1e-12)
+        _same_as_event_mode(ctx, 20_000)
