@@ -391,7 +391,10 @@ extern "C" int mcg_batch_run(mcg_context *ctx)
     return mcg_sync(ctx);
   }
   cudaError_t e;
-  if (!B->graph_valid) {
+  /* mcg_set_mode, _tally_scale, _launch and _step_limit leave the graph alone */
+  if (!B->graph_valid || B->graph_mode != ctx->mode || B->graph_scale != ctx->log2_scale ||
+      B->graph_refill != ctx->refill || B->graph_steps != ctx->max_steps) {
+    B->graph_valid = false;
     if (B->graph) {
       cudaGraphExecDestroy(B->graph);
       B->graph = nullptr;
@@ -412,6 +415,10 @@ extern "C" int mcg_batch_run(mcg_context *ctx)
     cudaGraphDestroy(g);
     if (e != cudaSuccess)
       return mcg_cuda_fail(e, "mcg_batch_run: instantiate");
+    B->graph_mode = ctx->mode;
+    B->graph_scale = ctx->log2_scale;
+    B->graph_refill = ctx->refill;
+    B->graph_steps = ctx->max_steps;
     B->graph_valid = true;
   }
   cudaEventRecord(ctx->ev0, ctx->stream);

@@ -39,6 +39,9 @@ struct mcg_batch_state {
   /* CUDA graph of one run (memset of the item counter + the kernel) */
   cudaGraphExec_t graph = nullptr;
   bool graph_valid = false;
+  /* the context's settings that the graph's kernel holds by value */
+  int graph_mode = -1, graph_scale = 0, graph_refill = 0;
+  uint32_t graph_steps = 0;
   int64_t items_built_for = -1; /* item size, grid and share of the histories the list is for */
   int items_grid = 0;
   double items_fraction = 1.0;

@@ -1,0 +1,57 @@
+"""Settings and state that outlive one call: what a context keeps between runs
+must follow its setters, and contexts must not disturb one another."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+f32 = np.float32
+
+
+def _batch(n_slabs=12, low=10, high=200, histories=500, seed=3):
+    rng = np.random.default_rng(seed)
+    cells = rng.integers(low, high + 1, n_slabs)
+    total = int(cells.sum())
+    slabs = [dict(n_cells=int(k), n_histories=histories, base_seed=31 + s, seed_mode=s % 2,
+                  isotropic=s % 3, mu0=1.0, w0=1.0) for s, k in enumerate(cells)]
+    return slabs, rng.uniform(0.5, 5, total).astype(f32), rng.uniform(0.1, 0.9, total).astype(f32)
+
+
+@pytest.mark.parametrize("first", ["strict", "fast"])
+def test_batch_follows_settings_made_after_its_first_run(mcg, first):
+    """The captured graph holds the arithmetic, the tally scale, the step limit
+    and the tile window by value: after each setter a run gives what a fresh
+    context with those settings gives."""
+    slabs, sigs, rates = _batch()
+    other = {"strict": "fast", "fast": "strict"}[first]
+
+    def fresh(mode, scale, limit):
+        with mcg.Context(mode=mode) as c:
+            c.set_tally_scale(scale)
+            mcg._check(c.lib.mcg_set_step_limit(c.h, limit))
+            c.batch_set(slabs, sigs, rates, 1e-12)
+            try:
+                c.batch_run()
+                code = 0
+            except mcg.MCGError as e:
+                code = e.code
+            return c.batch_tally_q(), c.counters()["steps"], code
+
+    with mcg.Context(mode=first) as c:
+        c.batch_set(slabs, sigs, rates, 1e-12)
+        c.batch_run()
+        for mode, scale, limit, window in ((first, 33, 1 << 28, 0), (other, 33, 1 << 28, 5),
+                                           (other, 33, 40, 5), (first, 40, 1 << 28, 0)):
+            c.set_mode(mode)
+            c.set_tally_scale(scale)
+            mcg._check(c.lib.mcg_set_step_limit(c.h, limit))
+            c.set_launch(refill_steps=window)
+            c.batch_tally_reset()
+            try:
+                c.batch_run()
+                code = 0
+            except mcg.MCGError as e:
+                code = e.code
+            q, steps, want = fresh(mode, scale, limit)
+            assert np.array_equal(c.batch_tally_q(), q)
+            assert (c.counters()["steps"], code) == (steps, want)
+            assert (code != 0) == (limit == 40)
