@@ -295,8 +295,9 @@ static int batch_configure(mcg_context *ctx, mcg_batch_state *B, int64_t item, d
   else
     L.kern = tm == MCG_TALLY_GLOBAL ? mcg_batch_kernel<false, MCG_TALLY_GLOBAL>
                                     : mcg_batch_kernel<false, MCG_TALLY_SMEM64>;
+  /* the opt-in maximum on every call (mcg_track_launch) */
   cudaError_t e = cudaFuncSetAttribute(L.kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       (int)L.smem);
+                                       ctx->smem_optin);
   int bps = 0;
   if (e == cudaSuccess)
     e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, L.kern, L.block, L.smem);
@@ -471,7 +472,7 @@ extern "C" int mcg_batch_run_per_slab(mcg_context *ctx)
                        : (shape.global ? mcg_track_kernel<false, MCG_TALLY_GLOBAL, false>
                                        : mcg_track_kernel<false, MCG_TALLY_SMEM32, false>);
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)smem);
+                                         ctx->smem_optin);
     int bps = 1;
     if (e == cudaSuccess)
       e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, kern, block, smem);

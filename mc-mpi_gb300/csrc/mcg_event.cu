@@ -571,11 +571,11 @@ static int ev_run_t(mcg_context *ctx, mcg_ev_params &P, unsigned long long total
   if (e != cudaSuccess)
     return mcg_cuda_fail(e, "event counters");
   const size_t smem = SMEM ? (size_t)P.n_cells * 8 : 0;
-  if (SMEM)
+  if (SMEM) /* half the opt-in maximum, mcg_event_run's limit, on every call (mcg_track_launch) */
     for (const void *k : {(const void *)mcg_ev_flight_kernel<STRICT, SLABS, SMEM>,
                           (const void *)mcg_ev_drain_kernel<STRICT, SLABS, SMEM>})
-      if ((e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)) !=
-          cudaSuccess)
+      if ((e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                    ctx->smem_optin / 2)) != cudaSuccess)
         return mcg_cuda_fail(e, "event kernels: shared memory");
   int bps = 1;
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, mcg_ev_flight_kernel<STRICT, SLABS, SMEM>,

@@ -1254,12 +1254,12 @@ template <typename K>
 static cudaError_t mcg_grad_shape(K kern, int block, int limit, size_t *smem, int32_t *jumps, int *bps)
 {
   const size_t more = (*smem + 7) / 8 * 8 + sizeof(mcg_chain_jumps);
-  const size_t top = more <= (size_t)limit ? more : *smem;
-  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)top);
+  /* the opt-in maximum on every call (mcg_track_launch) */
+  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, limit);
   if (e == cudaSuccess)
     e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(bps, kern, block, *smem);
   int with = 0;
-  if (e == cudaSuccess && top == more)
+  if (e == cudaSuccess && more <= (size_t)limit)
     e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&with, kern, block, more);
   *jumps = with > 0 && with == *bps;
   if (*jumps)

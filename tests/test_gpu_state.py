@@ -1,5 +1,7 @@
 """Settings and state that outlive one call: what a context keeps between runs
 must follow its setters, and contexts must not disturb one another."""
+import threading
+
 import numpy as np
 import pytest
 
@@ -55,3 +57,63 @@ def test_batch_follows_settings_made_after_its_first_run(mcg, first):
             assert np.array_equal(c.batch_tally_q(), q)
             assert (c.counters()["steps"], code) == (steps, want)
             assert (code != 0) == (limit == 40)
+
+
+@pytest.mark.parametrize("kind", ["batch", "per_slab", "adjoint", "fit", "event"])
+def test_contexts_of_two_threads_do_not_lower_each_others_shared_memory(mcg, kind):
+    """A launch's limit of shared memory belongs to the kernel, not to the
+    context: one host thread runs small problems while another runs large ones of
+    the same kernels.  A lowered limit is a failed launch (an error code)."""
+    def runner(m, n):
+        c = mcg.Context(mode="fast")
+        sa = np.full(m, 0.002 * m, f32)
+        slabs = [dict(n_cells=m, n_histories=n, base_seed=5, seed_mode=0, isotropic=0, mu0=1.0, w0=1.0)]
+        if kind in ("batch", "per_slab"):
+            c.batch_set(slabs, 2 * sa, np.full(m, 0.5, f32), 1e-12)
+
+            def run():
+                if kind == "per_slab":
+                    c.batch_run_per_slab()
+                    return
+                c.batch_set_launch(block=512)  # configured and captured anew
+                c.batch_run()
+        elif kind == "fit":
+            c.fit_set(slabs, sa, sa, np.zeros(m), max_steps=1)
+
+            def run():
+                c.fit_gradient(np.ones(m))
+        else:
+            c.set_layers_xs([0], [m], [f32(1.0 / m)], sa, sa, 1e-12)
+            if kind == "event":
+                c.set_algorithm("event", 4)
+
+                def run():
+                    c.simulate_source(0, n)
+            else:
+                c.adjoint_set_weights(np.ones(m, f32))
+
+                def run():
+                    c.adjoint_run(0, n)
+        return c, run
+
+    failed = []
+
+    def loop(run, times):
+        try:
+            for _ in range(times):
+                run()
+        except mcg.MCGError as e:
+            failed.append(str(e))
+
+    (a, small), (b, large) = runner(300, 20), runner(10_000, 20)
+    try:
+        times = 100 if kind == "event" else 400
+        threads = [threading.Thread(target=loop, args=(f, times)) for f in (small, large)]
+        for t in threads:
+            t.start()
+        for t in threads:
+            t.join()
+    finally:
+        a.close()
+        b.close()
+    assert not failed
