@@ -6,12 +6,12 @@
  *   uint32_t log_pairs[2 * n_log]   (argument bits, host logf result bits)
  *   uint32_t exp_pairs[2 * n_exp]   (argument bits, host expf result bits)
  *
- * The fingerprint hashes the host library's logf/expf, and the float-float
- * evaluators of exact_libm.h (value and midpoint distance), on a fixed set
- * of arguments; the loader recomputes it, so a table made against another C
- * library (another machine) or by another version of the evaluators is
- * refused instead of silently used.  Host-only header; include exact_libm.h
- * first.
+ * The fingerprint hashes the host library's logf/expf, the float-float
+ * evaluators of exact_libm.h (value and midpoint distance) and its short forms
+ * (value, residue, acceptance bounds), on a fixed set of arguments; the loader
+ * recomputes it, so a table made against another C library (another machine) or
+ * by another version of the forms is refused instead of silently used.
+ * Host-only header; include exact_libm.h first.
  */
 #ifndef MCG_LIBM_FILE_H
 #define MCG_LIBM_FILE_H
@@ -99,7 +99,9 @@ static inline uint64_t mcg_fnv_word(uint64_t h, float v)
 
 /* FNV-1a over the bits of logf/expf and of the evaluators at 8192
  * arguments spread over both domains by a 32-bit LCG (the exp arguments
- * cover both evaluator paths and both signs). */
+ * cover both evaluator paths and both signs), and of the short forms with
+ * their residues and acceptance bounds: a table is only good for the forms that
+ * were checked when it was made. */
 static inline uint64_t mcg_libm_fingerprint(const mcg_libm_tab *T)
 {
   uint64_t h = 1469598103934665603ull;
@@ -114,6 +116,28 @@ static inline uint64_t mcg_libm_fingerprint(const mcg_libm_tab *T)
     h = mcg_fnv_word(h, (i & 1) ? expf(t) : logf(x));
     h = mcg_fnv_word(h, (i & 1) ? mcg_exp_ff(t, &d, T) : mcg_log_ff(x, &d, T));
     h = mcg_fnv_word(h, d);
+  }
+  float tau[MCG_TAU_BUCKETS]; /* some distances, growing with u^2: the bounds' formula counts */
+  for (uint32_t b = 0; b < MCG_TAU_BUCKETS; ++b) {
+    float lo;
+    uint32_t ul = (b << 19) & 0x7fffffffu;
+    memcpy(&lo, &ul, 4);
+    tau[b] = lo >= 0x1p-14f && lo < MCG_OM_MID_MAX ? (float)(1 + b % 7) * (lo * lo) : -1.0f;
+  }
+  const mcg_run_bounds_t B = mcg_run_bounds(tau);
+  h = mcg_fnv_word(mcg_fnv_word(mcg_fnv_word(h, B.b_thin), B.c_thin), B.b_mid);
+  h = mcg_fnv_word(mcg_fnv_word(h, MCG_OM_THIN_MAX), MCG_OM_MID_MAX);
+  for (int i = 0; i < 8192; ++i) {
+    float u, r;
+    s = s * 1664525u + 1013904223u;
+    uint32_t ux = 0x33800000u + (s >> 2) % (0x3d800000u - 0x33800000u); /* [2^-24, 2^-4) */
+    memcpy(&u, &ux, 4);
+    h = mcg_fnv_word(h, mcg_om_mid(u, u * u, &r));
+    h = mcg_fnv_word(h, r);
+    if (u < MCG_OM_THIN_MAX) {
+      h = mcg_fnv_word(h, mcg_om_thin(u, u * u, &r));
+      h = mcg_fnv_word(h, r);
+    }
   }
   return h;
 }
