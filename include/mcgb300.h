@@ -396,7 +396,9 @@ int mcg_rnd_real_device(mcg_context *ctx, uint64_t *d_seeds, float *d_reals, int
  * fn 4 the hardware log2, fn 5 the fast arithmetic's collision probability
  * 1 - e^-tau of a flight of optical depth tau >= 0, fn 6 the fast
  * arithmetic's log2 of the flight sample whose state has top 32 bits t
- * (t passed as the argument's bit pattern). */
+ * (t passed as the argument's bit pattern); fn 7, 8, 9 the absorbed fraction
+ * 1 - e^-u of a step of optical width u in the tiles' packed arithmetic (strict
+ * on thin chains, strict, fast), NaN where the tiles leave it to the full step. */
 int mcg_libm_eval_device(mcg_context *ctx, int fn, const float *d_in, float *d_out, int64_t n);
 
 /* Check of the strict tracker's division by a cached reciprocal against the

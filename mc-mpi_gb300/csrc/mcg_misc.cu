@@ -1,11 +1,11 @@
 /*
  * mcg_misc.cu - small device entry points: the reference's rnd_real kernel
  * (src/curandom.cu:7-14), an evaluator of the strict libm, used to check
- * the device arithmetic against the host C library exhaustively, and the
- * check of the tracker's division by a cached reciprocal.
+ * the device arithmetic against the host C library exhaustively, with the
+ * tiles' packed absorption forms, and the check of the tracker's division by a cached reciprocal.
  */
 #include "mcg_internal.h"
-
+#include "mcg_track.cuh"
 
 __global__ void mcg_rnd_real_kernel(uint64_t *seeds, float *reals, int64_t n)
 {
@@ -57,6 +57,32 @@ __global__ void mcg_libm_eval_kernel(int fn, const float *in, float *out, int64_
   }
 }
 
+/* The tiles' absorbed fraction of optical width v (mcg_tile_steps: a cell of
+ * sig_a = v and sig_i = 0, crossed over a length of one by a flight that no
+ * sample ends), NaN where it is left to the full step; fn 7 strict and thin, 8
+ * strict, 9 fast.  Even arguments in the first half of the pair, odd ones in the
+ * second. */
+__global__ void mcg_tile_eval_kernel(int fn, const float *in, float *out, int64_t n, mcg_run_consts R)
+{
+  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n;
+       i += (int64_t)gridDim.x * blockDim.x) {
+    const float v = in[i], other = in[n - 1 - i];
+    const mcg_f2 one = f2_both(1.0f), rcp = f2_both(-1.0f);
+    const mcg_f2 sig_a = i & 1 ? f2_make(other, v) : f2_make(v, other);
+    const float bound = __fmaf_rn(__fmul_rn(v, v), -R.c_thin, R.b_thin); /* mcg_thin_tests */
+    float om0, om1;
+    mcg_f2 nde;
+    if (fn == 7)
+      mcg_tile_steps<true, true>(one, one, rcp, sig_a, f2_both(0.0f), 0u, 0u,
+                                 v < MCG_OM_THIN_MAX ? MCG_TILE_K : -1.0f, bound, R, om0, om1, nde);
+    else if (fn == 8)
+      mcg_tile_steps<true, false>(one, one, rcp, sig_a, f2_both(0.0f), 0u, 0u, 0.0f, 0.0f, R, om0, om1, nde);
+    else
+      mcg_tile_steps<false, false>(one, one, rcp, sig_a, f2_both(0.0f), 0u, 0u, 0.0f, 0.0f, R, om0, om1, nde);
+    out[i] = -(i & 1 ? om1 : om0);
+  }
+}
+
 extern "C" int mcg_rnd_real_device(mcg_context *ctx, uint64_t *d_seeds, float *d_reals, int64_t n)
 {
   if (!ctx || n < 0 || (n > 0 && (!d_seeds || !d_reals)))
@@ -75,7 +101,7 @@ extern "C" int mcg_rnd_real_device(mcg_context *ctx, uint64_t *d_seeds, float *d
 extern "C" int mcg_libm_eval_device(mcg_context *ctx, int fn, const float *d_in, float *d_out,
                                     int64_t n)
 {
-  if (!ctx || fn < 0 || fn > 6 || n < 0 || (n > 0 && (!d_in || !d_out)))
+  if (!ctx || fn < 0 || fn > 9 || n < 0 || (n > 0 && (!d_in || !d_out)))
     return mcg_fail(MCG_ERR_ARG, "mcg_libm_eval_device: bad arguments");
   if (!ctx->libm_loaded)
     return mcg_fail(MCG_ERR_STATE, "mcg_libm_eval_device: needs a strict context");
@@ -83,7 +109,11 @@ extern "C" int mcg_libm_eval_device(mcg_context *ctx, int fn, const float *d_in,
     return MCG_OK;
   cudaSetDevice(ctx->device);
   int grid = (int)std::min<int64_t>((n + 255) / 256, (int64_t)ctx->sm_count * 8);
-  mcg_libm_eval_kernel<<<grid, 256, 0, ctx->stream>>>(fn, d_in, d_out, n, ctx->libm_tab, ctx->libm);
+  if (fn >= 7)
+    mcg_tile_eval_kernel<<<grid, 256, 0, ctx->stream>>>(
+        fn, d_in, d_out, n, mcg_run_setup(ctx->log2_scale, 0.0f, ctx->run_bounds));
+  else
+    mcg_libm_eval_kernel<<<grid, 256, 0, ctx->stream>>>(fn, d_in, d_out, n, ctx->libm_tab, ctx->libm);
   cudaError_t e = cudaGetLastError();
   if (e == cudaSuccess)
     e = cudaStreamSynchronize(ctx->stream);
