@@ -378,12 +378,13 @@ int mcg_simulate_fast_noalloc(int n_layers, const int32_t *h_index_start, const 
 int mcg_measure_conversion_rates(mcg_context *ctx, double *h_rates);
 
 /* Testing aid (no counterpart in the reference): the after-th next device
- * allocation of the geometry set-up (mcg_set_layers, mcg_set_layers_xs,
- * mcg_set_slab, mcg_batch_set; 0 = the next one) reports
- * cudaErrorMemoryAllocation without being attempted, so tests can check that
- * a failed set-up leaves the context with no geometry (later launches and
- * reads return MCG_ERR_STATE) and that a new set-up recovers it.  A negative
- * value disables it.  Process-wide. */
+ * allocation of a set-up (mcg_set_layers, mcg_set_layers_xs, mcg_set_slab,
+ * mcg_batch_set, mcg_fit_set) or of the sums between a forward pass and its
+ * replay (0 = the next one) reports cudaErrorMemoryAllocation without being
+ * attempted, so tests can check that a failed set-up leaves the context with no
+ * geometry or fit (later launches and reads return MCG_ERR_STATE), that a new
+ * set-up recovers it, and that the sums make do with less.  A negative value
+ * disables it.  Process-wide. */
 int mcg_testing_fail_allocation(int32_t after);
 
 /* One rnd_real step on n device seeds (src/curandom.cu:7-14). */

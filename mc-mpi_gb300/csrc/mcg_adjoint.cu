@@ -601,7 +601,7 @@ extern "C" int mcg_adjoint_run(mcg_context *ctx, const mcg_source *src, int64_t 
         cudaFree(A->d_sum);
       A->d_sum = nullptr;
       A->sums = 0;
-      if ((e = cudaMalloc(&A->d_sum, (size_t)part * sizeof(float2))) == cudaSuccess) {
+      if ((e = mcg_dev_malloc((void **)&A->d_sum, (size_t)part * sizeof(float2))) == cudaSuccess) {
         A->sums = part;
       } else {
         cudaGetLastError();

@@ -285,7 +285,6 @@ extern "C" int mcg_fit_set(mcg_context *ctx, int32_t n_slabs, const mcg_slab *h_
     return mcg_fail(MCG_ERR_ARG, "mcg_fit_set: bad arguments");
   cudaSetDevice(ctx->device);
   mcg_fit_release(ctx);
-  mcg_fit_state *F = fit_of(ctx, true);
   int total = 0, maxc = 0;
   for (int s = 0; s < n_slabs; ++s) {
     if (h_slabs[s].n_cells <= 0 || h_slabs[s].n_histories <= 0)
@@ -314,16 +313,22 @@ extern "C" int mcg_fit_set(mcg_context *ctx, int32_t n_slabs, const mcg_slab *h_
   const size_t o_cs = take(total * 4), o_t = take(total * 8), o_g = take(total * 8);
   const size_t o_lh = take(max_steps * 8), o_sa = take(total * 4), o_m1 = take(total * 4);
   const size_t o_m2 = take(total * 4), o_ta = take(total * 8), o_in = take(16), o_st = take(8);
-  cudaError_t e = cudaMalloc(&F->dev, off);
+  mcg_fit_state *F = fit_of(ctx, true);
+  /* a failure from here on leaves no fit set and nothing allocated */
+  auto fail = [&](cudaError_t err, const char *what) {
+    mcg_fit_release(ctx);
+    return mcg_cuda_fail(err, what);
+  };
+  cudaError_t e = mcg_dev_malloc(&F->dev, off);
   if (e != cudaSuccess)
-    return mcg_cuda_fail(e, "mcg_fit_set: cudaMalloc");
+    return fail(e, "mcg_fit_set: cudaMalloc");
   for (F->part = (int)std::min<size_t>(items.size(), MCG_FIT_PART);; F->part /= 2) {
-    if ((e = cudaMalloc(&F->dev_sum, (size_t)F->part * MCG_ITEM_MOST * sizeof(float2))) == cudaSuccess)
+    if ((e = mcg_dev_malloc(&F->dev_sum, (size_t)F->part * MCG_ITEM_MOST * sizeof(float2))) == cudaSuccess)
       break;
     cudaGetLastError();
     F->dev_sum = nullptr;
     if (F->part <= 1)
-      return mcg_cuda_fail(e, "mcg_fit_set: cudaMalloc");
+      return fail(e, "mcg_fit_set: cudaMalloc");
   }
   char *b = static_cast<char *>(F->dev);
   F->cells = reinterpret_cast<float4 *>(b + o_cells);
@@ -368,7 +373,7 @@ extern "C" int mcg_fit_set(mcg_context *ctx, int32_t n_slabs, const mcg_slab *h_
       (e = cudaMemcpy(F->cell_slab, cs.data(), total * 4, cudaMemcpyHostToDevice)) != cudaSuccess ||
       (e = cudaMemcpy(F->target, h_target, total * 8, cudaMemcpyHostToDevice)) != cudaSuccess ||
       (e = cudaMemcpy(F->sig_a, h_sig_a0, total * 4, cudaMemcpyHostToDevice)) != cudaSuccess)
-    return mcg_cuda_fail(e, "mcg_fit_set: upload");
+    return fail(e, "mcg_fit_set: upload");
   F->n_slabs = n_slabs;
   F->n_cells = total;
   F->max_cells = maxc;

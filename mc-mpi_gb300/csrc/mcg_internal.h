@@ -159,9 +159,10 @@ struct mcg_context {
 };
 
 int mcg_fail(int code, const char *fmt, ...);
-/* cudaMalloc of the geometry set-up (mcg_set_layers, mcg_batch_set); a test
- * can make one of them report cudaErrorMemoryAllocation without attempting
- * it (mcg_testing_fail_allocation). */
+/* cudaMalloc of the set-up of a geometry or a fit (mcg_set_layers,
+ * mcg_batch_set, mcg_fit_set) and of the histories' sums; a test can make one
+ * of them report cudaErrorMemoryAllocation without attempting it
+ * (mcg_testing_fail_allocation). */
 cudaError_t mcg_dev_malloc(void **p, size_t bytes);
 int mcg_cuda_fail(cudaError_t e, const char *what);
 #define MCG_TAB_PAD 32 /* a tile reads past its chain's ends (mcg_tiles) */
