@@ -692,6 +692,72 @@ extern "C" int mcg_set_step_limit(mcg_context *ctx, int64_t max_steps)
 }
 
 /* ------------------------------------------------------------ launches */
+/* The largest |weight| of n particles, as its bits (a NaN is larger than any). */
+__global__ void mcg_heaviest_kernel(const mcg_particle *p, int64_t n, uint32_t *out)
+{
+  uint32_t top = 0;
+  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n;
+       i += (int64_t)gridDim.x * blockDim.x)
+    top = max(top, __float_as_uint(p[i].wmc) & 0x7fffffffu);
+  top = __reduce_max_sync(0xffffffffu, top);
+  if ((threadIdx.x & 31) == 0)
+    atomicMax(out, top);
+}
+
+/* One launch of the tracker in the given shape. */
+static int track_enqueue(mcg_context *ctx, mcg_track_params &P, const mcg_shape &shape)
+{
+  const bool strict = ctx->mode == MCG_MODE_STRICT, thin = shape.thin;
+  const int block = shape.block;
+  const size_t smem = shape.smem;
+  P.tally_copies = shape.copies;
+  const bool lanes = strict ? ctx->thick : ctx->thick_fast;
+  void (*kern)(mcg_track_params);
+  if (lanes && strict)
+    kern = shape.global ? mcg_track_kernel<true, MCG_TALLY_GLOBAL, false, true>
+           : ctx->tally_mode == MCG_TALLY_SMEM64 ? mcg_track_kernel<true, MCG_TALLY_SMEM64, false, true>
+                                                 : mcg_track_kernel<true, MCG_TALLY_SMEM32, false, true>;
+  else if (lanes)
+    kern = shape.global ? mcg_track_kernel<false, MCG_TALLY_GLOBAL, false, true>
+           : ctx->tally_mode == MCG_TALLY_SMEM64 ? mcg_track_kernel<false, MCG_TALLY_SMEM64, false, true>
+                                                 : mcg_track_kernel<false, MCG_TALLY_SMEM32, false, true>;
+  else if (strict)
+    kern = thin ? mcg_track_kernel<true, MCG_TALLY_LO32, true>
+           : shape.global ? mcg_track_kernel<true, MCG_TALLY_GLOBAL, false>
+           : ctx->tally_mode == MCG_TALLY_SMEM64 ? mcg_track_kernel<true, MCG_TALLY_SMEM64, false>
+                                                 : mcg_track_kernel<true, MCG_TALLY_SMEM32, false>;
+  else
+    kern = thin ? mcg_track_kernel<false, MCG_TALLY_LO32, true>
+           : shape.global ? mcg_track_kernel<false, MCG_TALLY_GLOBAL, false>
+           : ctx->tally_mode == MCG_TALLY_SMEM64 ? mcg_track_kernel<false, MCG_TALLY_SMEM64, false>
+                                                 : mcg_track_kernel<false, MCG_TALLY_SMEM32, false>;
+  /* the limit is raised to the device's opt-in maximum, the same value on
+   * every call, so launches of the same kernel from other host threads (other
+   * contexts, the no-allocation entry point) cannot lower it under this one */
+  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                       ctx->smem_optin);
+  if (e != cudaSuccess)
+    return mcg_cuda_fail(e, "cudaFuncSetAttribute");
+  int bps = ctx->blocks_per_sm;
+  if (bps <= 0) {
+    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, kern, block, smem);
+    if (e != cudaSuccess)
+      return mcg_cuda_fail(e, "occupancy");
+    bps = std::max(bps, 1);
+  }
+  const int grid = mcg_track_grid(ctx->sm_count * bps, block, P.n, lanes, P);
+  if ((e = cudaMemsetAsync(ctx->d_next, 0, sizeof(unsigned long long), ctx->stream)) != cudaSuccess)
+    return mcg_cuda_fail(e, "cudaMemsetAsync");
+  kern<<<grid, block, smem, ctx->stream>>>(P);
+  e = cudaGetLastError();
+  if (e != cudaSuccess)
+    return mcg_cuda_fail(e, "mcg_track_kernel launch");
+  ctx->last_grid = grid;
+  ctx->last_block = block;
+  ctx->launches++;
+  return MCG_OK;
+}
+
 int mcg_track_launch(mcg_context *ctx, mcg_particle *d_particles, int64_t n, int32_t *d_results,
                      int64_t *d_steps, int64_t *d_scatters, const mcg_source *src, int64_t first)
 {
@@ -730,63 +796,36 @@ int mcg_track_launch(mcg_context *ctx, mcg_particle *d_particles, int64_t n, int
     return mcg_event_run(ctx, P);
   }
   /* thin chains take the thin kernel with its tally unless the caller set
-   * the global tally or a larger block */
+   * the global tally or a larger block, or the weights are too large for it */
   const bool global = ctx->tally_mode == MCG_TALLY_GLOBAL;
+  const float heavy = mcg_heavy_weight(ctx);
   const bool try_thin = (strict ? ctx->thin : ctx->thin_fast) && !global &&
-                        ctx->block <= MCG_THIN_BLOCK;
-  const mcg_shape shape = mcg_track_shape(ctx->n_cells, ctx->block, global, try_thin,
-                                          (size_t)ctx->smem_optin);
-  const bool thin = shape.thin;
-  const int block = shape.block;
-  const size_t smem = shape.smem;
-  P.tally_copies = shape.copies;
-  const bool lanes = strict ? ctx->thick : ctx->thick_fast;
-  void (*kern)(mcg_track_params);
-  if (lanes && strict)
-    kern = shape.global ? mcg_track_kernel<true, MCG_TALLY_GLOBAL, false, true>
-           : ctx->tally_mode == MCG_TALLY_SMEM64 ? mcg_track_kernel<true, MCG_TALLY_SMEM64, false, true>
-                                                 : mcg_track_kernel<true, MCG_TALLY_SMEM32, false, true>;
-  else if (lanes)
-    kern = shape.global ? mcg_track_kernel<false, MCG_TALLY_GLOBAL, false, true>
-           : ctx->tally_mode == MCG_TALLY_SMEM64 ? mcg_track_kernel<false, MCG_TALLY_SMEM64, false, true>
-                                                 : mcg_track_kernel<false, MCG_TALLY_SMEM32, false, true>;
-  else if (strict)
-    kern = thin ? mcg_track_kernel<true, MCG_TALLY_LO32, true>
-           : shape.global ? mcg_track_kernel<true, MCG_TALLY_GLOBAL, false>
-           : ctx->tally_mode == MCG_TALLY_SMEM64 ? mcg_track_kernel<true, MCG_TALLY_SMEM64, false>
-                                                 : mcg_track_kernel<true, MCG_TALLY_SMEM32, false>;
-  else
-    kern = thin ? mcg_track_kernel<false, MCG_TALLY_LO32, true>
-           : shape.global ? mcg_track_kernel<false, MCG_TALLY_GLOBAL, false>
-           : ctx->tally_mode == MCG_TALLY_SMEM64 ? mcg_track_kernel<false, MCG_TALLY_SMEM64, false>
-                                                 : mcg_track_kernel<false, MCG_TALLY_SMEM32, false>;
-  /* the limit is raised to the device's opt-in maximum, the same value on
-   * every call, so launches of the same kernel from other host threads (other
-   * contexts, the no-allocation entry point) cannot lower it under this one */
-  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       ctx->smem_optin);
-  if (e != cudaSuccess)
-    return mcg_cuda_fail(e, "cudaFuncSetAttribute");
-  int bps = ctx->blocks_per_sm;
-  if (bps <= 0) {
-    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, kern, block, smem);
-    if (e != cudaSuccess)
-      return mcg_cuda_fail(e, "occupancy");
-    bps = std::max(bps, 1);
-  }
-  const int grid = mcg_track_grid(ctx->sm_count * bps, block, n, lanes, P);
-  if ((e = cudaMemsetAsync(ctx->d_next, 0, sizeof(unsigned long long), ctx->stream)) != cudaSuccess)
-    return mcg_cuda_fail(e, "cudaMemsetAsync");
+                        ctx->block <= MCG_THIN_BLOCK && !(src && std::fabs(src->w0) >= heavy);
+  mcg_shape shape = mcg_track_shape(ctx->n_cells, ctx->block, global, try_thin, (size_t)ctx->smem_optin);
   cudaEventRecord(ctx->ev0, ctx->stream);
-  kern<<<grid, block, smem, ctx->stream>>>(P);
-  e = cudaGetLastError();
+  if (shape.thin && d_particles) {
+    /* which of the two forms runs is decided on the device, from the particles:
+     * the other's launch returns at once */
+    uint32_t *heaviest = reinterpret_cast<uint32_t *>(ctx->d_next + 1);
+    cudaError_t e = cudaMemsetAsync(heaviest, 0, sizeof(uint32_t), ctx->stream);
+    if (e != cudaSuccess)
+      return mcg_cuda_fail(e, "cudaMemsetAsync");
+    mcg_heaviest_kernel<<<(int)std::min<int64_t>((n + 255) / 256, 4LL * ctx->sm_count), 256, 0,
+                          ctx->stream>>>(d_particles, n, heaviest);
+    P.heaviest = heaviest;
+    memcpy(&P.heavy_line, &heavy, 4);
+    if ((e = cudaGetLastError()) != cudaSuccess)
+      return mcg_cuda_fail(e, "mcg_heaviest_kernel launch");
+    ctx->launches++;
+    int rc = track_enqueue(ctx, P, shape);
+    if (rc != MCG_OK)
+      return rc;
+    P.heavy = 1;
+    shape = mcg_track_shape(ctx->n_cells, ctx->block, false, false, (size_t)ctx->smem_optin);
+  }
+  const int rc = track_enqueue(ctx, P, shape);
   cudaEventRecord(ctx->ev1, ctx->stream);
-  if (e != cudaSuccess)
-    return mcg_cuda_fail(e, "mcg_track_kernel launch");
-  ctx->last_grid = grid;
-  ctx->last_block = block;
-  ctx->launches++;
-  return MCG_OK;
+  return rc;
 }
 
 int mcg_sync(mcg_context *ctx)

@@ -24,6 +24,7 @@
  */
 #include <algorithm>
 #include <chrono>
+#include <cmath>
 #include <cstdio>
 #include <cstdlib>
 #include <thread>
@@ -1043,7 +1044,8 @@ extern "C" int mcg_worker_run_async(mcg_context *ctx, const mcg_source *src, int
 
   /* the largest block whose tiles fit beside the tally; the global tally where
    * not even 256 threads' do */
-  bool thin = strict ? ctx->thin : ctx->thin_fast, global = false;
+  bool thin = (strict ? ctx->thin : ctx->thin_fast) && std::fabs(src->w0) < mcg_heavy_weight(ctx);
+  bool global = false;
   int block = 1024;
   auto smem_of = [&](bool t) { return async_smem(P_, (size_t)ctx->n_cells, block, global, thin, t); };
   const bool tiled = (int64_t)ctx->n_cells >= (int64_t)MCG_AQ_SHORT * P_ ||

@@ -7,6 +7,8 @@ gives the same arithmetic by another path; results are exact."""
 import numpy as np
 import pytest
 
+from test_gpu_tiles import _particles
+
 pytestmark = pytest.mark.gpu
 f32 = np.float32
 
@@ -112,3 +114,80 @@ def test_uniform_decomposed_slab(mcg, mode):
     with mcg.Context(mode=mode) as ctx:
         ctx.set_layers_xs(st, lm, dx, np.full(m, wa * m), np.full(m, ws * m), 1e-12)
         _same_as_event_mode(ctx, 20_000)
+
+
+def _kernel_ms(ctx, n, **source):
+    times = []
+    for _ in range(4):
+        ctx.simulate_source(0, n, **source)
+        times.append(ctx.last_kernel_ms())
+    return min(times)
+
+
+@pytest.mark.parametrize("mode", ["strict", "fast"])
+@pytest.mark.parametrize("scale,w0", [(40, 30.0), (40, 1e6), (50, 1.0), (58, 1.0), (62, 1e-3), (62, 1.0), (0, 1e18)])
+def test_large_deposits(mcg, mode, scale, w0):
+    """Deposits around and above the 31 bits of a low word, up to beyond the 62
+    that the tiles take (sums wrap alike)."""
+    rng = np.random.default_rng(9)
+    m = 1000
+    sa, ss = rng.uniform(0.2, 1.0, (2, m)) * 1.5e-4 * m
+    sa[::9] = 0.0
+    with mcg.Context(mode=mode) as ctx:
+        ctx.set_layers_xs([0], [m], [f32(1.0 / m)], sa, ss, 1e-12)
+        ctx.set_tally_scale(scale)
+        _same_as_event_mode(ctx, 3000, w0=w0)
+
+
+@pytest.mark.parametrize("mode", ["strict", "fast"])
+def test_large_deposits_stay_in_the_tiles(mcg, mode):
+    """The same histories with a weight of 1000 and of 1, born or as particles: a
+    full step for every crossing takes 40 times as long, the form with wider
+    deposits two to three times."""
+    m, n = 10_000, 20_000
+    with mcg.Context(mode=mode) as ctx:
+        ctx.set_layers_xs([0], [m], [f32(1.0 / m)], np.full(m, 5e-5 * m), np.full(m, 2e-4 * m), 1e-12)
+        assert _kernel_ms(ctx, n, w0=1000.0) < 8 * _kernel_ms(ctx, n)
+        p = np.zeros(n, mcg.PARTICLE_DTYPE)
+        p["seed"] = np.arange(1, n + 1, dtype=np.uint64) * np.uint64(7919 * 10 ** 9)
+        p["mu"] = 1.0
+        times = []
+        for w in (1.0, 1000.0):
+            p["wmc"] = w
+            best = []
+            for _ in range(3):
+                ctx.simulate(p.copy())
+                best.append(ctx.last_kernel_ms())
+            times.append(min(best))
+        assert times[1] < 8 * times[0]
+
+
+@pytest.mark.parametrize("mode", ["strict", "fast"])
+@pytest.mark.parametrize("heavy", [False, True])
+@pytest.mark.parametrize("m", [1, 31, 33, 700])
+def test_thin_particles(mcg, mode, heavy, m):
+    """Host particles on both sides of the line between the two forms, which is
+    drawn on the device from their weights: one heavy particle decides."""
+    rng = np.random.default_rng(m)
+    sa, ss = rng.uniform(0.2, 1.0, (2, m)) * 1.5e-4 * m
+    p = _particles(mcg, rng, m, 1.0 / m, 2500)
+    p["wmc"] = np.minimum(p["wmc"], 1.0)
+    if heavy:
+        p["wmc"][1234] = -1e9 if m == 31 else np.nan if m == 33 else 1e9
+    with mcg.Context(mode=mode) as ctx:
+        for min_w, scale in ((1e-12, 40), (-np.inf, 35), (0.3, 30)):
+            ctx.set_layers_xs([0], [m], [f32(1.0 / m)], sa, ss, min_w)
+            ctx.set_tally_scale(scale)
+            out = []
+            for algorithm in ("history", "event"):
+                ctx.set_algorithm(algorithm, 1)
+                ctx.tally_reset()
+                q = p.copy()
+                r = ctx.simulate(q)
+                out.append((q, r, ctx.tally_q(), ctx.counters()))
+            (pa, ra, qa, ca), (pb, rb, qb, cb) = out
+            assert pa.tobytes() == pb.tobytes()
+            for key in ("results", "steps", "scatters"):
+                assert np.array_equal(ra[key], rb[key]), key
+            assert np.array_equal(qa, qb)
+            assert ca == cb
