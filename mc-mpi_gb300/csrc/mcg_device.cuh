@@ -17,6 +17,10 @@
 struct mcg_run_consts {
   float scale, inv_scale;
   float min_w; /* the minimum weight times the scale */
+  /* weights of less than this are not scaled in the tiles, so that they round as
+   * the reference's do below the normal numbers, and their deposits are 0; 0
+   * where a positive minimum weight or a large scale leaves none */
+  float tiny;
   float b_thin, c_thin, b_mid;
   float w_a, w_i; /* thin chains: the largest sig_a and sig_i cell widths */
 };
@@ -30,6 +34,7 @@ inline mcg_run_consts mcg_run_setup(int log2_scale, float min_w, const float *b,
   R.scale = ldexpf(1.0f, log2_scale);
   R.inv_scale = ldexpf(1.0f, -log2_scale);
   R.min_w = min_w * R.scale;
+  R.tiny = log2_scale <= 58 && min_w <= 0.0f ? 0x1p-60f : 0.0f;
   R.b_thin = b ? b[0] : 0.0f;
   R.c_thin = b ? b[1] : 0.0f;
   R.b_mid = b ? b[2] : 0.0f;
