@@ -388,10 +388,12 @@ static void update_thin(mcg_context *ctx)
   }
   ctx->width_a = wa;
   ctx->width_i = wi;
-  ctx->thin = !ctx->cells_strict.empty() && wa <= (depth < 1.2 ? 7e-5f : 2e-4f);
-  ctx->thin_fast = !ctx->cells_strict.empty() && std::max(wa, wi) <= 4e-4f;
-  ctx->thick = mcg_thick(ctx->cells_strict.data(), (int)ctx->cells_strict.size(), true);
-  ctx->thick_fast = mcg_thick(ctx->cells_strict.data(), (int)ctx->cells_strict.size(), false);
+  ctx->thick = mcg_thick(ctx->cells_strict.data(), n, true);
+  ctx->thick_fast = mcg_thick(ctx->cells_strict.data(), n, false);
+  /* a chain of thick cells that hardly any flight may enter in the tiles is both:
+   * it takes lanes, whose launch has no thin shape */
+  ctx->thin = n > 0 && !ctx->thick && wa <= (depth < 1.2 ? 7e-5f : 2e-4f);
+  ctx->thin_fast = n > 0 && !ctx->thick_fast && std::max(wa, wi) <= 4e-4f;
 }
 
 /* Chains on which a lane per history is faster than tiles: by the cells' mean

@@ -116,6 +116,33 @@ def test_uniform_decomposed_slab(mcg, mode):
         _same_as_event_mode(ctx, 20_000)
 
 
+@pytest.mark.parametrize("mode", ["strict", "fast"])
+def test_thick_cells_with_short_entries(mcg, mode):
+    """Layers of one cell whose right faces coincide: no flight to the right has a
+    length, and those to the left are 1 / g of the cells' own width, so that the
+    chain is thin by the tiles' lengths and thick by its cells."""
+    m = 1000
+    g = np.arange(m)
+    dx = 1.0 / (g + 1)
+    left, right = _entry_widths(g, np.ones(m, int), dx)
+    assert np.abs(left[1:]).max() < 1e-3 and np.median(right) < 1e-2
+    sa = 1e-4 * (g + 1) * (g + 2)
+    sa[0] = sa[-1] = 0.0
+    with mcg.Context(mode=mode) as ctx:
+        ctx.set_layers_xs(g, np.ones(m, int), dx, sa, 0.9 * sa, 1e-12)
+        p = _particles(mcg, np.random.default_rng(1), m, 1.0, 1500)
+        p["x"] = ((p["index"] + 0.5) * dx[np.clip(p["index"], 0, m - 1)]).astype(f32)
+        out = []
+        for algorithm in ("event", "history"):
+            ctx.set_algorithm(algorithm, 1)
+            ctx.tally_reset()
+            q = p.copy()
+            ctx.simulate(q)
+            out.append((q.tobytes(), ctx.tally_q().tobytes(), ctx.counters()))
+        assert out[0] == out[1]
+        _same_as_event_mode(ctx, 3000)
+
+
 def _kernel_ms(ctx, n, **source):
     times = []
     for _ in range(4):
