@@ -371,8 +371,11 @@ static void update_thin(mcg_context *ctx)
 {
   float wa = 0.0f, wi = 0.0f;
   double depth = 0.0; /* of the chain, both cross sections */
+  ctx->depth_i = 0.0;
   for (const float4 &c : ctx->cells_strict) {
-    depth += ((double)std::fabs(c.x) + std::fabs(c.y)) * ((double)c.w - c.z);
+    const double len = (double)c.w - c.z;
+    depth += ((double)std::fabs(c.x) + std::fabs(c.y)) * len;
+    ctx->depth_i += c.y > 1e-4f ? c.y * len : 0.0;
   }
   /* the widths that bound a whole flight (mcg_thin_tests): of the lengths that
    * the tiles use, since a cell entered from another layer's face may be wider
@@ -396,19 +399,51 @@ static void update_thin(mcg_context *ctx)
   ctx->thin_fast = n > 0 && !ctx->thick_fast && std::max(wa, wi) <= 4e-4f;
 }
 
-/* Chains on which a lane per history is faster than tiles: by the cells' mean
+/* Whether the thin form pays for n histories.  It halves the rounds of a history,
+ * but its one block of 768 threads per SM holds fewer of them, which short chains
+ * feel, and a flight with |mu| < `slant`, which leaves the short forms' range, takes
+ * a full step and a round (1.2 to 1.5 us) per cell, `far` of them until it collides
+ * or leaves, where the other tiles take 16 at a time: the end of a launch waits for
+ * one, and all of them (4e-10 s per round over the GPU) add up.  Thin time / other:
+ * without collisions .7 to .8 from 200 cells on, 1.0 at 100, 1.3 at 64, 1.85 at 32,
+ * but .75 there for 1e6 cells times histories; widths 1e-4 in both sections, 6e8
+ * cells times histories, strict: 1.06 at 300 cells, 1.3 at 1000, 1.7 at 2000, .76 at
+ * 10,000; 1e7: 4.3, 5.1, 1.7 and .88; fast, as many: .94, 1.17, 1.12, .57; 3.3, 2.5,
+ * 1.6, .73. */
+static bool thin_pays(const mcg_context *ctx, bool strict, int64_t n, bool isotropic)
+{
+  const double m = ctx->n_cells;
+  if (m < (n > 65536 ? 100.0 : 16.0))
+    return false;
+  const double slant = strict ? ctx->width_a / MCG_OM_THIN_MAX : std::max(ctx->width_a, ctx->width_i) * 128.0;
+  /* histories with such a flight */
+  const double slanted = (double)n * (ctx->depth_i + (isotropic ? 1.0 : 0.0)) * slant;
+  if (slanted < 1.5)
+    return true;
+  const double far = std::min(0.5 * m, slant * m / ctx->depth_i);
+  return 7e-13 * (double)n * m * (1.0 + ctx->depth_i) + 1e-7 * m > far * (1.2e-6 + 4e-10 * slanted);
+}
+
+/* Chains on which a lane per history is faster than tiles.  By the cells' mean
  * optical widths, in absorption (strict, whose tiles need u < 2^-4) or both
- * together.  Kernel times of 2e6 histories, lanes / tiles, at mean widths
+ * together: kernel times of 2e6 histories, lanes / tiles, at mean widths
  * sig_a (+ sig_i): strict .069 753 / 1454 us, .031 1053 / 1308, .028 1351 / 1709,
  * .021 1338 / 1247, .014 tiles; fast .131 424 / 610, .156 555 / 792,
- * .088 569 / 611, .104 797 / 775, .053 tiles. */
+ * .088 569 / 611, .104 797 / 775, .053 tiles.  Strict, where a history scatters
+ * every other cell and the chain is short: tiles 1.3 to 1.5 times the lanes' time up
+ * to 48 cells of sig_i width .5, .99 at 100.  And chains of one to five cells, on
+ * which a tile is a step or two: 1.25 times at one cell, 1.1 at four, .95 at eight. */
 bool mcg_thick(const float4 *cells, int n, bool strict)
 {
-  double sum = 0.0;
-  for (int c = 0; c < n; ++c)
-    sum += (std::fabs((double)cells[c].x) + (strict ? 0.0 : std::fabs((double)cells[c].y))) *
-           ((double)cells[c].w - cells[c].z);
-  return n > 0 && sum > (strict ? 0.02 : 0.08) * n;
+  if (n < 6)
+    return n > 0;
+  double a = 0.0, i = 0.0;
+  for (int c = 0; c < n; ++c) {
+    const double len = (double)cells[c].w - cells[c].z;
+    a += std::fabs((double)cells[c].x) * len;
+    i += std::fabs((double)cells[c].y) * len;
+  }
+  return strict ? a > 0.02 * n || (n < 80 && i > 0.25 * n) : a + i > 0.08 * n;
 }
 
 /* The cells and their tile table to the device; `tab` holds the latter until
@@ -750,6 +785,8 @@ static int track_enqueue(mcg_context *ctx, mcg_track_params &P, const mcg_shape 
   const int grid = mcg_track_grid(ctx->sm_count * bps, block, P.n, lanes, P);
   if ((e = cudaMemsetAsync(ctx->d_next, 0, sizeof(unsigned long long), ctx->stream)) != cudaSuccess)
     return mcg_cuda_fail(e, "cudaMemsetAsync");
+  if (!P.heaviest) /* else the run's time starts with the look at the weights */
+    cudaEventRecord(ctx->ev0, ctx->stream);
   kern<<<grid, block, smem, ctx->stream>>>(P);
   e = cudaGetLastError();
   if (e != cudaSuccess)
@@ -797,14 +834,15 @@ int mcg_track_launch(mcg_context *ctx, mcg_particle *d_particles, int64_t n, int
     ctx->launches++;
     return mcg_event_run(ctx, P);
   }
-  /* thin chains take the thin kernel with its tally unless the caller set
-   * the global tally or a larger block, or the weights are too large for it */
+  /* thin chains take the thin kernel with its tally unless it does not pay (with
+   * a block size of the caller's it is taken all the same), the caller set the
+   * global tally or a larger block, or the weights are too large for it */
   const bool global = ctx->tally_mode == MCG_TALLY_GLOBAL;
   const float heavy = mcg_heavy_weight(ctx);
   const bool try_thin = (strict ? ctx->thin : ctx->thin_fast) && !global &&
-                        ctx->block <= MCG_THIN_BLOCK && !(src && std::fabs(src->w0) >= heavy);
+                        ctx->block <= MCG_THIN_BLOCK && !(src && std::fabs(src->w0) >= heavy) &&
+                        (ctx->block || thin_pays(ctx, strict, n, src && src->isotropic));
   mcg_shape shape = mcg_track_shape(ctx->n_cells, ctx->block, global, try_thin, (size_t)ctx->smem_optin);
-  cudaEventRecord(ctx->ev0, ctx->stream);
   if (shape.thin && d_particles) {
     /* which of the two forms runs is decided on the device, from the particles:
      * the other's launch returns at once */
@@ -812,6 +850,7 @@ int mcg_track_launch(mcg_context *ctx, mcg_particle *d_particles, int64_t n, int
     cudaError_t e = cudaMemsetAsync(heaviest, 0, sizeof(uint32_t), ctx->stream);
     if (e != cudaSuccess)
       return mcg_cuda_fail(e, "cudaMemsetAsync");
+    cudaEventRecord(ctx->ev0, ctx->stream);
     mcg_heaviest_kernel<<<(int)std::min<int64_t>((n + 255) / 256, 4LL * ctx->sm_count), 256, 0,
                           ctx->stream>>>(d_particles, n, heaviest);
     P.heaviest = heaviest;

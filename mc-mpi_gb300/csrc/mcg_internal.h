@@ -119,6 +119,7 @@ struct mcg_context {
   bool thin_fast = false; /* sig_a and sig_i widths <= 4e-4 (fast THIN) */
   bool thick = false, thick_fast = false; /* mcg_thick, strict and fast */
   float width_a = 0.f, width_i = 0.f; /* those largest widths */
+  double depth_i = 0.0;               /* the chain's optical depth in sig_i */
   float4 *d_cells_strict = nullptr, *d_cells_fast = nullptr;
   /* the tiles' per-cell parameters (mcg_tile_table), MCG_TAB_PAD entries
    * before and after; of the thin form one such array per direction, in the

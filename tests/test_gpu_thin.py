@@ -27,15 +27,19 @@ def _entry_widths(st, m, dx):
 
 
 def _same_as_event_mode(ctx, n, **source):
+    """In the launch shape of the library's choice, and with a block size that
+    makes a thin chain take the thin form whether it pays or not."""
     out = []
-    for algorithm in ("event", "history"):
+    for algorithm, launch in (("event", {}), ("history", {}), ("history", dict(block=768))):
         ctx.set_algorithm(algorithm, 1)
+        ctx.set_launch(**launch)
         ctx.tally_reset()
         ctx.simulate_source(0, n, **source)
         out.append((ctx.tally_q(), ctx.counters()))
-    ctx.set_algorithm("history")
-    assert np.array_equal(out[0][0], out[1][0])
-    assert out[0][1] == out[1][1]
+    ctx.set_launch()
+    for q, c in out[1:]:
+        assert np.array_equal(out[0][0], q)
+        assert out[0][1] == c
     ctx.tally_reset()
     ctx.worker_run_async(n, **source)
     assert np.array_equal(out[0][0], ctx.tally_q())
@@ -206,15 +210,30 @@ def test_thin_particles(mcg, mode, heavy, m):
             ctx.set_layers_xs([0], [m], [f32(1.0 / m)], sa, ss, min_w)
             ctx.set_tally_scale(scale)
             out = []
-            for algorithm in ("history", "event"):
+            for algorithm, launch in (("event", {}), ("history", {}), ("history", dict(block=512))):
                 ctx.set_algorithm(algorithm, 1)
+                ctx.set_launch(**launch)
                 ctx.tally_reset()
                 q = p.copy()
                 r = ctx.simulate(q)
                 out.append((q, r, ctx.tally_q(), ctx.counters()))
-            (pa, ra, qa, ca), (pb, rb, qb, cb) = out
-            assert pa.tobytes() == pb.tobytes()
-            for key in ("results", "steps", "scatters"):
-                assert np.array_equal(ra[key], rb[key]), key
-            assert np.array_equal(qa, qb)
-            assert ca == cb
+            pa, ra, qa, ca = out[0]
+            for pb, rb, qb, cb in out[1:]:
+                assert pa.tobytes() == pb.tobytes()
+                for key in ("results", "steps", "scatters"):
+                    assert np.array_equal(ra[key], rb[key]), key
+                assert np.array_equal(qa, qb)
+                assert ca == cb
+
+
+@pytest.mark.parametrize("mode", ["strict", "fast"])
+@pytest.mark.parametrize("m", [1, 16, 64, 300])
+def test_short_chains_are_not_slower_for_being_thin(mcg, mode, m):
+    """Two million histories through chains of almost nothing, on which the thin
+    form's one block per SM took twice as long as cells of width 5e-3 do."""
+    times = []
+    with mcg.Context(mode=mode) as ctx:
+        for width in (1e-7, 5e-3):
+            ctx.set_layers_xs([0], [m], [f32(1.0 / m)], np.full(m, width * m), np.full(m, width * m), 1e-12)
+            times.append(_kernel_ms(ctx, 2_000_000 if m < 64 else 500_000))
+    assert times[0] < 1.25 * times[1], times
