@@ -244,7 +244,7 @@ static void free_geometry(mcg_context *ctx)
   ctx->rates.clear();
   ctx->cells_strict.clear();
   ctx->cells_fast.clear();
-  ctx->thin = ctx->thin_fast = false;
+  ctx->thin = ctx->thin_fast = ctx->thin_step = false;
 }
 
 /* Allocations still to succeed before one is made to fail (-1: none). */
@@ -370,12 +370,14 @@ void mcg_tile_table(const float4 *c, int n, float4 *tab, float2 *right, float2 *
 static void update_thin(mcg_context *ctx)
 {
   float wa = 0.0f, wi = 0.0f;
+  float own = 0.0f;   /* the widest cell between its own faces, in sig_a */
   double depth = 0.0; /* of the chain, both cross sections */
   ctx->depth_i = 0.0;
   for (const float4 &c : ctx->cells_strict) {
     const double len = (double)c.w - c.z;
     depth += ((double)std::fabs(c.x) + std::fabs(c.y)) * len;
     ctx->depth_i += c.y > 1e-4f ? c.y * len : 0.0;
+    own = std::max(own, std::fabs(c.x) * (c.w - c.z));
   }
   /* the widths that bound a whole flight (mcg_thin_tests): of the lengths that
    * the tiles use, since a cell entered from another layer's face may be wider
@@ -391,6 +393,7 @@ static void update_thin(mcg_context *ctx)
   }
   ctx->width_a = wa;
   ctx->width_i = wi;
+  ctx->thin_step = n > 0 && own <= 5e-4f;
   ctx->thick = mcg_thick(ctx->cells_strict.data(), n, true);
   ctx->thick_fast = mcg_thick(ctx->cells_strict.data(), n, false);
   /* a chain of thick cells that hardly any flight may enter in the tiles is both:

@@ -115,6 +115,7 @@ struct mcg_context {
   std::vector<int32_t> layer_start, layer_m;
   std::vector<float> layer_dx, sigs, rates;
   std::vector<float4> cells_strict, cells_fast;
+  bool thin_step = false; /* mcg_strict_thin */
   bool thin = false;      /* every cell's sig_a width <= 2e-4 (strict THIN) */
   bool thin_fast = false; /* sig_a and sig_i widths <= 4e-4 (fast THIN) */
   bool thick = false, thick_fast = false; /* mcg_thick, strict and fast */
@@ -186,13 +187,15 @@ inline unsigned long long mcg_event_drain_below(const mcg_context *ctx)
 {
   return (unsigned long long)ctx->sm_count * 1024;
 }
-/* The strict thin-cell step applies: a thin chain, and exception-table
- * thresholds small enough for its test on |yl| (that test implies the
- * midpoint-distance test for thresholds below 0.4; the tables' are about
- * 0.002). */
+/* The strict thin-cell step applies (mcg_step THIN, the workers' cycles): every
+ * cell's sig_a width is at most 5e-4, so that a crossing has |sig_a d_edge| >=
+ * MCG_EXP_SMALL_T only for |mu| < 0.093, under 1 % of the crossings, and
+ * exception-table thresholds small enough for its test on |yl| (that test implies
+ * the midpoint-distance test for thresholds below 0.4; the tables' are about
+ * 0.002).  Not the tiles' line: each step tests its own argument. */
 inline bool mcg_strict_thin(const mcg_context *ctx)
 {
-  return ctx->thin && ctx->libm.tau_exp_max < 0.25f;
+  return ctx->thin_step && ctx->libm.tau_exp_max < 0.25f;
 }
 int mcg_event_run(mcg_context *ctx, mcg_track_params &P);
 int mcg_event_run_slabs(mcg_context *ctx, const float4 *cells, unsigned long long *tally,

@@ -117,3 +117,24 @@ def test_contexts_of_two_threads_do_not_lower_each_others_shared_memory(mcg, kin
         a.close()
         b.close()
     assert not failed
+
+
+@pytest.mark.parametrize("width", [1e-4, 3e-4, 4.9e-4, 5.1e-4, 2e-3])
+def test_synchronous_workers_around_the_thin_step(mcg, width):
+    """Strict workers' cycles on both sides of the line of the thin-cell step
+    (5e-4) and of the tiles' lower one, against event mode."""
+    m, layers, n = 1000, 8, 3000
+    rng = np.random.default_rng(4)
+    st, lm, dx, _, _ = mcg.layer_decomposition(0.0, 1.0, m, layers)
+    sa, ss = rng.uniform(0.3, 1.0, (2, m)) * width * m
+    sa[500] = width * m
+    with mcg.Context(mode="strict") as ctx:
+        ctx.set_layers_xs(st, lm, dx, sa, ss, 1e-12)
+        ctx.set_algorithm("event", 1)
+        ctx.simulate_source(0, n)
+        want, c = ctx.tally_q(), ctx.counters()
+        ctx.set_algorithm("history")
+        ctx.tally_reset()
+        ctx.worker_run(n, per_cycle=500)
+        assert np.array_equal(ctx.tally_q(), want)
+        assert all(ctx.counters()[k] == c[k] for k in ("steps", "scatters"))
