@@ -1380,27 +1380,26 @@ inline mcg_shape mcg_track_shape(int n_cells, int block, bool global, bool thin,
   return s;
 }
 
-/* Counters of a finished history: result r, final weight. */
+/* Counters of a finished history: result r, final weight.  In 32-bit halves:
+ * 64-bit shared-memory adds whose result is not used are compare-and-swap loops,
+ * which all lanes of a block run on the same few words (short histories are little
+ * else: 1e7 of one or two steps in 2-cell slabs 2.46 ms so, and half the
+ * instructions waited for them). */
 template <bool STRICT>
 __device__ __forceinline__ void mcg_count_end(unsigned long long *s_cnt, int r, float wmc,
                                               float wres, int qs)
 {
-  atomicAdd(&s_cnt[MCG_CNT_HIST], 1ull);
   long long wq = mcg_to_fixed(wmc, qs);
   if (!STRICT)
     wq += mcg_to_fixed(wres, qs); /* the weight's float-float remainder */
-  if (r == -1) {
-    atomicAdd(&s_cnt[MCG_CNT_LEFT], 1ull);
-    atomicAdd(&s_cnt[MCG_CNT_WLEFT], (unsigned long long)wq);
-  } else if (r == 1) {
-    atomicAdd(&s_cnt[MCG_CNT_RIGHT], 1ull);
-    atomicAdd(&s_cnt[MCG_CNT_WRIGHT], (unsigned long long)wq);
-  } else if (r == 0) {
-    atomicAdd(&s_cnt[MCG_CNT_KILL], 1ull);
-    atomicAdd(&s_cnt[MCG_CNT_WKILL], (unsigned long long)wq);
-  } else {
-    atomicOr(&s_cnt[MCG_CNT_ERR], 1ull);
+  mcg_tally_add<MCG_TALLY_SMEM32>(&s_cnt[MCG_CNT_HIST], 1);
+  if (r == 2) {
+    atomicOr(reinterpret_cast<unsigned *>(&s_cnt[MCG_CNT_ERR]), 1u);
+    return;
   }
+  const int side = r == -1 ? 0 : r == 1 ? 1 : 2; /* left, right, killed */
+  mcg_tally_add<MCG_TALLY_SMEM32>(&s_cnt[MCG_CNT_LEFT + side], 1);
+  mcg_tally_add<MCG_TALLY_SMEM32>(&s_cnt[MCG_CNT_WLEFT + side], wq);
 }
 
 /* The chain that a warp's newborns run in; with MULTI the slab, whose cells
