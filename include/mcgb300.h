@@ -264,7 +264,8 @@ int mcg_batch_tally_reset(mcg_context *ctx);
 int mcg_batch_tally_read(mcg_context *ctx, int64_t *h_q, double *h_f64);
 /* Launch shape of mcg_batch_run: threads per block (256, 512 or 1024),
  * most histories per work item (a block takes one item at a time), tally mode
- * (as mcg_set_tally_mode). 0 keeps the current value. */
+ * (as mcg_set_tally_mode; 0 and 1 run the same kernel). 0 keeps the current value.
+ * Short and thick slabs take a lane per history in blocks of 256 beside it. */
 int mcg_batch_set_launch(mcg_context *ctx, int32_t block, int64_t item_histories,
                          int32_t tally_mode);
 /* Deferral of the full step in mcg_batch_run: a lane whose step is not a certain

@@ -371,11 +371,11 @@ static void update_thin(mcg_context *ctx)
 {
   float wa = 0.0f, wi = 0.0f;
   float own = 0.0f;   /* the widest cell between its own faces, in sig_a */
-  double depth = 0.0; /* of the chain, both cross sections */
   ctx->depth_i = 0.0;
+  mcg_widths sum;
   for (const float4 &c : ctx->cells_strict) {
+    sum.add(c);
     const double len = (double)c.w - c.z;
-    depth += ((double)std::fabs(c.x) + std::fabs(c.y)) * len;
     ctx->depth_i += c.y > 1e-4f ? c.y * len : 0.0;
     own = std::max(own, std::fabs(c.x) * (c.w - c.z));
   }
@@ -394,11 +394,11 @@ static void update_thin(mcg_context *ctx)
   ctx->width_a = wa;
   ctx->width_i = wi;
   ctx->thin_step = n > 0 && own <= 5e-4f;
-  ctx->thick = mcg_thick(ctx->cells_strict.data(), n, true);
-  ctx->thick_fast = mcg_thick(ctx->cells_strict.data(), n, false);
+  ctx->thick = mcg_thick(sum, n, true);
+  ctx->thick_fast = mcg_thick(sum, n, false);
   /* a chain of thick cells that hardly any flight may enter in the tiles is both:
    * it takes lanes, whose launch has no thin shape */
-  ctx->thin = n > 0 && !ctx->thick && wa <= (depth < 1.2 ? 7e-5f : 2e-4f);
+  ctx->thin = n > 0 && !ctx->thick && wa <= (sum.a + sum.i < 1.2 ? 7e-5f : 2e-4f);
   ctx->thin_fast = n > 0 && !ctx->thick_fast && std::max(wa, wi) <= 4e-4f;
 }
 
@@ -427,26 +427,23 @@ static bool thin_pays(const mcg_context *ctx, bool strict, int64_t n, bool isotr
   return 7e-13 * (double)n * m * (1.0 + ctx->depth_i) + 1e-7 * m > far * (1.2e-6 + 4e-10 * slanted);
 }
 
-/* Chains on which a lane per history is faster than tiles.  By the cells' mean
- * optical widths, in absorption (strict, whose tiles need u < 2^-4) or both
- * together: kernel times of 2e6 histories, lanes / tiles, at mean widths
- * sig_a (+ sig_i): strict .069 753 / 1454 us, .031 1053 / 1308, .028 1351 / 1709,
- * .021 1338 / 1247, .014 tiles; fast .131 424 / 610, .156 555 / 792,
- * .088 569 / 611, .104 797 / 775, .053 tiles.  Strict, where a history scatters
- * every other cell and the chain is short: tiles 1.3 to 1.5 times the lanes' time up
- * to 48 cells of sig_i width .5, .99 at 100.  And chains of one to five cells, on
- * which a tile is a step or two: 1.25 times at one cell, 1.1 at four, .95 at eight. */
-bool mcg_thick(const float4 *cells, int n, bool strict)
+/* Chains on which a lane per history is faster than tiles: of up to seven cells, on
+ * which a tile is a few steps, and of thick cells, by their mean optical widths,
+ * which end a tile's flights or (strict, u < 2^-4) its crossings after a step or
+ * two; where absorption ends histories in a few cells, also long chains.  Tiles /
+ * lanes, widths sig_a and sig_i: almost nothing 2.2 at one cell, 1.6 at four, 1.15 at
+ * eight, .9 at twelve.  Strict .02 and .02 .65 to 1.0; .05, .05 1.5 to 1.7 from 8 to
+ * 64 cells, 1.1 at 100, .8 at 200, .6 at 400; .3, .3 2.0 at 24, .86 at 100; .01, .5 1.3
+ * at 24, .96 at 64; .1, .01 3.0 at 100, 2.1 at 200, 1.1 at 400.  Fast .05, .05 1.0 at
+ * 24, .7 at 100; .1, .1 1.5 at 24, .8 at 100; .01, .1 1.2 at 16, .86 at 48; .05, .3
+ * 1.4 at 100, 1.1 at 200; .3, .001 4.3 at 200, 1.7 at 400. */
+bool mcg_thick(const mcg_widths &w, int n, bool strict)
 {
-  if (n < 6)
+  if (n < 8)
     return n > 0;
-  double a = 0.0, i = 0.0;
-  for (int c = 0; c < n; ++c) {
-    const double len = (double)cells[c].w - cells[c].z;
-    a += std::fabs((double)cells[c].x) * len;
-    i += std::fabs((double)cells[c].y) * len;
-  }
-  return strict ? a > 0.02 * n || (n < 80 && i > 0.25 * n) : a + i > 0.08 * n;
+  if (n < 100)
+    return strict ? w.a > 0.025 * n || (n < 80 && w.i > 0.25 * n) : w.a + w.i > 0.08 * n;
+  return strict ? w.a > 0.05 * n && w.a > 3.0 * w.i : w.a + w.i > 0.25 * n;
 }
 
 /* The cells and their tile table to the device; `tab` holds the latter until

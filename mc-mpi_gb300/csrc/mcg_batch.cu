@@ -15,10 +15,15 @@
  * Waiting for them instead, an item's end cost its block up to 3 ms (the
  * longest of its histories): 4096 slabs of up to 50,000 histories, strict,
  * took 285 ms with that, 278 without, 36 more of it per halving of the items.
- * Issue-bound (66 % of the slots; 5 warp instructions per step and lane, 40 %
+ * Issue-bound (75 % of the slots; 4.65 warp instructions per step and lane, 40 %
  * in forming the steps, 20 % in the deposits, 16 % in full steps), then the
  * loads of the 136 MB step table through L2.  Whole run: 410 -> 206 ms strict,
  * 247 -> 155 ms fast.
+ *
+ * Short and thick slabs, whose histories take a few steps or end their flights
+ * at every other one, go to a second kernel with a lane per history
+ * (mcg_batch_lanes): 2000 slabs of 16 to 64 cells of width .5 (2000 histories each)
+ * strict 6.8 ms by tiles, 3.2 so, fast 5.1 and 1.5; of width 1e-4 2.0 and .77.
  */
 #include <algorithm>
 #include <new>
@@ -41,6 +46,12 @@ __global__ void __launch_bounds__(1024) mcg_batch_kernel(mcg_batch_params P)
   mcg_batch_body<STRICT, TALLY, false>(P);
 }
 
+template <bool STRICT, int TALLY>
+__global__ void __launch_bounds__(MCG_LANES_BLOCK, 4) mcg_batch_lanes_kernel(mcg_batch_params P)
+{
+  mcg_batch_lanes_body<STRICT, TALLY, false>(P);
+}
+
 /* ------------------------------------------------------------ host side */
 static mcg_batch_state *batch_of(mcg_context *ctx)
 {
@@ -58,6 +69,11 @@ static void batch_free(mcg_batch_state *B)
       cudaFree(p);
   if (B->graph)
     cudaGraphExecDestroy(B->graph);
+  if (B->side)
+    cudaStreamDestroy(B->side);
+  for (cudaEvent_t ev : {B->fork, B->join})
+    if (ev)
+      cudaEventDestroy(ev);
   *B = mcg_batch_state();
 }
 
@@ -88,6 +104,17 @@ __global__ void mcg_batch_tables(const float4 *strict, float4 *fast, float4 *tab
     fast[k] = make_float4(c.x, c.y > 1e-4f ? c.y : 0.0f, c.z, c.w);
     tab[k] = mcg_tile_cell(fast[k]);
   }
+}
+
+/* Slabs whose histories take a lane each: up to 100 cells, and thick ones.  Batches
+ * of up to 3000 slabs, tiles / lanes, strict: 20 cells of width .005 in both sections
+ * 1.8 times, 40 1.2, 80 .8 (3000 histories each) to 2.4 (100,000), 160 .8, 320 .5; 80
+ * cells of .1 and .01 3.3, 320 2.4; 320 of .05 1.2, of .02 .7; 200 to 800 of .03 .93.
+ * Fast: 80 cells of .005 .8 to 3.1, 160 .7, 320 .5; 320 of .05 .7, of .1 1.0, of .01
+ * and .5 2.4. */
+bool mcg_batch_lanes(const mcg_widths &w, int n, bool strict)
+{
+  return n <= 100 || (strict ? w.a > 0.04 * n || w.i > 0.25 * n : w.a + w.i > 0.15 * n);
 }
 
 extern "C" int mcg_batch_set(mcg_context *ctx, int32_t n_slabs, const mcg_slab *h_slabs,
@@ -137,14 +164,18 @@ extern "C" int mcg_batch_set(mcg_context *ctx, int32_t n_slabs, const mcg_slab *
   B->min_w = particle_min_weight;
   B->slabs.assign(h_slabs, h_slabs + n_slabs);
   B->cell_off.resize(n_slabs);
+  B->slab_lanes.resize(n_slabs);
   int64_t off = 0;
   for (int s = 0; s < n_slabs; ++s) {
     const mcg_slab &sl = h_slabs[s];
     B->cell_off[s] = (int32_t)off;
     const float dx = (1.0f - 0.0f) / (float)sl.n_cells; /* Layer(0, 1, 0, m): src/layer.cpp:47 */
     float4 fast;
-    for (int j = 0; j < sl.n_cells; ++j)
+    mcg_widths widths;
+    for (int j = 0; j < sl.n_cells; ++j) {
       mcg_cell_params(h_sigs[off + j], h_rates[off + j], j, dx, cs[off + j], fast);
+      widths.add(cs[off + j]);
+    }
     sd[s].cell_off = (int32_t)off;
     sd[s].m = sl.n_cells;
     sd[s].n_hist = sl.n_histories;
@@ -155,6 +186,10 @@ extern "C" int mcg_batch_set(mcg_context *ctx, int32_t n_slabs, const mcg_slab *
     sd[s].src.mu0 = sl.mu0;
     sd[s].src.w0 = sl.w0;
     sd[s].src.cell0 = 0;
+    B->slab_lanes[s] = (mcg_batch_lanes(widths, sl.n_cells, true) ? 1 : 0) |
+                       (mcg_batch_lanes(widths, sl.n_cells, false) ? 2 : 0) |
+                       (mcg_thick(widths, sl.n_cells, true) ? 4 : 0) |
+                       (mcg_thick(widths, sl.n_cells, false) ? 8 : 0);
     off += sl.n_cells;
   }
   /* any failure from here on leaves no slabs set (launches return
@@ -192,28 +227,36 @@ extern "C" int mcg_batch_set(mcg_context *ctx, int32_t n_slabs, const mcg_slab *
  * is also at most a sixteenth of a block's even share of the run (cost: histories
  * x cells), so a small run still has an item for every block and the last ones
  * are short: 37 slabs of up to 20,000 histories took 34 ms with the 40 items
- * that 16,384 histories make of them.  Not below 64 histories: each item loads
- * and adds its slab's tally. */
+ * that 16,384 histories make of them.  Not below 64 histories (512 for a lane
+ * each, two rounds of a block): each item loads and adds its slab's tally.  The
+ * items of the second kernel come last, and there are none unless they are a tenth
+ * of the work: 37 slabs with three of them took 4 % longer in two launches. */
 static int build_items(mcg_context *ctx, mcg_batch_state *B, int64_t item, double fraction, int grid)
 {
   std::vector<mcg_batch_item> items;
   std::vector<double> cost;
+  const bool strict = ctx->mode == MCG_MODE_STRICT;
   auto histories = [&](int s) {
     const int64_t n = B->slabs[s].n_histories;
     return fraction < 1.0 ? std::max<int64_t>(std::min<int64_t>(n, 32), (int64_t)std::ceil(n * fraction))
                           : n;
   };
-  double total = 0.0;
-  for (int s = 0; s < B->n_slabs; ++s)
+  double total = 0.0, by_lanes = 0.0;
+  for (int s = 0; s < B->n_slabs; ++s) {
     total += (double)histories(s) * B->slabs[s].n_cells;
+    if (B->slab_lanes[s] & (strict ? 1 : 2))
+      by_lanes += (double)histories(s) * B->slabs[s].n_cells;
+  }
+  const bool mixed = by_lanes > 0.1 * total;
   for (int s = 0; s < B->n_slabs; ++s) {
     const int64_t n = histories(s);
     const int64_t share = (int64_t)(total / (16.0 * grid) / B->slabs[s].n_cells);
-    const int64_t step = std::min(item, std::max<int64_t>(64, share));
+    const bool lanes = mixed && (B->slab_lanes[s] & (strict ? 1 : 2));
+    const int64_t step = std::min(item, std::max<int64_t>(lanes ? 512 : 64, share));
     for (int64_t f = 0; f < n; f += step) {
       mcg_batch_item it;
       it.slab = s;
-      it.pad = 0;
+      it.lanes = lanes;
       it.first = f;
       it.count = std::min(step, n - f);
       items.push_back(it);
@@ -223,7 +266,9 @@ static int build_items(mcg_context *ctx, mcg_batch_state *B, int64_t item, doubl
   std::vector<size_t> order(items.size());
   for (size_t i = 0; i < order.size(); ++i)
     order[i] = i;
-  std::stable_sort(order.begin(), order.end(), [&](size_t a, size_t b) { return cost[a] > cost[b]; });
+  std::stable_sort(order.begin(), order.end(), [&](size_t a, size_t b) {
+    return items[a].lanes != items[b].lanes ? items[a].lanes < items[b].lanes : cost[a] > cost[b];
+  });
   std::vector<mcg_batch_item> sorted(items.size());
   for (size_t i = 0; i < order.size(); ++i)
     sorted[i] = items[order[i]];
@@ -240,8 +285,15 @@ static int build_items(mcg_context *ctx, mcg_batch_state *B, int64_t item, doubl
                              cudaMemcpyHostToDevice);
   if (e != cudaSuccess)
     return mcg_cuda_fail(e, "mcg_batch: upload items");
+  B->lane_cells = 0;
+  for (int s = 0; s < B->n_slabs; ++s)
+    if (B->slab_lanes[s] & (strict ? 1 : 2))
+      B->lane_cells = std::max(B->lane_cells, B->slabs[s].n_cells);
   B->n_items = (int)sorted.size();
+  B->n_tiled = (int)std::count_if(sorted.begin(), sorted.end(),
+                                  [](const mcg_batch_item &it) { return !it.lanes; });
   B->items_built_for = item;
+  B->items_strict = strict;
   B->items_grid = grid;
   B->items_fraction = fraction;
   B->graph_valid = false;
@@ -253,6 +305,11 @@ struct mcg_batch_launch {
   mcg_batch_params P;
   size_t smem;
   int grid, block;
+  /* the items that take a lane per history, beside the others */
+  void (*lanes_kern)(mcg_batch_params);
+  mcg_batch_params lanes;
+  size_t lanes_smem;
+  int lanes_grid;
 };
 
 /* Lanes waiting for the full step that trigger it (mcg_batch_set_deferral 0):
@@ -304,28 +361,73 @@ static int batch_configure(mcg_context *ctx, mcg_batch_state *B, int64_t item, d
   if (e != cudaSuccess)
     return mcg_cuda_fail(e, "mcg_batch: launch set-up");
   L.grid = ctx->sm_count * std::max(bps, 1);
-  if (B->items_built_for != item || B->items_grid != L.grid || B->items_fraction != fraction) {
+  if (B->items_built_for != item || B->items_grid != L.grid || B->items_fraction != fraction ||
+      B->items_strict != strict) {
     int rc = build_items(ctx, B, item, fraction, L.grid);
     if (rc != MCG_OK)
       return rc;
   }
   P.items = static_cast<const mcg_batch_item *>(B->d_items);
-  P.n_items = B->n_items;
+  P.n_items = B->n_tiled;
+  L.lanes = P;
+  L.lanes.items = P.items + B->n_tiled;
+  L.lanes.n_items = B->n_items - B->n_tiled;
+  L.lanes.item_next = P.item_next + 1;
+  if (L.lanes.n_items == 0)
+    return MCG_OK;
+  const bool global = B->tally_mode == MCG_TALLY_GLOBAL ||
+                      mcg_batch_lanes_smem(B->lane_cells, true) > (size_t)ctx->smem_optin;
+  L.lanes_smem = mcg_batch_lanes_smem(B->lane_cells, !global);
+  if (strict)
+    L.lanes_kern = global ? mcg_batch_lanes_kernel<true, MCG_TALLY_GLOBAL>
+                          : mcg_batch_lanes_kernel<true, MCG_TALLY_SMEM32>;
+  else
+    L.lanes_kern = global ? mcg_batch_lanes_kernel<false, MCG_TALLY_GLOBAL>
+                          : mcg_batch_lanes_kernel<false, MCG_TALLY_SMEM32>;
+  e = cudaFuncSetAttribute(L.lanes_kern, cudaFuncAttributeMaxDynamicSharedMemorySize, ctx->smem_optin);
+  if (e == cudaSuccess)
+    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, L.lanes_kern, MCG_LANES_BLOCK, L.lanes_smem);
+  if (e == cudaSuccess && !B->side)
+    e = cudaStreamCreateWithFlags(&B->side, cudaStreamNonBlocking);
+  for (cudaEvent_t *ev : {&B->fork, &B->join})
+    if (e == cudaSuccess && !*ev)
+      e = cudaEventCreateWithFlags(ev, cudaEventDisableTiming);
+  if (e != cudaSuccess)
+    return mcg_cuda_fail(e, "mcg_batch: launch set-up");
+  L.lanes_grid = std::min(ctx->sm_count * std::max(bps, 1), L.lanes.n_items);
   return MCG_OK;
 }
 
+/* The two kernels side by side: the lane form's blocks come first, the others fill
+ * the SMs that those leave. */
 static int batch_enqueue(mcg_context *ctx, mcg_batch_state *B, const mcg_batch_launch &L)
 {
-  cudaError_t e;
-  if ((e = cudaMemsetAsync(B->d_item_next, 0, 8, ctx->stream)) != cudaSuccess)
-    return mcg_cuda_fail(e, "mcg_batch: memset");
-  L.kern<<<L.grid, L.block, L.smem, ctx->stream>>>(L.P);
-  if ((e = cudaGetLastError()) != cudaSuccess)
-    return mcg_cuda_fail(e, "mcg_batch_kernel launch");
-  ctx->last_grid = L.grid;
-  ctx->last_block = L.block;
-  ctx->launches++;
-  return MCG_OK;
+  cudaError_t e = cudaMemsetAsync(B->d_item_next, 0, 16, ctx->stream);
+  if (L.lanes.n_items) {
+    const bool beside = L.P.n_items > 0;
+    cudaStream_t st = beside ? B->side : ctx->stream;
+    if (e == cudaSuccess && beside && (e = cudaEventRecord(B->fork, ctx->stream)) == cudaSuccess)
+      e = cudaStreamWaitEvent(st, B->fork, 0);
+    if (e == cudaSuccess) {
+      L.lanes_kern<<<L.lanes_grid, MCG_LANES_BLOCK, L.lanes_smem, st>>>(L.lanes);
+      e = cudaGetLastError();
+      ctx->last_grid = L.lanes_grid;
+      ctx->last_block = MCG_LANES_BLOCK;
+      ctx->launches++;
+    }
+    if (e == cudaSuccess && beside)
+      e = cudaEventRecord(B->join, st);
+  }
+  if (e == cudaSuccess && L.P.n_items) {
+    L.kern<<<L.grid, L.block, L.smem, ctx->stream>>>(L.P);
+    e = cudaGetLastError();
+    ctx->last_grid = L.grid;
+    ctx->last_block = L.block;
+    ctx->launches++;
+    if (e == cudaSuccess && L.lanes.n_items)
+      e = cudaStreamWaitEvent(ctx->stream, B->join, 0);
+  }
+  return e == cudaSuccess ? MCG_OK : mcg_cuda_fail(e, "mcg_batch_kernel launch");
 }
 
 /* First history of each slab for the event engine, with the same sampled
@@ -467,16 +569,24 @@ extern "C" int mcg_batch_run_per_slab(mcg_context *ctx)
     const int block = shape.block;
     const size_t smem = shape.smem;
     P.tally_copies = shape.copies;
-    auto kern = strict ? (shape.global ? mcg_track_kernel<true, MCG_TALLY_GLOBAL, false>
-                                       : mcg_track_kernel<true, MCG_TALLY_SMEM32, false>)
-                       : (shape.global ? mcg_track_kernel<false, MCG_TALLY_GLOBAL, false>
-                                       : mcg_track_kernel<false, MCG_TALLY_SMEM32, false>);
+    const bool lanes = B->slab_lanes[s] & (strict ? 4 : 8);
+    void (*kern)(mcg_track_params);
+    if (lanes)
+      kern = strict ? (shape.global ? mcg_track_kernel<true, MCG_TALLY_GLOBAL, false, true>
+                                    : mcg_track_kernel<true, MCG_TALLY_SMEM32, false, true>)
+                    : (shape.global ? mcg_track_kernel<false, MCG_TALLY_GLOBAL, false, true>
+                                    : mcg_track_kernel<false, MCG_TALLY_SMEM32, false, true>);
+    else
+      kern = strict ? (shape.global ? mcg_track_kernel<true, MCG_TALLY_GLOBAL, false>
+                                    : mcg_track_kernel<true, MCG_TALLY_SMEM32, false>)
+                    : (shape.global ? mcg_track_kernel<false, MCG_TALLY_GLOBAL, false>
+                                    : mcg_track_kernel<false, MCG_TALLY_SMEM32, false>);
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          ctx->smem_optin);
     int bps = 1;
     if (e == cudaSuccess)
       e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, kern, block, smem);
-    const int grid = mcg_track_grid(ctx->sm_count * std::max(bps, 1), block, sl.n_histories, false, P);
+    const int grid = mcg_track_grid(ctx->sm_count * std::max(bps, 1), block, sl.n_histories, lanes, P);
     if (e == cudaSuccess)
       e = cudaMemsetAsync(ctx->d_next, 0, 8, ctx->stream);
     if (e == cudaSuccess) {

@@ -12,6 +12,8 @@
 
 #define MCG_ITEM_MOST 8192 /* LOSS: most histories of an item */
 
+bool mcg_batch_lanes(const mcg_widths &w, int n, bool strict);
+
 /* A cell's entry of the tile table from its fast-arithmetic parameters
  * (mcg_tile_table: within a slab neighbours share their faces). */
 __host__ __device__ inline float4 mcg_tile_cell(const float4 c)
@@ -22,7 +24,7 @@ __host__ __device__ inline float4 mcg_tile_cell(const float4 c)
 }
 
 struct mcg_batch_item {
-  int32_t slab, pad;
+  int32_t slab, lanes; /* lanes: a lane per history (mcg_batch_lanes) */
   int64_t first, count;
 };
 
@@ -157,6 +159,105 @@ __device__ __forceinline__ void mcg_batch_body(const mcg_batch_params &P)
         return true;
       });
   __syncthreads();
+  flush();
+  if (LOSS)
+    return;
+  for (int o = 16; o > 0; o >>= 1) {
+    tot_steps += __shfl_down_sync(0xffffffffu, tot_steps, o);
+    tot_scat += __shfl_down_sync(0xffffffffu, tot_scat, o);
+  }
+  if (lane == 0) {
+    atomicAdd(&s_cnt[MCG_CNT_STEPS], tot_steps);
+    atomicAdd(&s_cnt[MCG_CNT_SCAT], tot_scat);
+  }
+  __syncthreads();
+  if (tid < MCG_CNT_N && s_cnt[tid]) {
+    if (tid == MCG_CNT_ERR)
+      atomicOr(&P.counters[tid], s_cnt[tid]);
+    else
+      atomicAdd(&P.counters[tid], s_cnt[tid]);
+  }
+}
+
+/* Shared memory of the lane form: libm tables, counters, the item and its history
+ * counter, jumps, the tally of one slab. */
+#define MCG_LANES_BLOCK 256
+inline size_t mcg_batch_lanes_smem(int cells, bool tally)
+{
+  return sizeof(mcg_libm_tab) + 16 * 8 + 16 + sizeof(mcg_chain_jumps) + (tally ? (size_t)cells * 8 : 0);
+}
+
+/* The items of slabs on which a lane per history is faster (mcg_batch_lanes), each
+ * by one block, to its end: such histories are short. */
+template <bool STRICT, int TALLY, bool LOSS>
+__device__ __forceinline__ void mcg_batch_lanes_body(const mcg_batch_params &P)
+{
+  extern __shared__ __align__(16) unsigned char smem[];
+  mcg_libm_tab *T = reinterpret_cast<mcg_libm_tab *>(smem);
+  unsigned long long *s_cnt = reinterpret_cast<unsigned long long *>(smem + sizeof(mcg_libm_tab));
+  unsigned long long *s_ctl = s_cnt + 16; /* item, histories handed out */
+  mcg_chain_jumps *s_chain = reinterpret_cast<mcg_chain_jumps *>(s_ctl + 2);
+  unsigned long long *s_tally = reinterpret_cast<unsigned long long *>(s_chain + 1);
+  const int tid = threadIdx.x, lane = tid & 31;
+  mcg_fill_chain_jumps(s_chain);
+  if (STRICT) {
+    const float *src = reinterpret_cast<const float *>(P.libm_tab);
+    float *dst = reinterpret_cast<float *>(T);
+    for (int i = tid; i < (int)(sizeof(mcg_libm_tab) / 4); i += blockDim.x)
+      dst[i] = src[i];
+  }
+  if (tid < 16)
+    s_cnt[tid] = 0ull;
+  int off = -1, m = 0;
+  auto flush = [&] {
+    if (TALLY != MCG_TALLY_GLOBAL)
+      for (int i = tid; i < m; i += blockDim.x)
+        if (s_tally[i])
+          atomicAdd(&P.tally[off + i], s_tally[i]);
+  };
+  unsigned long long tot_steps = 0, tot_scat = 0;
+  for (;;) {
+    __syncthreads();
+    if (tid == 0) {
+      s_ctl[0] = atomicAdd(P.item_next, 1ull);
+      s_ctl[1] = 0;
+    }
+    __syncthreads();
+    const long long item = (long long)s_ctl[0];
+    if (item >= P.n_items)
+      break;
+    const mcg_batch_item it = P.items[item];
+    const mcg_batch_slab_dev sd = P.slabs[it.slab];
+    if (sd.cell_off != off) {
+      flush(); /* and then zero, each thread its own words */
+      off = sd.cell_off;
+      m = sd.m;
+      if (TALLY != MCG_TALLY_GLOBAL) {
+        __syncthreads();
+        for (int i = tid; i < m; i += blockDim.x)
+          s_tally[i] = 0ull;
+        __syncthreads();
+      }
+    }
+    const int64_t first = it.first + (LOSS ? *P.step * sd.n_hist : 0);
+    mcg_lane_histories<STRICT, TALLY, LOSS>(
+        m, P.cells + off, LOSS ? P.aux + off : nullptr, TALLY == MCG_TALLY_GLOBAL ? P.tally + off : s_tally,
+        P.rules, T, P.libm, &s_ctl[1], it.count, 0,
+        [&](long long my, uint64_t &seed, float &x, float &mu, float &wmc, int &idx) {
+          mcg_born(s_chain, sd.src, first + my, seed, x, mu, wmc, idx);
+          return LOSS ? item * MCG_ITEM_MOST + my : my;
+        },
+        [&](long long hid, int r, const mcg_lane &p, int) {
+          if (LOSS) {
+            if (P.loss)
+              P.loss[hid] = make_float2(p.G_hi, p.G_lo);
+            return;
+          }
+          mcg_count_end<STRICT>(s_cnt, r, p.wmc, p.wres, P.rules.q_log2);
+          tot_steps += p.nst;
+          tot_scat += p.nsc;
+        });
+  }
   flush();
   if (LOSS)
     return;

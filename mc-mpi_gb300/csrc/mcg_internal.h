@@ -20,9 +20,13 @@ struct mcg_batch_state {
   int64_t total_histories = 0;
   std::vector<mcg_slab> slabs;
   std::vector<int32_t> cell_off;
+  /* slabs that take a lane per history, strict and fast: 1 and 2 in the batch
+   * (mcg_batch_lanes), 4 and 8 in a launch of their own (mcg_thick) */
+  std::vector<uint8_t> slab_lanes;
   void *d_slabs = nullptr;  /* mcg_batch_slab_dev[] */
   void *d_items = nullptr;  /* mcg_batch_item[] */
-  int n_items = 0, items_cap = 0;
+  int n_items = 0, n_tiled = 0, items_cap = 0; /* the first n_tiled by tiles */
+  int lane_cells = 0; /* of the longest slab of the others */
   float4 *d_cells_strict = nullptr, *d_cells_fast = nullptr;
   float4 *d_tab = nullptr; /* the tiles' per-cell parameters */
   unsigned long long *d_tally = nullptr;
@@ -39,11 +43,15 @@ struct mcg_batch_state {
   /* CUDA graph of one run (memset of the item counter + the kernel) */
   cudaGraphExec_t graph = nullptr;
   bool graph_valid = false;
-  /* the context's settings that the graph's kernel holds by value */
+  cudaStream_t side = nullptr; /* the lane form's, between fork and join */
+  cudaEvent_t fork = nullptr, join = nullptr;
+  /* the context's settings that the graph's kernels hold by value */
   int graph_mode = -1, graph_scale = 0, graph_refill = 0;
   uint32_t graph_steps = 0;
-  int64_t items_built_for = -1; /* item size, grid and share of the histories the list is for */
+  int64_t items_built_for = -1; /* item size, launch, arithmetic and share of the histories
+                                   the list is for */
   int items_grid = 0;
+  bool items_strict = false;
   double items_fraction = 1.0;
 };
 
@@ -168,7 +176,17 @@ int mcg_fail(int code, const char *fmt, ...);
 cudaError_t mcg_dev_malloc(void **p, size_t bytes);
 int mcg_cuda_fail(cudaError_t e, const char *what);
 #define MCG_TAB_PAD 32 /* a tile reads past its chain's ends (mcg_tiles) */
-bool mcg_thick(const float4 *cells, int n, bool strict);
+/* Sums of a chain's optical widths, sig_a and sig_i: its optical depths. */
+struct mcg_widths {
+  double a = 0.0, i = 0.0;
+  void add(const float4 &c)
+  {
+    const double len = (double)c.w - c.z;
+    a += (c.x < 0.0f ? -c.x : c.x) * len;
+    i += (c.y < 0.0f ? -c.y : c.y) * len;
+  }
+};
+bool mcg_thick(const mcg_widths &w, int n, bool strict);
 cudaError_t mcg_read_tally(mcg_context *ctx, const unsigned long long *d, size_t n, int64_t *h_q,
                            double *h_f64);
 void mcg_tile_table(const float4 *cells_fast, int n, float4 *tab, float2 *right = nullptr,

@@ -138,7 +138,10 @@ extern "C" int mcg_simulate_fast_noalloc(int n_layers, const int32_t *h_index_st
     const int block = shape.block;
     const size_t smem = shape.smem;
     P.tally_copies = shape.copies;
-    const bool lanes = mcg_thick(cf.data(), total, false);
+    mcg_widths widths;
+    for (const float4 &c : cf)
+      widths.add(c);
+    const bool lanes = mcg_thick(widths, total, false);
     auto kern = lanes ? (smem_tally ? mcg_track_kernel<false, MCG_TALLY_SMEM32, false, true>
                                     : mcg_track_kernel<false, MCG_TALLY_GLOBAL, false, true>)
                       : (smem_tally ? mcg_track_kernel<false, MCG_TALLY_SMEM32, false>

@@ -1601,12 +1601,12 @@ __device__ __forceinline__ void mcg_histories(mcg_geometry &geo, mcg_sink &D, co
   }
 }
 
-/* Histories of a chain of thick cells (update_thin in mcg_api.cu): one lane
- * each through every step, MCG_LANES_STEPS of them between two looks for new
- * ones.  Collisions and steep absorptions leave the tiles a step or two each. */
+/* Histories of a chain of thick cells (mcg_thick): one lane each through every
+ * step, MCG_LANES_STEPS of them between two looks for new ones.  Collisions and
+ * steep absorptions leave the tiles a step or two each.  LOSS as in mcg_tiles. */
 #define MCG_LANES_STEPS 8
-template <bool STRICT, int TALLY, class BIRTH, class END>
-__device__ __forceinline__ void mcg_lane_histories(int ncell, const float4 *cells,
+template <bool STRICT, int TALLY, bool LOSS, class BIRTH, class END>
+__device__ __forceinline__ void mcg_lane_histories(int ncell, const float4 *cells, const float2 *aux,
                                                    unsigned long long *tally, const mcg_rules &R,
                                                    const mcg_libm_tab *T, const mcg_libm_dev &libm,
                                                    unsigned long long *counter, long long n, int chunk,
@@ -1627,6 +1627,7 @@ __device__ __forceinline__ void mcg_lane_histories(int ncell, const float4 *cell
         p.inv_mu = mcg_flight_rcp(p.mu);
         p.wres = 0.f;
         p.nst = p.nsc = 0;
+        p.G_hi = p.G_lo = 0.f;
         active = true;
       }
     }
@@ -1636,10 +1637,17 @@ __device__ __forceinline__ void mcg_lane_histories(int ncell, const float4 *cell
       const int kmax = (int)min((uint32_t)MCG_LANES_STEPS, R.max_steps - p.nst);
       int k = 0;
 #pragma unroll 1
-      for (; k < kmax && (p.wmc >= R.min_w) & ((unsigned)p.idx < (unsigned)ncell); ++k)
+      for (; k < kmax && (p.wmc >= R.min_w) & ((unsigned)p.idx < (unsigned)ncell); ++k) {
+        const int cell = p.idx;
+        float len, dep;
+        bool coll;
         mcg_step<STRICT, TALLY, false>(seed, p.x, p.mu, p.wmc, p.inv_mu, p.idx, p.nsc,
-                                       __ldg(cells + p.idx), tally + p.idx, R.q_log2, T, libm, nullptr,
-                                       nullptr, nullptr, STRICT ? nullptr : &p.wres);
+                                       __ldg(cells + cell), tally + cell, R.q_log2, T, libm,
+                                       LOSS ? &len : nullptr, LOSS ? &coll : nullptr,
+                                       LOSS ? &dep : nullptr, STRICT || LOSS ? nullptr : &p.wres);
+        if (LOSS)
+          mcg_ff_add(p.G_hi, p.G_lo, __fmul_rn(__ldg(&aux[cell].x), dep));
+      }
       p.nst += (uint32_t)k;
       if (!p.living(R)) {
         p.s2 = seed << 1;
@@ -1717,8 +1725,9 @@ __global__ void __launch_bounds__(THIN ? MCG_THIN_BLOCK : 1024) mcg_track_kernel
     tot_scat += p.nsc;
   };
   if constexpr (LANES)
-    mcg_lane_histories<STRICT, TALLY>(ncell, P.cells, TALLY == MCG_TALLY_GLOBAL ? P.tally : my_tally,
-                                      P.rules, T, P.libm, P.next, P.n, P.chunk, birth, end);
+    mcg_lane_histories<STRICT, TALLY, false>(ncell, P.cells, nullptr,
+                                             TALLY == MCG_TALLY_GLOBAL ? P.tally : my_tally, P.rules, T,
+                                             P.libm, P.next, P.n, P.chunk, birth, end);
   else
     mcg_histories<STRICT, THIN, TALLY, false, false>(
         geo, sink, P.cells, P.tab, my_tally, P.rules, tiles, s_real, T, P.libm, P.next,
