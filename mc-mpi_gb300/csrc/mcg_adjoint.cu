@@ -63,11 +63,14 @@ struct mcg_adj_params {
 /* Shared memory of the forward kernel: the tracker's, with the tiles' loss
  * weights. */
 #define MCG_ADJ_FORWARD_BLOCK 1024
-#define MCG_ADJ_SHORT 256 /* cells of the longest chain that mcg_adjoint_fused takes */
+#define MCG_ADJ_LANES_BLOCK 512
+#define MCG_ADJ_SHORT 256 /* cells of the longest chain that mcg_adjoint_fused takes whatever their widths */
 #define MCG_ADJ_FUSED_STEPS 8 /* its steps between two looks for new histories */
 #define MCG_ADJ_PART (1 << 24) /* most histories between a forward pass and its replay */
-static size_t adj_forward_smem(int n_cells, int block)
+static size_t adj_forward_smem(int n_cells, int block, bool lanes)
 {
+  if (lanes)
+    return mcg_track_smem(n_cells, 0, false);
   return mcg_track_smem(n_cells, block, false) +
          (size_t)(block / 32) * (sizeof(mcg_loss_smem) - sizeof(mcg_tile_smem<false>));
 }
@@ -77,8 +80,9 @@ static size_t adj_forward_smem(int n_cells, int block)
  * of the serial phase.  Bound: instruction issue, as the tracker.  1000 cells, 2e6
  * histories, strict: 18.3 ms with a lane per history, 14.3 ms so.
  */
-template <bool STRICT>
-__global__ void __launch_bounds__(1024) mcg_adjoint_forward(mcg_adj_params P)
+template <bool STRICT, bool LANES>
+__global__ void __launch_bounds__(LANES ? MCG_ADJ_LANES_BLOCK : 1024, LANES ? 2 : 1)
+mcg_adjoint_forward(mcg_adj_params P)
 {
   extern __shared__ __align__(16) unsigned char smem[];
   mcg_libm_tab *T = reinterpret_cast<mcg_libm_tab *>(smem);
@@ -101,29 +105,34 @@ __global__ void __launch_bounds__(1024) mcg_adjoint_forward(mcg_adj_params P)
   for (int i = tid; i < ncell; i += blockDim.x)
     s_tally[i] = 0ull;
   __syncthreads();
-  const mcg_tile_warp<false> tiles(tile, s_real);
-  mcg_geometry geo = {0, ncell};
-  mcg_sink sink = {(uint32_t)__cvta_generic_to_shared(s_tally), P.tally};
   unsigned long long tot_steps = 0, tot_scat = 0, loss = 0, hist = 0;
-  mcg_histories<STRICT, false, MCG_TALLY_SMEM32, false, true>(
-      geo, sink, P.cells, {P.tab, nullptr, 0, P.aux}, s_tally, P.rules, tiles, s_real, T, P.libm, P.next,
-      [&] { return (long long)P.n; }, P.chunk,
-      [&](long long my, uint64_t &seed, float &x, float &mu, float &wmc, int &idx) {
-        mcg_born(s_chain, P.src, P.first + my, seed, x, mu, wmc, idx);
-        idx -= lo;
-        return my;
-      },
-      [&](long long hid, int r, const mcg_lane &p, int) {
-        if (r == 2)
-          atomicOr(&s_cnt[MCG_CNT_ERR], 1ull); /* the step limit */
-        if (P.sum)
-          P.sum[hid] = make_float2(p.G_hi, p.G_lo);
-        loss += (unsigned long long)(mcg_to_fixed(p.G_hi, gs) + mcg_to_fixed(p.G_lo, gs));
-        ++hist;
-        tot_steps += p.nst;
-        tot_scat += p.nsc;
-      },
-      [] { return true; }, [] { return false; });
+  auto birth = [&](long long my, uint64_t &seed, float &x, float &mu, float &wmc, int &idx) {
+    mcg_born(s_chain, P.src, P.first + my, seed, x, mu, wmc, idx);
+    idx -= lo;
+    return my;
+  };
+  auto end = [&](long long hid, int r, const mcg_lane &p, int) {
+    if (r == 2)
+      atomicOr(&s_cnt[MCG_CNT_ERR], 1ull); /* the step limit */
+    if (P.sum)
+      P.sum[hid] = make_float2(p.G_hi, p.G_lo);
+    loss += (unsigned long long)(mcg_to_fixed(p.G_hi, gs) + mcg_to_fixed(p.G_lo, gs));
+    ++hist;
+    tot_steps += p.nst;
+    tot_scat += p.nsc;
+  };
+  if constexpr (LANES) {
+    mcg_lane_histories<STRICT, MCG_TALLY_SMEM32, true>(ncell, P.cells, P.aux, s_tally, P.rules, T, P.libm,
+                                                       P.next, P.n, P.chunk, birth, end);
+  } else {
+    const mcg_tile_warp<false> tiles(tile, s_real);
+    mcg_geometry geo = {0, ncell};
+    mcg_sink sink = {(uint32_t)__cvta_generic_to_shared(s_tally), P.tally};
+    mcg_histories<STRICT, false, MCG_TALLY_SMEM32, false, true>(
+        geo, sink, P.cells, {P.tab, nullptr, 0, P.aux}, s_tally, P.rules, tiles, s_real, T, P.libm,
+        P.next, [&] { return (long long)P.n; }, P.chunk, birth, end, [] { return true; },
+        [] { return false; });
+  }
   for (int o = 16; o > 0; o >>= 1) {
     loss += __shfl_down_sync(0xffffffffu, loss, o);
     hist += __shfl_down_sync(0xffffffffu, hist, o);
@@ -293,8 +302,8 @@ __global__ void __launch_bounds__(1024) mcg_adjoint_replay(mcg_adj_params P)
 }
 
 /*
- * Short chains: forward pass and replay in one kernel, every lane through the
- * whole step.  A short history is mostly its birth and its end, which the two
+ * Short chains, and those of thick cells (adj_thick): forward pass and replay in one
+ * kernel, every lane through the whole step.  A short history is mostly its birth and its end, which the two
  * kernels pay twice (50 cells, 1e6 histories, strict: 4.8 ms here, 5.4 ms there;
  * 100 cells: 7.7 against 7.2), and where thousands of histories add to the same
  * few floats the order of the additions shows: rounds in which colliding
@@ -528,6 +537,25 @@ extern "C" int mcg_adjoint_reset(mcg_context *ctx)
   return mcg_tally_reset(ctx);
 }
 
+/* Chains of thick cells, on which most steps are full ones: with a gradient the one
+ * kernel with every lane through the whole step (rounds gather too little there),
+ * without one a forward pass with a lane per history.  Two kernels / one, widths
+ * sig_a and sig_i, 300 to 1500 cells: strict .02, .02 .7, .05, .05 1.1, .1, .1 1.2,
+ * .1, .01 1.3 to 1.7, .01, .1 .6; fast .05, .05 .8, .01, .1 .85, .1, .01 1.2, .1, .1
+ * 1.2, .3, .3 1.5, .05, .3 1.7.  Forward pass, tiles / lanes, 40 and 300 cells: strict
+ * .02, .02 1.0 and .6, .05, .05 1.9 and 1.2, .1, .01 4.5 and 3.7; fast .05, .05 1.0 and
+ * .6, .1, .1 1.5 and .9, .3, .3 3.2 and 2.2, ten cells of .1, .1 1.7.  Below eight cells
+ * lanes (two cells: 2.1). */
+static bool adj_thick(const mcg_widths &w, int n, bool strict, bool gradient)
+{
+  if (n < 8)
+    return true;
+  if (strict)
+    return w.a > 0.035 * n || w.i > 0.25 * n;
+  return gradient ? w.a > 0.06 * n || w.a + w.i > 0.15 * n
+                  : w.a + w.i > (n < 32 ? 0.1 : 0.25) * n;
+}
+
 extern "C" int mcg_adjoint_run(mcg_context *ctx, const mcg_source *src, int64_t first, int64_t n,
                                int32_t with_gradient)
 {
@@ -568,20 +596,24 @@ extern "C" int mcg_adjoint_run(mcg_context *ctx, const mcg_source *src, int64_t 
   if (sizeof(mcg_libm_tab) + 16 * 8 + 2 * (size_t)ctx->n_cells * 8 > (size_t)ctx->smem_optin)
     return mcg_fail(MCG_ERR_ARG, "mcg_adjoint_run: chain of %d cells too long (max %d)",
                     ctx->n_cells, (int)((ctx->smem_optin - 2048 - 128) / 16));
-  auto forward = strict ? mcg_adjoint_forward<true> : mcg_adjoint_forward<false>;
+  const bool thick = adj_thick(ctx->widths, ctx->n_cells, strict, with_gradient), lanes = thick && !with_gradient;
+  auto forward = strict ? (lanes ? mcg_adjoint_forward<true, true> : mcg_adjoint_forward<true, false>)
+                        : (lanes ? mcg_adjoint_forward<false, true> : mcg_adjoint_forward<false, false>);
   auto replay = strict ? mcg_adjoint_replay<true> : mcg_adjoint_replay<false>;
   auto short_chain = strict ? mcg_adjoint_fused<true> : mcg_adjoint_fused<false>;
-  const bool fused = with_gradient && ctx->n_cells <= MCG_ADJ_SHORT;
-  int f_block = MCG_ADJ_FORWARD_BLOCK, f_bps = 1, bps = 1;
-  while (f_block > 128 && adj_forward_smem(ctx->n_cells, f_block) > (size_t)ctx->smem_optin)
+  const bool fused = with_gradient && (ctx->n_cells <= MCG_ADJ_SHORT || thick);
+  int f_block = lanes ? MCG_ADJ_LANES_BLOCK : MCG_ADJ_FORWARD_BLOCK, f_bps = 1, bps = 1;
+  while (f_block > 128 && adj_forward_smem(ctx->n_cells, f_block, lanes) > (size_t)ctx->smem_optin)
     f_block -= 128;
-  const size_t f_smem = adj_forward_smem(ctx->n_cells, f_block);
+  const size_t f_smem = adj_forward_smem(ctx->n_cells, f_block, lanes);
   const int block = ctx->block ? ctx->block : 512;
   size_t smem = sizeof(mcg_libm_tab) + (size_t)ctx->n_cells * 8;
-  const size_t fused_smem = sizeof(mcg_libm_tab) + 16 * 8 + 2 * (size_t)ctx->n_cells * 8; /* < 48 KB */
+  const size_t fused_smem = sizeof(mcg_libm_tab) + 16 * 8 + 2 * (size_t)ctx->n_cells * 8;
   cudaError_t e = cudaFuncSetAttribute(forward, cudaFuncAttributeMaxDynamicSharedMemorySize, ctx->smem_optin);
   if (e == cudaSuccess)
     e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&f_bps, forward, f_block, f_smem);
+  if (e == cudaSuccess && fused)
+    e = cudaFuncSetAttribute(short_chain, cudaFuncAttributeMaxDynamicSharedMemorySize, ctx->smem_optin);
   if (e == cudaSuccess)
     e = fused ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, short_chain, block, fused_smem)
               : mcg_grad_shape(replay, block, ctx->smem_optin, &smem, &P.jumps, &bps);
@@ -629,7 +661,7 @@ extern "C" int mcg_adjoint_run(mcg_context *ctx, const mcg_source *src, int64_t 
     P.first = first + at;
     P.n = std::min(part, n - at);
     const int64_t warps = (int64_t)ctx->sm_count * std::max(f_bps, 1) * (f_block / 32);
-    P.chunk = (int)std::min<int64_t>(32, (P.n + warps - 1) / warps);
+    P.chunk = lanes ? 32 : (int)std::min<int64_t>(32, (P.n + warps - 1) / warps);
     if ((e = cudaMemsetAsync(ctx->d_next, 0, 8, ctx->stream)) != cudaSuccess)
       return mcg_cuda_fail(e, "mcg_adjoint_run: memset");
     forward<<<(int)std::min<int64_t>((int64_t)ctx->sm_count * std::max(f_bps, 1), P.n), f_block, f_smem,

@@ -393,6 +393,7 @@ static void update_thin(mcg_context *ctx)
   }
   ctx->width_a = wa;
   ctx->width_i = wi;
+  ctx->widths = sum;
   ctx->thin_step = n > 0 && own <= 5e-4f;
   ctx->thick = mcg_thick(sum, n, true);
   ctx->thick_fast = mcg_thick(sum, n, false);

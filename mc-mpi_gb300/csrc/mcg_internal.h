@@ -108,6 +108,17 @@ struct mcg_batch_slab_dev {
   mcg_source src;
 };
 
+/* Sums of a chain's optical widths, sig_a and sig_i: its optical depths. */
+struct mcg_widths {
+  double a = 0.0, i = 0.0;
+  void add(const float4 &c)
+  {
+    const double len = (double)c.w - c.z;
+    a += (c.x < 0.0f ? -c.x : c.x) * len;
+    i += (c.y < 0.0f ? -c.y : c.y) * len;
+  }
+};
+
 struct mcg_context {
   int device = 0, mode = MCG_MODE_STRICT;
   int sm_count = 0, smem_optin = 0, cc_major = 0, cc_minor = 0;
@@ -128,7 +139,8 @@ struct mcg_context {
   bool thin_fast = false; /* sig_a and sig_i widths <= 4e-4 (fast THIN) */
   bool thick = false, thick_fast = false; /* mcg_thick, strict and fast */
   float width_a = 0.f, width_i = 0.f; /* those largest widths */
-  double depth_i = 0.0;               /* the chain's optical depth in sig_i */
+  double depth_i = 0.0;               /* the chain's optical depth in sig_i, where it scatters */
+  mcg_widths widths;
   float4 *d_cells_strict = nullptr, *d_cells_fast = nullptr;
   /* the tiles' per-cell parameters (mcg_tile_table), MCG_TAB_PAD entries
    * before and after; of the thin form one such array per direction, in the
@@ -176,16 +188,6 @@ int mcg_fail(int code, const char *fmt, ...);
 cudaError_t mcg_dev_malloc(void **p, size_t bytes);
 int mcg_cuda_fail(cudaError_t e, const char *what);
 #define MCG_TAB_PAD 32 /* a tile reads past its chain's ends (mcg_tiles) */
-/* Sums of a chain's optical widths, sig_a and sig_i: its optical depths. */
-struct mcg_widths {
-  double a = 0.0, i = 0.0;
-  void add(const float4 &c)
-  {
-    const double len = (double)c.w - c.z;
-    a += (c.x < 0.0f ? -c.x : c.x) * len;
-    i += (c.y < 0.0f ? -c.y : c.y) * len;
-  }
-};
 bool mcg_thick(const mcg_widths &w, int n, bool strict);
 cudaError_t mcg_read_tally(mcg_context *ctx, const unsigned long long *d, size_t n, int64_t *h_q,
                            double *h_f64);
