@@ -58,6 +58,7 @@ struct mcg_adj_params {
   const mcg_libm_tab *libm_tab;
   int32_t chunk, jumps; /* jumps: the seed chain's table fits in shared memory (replay) */
   float b_mid; /* mcg_run_consts */
+  int32_t refill; /* fused: steps between two looks for new histories */
 };
 
 /* Shared memory of the forward kernel: the tracker's, with the tiles' loss
@@ -65,7 +66,7 @@ struct mcg_adj_params {
 #define MCG_ADJ_FORWARD_BLOCK 1024
 #define MCG_ADJ_LANES_BLOCK 512
 #define MCG_ADJ_SHORT 256 /* cells of the longest chain that mcg_adjoint_fused takes whatever their widths */
-#define MCG_ADJ_FUSED_STEPS 8 /* its steps between two looks for new histories */
+#define MCG_ADJ_FUSED_STEPS 8 /* its steps between two looks for new histories (mcg_set_launch 0) */
 #define MCG_ADJ_PART (1 << 24) /* most histories between a forward pass and its replay */
 static size_t adj_forward_smem(int n_cells, int block, bool lanes)
 {
@@ -388,9 +389,9 @@ __global__ void __launch_bounds__(1024) mcg_adjoint_fused(mcg_adj_params P)
       break;
 
     if (active) {
-      /* up to refill_steps steps, never past the step limit; idx is local
+      /* up to P.refill steps, never past the step limit; idx is local
        * to the chain */
-      const int kmax = (int)min((uint32_t)MCG_ADJ_FUSED_STEPS, P.rules.max_steps - nst);
+      const int kmax = (int)min((uint32_t)P.refill, P.rules.max_steps - nst);
       int k = 0;
       bool going = true;
       for (; k < kmax; ++k) {
@@ -592,6 +593,7 @@ extern "C" int mcg_adjoint_run(mcg_context *ctx, const mcg_source *src, int64_t 
   P.libm = ctx->libm;
   P.libm_tab = ctx->libm_tab;
   P.b_mid = ctx->run_bounds[2];
+  P.refill = ctx->refill ? ctx->refill : MCG_ADJ_FUSED_STEPS;
   /* the longest chain: that of the replay's arrays beside a tally */
   if (sizeof(mcg_libm_tab) + 16 * 8 + 2 * (size_t)ctx->n_cells * 8 > (size_t)ctx->smem_optin)
     return mcg_fail(MCG_ERR_ARG, "mcg_adjoint_run: chain of %d cells too long (max %d)",

@@ -54,3 +54,20 @@ def test_forward_pass_costs_what_the_tracker_does(mcg, mode):
                 best.append(ctx.last_kernel_ms())
             times.append(min(best))
     assert times[1] < 2 * times[0], times
+
+
+@pytest.mark.parametrize("mode", ["strict", "fast"])
+@pytest.mark.parametrize("refill", [1, 3, 200])
+def test_refill_steps_of_the_one_kernel(mcg, mode, refill):
+    """mcg_set_launch's steps between two looks for new histories: the same sums."""
+    m, n = 40, 3000
+    with mcg.Context(mode=mode) as ctx:
+        ctx.set_layers_xs([0], [m], [f32(1.0 / m)], np.full(m, 0.3 * m), np.full(m, 0.3 * m), 1e-12)
+        ctx.adjoint_set_weights(np.ones(m, f32))
+        out = []
+        for steps in (0, refill):
+            ctx.set_launch(refill_steps=steps)
+            ctx.adjoint_reset()
+            ctx.adjoint_run(0, n)
+            out.append((ctx.tally_q().tobytes(), ctx.adjoint_read()[0], ctx.counters()))
+        assert out[0] == out[1]
