@@ -548,10 +548,9 @@ def bench_fit(mcg, device, scale=1.0, n_steps=200):
         ms = ctx.last_kernel_ms()
         sig, loss = ctx.fit_read()
     hist = n_steps * sum(d["n_histories"] for d in slabs)
-    # a step: forward pass and replay (in turns of 2048 items of 8192
-    # histories), the weights and the Adam update
-    items = sum(-(-d["n_histories"] // 8192) for d in slabs)
-    per_step = 2 * -(-items // 2048) + 2
+    # a step: forward pass and replay (in turns of at most 2^24 histories),
+    # the weights and the Adam update
+    per_step = 2 * -(-sum(d["n_histories"] for d in slabs) // 2 ** 24) + 2
     err0 = float(np.linalg.norm(1.0 - hidden) / np.linalg.norm(hidden))
     err = float(np.linalg.norm(sig - hidden) / np.linalg.norm(hidden))
     return {"value": hist / (ms / 1e3), "unit": "histories/s", "adam_steps": n_steps,

@@ -257,6 +257,7 @@ static int build_items(mcg_context *ctx, mcg_batch_state *B, int64_t item, doubl
       mcg_batch_item it;
       it.slab = s;
       it.lanes = lanes;
+      it.sum = 0;
       it.first = f;
       it.count = std::min(step, n - f);
       items.push_back(it);

@@ -10,8 +10,6 @@
 
 #include "mcg_track.cuh"
 
-#define MCG_ITEM_MOST 8192 /* LOSS: most histories of an item */
-
 bool mcg_batch_lanes(const mcg_widths &w, int n, bool strict);
 
 /* A cell's entry of the tile table from its fast-arithmetic parameters
@@ -26,12 +24,13 @@ __host__ __device__ inline float4 mcg_tile_cell(const float4 c)
 struct mcg_batch_item {
   int32_t slab, lanes; /* lanes: a lane per history (mcg_batch_lanes) */
   int64_t first, count;
+  int64_t sum; /* LOSS: its first history's place in `loss` */
 };
 
 struct mcg_batch_params {
   const float4 *cells, *tab;
   const float2 *aux;      /* LOSS: loss weights, {w_c, .} */
-  float2 *loss;           /* LOSS: a history's sum, at item x MCG_ITEM_MOST + its number in the item */
+  float2 *loss;           /* LOSS: the histories' sums; null: not wanted */
   const long long *step;  /* LOSS: histories of earlier steps precede this one's (null: none) */
   const mcg_batch_slab_dev *slabs;
   const mcg_batch_item *items;
@@ -48,10 +47,9 @@ struct mcg_batch_params {
 /* The item that a block works on (shared memory). */
 struct mcg_batch_work {
   unsigned long long taken; /* histories handed out */
-  long long item, first, count;
+  long long item, first, count, sum;
   int32_t off, m;
   mcg_source src;
-  long long pad;
 };
 
 /* Shared memory: libm tables, counters, the item, jumps, the tally of one slab,
@@ -107,7 +105,7 @@ __device__ __forceinline__ void mcg_batch_body(const mcg_batch_params &P)
       &work->taken, [&] { return work->count; }, 0,
       [&](long long my, uint64_t &seed, float &x, float &mu, float &wmc, int &idx) {
         mcg_born(s_chain, work->src, work->first + my, seed, x, mu, wmc, idx);
-        return LOSS ? work->item * MCG_ITEM_MOST + my : my;
+        return LOSS ? work->sum + my : my;
       },
       [&](long long hid, int r, const mcg_lane &p, int) {
         if (LOSS) {
@@ -136,6 +134,7 @@ __device__ __forceinline__ void mcg_batch_body(const mcg_batch_params &P)
             const mcg_batch_slab_dev sd = P.slabs[it.slab];
             work->first = it.first + (LOSS ? *P.step * sd.n_hist : 0);
             work->count = it.count;
+            work->sum = it.sum;
             work->off = sd.cell_off;
             work->m = sd.m;
             work->src = sd.src;
@@ -245,7 +244,7 @@ __device__ __forceinline__ void mcg_batch_lanes_body(const mcg_batch_params &P)
         P.rules, T, P.libm, &s_ctl[1], it.count, 0,
         [&](long long my, uint64_t &seed, float &x, float &mu, float &wmc, int &idx) {
           mcg_born(s_chain, sd.src, first + my, seed, x, mu, wmc, idx);
-          return LOSS ? item * MCG_ITEM_MOST + my : my;
+          return LOSS ? it.sum + my : my;
         },
         [&](long long hid, int r, const mcg_lane &p, int) {
           if (LOSS) {

@@ -38,11 +38,23 @@ struct mcg_fit_params {
   uint32_t max_steps;
 };
 
+#define MCG_FIT_ITEM 8192   /* most histories of an item */
+#define MCG_FIT_LANES 2048  /* ... of a slab whose histories take a lane each */
+#define MCG_FIT_PART (1 << 24) /* most histories between a forward pass and its replay: 128 MB of losses */
+
 /* Forward pass: the batched tracker with the losses.  64 slabs of up to 1024
  * cells, 1e5 histories each: 17.5 ms; 24 ms with a lane per history. */
 __global__ void __launch_bounds__(1024) mcg_fit_forward(mcg_batch_params P)
 {
   mcg_batch_body<false, MCG_TALLY_SMEM64, true>(P);
+}
+
+/* ... and its second kernel, for short and thick slabs (mcg_batch_lanes).  A gradient
+ * of 64 slabs of 16 to 64 cells, 50,000 histories each, replay included: width .3
+ * 10.1 ms by tiles, 5.6 so, .05 4.5 and 3.9; three such slabs 2.4 and 1.0. */
+__global__ void __launch_bounds__(MCG_LANES_BLOCK, 4) mcg_fit_forward_lanes(mcg_batch_params P)
+{
+  mcg_batch_lanes_body<false, MCG_TALLY_SMEM32, true>(P);
 }
 
 /*
@@ -99,7 +111,7 @@ __global__ void __launch_bounds__(512, 2) mcg_fit_replay(mcg_fit_params P)
       __syncthreads();
     }
     const int64_t src_base = step * sd.n_hist + it.first;
-    const float2 *sum = P.sum + item * MCG_ITEM_MOST;
+    const float2 *sum = P.sum + it.sum;
 
     uint64_t seed = 0;
     float x = 0.f, mu = 0.f, wmc = 0.f, inv_mu = 0.f;
@@ -232,14 +244,18 @@ __global__ void mcg_fit_adam_kernel(int n_cells, const int32_t *cell_slab,
 }
 
 /* ------------------------------------------------------------ host side */
-#define MCG_FIT_PART 2048 /* most items between a forward pass and its replay: 128 MB of losses */
+/* Items that go through a forward pass and its replay together, the first `tiled`
+ * by tiles. */
+struct mcg_fit_turn {
+  int first, items, tiled;
+};
 
 struct mcg_fit_state {
-  int n_slabs = 0, n_cells = 0, max_cells = 0, n_items = 0, max_steps = 0;
+  int n_slabs = 0, n_cells = 0, max_cells = 0, lane_cells = 0, max_steps = 0;
+  std::vector<mcg_fit_turn> turns;
   std::vector<int32_t> cell_off;
   void *dev = nullptr; /* one allocation for everything below */
-  void *dev_sum = nullptr; /* losses of `part` items, forward pass -> replay */
-  int part = 0;
+  void *dev_sum = nullptr; /* losses of a turn's histories, forward pass -> replay */
   float4 *cells = nullptr, *tab = nullptr; /* tab: mcg_tile_cell of cells */
   float2 *aux = nullptr;
   mcg_batch_slab_dev *slabs = nullptr;
@@ -294,13 +310,31 @@ extern "C" int mcg_fit_set(mcg_context *ctx, int32_t n_slabs, const mcg_slab *h_
   }
   if (16 * 4 + (size_t)maxc * 12 > (size_t)ctx->smem_optin)
     return mcg_fail(MCG_ERR_ARG, "mcg_fit_set: slab of %d cells too large", maxc);
-  /* items of up to MCG_ITEM_MOST histories, largest first */
+  /* items, largest first, those with a lane per history last */
   std::vector<mcg_batch_item> items;
-  for (int s = 0; s < n_slabs; ++s)
-    for (int64_t f = 0; f < h_slabs[s].n_histories; f += MCG_ITEM_MOST)
-      items.push_back({s, 0, f, std::min<int64_t>(MCG_ITEM_MOST, h_slabs[s].n_histories - f)});
+  std::vector<uint8_t> lanes(n_slabs);
+  double work = 0.0, by_lanes = 0.0;
+  for (int s = 0, k = 0; s < n_slabs; ++s) {
+    const int m = h_slabs[s].n_cells;
+    mcg_widths w;
+    for (int j = 0; j < m; ++j, ++k)
+      w.add(make_float4(h_sig_a0[k], h_sig_s[k], 0.0f, 1.0f / (float)m));
+    lanes[s] = mcg_batch_lanes(w, m, false);
+    work += (double)h_slabs[s].n_histories * m;
+    by_lanes += lanes[s] ? (double)h_slabs[s].n_histories * m : 0.0;
+  }
+  int lane_cells = 0;
+  for (int s = 0; s < n_slabs; ++s) {
+    if (!(by_lanes > 0.1 * work)) /* as in the batch (build_items) */
+      lanes[s] = 0;
+    lane_cells = std::max(lane_cells, lanes[s] ? h_slabs[s].n_cells : 0);
+    const int64_t step = lanes[s] ? MCG_FIT_LANES : MCG_FIT_ITEM;
+    for (int64_t f = 0; f < h_slabs[s].n_histories; f += step)
+      items.push_back({s, lanes[s], f, std::min(step, h_slabs[s].n_histories - f), 0});
+  }
   std::stable_sort(items.begin(), items.end(), [&](const mcg_batch_item &a, const mcg_batch_item &b) {
-    return a.count * h_slabs[a.slab].n_cells > b.count * h_slabs[b.slab].n_cells;
+    return a.lanes != b.lanes ? a.lanes < b.lanes
+                              : a.count * h_slabs[a.slab].n_cells > b.count * h_slabs[b.slab].n_cells;
   });
   /* carve one allocation */
   size_t off = 0;
@@ -312,7 +346,7 @@ extern "C" int mcg_fit_set(mcg_context *ctx, int32_t n_slabs, const mcg_slab *h_
   const size_t o_items = take(items.size() * sizeof(mcg_batch_item));
   const size_t o_cs = take(total * 4), o_t = take(total * 8), o_g = take(total * 8);
   const size_t o_lh = take(max_steps * 8), o_sa = take(total * 4), o_m1 = take(total * 4);
-  const size_t o_m2 = take(total * 4), o_ta = take(total * 8), o_in = take(16), o_st = take(8);
+  const size_t o_m2 = take(total * 4), o_ta = take(total * 8), o_in = take(24), o_st = take(8);
   mcg_fit_state *F = fit_of(ctx, true);
   /* a failure from here on leaves no fit set and nothing allocated */
   auto fail = [&](cudaError_t err, const char *what) {
@@ -322,13 +356,30 @@ extern "C" int mcg_fit_set(mcg_context *ctx, int32_t n_slabs, const mcg_slab *h_
   cudaError_t e = mcg_dev_malloc(&F->dev, off);
   if (e != cudaSuccess)
     return fail(e, "mcg_fit_set: cudaMalloc");
-  for (F->part = (int)std::min<size_t>(items.size(), MCG_FIT_PART);; F->part /= 2) {
-    if ((e = mcg_dev_malloc(&F->dev_sum, (size_t)F->part * MCG_ITEM_MOST * sizeof(float2))) == cudaSuccess)
-      break;
+  /* turns of as many histories as there is memory for, at least one item each */
+  int64_t most = 0, all = 0;
+  for (const mcg_batch_item &it : items) {
+    most = std::max(most, it.count);
+    all += it.count;
+  }
+  int64_t part = std::max<int64_t>(most, std::min<int64_t>(all, MCG_FIT_PART));
+  while ((e = mcg_dev_malloc(&F->dev_sum, (size_t)part * sizeof(float2))) != cudaSuccess) {
     cudaGetLastError();
     F->dev_sum = nullptr;
-    if (F->part <= 1)
+    if (part == most)
       return fail(e, "mcg_fit_set: cudaMalloc");
+    part = std::max(most, part / 2);
+  }
+  int64_t at = part;
+  for (int i = 0; i < (int)items.size(); ++i) {
+    if (at + items[i].count > part) {
+      F->turns.push_back({i, 0, 0});
+      at = 0;
+    }
+    items[i].sum = at;
+    at += items[i].count;
+    F->turns.back().items++;
+    F->turns.back().tiled += !items[i].lanes;
   }
   char *b = static_cast<char *>(F->dev);
   F->cells = reinterpret_cast<float4 *>(b + o_cells);
@@ -377,13 +428,13 @@ extern "C" int mcg_fit_set(mcg_context *ctx, int32_t n_slabs, const mcg_slab *h_
   F->n_slabs = n_slabs;
   F->n_cells = total;
   F->max_cells = maxc;
-  F->n_items = (int)items.size();
+  F->lane_cells = lane_cells;
   F->max_steps = max_steps;
   F->min_w = particle_min_weight;
   return MCG_OK;
 }
 
-/* The forward pass and (with_grad) the replay, in turns of F->part items. */
+/* The forward pass and (with_grad) the replay, in turns. */
 static int fit_launch_track(mcg_context *ctx, mcg_fit_state *F, int with_grad)
 {
   mcg_batch_params B;
@@ -395,7 +446,6 @@ static int fit_launch_track(mcg_context *ctx, mcg_fit_state *F, int with_grad)
   B.step = F->step;
   B.slabs = F->slabs;
   B.max_cells = F->max_cells;
-  B.item_next = F->item_next;
   B.tally = F->tally;
   B.rules = mcg_rules_setup(ctx, F->min_w);
   mcg_fit_params P;
@@ -411,7 +461,7 @@ static int fit_launch_track(mcg_context *ctx, mcg_fit_state *F, int with_grad)
   P.min_w = F->min_w;
   P.q_log2 = ctx->log2_scale;
   P.max_steps = ctx->max_steps;
-  int block = 1024, f_bps = 1, bps = 1;
+  int block = 1024, f_bps = 1, l_bps = 1, bps = 1;
   while (block > 128 && mcg_batch_smem(F->max_cells, block, true, true) > (size_t)ctx->smem_optin)
     block -= 128;
   const size_t f_smem = mcg_batch_smem(F->max_cells, block, true, true);
@@ -420,6 +470,11 @@ static int fit_launch_track(mcg_context *ctx, mcg_fit_state *F, int with_grad)
                                        ctx->smem_optin);
   if (e == cudaSuccess)
     e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&f_bps, mcg_fit_forward, block, f_smem);
+  const size_t l_smem = mcg_batch_lanes_smem(F->lane_cells, true); /* fewer cells than mcg_fit_set's limit */
+  if (e == cudaSuccess)
+    e = cudaFuncSetAttribute(mcg_fit_forward_lanes, cudaFuncAttributeMaxDynamicSharedMemorySize, ctx->smem_optin);
+  if (e == cudaSuccess)
+    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&l_bps, mcg_fit_forward_lanes, MCG_LANES_BLOCK, l_smem);
   if (e == cudaSuccess)
     e = mcg_grad_shape(mcg_fit_replay, 512, ctx->smem_optin, &smem, &P.jumps, &bps);
   if (e != cudaSuccess)
@@ -427,13 +482,26 @@ static int fit_launch_track(mcg_context *ctx, mcg_fit_state *F, int with_grad)
   /* two blocks: their accumulators take what they took before the forward
    * pass had its own kernel */
   bps = std::min(std::max(bps, 1), 2);
-  for (int i = 0; i < F->n_items; i += F->part) {
-    B.items = P.items = F->items + i;
-    B.n_items = P.n_items = std::min(F->part, F->n_items - i);
-    if ((e = cudaMemsetAsync(F->item_next, 0, 16, ctx->stream)) != cudaSuccess)
+  for (const mcg_fit_turn &t : F->turns) {
+    if ((e = cudaMemsetAsync(F->item_next, 0, 24, ctx->stream)) != cudaSuccess)
       return mcg_cuda_fail(e, "mcg_fit: memset");
-    mcg_fit_forward<<<ctx->sm_count * std::max(f_bps, 1), block, f_smem, ctx->stream>>>(B);
-    ctx->launches++;
+    P.items = F->items + t.first;
+    P.n_items = t.items;
+    B.items = P.items;
+    B.n_items = t.tiled;
+    B.item_next = F->item_next;
+    if (t.tiled) {
+      mcg_fit_forward<<<ctx->sm_count * std::max(f_bps, 1), block, f_smem, ctx->stream>>>(B);
+      ctx->launches++;
+    }
+    B.items = P.items + t.tiled;
+    B.n_items = t.items - t.tiled;
+    B.item_next = F->item_next + 2;
+    if (B.n_items) {
+      mcg_fit_forward_lanes<<<std::min(ctx->sm_count * std::max(l_bps, 1), B.n_items), MCG_LANES_BLOCK, l_smem,
+                              ctx->stream>>>(B);
+      ctx->launches++;
+    }
     if (with_grad) {
       mcg_fit_replay<<<ctx->sm_count * bps, 512, smem, ctx->stream>>>(P);
       ctx->launches++;
@@ -498,7 +566,7 @@ extern "C" int mcg_fit_run(mcg_context *ctx, int32_t n_steps, float lr, float be
   if (e != cudaSuccess || e2 != cudaSuccess)
     return mcg_cuda_fail(e != cudaSuccess ? e : e2, "mcg_fit_run");
   cudaEventElapsedTime(&ctx->last_ms, ctx->ev0, ctx->ev1);
-  ctx->launches += (2LL * ((F->n_items + F->part - 1) / F->part) + 2) * n_steps;
+  ctx->launches += (2LL * (long long)F->turns.size() + 2) * n_steps;
   return MCG_OK;
 }
 

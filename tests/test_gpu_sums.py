@@ -20,8 +20,8 @@ def _close(a, b):
     assert np.abs(a - b).max() <= 1e-4 * np.abs(b).max()
 
 
-def test_fit_of_more_items_than_one_turn(mcg):
-    """2100 items take two turns; the same slabs in two halves take one each."""
+def test_fit_of_many_items(mcg):
+    """2100 items, and the same slabs in two halves."""
     rng = np.random.default_rng(8)
     cells = rng.integers(1, 9, 2100)
     slabs, sa, ss = _fit(rng, cells, rng.integers(1, 60, 2100))
@@ -43,6 +43,38 @@ def test_fit_of_more_items_than_one_turn(mcg):
             far = np.abs(ctx.fit_read()[0] - sig[k]) > 1e-3
             assert far.sum() <= 0.01 * far.size
     assert loss.shape == (2,) and np.isfinite(loss).all()
+
+
+@pytest.mark.parametrize("turns", [1, 3])
+def test_fit_of_long_short_and_thick_slabs(mcg, fail_allocation, turns):
+    """Slabs that go to the two forward kernels of the fit, in one turn and in
+    several (a failed allocation halves the sums): the tracker's tallies, and the
+    adjoint's gradients but for the order of the float32 sums."""
+    rng = np.random.default_rng(6)
+    cells = np.array([1, 20, 64, 100, 101, 300, 500, 40])
+    histories = [5000, 9000, 2048, 2049, 3000, 8193, 700, 1]
+    width = [.2, .01, .3, 1e-3, .005, .3, .002, .1]
+    per = np.repeat(cells, cells)
+    sa = (np.repeat(width, cells) * per * rng.uniform(0.5, 1.5, per.size)).astype(f32)
+    ss = (0.7 * np.repeat(width, cells) * per * rng.uniform(0.5, 1.5, per.size)).astype(f32)
+    w = rng.standard_normal(per.size).astype(f32)
+    slabs = [dict(n_cells=int(m), n_histories=int(n), base_seed=11 + s, seed_mode=0, isotropic=0, mu0=1.0, w0=1.0)
+             for s, (m, n) in enumerate(zip(cells, histories))]
+    with mcg.Context(mode="fast") as ctx:
+        if turns > 1:
+            fail_allocation(1)
+        ctx.fit_set(slabs, sa, ss, np.zeros(per.size), max_steps=1)
+        t, g = ctx.fit_gradient(w)
+    o = 0
+    for d in slabs:
+        m, n, k = d["n_cells"], d["n_histories"], slice(o, o + d["n_cells"])
+        o += m
+        with mcg.Context(mode="fast") as ctx:
+            ctx.set_layers_xs([0], [m], [f32(1.0 / m)], sa[k], ss[k], 1e-12)
+            ctx.adjoint_set_weights(w[k])
+            ctx.adjoint_run(0, n, base_seed=d["base_seed"])
+            assert np.array_equal(t[k], ctx.tally() / n)
+            _close(g[k], ctx.adjoint_read()[1])
 
 
 @pytest.fixture
