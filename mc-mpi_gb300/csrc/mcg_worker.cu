@@ -549,8 +549,8 @@ static constexpr size_t mcg_lq_bytes(bool tiles)
 #define MCG_AQ_ROUND_IDLE 12
 #define MCG_AQ_ROUND_TILES 16
 /* ... and of short sub-domains (fewer than MCG_AQ_SHORT cells each on average),
- * where a tile is a few steps and a hand-over follows: a lane per particle through
- * every step, MCG_AQ_WINDOW of them between two votes, at most
+ * where a tile is a few steps and a hand-over follows (and of others, async_lanes): a
+ * lane per particle through every step, MCG_AQ_WINDOW of them between two votes, at most
  * MCG_AQ_ROUND_STEPS, and MCG_AQ_LANES_IDLE lanes that end the round, in blocks
  * of 1024 threads.  2e6 histories, lanes / tiles: 8 cells each 2.0 / 3.5 ms
  * (strict) and 2.2 / 3.9 (fast), 13 cells 2.2 / 2.9, 40 cells 4.2 / 2.7. */
@@ -997,6 +997,26 @@ __global__ void mcg_aq_init(unsigned long long *seq, unsigned long long total, u
     seq[i] = i % cap;
 }
 
+/* A lane per particle: in short sub-domains (MCG_AQ_SHORT), on thick cells, as the
+ * tracker does (mcg_thick), and where many histories stream through a short chain
+ * and reach its few inner faces together.  Kernel times, tiles / lanes, widths sig_a
+ * and sig_i, strict: 30 cells in one .05, .05 1.7 (fast 1.05), .1, .01 4.1 (1.4), .02,
+ * .02 1.1 (.9); 1000 in 8 .05, .05 1.2 (.6), .1, .01 3.2 (1.15), .02, .02 .7 (.5); fast
+ * 100 in 2 .1, .1 1.2, .3, .3 2.5.  5e5 histories through 60 cells in 2 of almost
+ * nothing 2.1, of .001 2.7, of .005 1.0; 3e5 through 100 in 2 1.65, 1.1, .76; 1e5
+ * through 300 in 2 and 10 of 1e-4 1.7 and 1.4, of .001 .5 and 1.0; 30 times fewer
+ * histories .6 to 1.0. */
+static bool async_lanes(const mcg_context *ctx, bool strict, bool thin, int layers, int64_t n)
+{
+  const mcg_widths &w = ctx->widths;
+  const int m = ctx->n_cells;
+  if ((int64_t)m < (int64_t)MCG_AQ_SHORT * layers)
+    return true;
+  if (strict ? w.a > 0.03 * m || w.i > 0.25 * m : w.a > 0.09 * m || w.a + w.i > 0.15 * m)
+    return true;
+  return layers > 1 && n >= 65536 && w.a + w.i < 0.004 * m && (m <= 100 || (thin && m < 500));
+}
+
 extern "C" int mcg_worker_run_async(mcg_context *ctx, const mcg_source *src, int64_t n,
                                     int64_t queue_capacity, int64_t *h_handoffs)
 {
@@ -1048,7 +1068,7 @@ extern "C" int mcg_worker_run_async(mcg_context *ctx, const mcg_source *src, int
   bool global = false;
   int block = 1024;
   auto smem_of = [&](bool t) { return async_smem(P_, (size_t)ctx->n_cells, block, global, thin, t); };
-  const bool tiled = (int64_t)ctx->n_cells >= (int64_t)MCG_AQ_SHORT * P_ ||
+  const bool tiled = !async_lanes(ctx, strict, thin, P_, n) ||
                      async_smem(P_, 0, 1024, true, false, false) > (size_t)ctx->smem_optin;
   if (tiled) {
     block = MCG_AQ_BLOCK;
