@@ -231,19 +231,17 @@ extern "C" int mcg_create(int device, int mode, mcg_context **out)
 static void free_geometry(mcg_context *ctx)
 {
   for (void *p : {(void *)ctx->d_cells_strict, (void *)ctx->d_cells_fast, (void *)ctx->d_tab,
-                  (void *)ctx->d_tally})
+                  (void *)ctx->d_thin, (void *)ctx->d_tally})
     if (p)
       cudaFree(p);
   ctx->d_cells_strict = ctx->d_cells_fast = ctx->d_tab = nullptr;
+  ctx->d_thin = nullptr;
   ctx->d_tally = nullptr;
   ctx->n_layers = ctx->n_cells = ctx->cell_lo = 0;
   ctx->layer_start.clear();
   ctx->layer_m.clear();
   ctx->layer_dx.clear();
-  ctx->sigs.clear();
-  ctx->rates.clear();
   ctx->cells_strict.clear();
-  ctx->cells_fast.clear();
   ctx->thin = ctx->thin_fast = ctx->thin_step = false;
 }
 
@@ -332,28 +330,34 @@ void mcg_cell_params(float sig, float rate, int gi, float dx, float4 &strict, fl
                      elo, ehi);
 }
 
-/* The tiles' parameters of n consecutive cells (mcg_tiles): {sig_a, sig_i, length
- * of a flight that enters the cell by its left face, by its right face}, the
- * float differences of the faces that mcg_step_cross forms (entered at a
- * neighbour's face, which between layers of different spacing differs from
- * the cell's own in the last bits).  Lengths outside the range in which the
- * cached-reciprocal division is exact, and those of cells that would amplify
- * the weight, are NaN: such steps take the full form.
- * sig_i <= EPS is 0 in both arithmetics: the flight always crosses. */
-static inline float4 tile_entry(const float4 *c, int n, int k)
+/* On the host (mcg_simulate_fast_noalloc). */
+void mcg_tile_table(const float4 *c, int n, float4 *tab)
 {
-  auto length = [&](float a) { return a >= 0x1p-90f && a <= 0x1p90f && c[k].x >= 0.0f ? a : NAN; };
-  return make_float4(c[k].x, c[k].y, length(c[k].w - (k ? c[k - 1].w : c[k].z)),
-                     length((k + 1 < n ? c[k + 1].z : c[k].w) - c[k].z));
+  for (int k = 0; k < n; ++k)
+    tab[k] = mcg_tile_entry(c, n, k);
 }
 
-void mcg_tile_table(const float4 *c, int n, float4 *tab, float2 *right, float2 *left)
+/* The fast arithmetic's cells (mcg_cell_params), the tile table and, where wanted, a
+ * thin chain's two, from the strict cells and with zeros beyond the ends: made on the
+ * host and uploaded they were 56 of the 72 bytes per cell (2e6 cells: 26 ms for
+ * mcg_set_layers; 15 before there were tiles, 11 so). */
+__global__ void mcg_chain_tables(const float4 *strict, int n, float4 *fast, float4 *tab, float2 *thin)
 {
-  for (int k = 0; k < n; ++k) {
-    tab[k] = tile_entry(c, n, k);
-    if (right) {
-      right[k] = make_float2(tab[k].x, tab[k].z);
-      left[k] = make_float2(tab[k].x, tab[k].w);
+  const int row = n + 2 * MCG_TAB_PAD;
+  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < row;
+       i += (int64_t)gridDim.x * blockDim.x) {
+    const int k = (int)i - MCG_TAB_PAD;
+    float4 t = make_float4(0.f, 0.f, 0.f, 0.f);
+    if ((unsigned)k < (unsigned)n) {
+      const float4 c = strict[k];
+      t = mcg_tile_entry(strict, n, k);
+      t.y = c.y > 1e-4f ? c.y : 0.0f;
+      fast[k] = make_float4(c.x, t.y, c.z, c.w);
+    }
+    tab[i] = t;
+    if (thin) {
+      thin[i] = make_float2(t.x, t.z);
+      thin[row + i] = make_float2(t.x, t.w);
     }
   }
 }
@@ -369,27 +373,27 @@ void mcg_tile_table(const float4 *c, int n, float4 *tab, float2 *right, float2 *
  * 1.4e-4 27.6 / 35.1, at 2.5 and 1.5e-4 15.3 / 18.8. */
 static void update_thin(mcg_context *ctx)
 {
-  float wa = 0.0f, wi = 0.0f;
-  float own = 0.0f;   /* the widest cell between its own faces, in sig_a */
-  ctx->depth_i = 0.0;
-  mcg_widths sum;
-  for (const float4 &c : ctx->cells_strict) {
-    sum.add(c);
-    const double len = (double)c.w - c.z;
-    ctx->depth_i += c.y > 1e-4f ? c.y * len : 0.0;
-    own = std::max(own, std::fabs(c.x) * (c.w - c.z));
-  }
-  /* the widths that bound a whole flight (mcg_thin_tests): of the lengths that
-   * the tiles use, since a cell entered from another layer's face may be wider
-   * than its own faces are apart (3.7 % at some sub-domains' ends of 10,000
-   * cells in 64, without limit between layers of different spacing).  A NaN
-   * length has no step in the tiles. */
+  const float4 *cells = ctx->cells_strict.data();
   const int n = (int)ctx->cells_strict.size();
+  float wa = 0.0f, wi = 0.0f;
+  float own = 0.0f; /* the widest cell between its own faces, in sig_a */
+  mcg_widths sum;
+  ctx->depth_i = 0.0;
   for (int k = 0; k < n; ++k) {
-    const float4 t = tile_entry(ctx->cells_strict.data(), n, k);
-    const float len = std::fmax(std::fmax(t.z, t.w), 0.0f);
-    wa = std::max(wa, std::fabs(t.x) * len);
-    wi = std::max(wi, std::fabs(t.y) * len);
+    const float4 c = cells[k];
+    const float len = c.w - c.z;
+    sum.add(c);
+    ctx->depth_i += c.y > 1e-4f ? (double)c.y * len : 0.0;
+    own = std::max(own, std::fabs(c.x) * len);
+    /* the widths that bound a whole flight (mcg_thin_tests): of the lengths that
+     * the tiles use, since a cell entered from another layer's face may be wider
+     * than its own faces are apart (3.7 % at some sub-domains' ends of 10,000
+     * cells in 64, without limit between layers of different spacing).  A NaN
+     * length has no step in the tiles. */
+    const float4 t = mcg_tile_entry(cells, n, k);
+    const float entry = t.z > t.w ? t.z : t.w > 0.0f ? t.w : t.z > 0.0f ? t.z : 0.0f;
+    wa = std::max(wa, std::fabs(c.x) * entry);
+    wi = std::max(wi, std::fabs(c.y) * entry);
   }
   ctx->width_a = wa;
   ctx->width_i = wi;
@@ -447,94 +451,101 @@ bool mcg_thick(const mcg_widths &w, int n, bool strict)
   return strict ? w.a > 0.05 * n && w.a > 3.0 * w.i : w.a + w.i > 0.25 * n;
 }
 
-/* The cells and their tile table to the device; `tab` holds the latter until
- * the stream is synchronised. */
-static cudaError_t upload_cells(mcg_context *ctx, std::vector<float4> &tab)
+/* The chain: layers checked, and its cells' two cross sections either from sigs and
+ * rates (Layer, mcg_cell_params) or given (xs). */
+static int set_geometry(mcg_context *ctx, const char *who, int n_layers, const int32_t *h_index_start,
+                        const int32_t *h_m, const float *h_dx, const float *h_a, const float *h_b, bool xs,
+                        float particle_min_weight)
 {
-  /* n + 2 PAD float4, then twice n + 2 PAD float2 */
-  const size_t n = ctx->cells_fast.size(), row = n + 2 * MCG_TAB_PAD;
-  tab.assign(2 * row, make_float4(0, 0, 0, 0));
-  float2 *thin = reinterpret_cast<float2 *>(&tab[row]);
-  mcg_tile_table(ctx->cells_fast.data(), (int)n, &tab[MCG_TAB_PAD], thin + MCG_TAB_PAD,
-                 thin + row + MCG_TAB_PAD);
-  ctx->d_thin = reinterpret_cast<float2 *>(ctx->d_tab + row);
-  cudaError_t e = cudaMemcpyAsync(ctx->d_cells_strict, ctx->cells_strict.data(), n * sizeof(float4),
-                                  cudaMemcpyHostToDevice, ctx->stream);
+  if (!ctx || n_layers <= 0 || !h_index_start || !h_m || !h_dx || !h_a || !h_b)
+    return mcg_fail(MCG_ERR_ARG, "%s: bad arguments", who);
+  int64_t total64 = 0;
+  for (int l = 0; l < n_layers; ++l) {
+    if (h_m[l] <= 0)
+      return mcg_fail(MCG_ERR_ARG, "%s: layer %d has %d cells", who, l, h_m[l]);
+    if (l > 0 && (int64_t)h_index_start[l] != (int64_t)h_index_start[l - 1] + h_m[l - 1])
+      return mcg_fail(MCG_ERR_ARG, "%s: layer %d is not contiguous", who, l);
+    total64 += h_m[l];
+    if (total64 > INT32_MAX)
+      return mcg_fail(MCG_ERR_ARG, "%s: more than 2^31 - 1 cells", who);
+  }
+  const int total = (int)total64;
+  int rc = ensure_device(ctx);
+  if (rc != MCG_OK)
+    return rc;
+  std::vector<float4> cells;
+  std::vector<int32_t> start, m;
+  std::vector<float> dx;
+  try {
+    cells.resize(total);
+    start.assign(h_index_start, h_index_start + n_layers);
+    m.assign(h_m, h_m + n_layers);
+    dx.assign(h_dx, h_dx + n_layers);
+  } catch (const std::bad_alloc &) {
+    return mcg_fail(MCG_ERR_ARG, "%s: no host memory for %d cells", who, total);
+  }
+  int k = 0;
+  float4 fast;
+  for (int l = 0; l < n_layers; ++l)
+    for (int j = 0; j < h_m[l]; ++j, ++k)
+      if (xs) {
+        const int gi = h_index_start[l] + j;
+        cells[k] = make_float4(h_a[k], h_b[k], (float)gi * h_dx[l], (float)(gi + 1) * h_dx[l]);
+      } else {
+        mcg_cell_params(h_a[k], h_b[k], h_index_start[l] + j, h_dx[l], cells[k], fast);
+      }
+  cudaStreamSynchronize(ctx->stream);
+  /* a chain of as many cells takes over the buffers (with the copies on the
+   * stream and one synchronisation, a call of the reference's seam with 100
+   * cells and 1000 particles takes 167 us instead of 204); otherwise the old
+   * geometry goes first; any failure below leaves no geometry */
+  cudaError_t e = cudaSuccess;
+  if (!ctx->d_tally || ctx->n_cells != total) {
+    free_geometry(ctx);
+    if ((e = mcg_dev_malloc((void **)&ctx->d_cells_strict, total * sizeof(float4))) == cudaSuccess &&
+        (e = mcg_dev_malloc((void **)&ctx->d_cells_fast, total * sizeof(float4))) == cudaSuccess &&
+        (e = mcg_dev_malloc((void **)&ctx->d_tab, (total + 2 * (size_t)MCG_TAB_PAD) * sizeof(float4))) == cudaSuccess)
+      e = mcg_dev_malloc((void **)&ctx->d_tally, total * sizeof(unsigned long long));
+  }
+  ctx->n_layers = n_layers;
+  ctx->layer_start.swap(start);
+  ctx->layer_m.swap(m);
+  ctx->layer_dx.swap(dx);
+  ctx->cells_strict.swap(cells);
+  update_thin(ctx);
+  /* the thin tables, for chains that the thin kernel can hold */
+  const bool thin = (ctx->thin || ctx->thin_fast) &&
+                    mcg_track_shape(total, 256, false, true, (size_t)ctx->smem_optin).thin;
+  if (!thin)
+    ctx->thin = ctx->thin_fast = false;
+  else if (e == cudaSuccess && !ctx->d_thin)
+    e = mcg_dev_malloc((void **)&ctx->d_thin, 2 * (total + 2 * (size_t)MCG_TAB_PAD) * sizeof(float2));
   if (e == cudaSuccess)
-    e = cudaMemcpyAsync(ctx->d_cells_fast, ctx->cells_fast.data(), n * sizeof(float4),
+    e = cudaMemcpyAsync(ctx->d_cells_strict, ctx->cells_strict.data(), total * sizeof(float4),
                         cudaMemcpyHostToDevice, ctx->stream);
-  if (e == cudaSuccess)
-    e = cudaMemcpyAsync(ctx->d_tab, tab.data(), tab.size() * sizeof(float4), cudaMemcpyHostToDevice,
-                        ctx->stream);
-  return e;
+  if (e == cudaSuccess) {
+    mcg_chain_tables<<<(int)std::min<int64_t>(((int64_t)total + 2 * MCG_TAB_PAD + 255) / 256, 8LL * ctx->sm_count),
+                       256, 0, ctx->stream>>>(ctx->d_cells_strict, total, ctx->d_cells_fast, ctx->d_tab,
+                                              thin ? ctx->d_thin : nullptr);
+    e = cudaGetLastError();
+  }
+  if (e != cudaSuccess) {
+    cudaStreamSynchronize(ctx->stream);
+    free_geometry(ctx);
+    return mcg_fail(MCG_ERR_CUDA, "%s: cudaMalloc(layers) or upload: %s", who, cudaGetErrorString(e));
+  }
+  ctx->n_cells = total;
+  ctx->cell_lo = h_index_start[0];
+  ctx->min_w = particle_min_weight;
+  return mcg_tally_reset(ctx); /* synchronises */
 }
 
 extern "C" int mcg_set_layers(mcg_context *ctx, int n_layers, const int32_t *h_index_start,
                               const int32_t *h_m, const float *h_dx, const float *h_sigs,
                               const float *h_rates, float particle_min_weight)
 {
-  if (!ctx || n_layers <= 0 || !h_index_start || !h_m || !h_dx || !h_sigs || !h_rates)
-    return mcg_fail(MCG_ERR_ARG, "mcg_set_layers: bad arguments");
-  int64_t total64 = 0;
-  for (int l = 0; l < n_layers; ++l) {
-    if (h_m[l] <= 0)
-      return mcg_fail(MCG_ERR_ARG, "mcg_set_layers: layer %d has %d cells", l, h_m[l]);
-    if (l > 0 && (int64_t)h_index_start[l] != (int64_t)h_index_start[l - 1] + h_m[l - 1])
-      return mcg_fail(MCG_ERR_ARG, "mcg_set_layers: layer %d is not contiguous", l);
-    total64 += h_m[l];
-    if (total64 > INT32_MAX)
-      return mcg_fail(MCG_ERR_ARG, "mcg_set_layers: more than 2^31 - 1 cells");
-  }
-  const int total = (int)total64;
-  int rc = ensure_device(ctx);
-  if (rc != MCG_OK)
-    return rc;
-  std::vector<float4> cs, cf;
-  try {
-    cs.resize(total);
-    cf.resize(total);
-  } catch (const std::bad_alloc &) {
-    return mcg_fail(MCG_ERR_ARG, "mcg_set_layers: no host memory for %d cells", total);
-  }
-  int k = 0;
-  for (int l = 0; l < n_layers; ++l)
-    for (int j = 0; j < h_m[l]; ++j, ++k)
-      mcg_cell_params(h_sigs[k], h_rates[k], h_index_start[l] + j, h_dx[l], cs[k], cf[k]);
-  cudaStreamSynchronize(ctx->stream);
-  /* a chain of as many cells takes over the buffers (with the copies on the
-   * stream and one synchronisation, a call of the reference's seam with 100
-   * cells and 1000 particles takes 167 us instead of 204); otherwise the old
-   * geometry goes first; any failure below leaves no geometry */
-  cudaError_t e;
-  if (!ctx->d_tally || ctx->n_cells != total) {
-    free_geometry(ctx);
-    if ((e = mcg_dev_malloc((void **)&ctx->d_cells_strict, total * sizeof(float4))) != cudaSuccess ||
-        (e = mcg_dev_malloc((void **)&ctx->d_cells_fast, total * sizeof(float4))) != cudaSuccess ||
-        (e = mcg_dev_malloc((void **)&ctx->d_tab, 2 * (total + 2 * (size_t)MCG_TAB_PAD) * sizeof(float4))) != cudaSuccess ||
-        (e = mcg_dev_malloc((void **)&ctx->d_tally, total * sizeof(unsigned long long))) != cudaSuccess) {
-      free_geometry(ctx);
-      return mcg_cuda_fail(e, "cudaMalloc(layers)");
-    }
-  }
-  ctx->n_layers = n_layers;
-  ctx->layer_start.assign(h_index_start, h_index_start + n_layers);
-  ctx->layer_m.assign(h_m, h_m + n_layers);
-  ctx->layer_dx.assign(h_dx, h_dx + n_layers);
-  ctx->sigs.assign(h_sigs, h_sigs + total);
-  ctx->rates.assign(h_rates, h_rates + total);
-  ctx->cells_strict.swap(cs);
-  ctx->cells_fast.swap(cf);
-  update_thin(ctx);
-  std::vector<float4> tab;
-  if ((e = upload_cells(ctx, tab)) != cudaSuccess) {
-    cudaStreamSynchronize(ctx->stream);
-    free_geometry(ctx);
-    return mcg_cuda_fail(e, "cudaMemcpy(layers)");
-  }
-  ctx->n_cells = total;
-  ctx->cell_lo = h_index_start[0];
-  ctx->min_w = particle_min_weight;
-  return mcg_tally_reset(ctx); /* synchronises */
+  return set_geometry(ctx, "mcg_set_layers", n_layers, h_index_start, h_m, h_dx, h_sigs, h_rates, false,
+                      particle_min_weight);
 }
 
 /* Same as mcg_set_layers with the two cross sections of particle_step given
@@ -543,46 +554,8 @@ extern "C" int mcg_set_layers_xs(mcg_context *ctx, int n_layers, const int32_t *
                                  const int32_t *h_m, const float *h_dx, const float *h_sig_a,
                                  const float *h_sig_s, float particle_min_weight)
 {
-  if (!ctx || n_layers <= 0 || !h_index_start || !h_m || !h_dx || !h_sig_a || !h_sig_s)
-    return mcg_fail(MCG_ERR_ARG, "mcg_set_layers_xs: bad arguments");
-  int64_t total64 = 0;
-  for (int l = 0; l < n_layers; ++l) {
-    if (h_m[l] <= 0 || (l > 0 && (int64_t)h_index_start[l] != (int64_t)h_index_start[l - 1] + h_m[l - 1]))
-      return mcg_fail(MCG_ERR_ARG, "mcg_set_layers_xs: layer %d is empty or not contiguous", l);
-    total64 += h_m[l];
-    if (total64 > INT32_MAX)
-      return mcg_fail(MCG_ERR_ARG, "mcg_set_layers_xs: more than 2^31 - 1 cells");
-  }
-  const int total = (int)total64;
-  std::vector<float> sigs(total), rates(total);
-  for (int c = 0; c < total; ++c) {
-    sigs[c] = h_sig_a[c] + h_sig_s[c];
-    rates[c] = sigs[c] > 0.0f ? h_sig_a[c] / sigs[c] : 0.0f;
-  }
-  int rc = mcg_set_layers(ctx, n_layers, h_index_start, h_m, h_dx, sigs.data(), rates.data(),
-                          particle_min_weight);
-  if (rc != MCG_OK)
-    return rc;
-  /* replace the derived cross sections by the given ones */
-  int k = 0;
-  for (int l = 0; l < n_layers; ++l)
-    for (int j = 0; j < h_m[l]; ++j, ++k) {
-      float4 &cs = ctx->cells_strict[k], &cf = ctx->cells_fast[k];
-      cs.x = cf.x = h_sig_a[k];
-      cs.y = h_sig_s[k];
-      cf.y = h_sig_s[k] > 1e-4f ? h_sig_s[k] : 0.0f;
-    }
-  update_thin(ctx);
-  std::vector<float4> tab;
-  cudaError_t e = upload_cells(ctx, tab);
-  const cudaError_t e2 = cudaStreamSynchronize(ctx->stream);
-  if (e == cudaSuccess)
-    e = e2;
-  if (e != cudaSuccess) {
-    free_geometry(ctx);
-    return mcg_cuda_fail(e, "mcg_set_layers_xs: upload");
-  }
-  return MCG_OK;
+  return set_geometry(ctx, "mcg_set_layers_xs", n_layers, h_index_start, h_m, h_dx, h_sig_a, h_sig_s, true,
+                      particle_min_weight);
 }
 
 extern "C" int mcg_set_slab(mcg_context *ctx, float x_min, float x_max, int32_t nb_cells,
@@ -814,7 +787,7 @@ int mcg_track_launch(mcg_context *ctx, mcg_particle *d_particles, int64_t n, int
   mcg_track_params P;
   memset(&P, 0, sizeof(P));
   P.cells = strict ? ctx->d_cells_strict : ctx->d_cells_fast;
-  P.tab = {ctx->d_tab + MCG_TAB_PAD, ctx->d_thin + MCG_TAB_PAD, ctx->n_cells + 2 * MCG_TAB_PAD};
+  P.tab = mcg_chain_tab(ctx);
   P.n_cells = ctx->n_cells;
   P.cell_lo = ctx->cell_lo;
   P.particles = d_particles;

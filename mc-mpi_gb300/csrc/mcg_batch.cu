@@ -94,7 +94,7 @@ void mcg_ext_destroy(mcg_context *ctx)
 }
 
 /* The fast arithmetic's cells (mcg_cell_params) and the tile table
- * (mcg_tile_table: within a slab neighbours share their faces) from the strict
+ * (mcg_tile_entry: within a slab neighbours share their faces) from the strict
  * cells, on the GPU: uploading all three took 27 ms longer for 8.5e6 cells. */
 __global__ void mcg_batch_tables(const float4 *strict, float4 *fast, float4 *tab, int64_t n)
 {

@@ -13,7 +13,7 @@
 bool mcg_batch_lanes(const mcg_widths &w, int n, bool strict);
 
 /* A cell's entry of the tile table from its fast-arithmetic parameters
- * (mcg_tile_table: within a slab neighbours share their faces). */
+ * (mcg_tile_entry: within a slab neighbours share their faces). */
 __host__ __device__ inline float4 mcg_tile_cell(const float4 c)
 {
   const float a = c.w - c.z;

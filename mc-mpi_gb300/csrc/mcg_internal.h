@@ -7,6 +7,7 @@
 
 #include <cuda_runtime.h>
 
+#include <cmath>
 #include <cstdint>
 #include <vector>
 
@@ -132,8 +133,8 @@ struct mcg_context {
   int n_layers = 0, n_cells = 0, cell_lo = 0;
   float min_w = 0.f;
   std::vector<int32_t> layer_start, layer_m;
-  std::vector<float> layer_dx, sigs, rates;
-  std::vector<float4> cells_strict, cells_fast;
+  std::vector<float> layer_dx;
+  std::vector<float4> cells_strict;
   bool thin_step = false; /* mcg_strict_thin */
   bool thin = false;      /* every cell's sig_a width <= 2e-4 (strict THIN) */
   bool thin_fast = false; /* sig_a and sig_i widths <= 4e-4 (fast THIN) */
@@ -142,9 +143,9 @@ struct mcg_context {
   double depth_i = 0.0;               /* the chain's optical depth in sig_i, where it scatters */
   mcg_widths widths;
   float4 *d_cells_strict = nullptr, *d_cells_fast = nullptr;
-  /* the tiles' per-cell parameters (mcg_tile_table), MCG_TAB_PAD entries
-   * before and after; of the thin form one such array per direction, in the
-   * same allocation */
+  /* the tiles' per-cell parameters (mcg_tile_entry), MCG_TAB_PAD entries before
+   * and after; of the thin form one such array per direction, for chains that may
+   * take it */
   float4 *d_tab = nullptr;
   float2 *d_thin = nullptr;
   unsigned long long *d_tally = nullptr;
@@ -191,8 +192,21 @@ int mcg_cuda_fail(cudaError_t e, const char *what);
 bool mcg_thick(const mcg_widths &w, int n, bool strict);
 cudaError_t mcg_read_tally(mcg_context *ctx, const unsigned long long *d, size_t n, int64_t *h_q,
                            double *h_f64);
-void mcg_tile_table(const float4 *cells_fast, int n, float4 *tab, float2 *right = nullptr,
-                    float2 *left = nullptr);
+/* The tiles' parameters of cell k of n consecutive ones (mcg_tiles): {sig_a, sig_i,
+ * length of a flight that enters the cell by its left face, by its right face}, the
+ * float differences of the faces that mcg_step_cross forms (entered at a neighbour's
+ * face, which between layers of different spacing differs from the cell's own).
+ * Lengths outside the range in which the cached-reciprocal division is exact, and
+ * those of cells that would amplify the weight, are NaN: such steps take the full
+ * form.  sig_i as in the cells: 0 when at most EPS in the fast ones. */
+__host__ __device__ inline float4 mcg_tile_entry(const float4 *c, int n, int k)
+{
+  const float4 p = c[k];
+  const float l = p.w - (k ? c[k - 1].w : p.z), r = (k + 1 < n ? c[k + 1].z : p.w) - p.z;
+  return make_float4(p.x, p.y, l >= 0x1p-90f && l <= 0x1p90f && p.x >= 0.0f ? l : NAN,
+                     r >= 0x1p-90f && r <= 0x1p90f && p.x >= 0.0f ? r : NAN);
+}
+void mcg_tile_table(const float4 *cells_fast, int n, float4 *tab);
 void mcg_cell_params(float sig, float rate, int gi, float dx, float4 &strict, float4 &fast);
 int mcg_track_launch(mcg_context *ctx, mcg_particle *d_particles, int64_t n, int32_t *d_results,
                      int64_t *d_steps, int64_t *d_scatters, const mcg_source *src, int64_t first);

@@ -35,6 +35,12 @@ struct mcg_tab {
   const float2 *aux; /* LOSS: {w_c, .}, readable as far */
 };
 
+inline mcg_tab mcg_chain_tab(const mcg_context *ctx)
+{
+  return {ctx->d_tab + MCG_TAB_PAD, ctx->d_thin ? ctx->d_thin + MCG_TAB_PAD : nullptr,
+          ctx->n_cells + 2 * MCG_TAB_PAD};
+}
+
 /* How a warp runs its histories (mcg_histories). */
 struct mcg_rules {
   float min_w;

@@ -1090,7 +1090,7 @@ extern "C" int mcg_worker_run_async(mcg_context *ctx, const mcg_source *src, int
   mcg_async_params A;
   memset(&A, 0, sizeof(A));
   A.cells = strict ? ctx->d_cells_strict : ctx->d_cells_fast;
-  A.tab = {ctx->d_tab + MCG_TAB_PAD, ctx->d_thin + MCG_TAB_PAD, ctx->n_cells + 2 * MCG_TAB_PAD};
+  A.tab = mcg_chain_tab(ctx);
   A.n_layers = P_;
   A.cell_lo = ctx->cell_lo;
   A.n_cells = ctx->n_cells;

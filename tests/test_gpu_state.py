@@ -138,3 +138,62 @@ def test_synchronous_workers_around_the_thin_step(mcg, width):
         ctx.worker_run(n, per_cycle=500)
         assert np.array_equal(ctx.tally_q(), want)
         assert all(ctx.counters()[k] == c[k] for k in ("steps", "scatters"))
+
+
+@pytest.mark.parametrize("xs", [False, True])
+def test_memory_and_time_of_a_long_chain(mcg, xs):
+    """A chain that is never thin keeps 56 bytes per cell (cells of both arithmetics,
+    tile table, tally), not the thin tables' 16 more; and its cross sections given
+    directly do not cost a second upload."""
+    import time
+    import torch
+    m = 2_000_000
+    a, b = np.full(m, 0.01 * m, f32), np.full(m, 0.5, f32)
+    with mcg.Context(mode="fast") as ctx:
+        ctx.set_layers([0], [10], [f32(0.1)], np.ones(10), np.full(10, 0.5), 1e-12)
+        free = torch.cuda.mem_get_info()[0]
+        (ctx.set_layers_xs if xs else ctx.set_layers)([0], [m], [f32(1.0 / m)], a, b, 1e-12)
+        assert free - torch.cuda.mem_get_info()[0] < 60 * m + (16 << 20)
+        times = []
+        for f in (ctx.set_layers, ctx.set_layers_xs):
+            best = []
+            for _ in range(4):
+                t = time.perf_counter()
+                f([0], [m], [f32(1.0 / m)], a, b, 1e-12)
+                best.append(time.perf_counter() - t)
+            times.append(min(best))
+        assert times[1] < 1.5 * times[0], times
+
+
+@pytest.mark.parametrize("mode", ["strict", "fast"])
+def test_chains_of_one_length_with_and_without_thin_tables(mcg, mode):
+    """The buffers are kept for as many cells; the thin tables come with the first
+    chain that may use them, and are that chain's own each time."""
+    m = 6000
+    with mcg.Context(mode=mode) as ctx:
+        for width in (0.01, 2e-5, 0.03, 5e-5, 5e-5, 0.005):
+            sa, ss = np.full(m, width * m), np.full(m, 0.7 * width * m)
+            if width == 5e-5:
+                sa[::2] = 0.0
+            ctx.set_layers_xs([0], [m], [f32(1.0 / m)], sa, ss, 1e-12)
+            out = []
+            for algorithm in ("event", "history"):
+                ctx.set_algorithm(algorithm, 1)
+                ctx.tally_reset()
+                ctx.simulate_source(0, 300)
+                out.append((ctx.tally_q().tobytes(), ctx.counters()))
+            assert out[0] == out[1]
+
+
+def test_chain_longer_than_the_thin_kernel_holds(mcg):
+    """100,000 thin cells: no thin tables, the other tiles."""
+    m = 100_000
+    with mcg.Context(mode="strict") as ctx:
+        ctx.set_layers_xs([0], [m], [f32(1.0 / m)], np.full(m, 1.0), np.full(m, 2.0), 1e-12)
+        out = []
+        for algorithm in ("event", "history"):
+            ctx.set_algorithm(algorithm, 1)
+            ctx.tally_reset()
+            ctx.simulate_source(0, 100)
+            out.append((ctx.tally_q().tobytes(), ctx.counters()))
+        assert out[0] == out[1]
