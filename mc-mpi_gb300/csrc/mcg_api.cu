@@ -104,7 +104,9 @@ int mcg_load_libm(mcg_context *ctx)
   if (!ok)
     return mcg_fail(MCG_ERR_TABLES, "malformed libm exception table %s", path.c_str());
   const mcg_libm_tab tab = MCG_LIBM_TAB_INIT;
-  if (hdr.fingerprint != mcg_libm_fingerprint(&tab))
+  /* of this process's C library and forms: one for all contexts (1 ms) */
+  static const uint64_t fingerprint = mcg_libm_fingerprint(&tab);
+  if (hdr.fingerprint != fingerprint)
     return mcg_fail(MCG_ERR_TABLES,
                     "libm exception table %s was made against another C library (%s) or "
                     "another version of the evaluators; rebuild",
@@ -363,14 +365,15 @@ __global__ void mcg_chain_tables(const float4 *strict, int n, float4 *fast, floa
 }
 
 /* thin: every cell's absorption optical width, sig_a times the longer of its
- * tile lengths, is at most 2e-4, so that a crossing has u >= MCG_OM_THIN_MAX (2^-8) only for
- * |mu| < 0.05, 0.3 % of the crossings (their share of directions is about
- * mu^2), which go to the full step; thin_fast: both optical widths at most
- * 4e-4 (the short series, below 2^-7, again for |mu| > 0.05).  A transparent
- * chain keeps its slanted particles longer, so the strict line is lower there:
- * 1e6 histories, thin form / other, at depth 0.63 and widths of 1.7e-4 8.1 / 5.6
- * ms, 1.25e-4 9.5 / 7.4, 8.3e-5 11.7 / 11.4, 5e-5 15.6 / 19.2; at depth 2.1 and
- * 1.4e-4 27.6 / 35.1, at 2.5 and 1.5e-4 15.3 / 18.8. */
+ * tile lengths, is at most 2e-4, so that a crossing has u >= MCG_OM_THIN_MAX (2^-8)
+ * only for |mu| < 0.05, 0.3 % of the crossings (their share of directions is about
+ * mu^2), which go to the full step; thin_fast: both optical widths at most 4e-4 (the
+ * short series, below 2^-7, again for |mu| > 0.05).  A transparent chain keeps its
+ * slanted particles longer, so the strict line is lower there.  Thin form / other:
+ * strict at depth 0.54 to 0.72, 3000 cells, widths (sig_a) 1.4e-4 1.01, 2e-4 1.12;
+ * 10,000 cells at depth 1.2 1e-4 .92, 1.8 1.4e-4 .89, 2.4 2e-4 .73; fast, both widths,
+ * 3000 and 10,000 cells: 2e-4 .79 and .59, 4e-4 .87 and .68, 6e-4 .92 and .85, 8e-4
+ * 1.13 and 1.09.  Whether a run takes it: thin_pays. */
 static void update_thin(mcg_context *ctx)
 {
   const float4 *cells = ctx->cells_strict.data();
