@@ -340,12 +340,16 @@ void mcg_tile_table(const float4 *c, int n, float4 *tab)
 }
 
 /* The fast arithmetic's cells (mcg_cell_params), the tile table and, where wanted, a
- * thin chain's two, from the strict cells and with zeros beyond the ends: made on the
+ * thin chain's two, from the strict cells and with zeros beyond the ends; the tally
+ * and the counters cleared (mcg_tally_reset's two launches).  Made on the
  * host and uploaded they were 56 of the 72 bytes per cell (2e6 cells: 26 ms for
  * mcg_set_layers; 15 before there were tiles, 11 so). */
-__global__ void mcg_chain_tables(const float4 *strict, int n, float4 *fast, float4 *tab, float2 *thin)
+__global__ void mcg_chain_tables(const float4 *strict, int n, float4 *fast, float4 *tab, float2 *thin,
+                                 unsigned long long *tally, unsigned long long *counters)
 {
   const int row = n + 2 * MCG_TAB_PAD;
+  if (blockIdx.x == 0 && threadIdx.x < 16)
+    counters[threadIdx.x] = 0ull;
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < row;
        i += (int64_t)gridDim.x * blockDim.x) {
     const int k = (int)i - MCG_TAB_PAD;
@@ -355,6 +359,7 @@ __global__ void mcg_chain_tables(const float4 *strict, int n, float4 *fast, floa
       t = mcg_tile_entry(strict, n, k);
       t.y = c.y > 1e-4f ? c.y : 0.0f;
       fast[k] = make_float4(c.x, t.y, c.z, c.w);
+      tally[k] = 0ull;
     }
     tab[i] = t;
     if (thin) {
@@ -529,18 +534,20 @@ static int set_geometry(mcg_context *ctx, const char *who, int n_layers, const i
   if (e == cudaSuccess) {
     mcg_chain_tables<<<(int)std::min<int64_t>(((int64_t)total + 2 * MCG_TAB_PAD + 255) / 256, 8LL * ctx->sm_count),
                        256, 0, ctx->stream>>>(ctx->d_cells_strict, total, ctx->d_cells_fast, ctx->d_tab,
-                                              thin ? ctx->d_thin : nullptr);
+                                              thin ? ctx->d_thin : nullptr, ctx->d_tally, ctx->d_counters);
     e = cudaGetLastError();
+    const cudaError_t e2 = cudaStreamSynchronize(ctx->stream);
+    if (e == cudaSuccess)
+      e = e2;
   }
   if (e != cudaSuccess) {
-    cudaStreamSynchronize(ctx->stream);
     free_geometry(ctx);
     return mcg_fail(MCG_ERR_CUDA, "%s: cudaMalloc(layers) or upload: %s", who, cudaGetErrorString(e));
   }
   ctx->n_cells = total;
   ctx->cell_lo = h_index_start[0];
   ctx->min_w = particle_min_weight;
-  return mcg_tally_reset(ctx); /* synchronises */
+  return MCG_OK;
 }
 
 extern "C" int mcg_set_layers(mcg_context *ctx, int n_layers, const int32_t *h_index_start,
