@@ -541,7 +541,7 @@ extern "C" int mcg_adjoint_reset(mcg_context *ctx)
 /* Chains of thick cells, on which most steps are full ones: with a gradient the one
  * kernel with every lane through the whole step (rounds gather too little there),
  * without one a forward pass with a lane per history.  Two kernels / one, widths
- * sig_a and sig_i, 300 to 1500 cells: strict .02, .02 .7, .05, .05 1.1, .1, .1 1.2,
+ * sig_a and sig_i, 300 to 1500 cells: strict .02, .02 .7, .03, .03 1.14, .05, .05 1.1, .1, .1 1.2,
  * .1, .01 1.3 to 1.7, .01, .1 .6; fast .05, .05 .8, .01, .1 .85, .1, .01 1.2, .1, .1
  * 1.2, .3, .3 1.5, .05, .3 1.7.  Forward pass, tiles / lanes, 40 and 300 cells: strict
  * .02, .02 1.0 and .6, .05, .05 1.9 and 1.2, .1, .01 4.5 and 3.7; fast .05, .05 1.0 and
@@ -552,7 +552,7 @@ static bool adj_thick(const mcg_widths &w, int n, bool strict, bool gradient)
   if (n < 8)
     return true;
   if (strict)
-    return w.a > 0.035 * n || w.i > 0.25 * n;
+    return w.a > 0.025 * n || w.i > 0.25 * n;
   return gradient ? w.a > 0.06 * n || w.a + w.i > 0.15 * n
                   : w.a + w.i > (n < 32 ? 0.1 : 0.25) * n;
 }
