@@ -52,9 +52,9 @@ METRIC = "histories/s on 1 GB300 (plain vs batched vs fwd+adjoint) at matched ta
 NB_CELLS, N_LAYERS, N_TOTAL = 10000, 64, 100_000_000
 BASE_SEED = 5127801
 MIN_W = 1e-12
-# DRAM bytes (read + write) per history of the strict tracker, from an ncu
-# capture of 3e6 histories of this workload
-DRAM_BYTES_PER_HISTORY = 112.44e6 / 3e6
+# DRAM bytes (read + write) per history of the strict tracker's thin kernel, from an
+# ncu capture of 3e6 histories of this workload
+DRAM_BYTES_PER_HISTORY = 110.96e6 / 3e6
 WORKLOAD = ("slab 10000 cells / 64 sub-domains (decompose_domain), sigma_a=0.5+0.4sin(6pi x), "
             "sigma_s=2+1.5cos(4pi x), 1e8 histories from x=0 mu=1 w=1, rnd_seed chain 5127801, "
             "min weight 1e-12")

@@ -577,8 +577,8 @@ __device__ __forceinline__ void mcg_step_rest(uint64_t &seed, float &x, float &m
  * loads and the tally atomics runs of consecutive cells (with scattered lanes
  * the L1 was the bound: 18 of 19 cycles of a warp step on the 10,000-cell
  * slab), keeps the lanes busy whatever the histories do, and a single history
- * takes about 30 cycles per step instead of 300, which is what the end of a
- * launch waits for.  Every step is exactly mcg_step_cross's. */
+ * takes about 100 cycles per step (3200 per tile of 32) instead of 300 to 500, which
+ * is what the end of a launch waits for.  Every step is exactly mcg_step_cross's. */
 /* Lanes per flight in phases 2 and 4 (G) and steps of a tile (2 G).  Thin chains
  * take 16 and 32: fewer rounds and shared-memory rows per step; others 8 and
  * 16: their flights are short, and what a tile has after its flight's end is

@@ -582,7 +582,7 @@ template <bool THIN> struct mcg_async_tiles<THIN, false> {
 /* TALLY and THIN as in mcg_track_kernel; TILES: see MCG_AQ_SHORT.  A warp advances its particles by the
  * tracker's tiles (mcg_advance); it was one lane per particle through the whole
  * step.  Bound: instruction issue, 80 warp instructions per step of 32 lanes (the
- * tracker's 54, and the rows of tiles that a sub-domain's end cuts short), with
+ * tracker's 64, and the rows of tiles that a sub-domain's end cuts short), with
  * the waits for the queues' global words.  10,000 cells in 64 sub-domains, 1e6
  * histories, strict: 65.2 ms -> 34.2 ms for the call. */
 template <bool STRICT, int TALLY, bool THIN, bool TILES>
