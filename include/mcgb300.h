@@ -158,8 +158,8 @@ int mcg_counters_read(mcg_context *ctx, mcg_counters *out);
 int mcg_last_kernel_ms(mcg_context *ctx, float *ms);
 
 /* Launch shape (0 = automatic): threads per block, resident blocks per SM,
- * most steps a history takes before its warp looks at its other histories.  With
- * a block size given, a chain of thin cells takes the thin form whether or not the
+ * most steps a history takes before its warp looks at its other histories (tiles
+ * take at least eight).  With a block size given, a chain of thin cells takes the thin form whether or not the
  * library's rule finds that it pays. */
 int mcg_set_launch(mcg_context *ctx, int32_t block, int32_t blocks_per_sm, int32_t refill_steps);
 

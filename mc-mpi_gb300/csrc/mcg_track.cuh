@@ -1788,13 +1788,16 @@ inline float mcg_heavy_weight(const mcg_context *ctx)
  * need them on 1 % of the tiles, others on a third of them) and ended histories
  * replaced for two; 2 to 16 and 1 to 8 were measured within 5 % of these on thin
  * chains and within 10 % on a 1000-cell one. */
+#define MCG_WINDOW_LEAST 8 /* a caller's refill_steps below it: a tile's fixed costs (1000 cells, 3e5
+                              histories, strict: 20 ms at 1, 5.5 at 4, 3.3 at 8, 2.1 at 32, where a lane
+                              per history had taken 5.9, 4.6, 4.4 and 4.1) */
 inline mcg_rules mcg_rules_setup(const mcg_context *ctx, float min_w)
 {
   mcg_rules R;
   R.min_w = min_w;
   R.q_log2 = ctx->log2_scale;
   R.max_steps = ctx->max_steps;
-  R.window = ctx->refill ? ctx->refill : MCG_TW_MAX;
+  R.window = ctx->refill ? std::max(ctx->refill, MCG_WINDOW_LEAST) : MCG_TW_MAX;
   R.pool_lanes = 4;
   R.refill_lanes = 2;
   R.run = mcg_run_setup(ctx->log2_scale, min_w, ctx->run_bounds, ctx->width_a, ctx->width_i);

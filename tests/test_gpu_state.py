@@ -197,3 +197,21 @@ def test_chain_longer_than_the_thin_kernel_holds(mcg):
             ctx.simulate_source(0, 100)
             out.append((ctx.tally_q().tobytes(), ctx.counters()))
         assert out[0] == out[1]
+
+
+@pytest.mark.parametrize("mode", ["strict", "fast"])
+def test_small_refill_steps_are_not_a_tile_each(mcg, mode):
+    """A caller's refill_steps of 1 or 4 took six and two times as long as 8, a tile's
+    fixed costs for as many steps."""
+    m = 1000
+    with mcg.Context(mode=mode) as ctx:
+        ctx.set_layers_xs([0], [m], [f32(1.0 / m)], np.full(m, 2.0), np.full(m, 2.0), 1e-12)
+        times = {}
+        for steps in (8, 4, 1):
+            ctx.set_launch(refill_steps=steps)
+            best = []
+            for _ in range(4):
+                ctx.simulate_source(0, 300_000)
+                best.append(ctx.last_kernel_ms())
+            times[steps] = min(best)
+        assert max(times[1], times[4]) < 1.3 * times[8], times
