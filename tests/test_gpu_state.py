@@ -215,3 +215,27 @@ def test_small_refill_steps_are_not_a_tile_each(mcg, mode):
                 best.append(ctx.last_kernel_ms())
             times[steps] = min(best)
         assert max(times[1], times[4]) < 1.3 * times[8], times
+
+
+@pytest.mark.parametrize("kept", [False, True])
+def test_failed_thin_tables_leave_no_geometry(mcg, kept):
+    """The thin tables' allocation fails: with buffers of the same chain length kept,
+    where it is the only one, or after four others."""
+    m = 300
+    thin = ([0], [m], [f32(1.0 / m)], np.full(m, 1e-5 * m), np.full(m, 1e-5 * m), 1e-12)
+    with mcg.Context(mode="fast") as ctx:
+        n = m if kept else m + 1
+        ctx.set_layers_xs([0], [n], [f32(1.0 / n)], np.full(n, 0.01 * n), np.full(n, 0.01 * n), 1e-12)
+        ctx.lib.mcg_testing_fail_allocation(0 if kept else 4)
+        try:
+            with pytest.raises(mcg.MCGError) as e:
+                ctx.set_layers_xs(*thin)
+            assert e.value.code == 2  # MCG_ERR_CUDA
+        finally:
+            ctx.lib.mcg_testing_fail_allocation(-1)
+        with pytest.raises(mcg.MCGError) as e:
+            ctx.simulate_source(0, 10)
+        assert e.value.code == 5  # MCG_ERR_STATE
+        ctx.set_layers_xs(*thin)
+        ctx.simulate_source(0, 1000)
+        assert ctx.counters()["histories"] == 1000
